@@ -1,0 +1,84 @@
+"""The radix sort at the edges of its tiles and dispatch rules against numpy's stable lexsort: one CTA
+up to 2048 rows, 4096-row tiles below 2^21 rows, 8192-row tiles above; keys whose varying digits lie in
+the low half, the high half, both or nowhere; several keys in one call."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 2, 2048, 2049, 4095, 4096, 4097, 8193, 65536, 100_003, (1 << 21) - 1, 1 << 21, (1 << 21) + 8193]
+
+
+def _image(a, desc):
+    """Order-preserving integers of a key column, one or more per row (most significant first)."""
+    if a.ndim == 2:
+        cols = [a[:, j].astype(np.int64) for j in range(a.shape[1])]
+    elif a.dtype == np.float64:
+        b = np.where(a == 0, 0.0, a)
+        u = b.view(np.uint64).copy()
+        neg = u >> np.uint64(63) == 1
+        v = np.where(neg, ~u, u | np.uint64(1 << 63))
+        v[np.isnan(a)] = np.uint64(2**64 - 2)
+        cols = [(v ^ np.uint64(1 << 63)).view(np.int64)]
+    else:
+        cols = [a.astype(np.int64)]
+    return [~c for c in cols] if desc else cols
+
+
+def _expected(keys, descs):
+    cols = [c for k, d in zip(keys, descs) for c in _image(k, d)]
+    return np.lexsort(cols[::-1])
+
+
+def _check(keys, descs, perm=None):
+    from tqpk.ops import argsort_keys
+    dev = [torch.from_numpy(k).cuda() for k in keys]
+    if perm is None:
+        exp = _expected(keys, descs)
+        got = argsort_keys(dev, descs)
+    else:
+        exp = perm[_expected([k[perm] for k in keys], descs)]
+        got = argsort_keys(dev, descs, torch.from_numpy(perm).cuda())
+    np.testing.assert_array_equal(got.cpu().numpy(), exp)
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_sizes(n):
+    rng = np.random.default_rng(n)
+    _check([rng.integers(0, max(2, n // 3), n).astype(np.int64)], [bool(n & 1)])
+    f = rng.integers(-3000, 3000, n) * 0.25
+    f[: min(n, 4)] = [-0.0, 0.0, np.nan, np.inf][: min(n, 4)]
+    _check([f, rng.integers(-5, 5, n).astype(np.int32)], [True, False], rng.permutation(n))
+
+
+@pytest.mark.parametrize("n", [2000, 5000, 300_001])
+@pytest.mark.parametrize("make", [lambda r, n: r.integers(-2**40, 2**40, n) << 20, lambda r, n: r.integers(0, 300, n) << 34,
+                                  lambda r, n: np.full(n, -7), lambda r, n: r.integers(-64, 1, n),
+                                  lambda r, n: r.integers(-2**63, 2**63 - 1, n)])
+def test_varying_digits(make, n):
+    rng = np.random.default_rng(7)
+    k = make(rng, n).astype(np.int64)
+    for desc in (False, True):
+        _check([k], [desc])
+
+
+@pytest.mark.parametrize("n", [1500, 27_600, 150_001])
+def test_many_keys(n):
+    rng = np.random.default_rng(n)
+    words = np.frombuffer(b"BRAND-11BRAND-12BRAND-45LARGE TI", np.int8).reshape(4, 8)
+    text = np.zeros((n, 25), np.int8)
+    text[:, 3:11] = words[rng.integers(0, 4, n)]
+    text[:, 17:25] = words[rng.integers(0, 4, n)]
+    raw = rng.integers(0, 256, (n, 3)).astype(np.uint8)
+    keys = [rng.integers(0, 5, n).astype(np.int64), text, raw, rng.integers(-100, 100, n).astype(np.int8),
+            rng.integers(0, 3, n).astype(np.uint8), rng.integers(0, 9, n).astype(np.int32)]
+    _check(keys, [True, False, True, True, False, False])
+    _check(keys[1:4], [True, False, False], rng.integers(0, n, n))     # rows may repeat
+
+
+def test_too_many_words_raise():
+    from tqpk.ops import argsort_keys
+    wide = torch.zeros((3000, 8 * 33), dtype=torch.int8, device="cuda")
+    with pytest.raises(NotImplementedError):
+        argsort_keys([wide], [False])

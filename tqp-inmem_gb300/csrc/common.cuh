@@ -774,7 +774,19 @@ int key_ranges(const tqpk_predicate* pred, const uint8_t* mask, int64_t n, int n
 size_t compact_status_bytes(int64_t n);
 int compact_launch(const tqpk_predicate* pred, const uint8_t* mask, int64_t n, const ColSet& C, int64_t* d_count,
                    void* ws, size_t ws_bytes, cudaStream_t s);
-size_t sort_ws_bytes(int64_t n);
+
+// One sort key: element e is row rows[e] (null: e) of a column; a string key (width > 0: int8/uint8
+// [n, width] rows) is the big-endian word of its bytes word*8 .. word*8+7.
+struct SortKey {
+  const void* col;
+  const int64_t* rows;
+  int dt, desc, width, word;
+};
+constexpr int kMaxSortKeys = 32;
+size_t sort_ws_bytes(int64_t n, int nk = 1);
+int sort_keys(const SortKey* keys, int nk, const int64_t* perm_in, int64_t n, int64_t* perm_out, void* ws,
+              size_t ws_bytes, cudaStream_t s);
+
 bool spec_cols_vec(const tqpk_groupby_spec* S);   // all spec columns 16-byte aligned
 
 // Grid of one full wave: resident CTAs per SM (occupancy API) x SMs, capped by
@@ -791,7 +803,5 @@ inline int occ_grid(K kernel, int64_t work_units, size_t smem = 0) {
   if (g > cap) g = cap;
   return (int)(g < 1 ? 1 : g);
 }
-int sort_pairs(const void* keys, int dt, int desc, const int64_t* perm_in, int64_t n, void* ws, size_t ws_bytes,
-               cudaStream_t s, const int64_t** result);
 
 }  // namespace tqpk

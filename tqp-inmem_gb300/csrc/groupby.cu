@@ -434,18 +434,20 @@ __global__ void k_emit_hash(const __grid_constant__ tqpk_groupby_spec S, GbDev G
   }
 }
 
-// Hash-mode workspace: [512 header][acc table A x C][keys C][packed keys C][slots C][sort workspace]
+// Hash-mode workspace: [512 header][acc table A x C][keys C][packed keys C][slots C][order C/2][sort workspace]
 struct HashLayout {
   uint64_t* gacc;
   unsigned long long* hkeys;
   int64_t* pk;
   int64_t* cslot;
+  int64_t* perm;
   void* sort_ws;
   size_t sort_bytes;
 };
 
 static size_t hash_ws_bytes(int64_t C, int A) {
-  return 512 + align_up((size_t)C * A * 8, 256) + 3 * align_up((size_t)C * 8, 256) + sort_ws_bytes(C / 2 + 1) + 256;
+  return 512 + align_up((size_t)C * A * 8, 256) + 3 * align_up((size_t)C * 8, 256) +
+         align_up((size_t)(C / 2 + 1) * 8, 256) + sort_ws_bytes(C / 2 + 1) + 256;
 }
 
 static HashLayout hash_layout(void* ws, int64_t C, int A) {
@@ -459,6 +461,8 @@ static HashLayout hash_layout(void* ws, int64_t C, int A) {
   p += align_up((size_t)C * 8, 256);
   H.cslot = reinterpret_cast<int64_t*>(p);
   p += align_up((size_t)C * 8, 256);
+  H.perm = reinterpret_cast<int64_t*>(p);
+  p += align_up((size_t)(C / 2 + 1) * 8, 256);
   H.sort_ws = p;
   H.sort_bytes = sort_ws_bytes(C / 2 + 1);
   return H;
@@ -742,11 +746,12 @@ extern "C" int tqpk_groupby_emit(const tqpk_groupby_spec* S, const tqpk_gb_plan*
     TQPK_CUDA(cudaMemsetAsync(counter, 0, 8, s));
     k_hash_collect<<<grid_for(K, 4), kBlock, 0, s>>>(H.gacc, H.hkeys, K, H.pk, H.cslot, counter, groups);
     TQPK_CHECK_LAUNCH();
-    const int64_t* perm = nullptr;
-    int rc2 = sort_pairs(H.pk, TQPK_I64, 0, nullptr, groups, H.sort_ws, H.sort_bytes, s, &perm);
+    if (groups > K / 2) return TQPK_EINVAL;       // the table has two slots per row
+    const SortKey by_packed{H.pk, nullptr, TQPK_I64, 0, 0, 0};
+    int rc2 = sort_keys(&by_packed, 1, nullptr, groups, H.perm, H.sort_ws, H.sort_bytes, s);
     if (rc2) return rc2;
     const GbDev G = to_dev(*plan, S->n_keys);
-    k_emit_hash<<<grid_for(groups, 4), kBlock, 0, s>>>(*S, G, H.gacc, groups, H.pk, H.cslot, perm, E);
+    k_emit_hash<<<grid_for(groups, 4), kBlock, 0, s>>>(*S, G, H.gacc, groups, H.pk, H.cslot, H.perm, E);
     TQPK_CHECK_LAUNCH();
     TQPK_CUDA(cudaStreamSynchronize(s));
     return TQPK_OK;

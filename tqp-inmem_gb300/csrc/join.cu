@@ -261,6 +261,7 @@ struct BuildLayout {
   int64_t* dir;
   int* cnt;
   int64_t* csr;
+  int64_t* rows;       // the passing build rows in row order (a masked build side)
   int64_t* ukeys;
   int64_t* ustart;
   int64_t* head;
@@ -277,6 +278,7 @@ static bool layout(const tqpk_join_plan& p, void* ws, size_t bytes, BuildLayout&
   L.dir = c.take<int64_t>(p.mode == TQPK_JOIN_DIRECT ? p.slots : 1);
   L.cnt = c.take<int>(p.mode == TQPK_JOIN_DIRECT ? p.slots : 1);
   L.csr = c.take<int64_t>(m);
+  L.rows = c.take<int64_t>(m);
   L.ukeys = c.take<int64_t>(p.mode == TQPK_JOIN_SORTED ? m : 1);
   L.ustart = c.take<int64_t>(p.mode == TQPK_JOIN_SORTED ? m + 1 : 1);
   L.head = c.take<int64_t>(p.mode == TQPK_JOIN_SORTED ? m : 1);
@@ -291,7 +293,7 @@ static size_t layout_bytes(const tqpk_join_plan& p) {
   size_t b = 256 + 256;
   if (p.mode == TQPK_JOIN_DIRECT) b += align_up(p.slots * 8, 256) + align_up(p.slots * 4, 256);
   else b += 512;
-  b += align_up(m * 8, 256);
+  b += 2 * align_up(m * 8, 256);
   if (p.mode == TQPK_JOIN_SORTED) b += align_up(m * 8, 256) + align_up((m + 1) * 8, 256) + align_up(m * 8, 256);
   else b += 768;
   b += align_up(((m + kTile - 1) / kTile + 1) * 8, 256);
@@ -374,21 +376,23 @@ extern "C" int tqpk_join_build(tqpk_join_plan* plan, const void* keys, int32_t d
   }
   if (need_sort && plan->nb_rows > 0) {
     plan->unique = 0;
-    // Passing build rows in row order, then a stable sort by key -> CSR.
-    ColSet C;
-    C.n = 1;
-    C.in[0] = nullptr;
-    C.out[0] = L.csr;
-    C.size[0] = 0;  // row ids
-    int64_t* d_m = L.nu + 1;
-    int rc = compact_launch(nullptr, mask, nb, C, d_m, L.sort_ws, L.sort_bytes, s);  // no mask: all rows
+    // Passing build rows in row order (all of them without a mask), then a stable sort by key -> CSR.
+    if (mask) {
+      ColSet C;
+      C.n = 1;
+      C.in[0] = nullptr;
+      C.out[0] = L.rows;
+      C.size[0] = 0;  // row ids
+      int64_t* d_m = L.nu + 1;
+      TQPK_CUDA(cudaMemsetAsync(L.rows, 0, plan->nb_rows * 8, s));   // row ids even if the compaction fails
+      int rc = compact_launch(nullptr, mask, nb, C, d_m, L.sort_ws, L.sort_bytes, s);
+      if (rc) return rc;
+      k_count_status<<<1, 1, 0, s>>>(d_m, L.hdr + 1);   // a failed compaction's status joins the error word
+      TQPK_CHECK_LAUNCH();
+    }
+    const SortKey by_key{keys, nullptr, dt, 0, 0, 0};
+    int rc = sort_keys(&by_key, 1, mask ? L.rows : nullptr, plan->nb_rows, L.csr, L.sort_ws, L.sort_bytes, s);
     if (rc) return rc;
-    k_count_status<<<1, 1, 0, s>>>(d_m, L.hdr + 1);   // a failed compaction's status joins the error word
-    TQPK_CHECK_LAUNCH();
-    const int64_t* sorted = nullptr;
-    rc = sort_pairs(keys, dt, 0, L.csr, plan->nb_rows, L.sort_ws, L.sort_bytes, s, &sorted);
-    if (rc) return rc;
-    TQPK_CUDA(cudaMemcpyAsync(L.csr, sorted, plan->nb_rows * 8, cudaMemcpyDeviceToDevice, s));
     const int direct = plan->mode == TQPK_JOIN_DIRECT;
     k_join_runs<<<grid_for(plan->nb_rows, 4), kBlock, 0, s>>>(keys, dt, L.csr, plan->nb_rows, plan->key_min, direct,
                                                              L.dir, L.head);

@@ -13,11 +13,11 @@
 //      fingerprint match is confirmed by comparing the whole key tuple with
 //      the representative row's, so distinct tuples never share a group.
 //   2. k_key_collect: occupied entries are numbered (group ids in table order).
-//   3. The groups are ordered by key tuple with the library's stable radix sort,
-//      least significant key first: one pass per numeric key, one per 8 bytes
-//      of a string key (big-endian words of the bytes, an int8 column's with
-//      the sign bit flipped, so unsigned word order is the byte order of the
-//      reference's stacked columns).
+//   3. The groups are ordered by key tuple with the library's stable radix sort
+//      (sort_keys over the representative rows): one key per numeric column, one
+//      per 8 bytes of a string column (big-endian words of the bytes, an int8
+//      column's with the sign bit flipped, so unsigned word order is the byte
+//      order of the reference's stacked columns).
 //   4. k_key_codes: every row gets the rank of its group; d_reps[rank] is the
 //      group's representative row.
 //
@@ -124,31 +124,6 @@ __global__ void __launch_bounds__(kBlock) k_key_collect(const uint64_t* __restri
   }
 }
 
-// Sort key of pass (k, word) for group g: a numeric key's value (sorted in its
-// own dtype) or one big-endian 8-byte word of a string key (as int64 whose
-// sign-flipped bits give the unsigned order).
-__global__ void k_key_sortword(const __grid_constant__ KeyTuple K, int k, int word, const int64_t* __restrict__ rep,
-                               int64_t G, int64_t* __restrict__ out) {
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < G; g += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = rep[g];
-    if (K.width[k]) {
-      const uint8_t* s = static_cast<const uint8_t*>(K.col[k]) + row * K.width[k];
-      const uint8_t flip = K.dt[k] == TQPK_I8 ? 0x80u : 0u;   // int8 bytes order as signed values
-      uint64_t w = 0;
-      for (int i = 0; i < 8; ++i) {
-        const int c = word * 8 + i;
-        const uint64_t b = c < K.width[k] ? static_cast<uint64_t>(s[c] ^ flip) : 0ull;
-        w = (w << 8) | b;
-      }
-      out[g] = static_cast<int64_t>(w ^ (1ull << 63));
-    } else if (K.dt[k] == TQPK_F64) {
-      out[g] = __double_as_longlong(static_cast<const double*>(K.col[k])[row]);
-    } else {
-      out[g] = ld_int(K.col[k], K.dt[k], row);
-    }
-  }
-}
-
 __global__ void k_key_rank(const int64_t* __restrict__ perm, int64_t G, const int64_t* __restrict__ rep_of_gid,
                            int64_t* __restrict__ rank_of_gid, int64_t* __restrict__ reps_out) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < G; i += (int64_t)gridDim.x * blockDim.x) {
@@ -211,7 +186,7 @@ using namespace tqpk;
 extern "C" size_t tqpk_key_encode_workspace_bytes(int64_t n) {
   if (n < 0) n = 0;
   const int64_t cap = key_capacity(n);
-  return align_up(cap * 8, 256) * 2 + align_up(n * 8, 256) * 6 + sort_ws_bytes(n) + 4096;
+  return align_up(cap * 8, 256) * 2 + align_up(n * 8, 256) * 5 + sort_ws_bytes(n, kMaxSortKeys) + 4096;
 }
 
 extern "C" int tqpk_key_encode(int32_t n_keys, const void* const* h_keys, const int32_t* h_dtypes,
@@ -245,9 +220,8 @@ extern "C" int tqpk_key_encode(int32_t n_keys, const void* const* h_keys, const 
   int64_t* rank_of_gid = ws.take<int64_t>(n);
   int64_t* perm_a = ws.take<int64_t>(n);
   int64_t* perm_b = ws.take<int64_t>(n);
-  int64_t* words = ws.take<int64_t>(n);
   int* ctl = ws.take<int>(4);
-  void* sort_ws = ws.take<char>(sort_ws_bytes(n));
+  void* sort_ws = ws.take<char>(sort_ws_bytes(n, kMaxSortKeys));
   if (!sort_ws || !ctl) return TQPK_ENOMEM;
   unsigned long long* counter = reinterpret_cast<unsigned long long*>(ctl);   // ctl[0..1]
   int* err = ctl + 2;
@@ -265,18 +239,24 @@ extern "C" int tqpk_key_encode(int32_t n_keys, const void* const* h_keys, const 
   if (e) return e;
   *h_groups = G;
   if (G == 0) return TQPK_OK;
-  // least significant pass first: keys from last to first, words of a string from last to first
+  // the groups by key tuple, each through its representative row; a tuple of more than kMaxSortKeys
+  // words is sorted in runs of words, least significant run first
+  int total = 0;
+  for (int k = 0; k < n_keys; ++k) total += K.width[k] ? (K.width[k] + 7) / 8 : 1;
   int64_t* cur = nullptr;
+  SortKey run[kMaxSortKeys];
+  int m = 0, left = total;
   for (int k = n_keys - 1; k >= 0; --k) {
     const int nw = K.width[k] ? (K.width[k] + 7) / 8 : 1;
-    const int dt = (K.width[k] == 0 && K.dt[k] == TQPK_F64) ? TQPK_F64 : TQPK_I64;
     for (int w = nw - 1; w >= 0; --w) {
-      k_key_sortword<<<grid_for(G, 4), kBlock, 0, s>>>(K, k, w, rep_of_gid, G, words);
-      TQPK_CHECK_LAUNCH();
-      int64_t* out = (cur == perm_a) ? perm_b : perm_a;
-      const int rc = tqpk_argsort_stable(words, dt, 0, cur, G, out, sort_ws, sort_ws_bytes(n), stream);
-      if (rc) return rc;
-      cur = out;
+      run[kMaxSortKeys - 1 - m++] = SortKey{K.col[k], rep_of_gid, K.dt[k], 0, K.width[k], w};
+      if (--left == 0 || m == kMaxSortKeys) {
+        int64_t* out = (cur == perm_a) ? perm_b : perm_a;
+        const int rc = sort_keys(run + kMaxSortKeys - m, m, cur, G, out, sort_ws, sort_ws_bytes(n, kMaxSortKeys), s);
+        if (rc) return rc;
+        cur = out;
+        m = 0;
+      }
     }
   }
   k_key_rank<<<grid_for(G, 4), kBlock, 0, s>>>(cur, G, rep_of_gid, rank_of_gid, d_reps);

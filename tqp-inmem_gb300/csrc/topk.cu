@@ -99,7 +99,7 @@ extern "C" int tqpk_debug_topk_barrier(int32_t spin_limit, int32_t missing) {
 extern "C" size_t tqpk_topk_workspace_bytes(int64_t n, int64_t k) {
   if (n < 0) n = 0;
   if (k <= 256) return topk_scratch_bytes((int)std::max<int64_t>(k, 1)) + 1024;
-  return sort_ws_bytes(n);
+  return sort_ws_bytes(n) + align_up((size_t)n * sizeof(int64_t), 256);
 }
 
 extern "C" int tqpk_topk_stable(const void* d_keys, int32_t dt, int32_t desc, const int64_t* d_perm_in, int64_t n,
@@ -111,10 +111,13 @@ extern "C" int tqpk_topk_stable(const void* d_keys, int32_t dt, int32_t desc, co
   if (ws_bytes < tqpk_topk_workspace_bytes(n, k)) return TQPK_ENOMEM;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (k > 256) {
-    const int64_t* res = nullptr;
-    int rc = sort_pairs(d_keys, dt, desc ? 1 : 0, d_perm_in, n, ws, ws_bytes, s, &res);
+    WsCursor full(ws, ws_bytes);
+    int64_t* order = full.take<int64_t>(n);
+    if (!order) return TQPK_ENOMEM;
+    const SortKey key{d_keys, nullptr, dt, desc ? 1 : 0, 0, 0};
+    int rc = sort_keys(&key, 1, d_perm_in, n, order, full.base + full.off, ws_bytes - full.off, s);
     if (rc) return rc;
-    TQPK_CUDA(cudaMemcpyAsync(d_perm_out, res, m * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+    TQPK_CUDA(cudaMemcpyAsync(d_perm_out, order, m * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
     return TQPK_OK;
   }
   const int grid = topk_grid_size();

@@ -2,13 +2,13 @@
 
 The reference runs one stable torch.sort per key, last key first, each time
 gathering the key through ``perm`` (:26-35), then slices ``perm[:limit]``
-(:41-42) and gathers every input column (:44-54).  Here each key is one
-tqpk_argsort_stable call that sorts keys[perm] and permutes perm in the same
-kernels; with a limit the first key uses the stable top-k, which returns the
-same rows as the full sort followed by the slice.  A [N, w] key (the
-reference ranks its rows with unique(dim=0)) is sorted as ceil(w/8) stable
-passes over 8-byte words of the rows, last word first, which gives the same
-lexicographic order and ties; [N, w] columns are gathered row by row.
+(:41-42) and gathers every input column (:44-54).  Here that loop is one
+tqpk_argsort_keys call; with a limit the first key uses the stable top-k, which
+returns the same rows as the full sort followed by the slice.  A [N, w] key (the
+reference ranks its rows with unique(dim=0)) is sorted by its 8-byte words,
+which gives the same lexicographic order and ties; keys of more words than one
+call takes are sorted key by key (tqpk_argsort_stable), last word of the last
+key first.  [N, w] columns are gathered row by row.
 When every input column comes from one tqp_hash_aggregate call, whose groups are
 in ascending key-tuple order, and the sort keys are a prefix of those group keys,
 all ascending, the stable sort is the identity: only the limit is applied.
@@ -17,9 +17,14 @@ from __future__ import annotations
 
 import torch
 
-from ..ops import argsort_stable, check_deferred, gather, gather_rows, string_words, topk_stable
+from .._lib import MAX_SORT_WORDS
+from ..ops import argsort_keys, argsort_stable, check_deferred, gather, gather_rows, sort_words, string_words, topk_stable
 from ..variable import make_like, wait_ready
 from .filter import _require_gpu
+
+
+def _is_text(col) -> bool:
+    return col.dim() == 2 and col.shape[1] > 1
 
 
 def tqp_sort(gpu_enable, tensor_group, args, with_limit, name="sort"):
@@ -47,6 +52,15 @@ def tqp_sort(gpu_enable, tensor_group, args, with_limit, name="sort"):
     wait_ready(*[tensor_group[k] for k in key_ids])
     perm = None                                           # identity until the first pass
     steps = []
+    cols = [tensor_group[k].tensor for k in key_ids]
+    if len(cols) == len(key_descs) and all(
+            c.is_cuda and (c.dim() == 1 or c.shape[1] == 1 or
+                           (c.shape[1] > 1 and c.dtype in (torch.int8, torch.uint8))) for c in cols):
+        # one call for every key, or for all but the first when a limit ends the sort in a top-k
+        many = list(zip(cols, key_descs))[1 if limit is not None else 0:]
+        if many and sort_words([c for c, _ in many]) <= MAX_SORT_WORDS and (limit is None or not _is_text(cols[0])):
+            perm = argsort_keys([c for c, _ in many], [d for _, d in many])
+            key_ids, key_descs = key_ids[:len(key_ids) - len(many)], key_descs[:len(key_descs) - len(many)]
     for key_id, desc in zip(reversed(key_ids), reversed(key_descs)):
         col = tensor_group[key_id].tensor
         if col.dim() == 2 and col.shape[1] > 1:

@@ -319,6 +319,33 @@ def argsort_stable(keys: torch.Tensor, descending: bool = False,
     return out
 
 
+def sort_words(cols: Sequence[torch.Tensor]) -> int:
+    """Sort words of a key list: one per 1-D column, one per eight bytes of a [N, w] column."""
+    return sum((c.shape[1] + 7) // 8 if c.dim() == 2 and c.shape[1] > 1 else 1 for c in cols)
+
+
+def argsort_keys(cols: Sequence[torch.Tensor], descs: Sequence[bool],
+                 perm_in: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Stable order by cols[0], then cols[1], ... in one library call (at most L.MAX_SORT_WORDS sort
+    words); a [N, w] int8/uint8 column compares byte by byte."""
+    lib = L.load()
+    cols = [c.contiguous() if c.dim() == 2 and c.shape[1] > 1 else _col1d(c) for c in cols]
+    _check_cuda(perm_in, *cols)
+    device = cols[0].device
+    n = int(perm_in.numel()) if perm_in is not None else int(cols[0].shape[0])
+    out = torch.empty(n, dtype=torch.int64, device=device)
+    if n == 0:
+        return out
+    dts = _i32_array([code_of(c.dtype) for c in cols])
+    widths = _i32_array([int(c.shape[1]) if c.dim() == 2 else 0 for c in cols])
+    ws = _ws(lib.tqpk_argsort_keys_workspace_bytes(n, len(cols), dts, widths) if n > 2048 else 0, device)
+    L.check(lib.tqpk_argsort_keys(len(cols), _vp_array([c.data_ptr() for c in cols]), dts, widths,
+                                  _i32_array([int(bool(d)) for d in descs]),
+                                  perm_in.data_ptr() if perm_in is not None else None, n, out.data_ptr(),
+                                  ws.data_ptr(), ws.numel(), _stream(device)), "tqpk_argsort_keys")
+    return out
+
+
 def topk_stable(keys: torch.Tensor, k: int, descending: bool = False,
                 perm_in: Optional[torch.Tensor] = None) -> torch.Tensor:
     """First k of the stable sort of keys[perm_in] (ties in input order)."""
