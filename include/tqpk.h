@@ -281,7 +281,8 @@ int tqpk_groupby_emit(const tqpk_groupby_spec* h_spec, const tqpk_gb_plan* h_pla
  * ties in input order (torch.sort(stable=True, descending=True)).
  * Float keys: -0.0 sorts equal to +0.0 and NaN sorts as the largest value.
  * n <= 2048 sorts in one CTA without a workspace (d_ws may be NULL) and
- * without a host synchronisation; larger sorts synchronise once.
+ * without a host synchronisation; sorts of more than 98304 rows synchronise
+ * once.
  * d_perm_out must not overlap d_perm_in.                                   */
 size_t tqpk_sort_workspace_bytes(int64_t n);
 int tqpk_argsort_stable(const void* d_keys, int32_t key_dtype, int32_t descending,

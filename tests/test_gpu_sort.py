@@ -1,13 +1,14 @@
 """The radix sort at the edges of its tiles and dispatch rules against numpy's stable lexsort: one CTA
-up to 2048 rows, 4096-row tiles below 2^21 rows, 8192-row tiles above; keys whose varying digits lie in
-the low half, the high half, both or nowhere; several keys in one call."""
+up to 2048 rows, one cluster up to 98304 (four rows a thread, or twelve above 32768), 4096-row tiles up to 1228800 rows, 6144-row tiles above; keys whose varying digits lie
+in the low half, the high half, both or nowhere, and more of them than a key is sorted by; several keys
+in one call."""
 import numpy as np
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 2048, 2049, 4095, 4096, 4097, 8193, 65536, 100_003, (1 << 21) - 1, 1 << 21, (1 << 21) + 8193]
+SIZES = [1, 2, 2048, 2049, 4095, 4096, 4097, 32_768, 32_769, 98_304, 98_305, 1_228_800, 1_228_801, 1_234_944, (1 << 21) + 8193]
 
 
 def _image(a, desc):
@@ -63,7 +64,7 @@ def test_varying_digits(make, n):
         _check([k], [desc])
 
 
-@pytest.mark.parametrize("n", [1500, 27_600, 150_001])
+@pytest.mark.parametrize("n", [1500, 2049, 27_600, 60_000, 150_001])
 def test_many_keys(n):
     rng = np.random.default_rng(n)
     words = np.frombuffer(b"BRAND-11BRAND-12BRAND-45LARGE TI", np.int8).reshape(4, 8)
@@ -75,6 +76,20 @@ def test_many_keys(n):
             rng.integers(0, 3, n).astype(np.uint8), rng.integers(0, 9, n).astype(np.int32)]
     _check(keys, [True, False, True, True, False, False])
     _check(keys[1:4], [True, False, False], rng.integers(0, n, n))     # rows may repeat
+
+
+@pytest.mark.parametrize("n", [5000, 98_305, 1_228_800, 1_228_801])
+@pytest.mark.parametrize("make", [
+    lambda r, n: r.integers(90000, 10495001, n) / 100.0,                      # decimals: equal rows beside each other
+    lambda r, n: r.random(n),                                                 # runs of two or three rows to reorder
+    lambda r, n: (1 << 52) * (r.integers(0, 3, n) + 1.0) + r.integers(0, 9, n),   # long runs out of order
+    lambda r, n: np.where(r.integers(0, 50, n) > 0, 0.07, r.random(n)),       # a long run of equal rows
+])
+def test_keys_of_more_digits_than_are_sorted_by(make, n):
+    rng = np.random.default_rng(11)
+    f = make(rng, n).astype(np.float64)
+    _check([f], [True])
+    _check([rng.integers(0, 3, n).astype(np.int32), f], [False, False], rng.permutation(n))
 
 
 def test_too_many_words_raise():

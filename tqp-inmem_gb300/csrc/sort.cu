@@ -6,6 +6,9 @@
 // keys are sorted last to first, each key's digits least significant first.
 // tqpk_argsort_stable is its one-key form.
 //
+// Up to 2048 rows are sorted by one CTA, up to 98304 by one cluster; more rows
+// by the tiled passes below.
+//
 // Every key has an order-preserving unsigned image (signed integers: sign bit
 // flipped in their own width; float64: sign-magnitude flip with -0.0 -> +0.0
 // and NaN as the largest value; eight bytes of a string row big-endian;
@@ -15,22 +18,34 @@
 //          columns; the last CTA of each key scans them into global digit
 //          offsets and records which digits vary (a digit that holds every
 //          row is no pass at all).
-//   pass : launch p runs the p-th varying digit; launches beyond the last one
-//          return at once, so the host never reads the digit masks.  A key's
-//          first pass gathers the key through the rows' current order and
-//          keeps it as a 32-bit word when its varying digits allow; the last
-//          pass writes the int64 permutation itself.
+//   pass : a key gets at most four launches; launch q sorts by the q-th of its
+//          four highest varying digits (fewer vary: the launch returns at once),
+//          so the host never reads the digit masks.  The key's first pass gathers
+//          the column through the rows' current order and keeps a 32-bit word of
+//          it; the sort's last pass writes the int64 permutation itself.
+//   fix  : a key of more than four varying digits (a price as float64 varies in
+//          seven) is then ordered by its four highest digits.  Rows that agree in
+//          those are already in order unless their low digits disagree with it,
+//          which in real columns happens to a few neighbours: runs of up to 32
+//          such rows are sorted in place.  A longer run raises a flag, and the
+//          host, which waits for the sort anyway, sorts again with every digit
+//          (as text is from the start).
 //
-// What bounds a pass: the tiles are L2-resident (8 B per row each way at 32-bit
-// keys), so it is the chain load -> rank -> look-back -> scatter of one tile.
-// Rows are ranked by match_any per warp, reordered by digit in shared memory
-// and written as runs (a 4096-row tile has 16-row runs; the direct scatter
-// they replace wrote 16 B per row to 32 places per warp store), and a digit's
-// look-back reads eight predecessors at a time (one at a time, 129 tiles took
-// ~15 of a pass's 23 us).
+// What bounds a pass: the tiles are L2-resident (8 B per row each way), so it is
+// the chain load -> rank -> look-back -> write of one tile (about 1.5, 2, 3 and
+// 2 us of a 4096-row tile's 9) and the instructions of the rank.  Rows are ranked
+// per warp by eight ballots (match_any of 32 different digits was slower),
+// reordered by digit in shared memory and written as runs, and a digit's
+// look-back reads eight predecessors at a time.
+#include <stddef.h>
+
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tqpk {
 
@@ -46,9 +61,11 @@ struct SortKeySet {
 
 struct SortCtl {
   int err;
+  int redo;                          // a key's four highest digits did not order it: sort by every digit
+  unsigned fixes[kMaxSortKeys];      // runs listed per key
+  unsigned tile_ctr[kMaxPasses];     // next tile of each pass
   unsigned mask[kMaxSortKeys];       // varying digits per key
   unsigned ticket[kMaxSortKeys];     // hist CTAs done
-  unsigned tile_ctr[kMaxPasses];     // next tile of each pass
 };
 
 __host__ __device__ __forceinline__ int sort_key_digits(const SortKey& K) {
@@ -208,34 +225,61 @@ __device__ __forceinline__ uint64_t radix_lookback(uint64_t* status, int64_t til
   return excl;
 }
 
-constexpr int kSortItems = 16;
+constexpr int kSortBlock = 512;
+constexpr int kSortWarps = kSortBlock / 32;
+constexpr int kKeyPasses = 4;                // launches of a key: its four highest varying digits
+constexpr int kFixRun = 32;                  // longest run of rows that k_sort_fix reorders
 
-template <int BLOCK, class V>
+// Shared memory of a pass: the tile's keys (32-bit words, or 64-bit in the every-digit form) and
+// positions, digit places, per-warp digit counts.
+template <int ITEMS, class V, class K>
 constexpr size_t pass_smem() {
-  return (size_t)BLOCK * kSortItems * (8 + sizeof(V)) + kRadix * 12 + (BLOCK / 32) * kRadix * 4;
+  return (size_t)kSortBlock * ITEMS * (sizeof(K) + sizeof(V)) + kRadix * 12 + kSortWarps * kRadix * 4;
+}
+
+// The digits of `mask` a key is sorted by: the four highest varying ones, or all of them.
+__device__ __forceinline__ unsigned sorted_digits(unsigned mask, bool every) {
+  if (every) return mask;
+  while (__popc(mask) > kKeyPasses) mask &= mask - 1;
+  return mask;
 }
 
 template <class V>
 struct PassArgs {
+  SortKey key;
   const int64_t* perm_in;    // element of position i (null: i)
   int64_t n;
-  uint64_t* kbuf[2];
+  void* kbuf[2];
   V* vbuf[2];
   int64_t* perm_out;
-  const int64_t* offsets;
+  const int64_t* offsets;    // of this key: [kDigits][kRadix]
   uint64_t* status;
   SortCtl* ctl;
-  int p;                     // which varying digit, counted over all keys from the last key up
+  int k, nk;                 // this key's index, and the number of keys
+  int q;                     // which of the key's digits
+  unsigned every;            // bit k: key k is sorted by every varying digit
 };
 
-// V: type of a row's position among the n rows (uint32 below 2^32 rows).
-template <int BLOCK, class V>
-__global__ void __launch_bounds__(BLOCK) k_sort_pass(const __grid_constant__ SortKeySet S, const PassArgs<V> A) {
-  constexpr int kTileN = BLOCK * kSortItems;
-  constexpr int kWarps = BLOCK / 32;
-  static_assert(BLOCK >= kRadix, "one thread per digit");
+// How many passes run before key k's, and in all.
+template <class V>
+__device__ __forceinline__ void pass_counts(const PassArgs<V>& A, int& before, int& total) {
+  before = 0;
+  total = 0;
+  for (int j = A.nk - 1; j >= 0; --j) {
+    const int c = __popc(sorted_digits(A.ctl->mask[j], (A.every >> j) & 1u));
+    total += c;
+    if (j > A.k) before += c;
+  }
+}
+
+// V: type of a row's position among the n rows (uint32 below 2^32 rows).  K: uint32, the key's four
+// highest varying digits packed, or uint64, the whole key, when every digit is sorted by.
+template <int ITEMS, class V, class K>
+__global__ void __launch_bounds__(kSortBlock, 2) k_sort_pass(const __grid_constant__ PassArgs<V> A) {
+  constexpr int kTileN = kSortBlock * ITEMS;
+  constexpr bool kEvery = sizeof(K) == 8;
   extern __shared__ __align__(16) unsigned char smem[];
-  uint64_t* s_key = reinterpret_cast<uint64_t*>(smem);
+  K* s_key = reinterpret_cast<K*>(smem);
   V* s_val = reinterpret_cast<V*>(s_key + kTileN);
   int64_t* s_gbase = reinterpret_cast<int64_t*>(s_val + kTileN);
   unsigned* s_dbase = reinterpret_cast<unsigned*>(s_gbase + kRadix);
@@ -243,91 +287,95 @@ __global__ void __launch_bounds__(BLOCK) k_sort_pass(const __grid_constant__ Sor
   __shared__ unsigned s_tile;
   __shared__ unsigned s_ws[kRadix / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the p-th varying digit, keys from last to first
-  int total = 0, key = -1, digit = 0;
-  unsigned kmask = 0;
-  for (int k = S.n - 1; k >= 0; --k) {
-    const unsigned m = A.ctl->mask[k];
-    const int c = __popc(m);
-    if (key < 0 && A.p < total + c) {
-      unsigned b = m;
-      for (int q = A.p - total; q > 0; --q) b &= b - 1;
-      key = k;
-      kmask = m;
-      digit = __ffs(b) - 1;
-    }
-    total += c;
-  }
+  const unsigned varying = A.ctl->mask[A.k];
+  const unsigned digits = sorted_digits(varying, kEvery);
   const int64_t n = A.n;
-  if (key < 0) {
-    if (A.p == 0)                    // no digit varies: the order stays as it is
-      for (int64_t i = blockIdx.x * (int64_t)BLOCK + threadIdx.x; i < n; i += (int64_t)gridDim.x * BLOCK)
+  int before, total;
+  pass_counts(A, before, total);
+  if (A.q >= __popc(digits)) {
+    if (total == 0 && A.k == 0 && A.q == 0)       // no digit varies: the order stays as it is
+      for (int64_t i = blockIdx.x * (int64_t)kSortBlock + threadIdx.x; i < n; i += (int64_t)gridDim.x * kSortBlock)
         A.perm_out[i] = A.perm_in ? A.perm_in[i] : i;
     return;
   }
-  const SortKey K = S.k[key];
-  const bool first = (kmask & ((1u << digit) - 1u)) == 0;     // the key's first pass reads the column
-  const bool keep = (kmask >> (digit + 1)) != 0;              // a later pass of the key reads kbuf
-  const bool final_pass = A.p == total - 1;
-  const bool low = (kmask >> 4) == 0, high = (kmask & 15u) == 0;
-  const bool narrow = low || high;                            // the key is kept as its low or high half
-  const int shift = 8 * (digit - (high ? 4 : 0));
-  const int from = (A.p + 1) & 1, to = A.p & 1;
+  const int p = before + A.q;
+  unsigned left = digits;
+  for (int q = A.q; q > 0; --q) left &= left - 1;
+  const int digit = __ffs(left) - 1;
+  const bool more = (left & (left - 1)) != 0;                 // a later pass of this key
+  const bool keep = more || varying != digits;                // that pass, or k_sort_check, reads kbuf
+  const bool final_pass = p == total - 1;
+  const bool keep_row = !final_pass || varying != digits;
+  // the 32-bit word of a key holds its sorted digits side by side
+  const int shift = kEvery ? 8 * digit : 8 * A.q;
+  const int from = (p + 1) & 1, to = p & 1;
   const int64_t tiles = (n + kTileN - 1) / kTileN;
-  const unsigned epoch = (unsigned)A.p + 1;
-  const int64_t* off = A.offsets + ((size_t)key * kDigits + digit) * kRadix;
+  const unsigned epoch = (unsigned)p + 1;
+  const int64_t* off = A.offsets + digit * kRadix;
   const unsigned lt = (1u << lane) - 1u;
   while (true) {
     __syncthreads();
-    if (threadIdx.x == 0) s_tile = atomicAdd(&A.ctl->tile_ctr[A.p], 1u);
-    for (int i = threadIdx.x; i < kWarps * kRadix; i += BLOCK) (&wcnt[0][0])[i] = 0;
+    if (threadIdx.x == 0) s_tile = atomicAdd(&A.ctl->tile_ctr[p], 1u);
+    for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortBlock) (&wcnt[0][0])[i] = 0;
     __syncthreads();
     const int64_t tile = s_tile;
     if (tile >= tiles) return;
     const int64_t tbase = tile * kTileN;
-    const int64_t wbase = tbase + (int64_t)warp * (32 * kSortItems);
-    uint64_t k[kSortItems];
-    V v[kSortItems];
-    unsigned rank[kSortItems];
+    const int64_t wbase = tbase + (int64_t)warp * (32 * ITEMS);
+    K k[ITEMS];
+    V v[ITEMS];
+    unsigned rank[ITEMS];
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
       const int64_t i = wbase + j * 32 + lane;
-      v[j] = i >= n ? V(0) : A.p == 0 ? (V)i : A.vbuf[from][i];
+      v[j] = i >= n ? V(0) : p == 0 ? (V)i : A.vbuf[from][i];
     }
-    if (first) {
+    if (A.q == 0) {
 #pragma unroll
-      for (int j = 0; j < kSortItems; ++j) {
+      for (int j = 0; j < ITEMS; ++j) {
         // after an expired look-back a position may be left over from other data: it stays in bounds,
         // and the call reports the error
         const int64_t e = (int64_t)v[j] < n ? (int64_t)v[j] : n - 1;
         k[j] = 0;
-        if (wbase + j * 32 + lane < n) k[j] = sort_image(K, A.perm_in ? A.perm_in[e] : e);
-        if (high) k[j] >>= 32;
-      }
-    } else if (narrow) {
+        if (wbase + j * 32 + lane < n) {
+          const uint64_t u = sort_image(A.key, A.perm_in ? A.perm_in[e] : e);
+          if (kEvery) {
+            k[j] = (K)u;
+          } else {
+            unsigned w = 0, d = digits;
 #pragma unroll
-      for (int j = 0; j < kSortItems; ++j) {
-        const int64_t i = wbase + j * 32 + lane;
-        k[j] = i < n ? reinterpret_cast<const unsigned*>(A.kbuf[from])[i] : 0;
+            for (int q = 0; q < kKeyPasses; ++q) {
+              if (d) w |= ((unsigned)(u >> (8 * (__ffs(d) - 1))) & 255u) << (8 * q);
+              d &= d - 1;
+            }
+            k[j] = (K)w;
+          }
+        }
       }
     } else {
+      const K* in = static_cast<const K*>(A.kbuf[from]);
 #pragma unroll
-      for (int j = 0; j < kSortItems; ++j) {
+      for (int j = 0; j < ITEMS; ++j) {
         const int64_t i = wbase + j * 32 + lane;
-        k[j] = i < n ? A.kbuf[from][i] : 0;
+        k[j] = i < n ? in[i] : 0;
       }
     }
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
       const bool ok = wbase + j * 32 + lane < n;
-      const unsigned d = ok ? (unsigned)(k[j] >> shift) & 255u : 256u + lane;   // out of range: a digit of its own
-      const unsigned peers = __match_any_sync(0xffffffffu, d);
-      unsigned base = 0;
-      if (ok) base = wcnt[warp][d];
+      const unsigned d = (unsigned)(k[j] >> shift) & 255u;
+      unsigned peers = __ballot_sync(0xffffffffu, ok);     // lanes of the warp with the same digit
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const bool set = (d >> b) & 1u;
+        const unsigned m = __ballot_sync(0xffffffffu, set);
+        peers &= set ? m : ~m;
+      }
+      const int leader = ok ? 31 - __clz(peers) : lane;
+      unsigned old = 0;
+      if (ok && lane == leader) old = atomicAdd(&wcnt[warp][d], (unsigned)__popc(peers));
+      rank[j] = __shfl_sync(0xffffffffu, old, leader) + __popc(peers & lt);
       __syncwarp();
-      if (ok && lane == 31 - __clz(peers)) wcnt[warp][d] = base + __popc(peers);
-      __syncwarp();
-      rank[j] = base + __popc(peers & lt);
     }
     __syncthreads();
     // thread d owns digit d: warp prefixes, the tile's count (published at once), then the digits'
@@ -336,7 +384,7 @@ __global__ void __launch_bounds__(BLOCK) k_sort_pass(const __grid_constant__ Sor
     if (threadIdx.x < kRadix) {
       const int d = threadIdx.x;
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
+      for (int w = 0; w < kSortWarps; ++w) {
         const unsigned c = wcnt[w][d];
         wcnt[w][d] = run;
         run += c;
@@ -347,14 +395,14 @@ __global__ void __launch_bounds__(BLOCK) k_sort_pass(const __grid_constant__ Sor
     }
     __syncthreads();
     if (threadIdx.x < kRadix) {
-      unsigned before = 0;
+      unsigned below = 0;
 #pragma unroll
-      for (int w = 0; w < kRadix / 32; ++w) before += w < warp ? s_ws[w] : 0;
-      s_dbase[threadIdx.x] = before + inc - run;
+      for (int w = 0; w < kRadix / 32; ++w) below += w < warp ? s_ws[w] : 0;
+      s_dbase[threadIdx.x] = below + inc - run;
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
       if (wbase + j * 32 + lane < n) {
         const unsigned d = (unsigned)(k[j] >> shift) & 255u;
         const unsigned at = s_dbase[d] + wcnt[warp][d] + rank[j];
@@ -370,21 +418,112 @@ __global__ void __launch_bounds__(BLOCK) k_sort_pass(const __grid_constant__ Sor
     }
     __syncthreads();
     const int count = (int)(n - tbase < kTileN ? n - tbase : kTileN);
-    for (int i = threadIdx.x; i < count; i += BLOCK) {
-      const uint64_t x = s_key[i];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < count; i += kSortBlock) {
+      const K x = s_key[i];
       const V src = s_val[i];
       int64_t pos = s_gbase[(unsigned)(x >> shift) & 255u] + i;
       pos = pos < n ? pos : n - 1;             // in bounds also after an expired look-back
-      if (keep) {
-        if (narrow) reinterpret_cast<unsigned*>(A.kbuf[to])[pos] = (unsigned)x;
-        else A.kbuf[to][pos] = x;
-      }
+      if (keep) static_cast<K*>(A.kbuf[to])[pos] = x;
       if (final_pass) {
         const int64_t e = (int64_t)src < n ? (int64_t)src : n - 1;
         A.perm_out[pos] = A.perm_in ? A.perm_in[e] : e;
-      } else {
-        A.vbuf[to][pos] = src;
       }
+      if (keep_row) A.vbuf[to][pos] = src;
+    }
+  }
+}
+
+template <class V>
+__device__ __forceinline__ int64_t pass_element(const PassArgs<V>& A, V v) {
+  const int64_t e = (int64_t)v < A.n ? (int64_t)v : A.n - 1;
+  return A.perm_in ? A.perm_in[e] : e;
+}
+
+// After the passes of a key that varies in more digits than it was sorted by: neighbours with one word
+// are compared by the whole key.  The first pair of a run (rows of one word) found out of order puts
+// the run's first row on the list that k_sort_fix works off (the free position buffer); a run longer
+// than kFixRun sets ctl->redo.
+template <class V>
+__global__ void __launch_bounds__(kBlock) k_sort_check(const __grid_constant__ PassArgs<V> A) {
+  const unsigned varying = A.ctl->mask[A.k];
+  if (varying == sorted_digits(varying, false)) return;
+  int before, total;
+  pass_counts(A, before, total);
+  const int at = (before + kKeyPasses - 1) & 1;
+  const unsigned* word = static_cast<const unsigned*>(A.kbuf[at]);
+  const V* pos = A.vbuf[at];
+  V* list = A.vbuf[at ^ 1];
+  const int64_t n = A.n;
+  const int lane = threadIdx.x & 31;
+  for (int64_t i0 = blockIdx.x * (int64_t)kBlock + (threadIdx.x & ~31); i0 < n; i0 += (int64_t)gridDim.x * kBlock) {
+    const int64_t i = i0 + lane;
+    const unsigned w = i < n ? word[i] : 0;
+    const bool joins = i > 0 && i < n && word[i - 1] == w;
+    const bool next = lane < 31 ? __shfl_down_sync(0xffffffffu, (int)joins, 1) : (__shfl_down_sync(0xffffffffu, (int)joins, 1), false);
+    uint64_t u = 0;
+    if (joins || next) u = sort_image(A.key, pass_element(A, pos[i]));
+    uint64_t prev = __shfl_up_sync(0xffffffffu, u, 1);
+    if (joins && lane == 0) prev = sort_image(A.key, pass_element(A, pos[i - 1]));
+    if (!joins || prev <= u) continue;
+    // out of order: the run's first such pair if every pair before it in the run is in order
+    int64_t head = i - 1;
+    uint64_t x = prev;
+    bool mine = true;
+    while (head > 0 && word[head - 1] == w) {
+      if (i - head >= kFixRun) {
+        A.ctl->redo = 1;
+        mine = false;
+        break;
+      }
+      const uint64_t y = sort_image(A.key, pass_element(A, pos[head - 1]));
+      if (y > x) {
+        mine = false;
+        break;
+      }
+      x = y;
+      --head;
+    }
+    if (mine) list[atomicAdd(&A.ctl->fixes[A.k], 1u)] = (V)head;
+  }
+}
+
+// Orders each listed run by the whole key: a stable insertion sort of at most kFixRun rows.
+template <class V>
+__global__ void __launch_bounds__(kBlock) k_sort_fix(const __grid_constant__ PassArgs<V> A) {
+  const int64_t fixes = A.ctl->fixes[A.k];
+  if (fixes == 0 || A.ctl->redo) return;
+  int before, total;
+  pass_counts(A, before, total);
+  const int at = (before + kKeyPasses - 1) & 1;
+  const unsigned* word = static_cast<const unsigned*>(A.kbuf[at]);
+  V* pos = A.vbuf[at];
+  const V* list = A.vbuf[at ^ 1];
+  for (int64_t f = blockIdx.x * (int64_t)kBlock + threadIdx.x; f < fixes; f += (int64_t)gridDim.x * kBlock) {
+    const int64_t i = (int64_t)list[f];
+    const unsigned w = word[i];
+    uint64_t key[kFixRun];
+    V row[kFixRun];
+    int m = 0;
+    for (int64_t j = i; j < A.n && word[j] == w; ++j) {
+      if (m == kFixRun) {
+        A.ctl->redo = 1;
+        m = 0;
+        break;
+      }
+      const V v = pos[j];
+      const uint64_t u = sort_image(A.key, pass_element(A, v));
+      int b = m++;
+      for (; b > 0 && key[b - 1] > u; --b) {
+        key[b] = key[b - 1];
+        row[b] = row[b - 1];
+      }
+      key[b] = u;
+      row[b] = v;
+    }
+    for (int a = 0; a < m; ++a) {
+      pos[i + a] = row[a];
+      if (before + kKeyPasses == total) A.perm_out[i + a] = pass_element(A, row[a]);
     }
   }
 }
@@ -452,11 +591,206 @@ __global__ void __launch_bounds__(1024) k_sort_small(const __grid_constant__ Sor
   for (int i = threadIdx.x; i < n; i += blockDim.x) perm_out[i] = perm_in ? perm_in[order[i]] : order[i];
 }
 
-// Tiles of 512 threads (8192 rows, 32-row runs) once they fill the SMs twice; 256 threads below.
-constexpr int64_t kBigSort = int64_t(1) << 21;
+// Mid-size sorts (the groups of an aggregate, small tables): the rows live in the shared memory of one
+// cluster of 16 CTAs for the whole sort, every key and digit of it in one launch.  As launches these
+// sorts were 60 passes of seven tiles: each ~15 us of latency for 0.3 MB of rows, two synchronisations a
+// key.  A pass here is rank, exchange of the CTAs' digit counts, and a scatter into the owning CTA's
+// buffer (distributed shared memory), with two hardware cluster barriers and no look-back.  Digits are
+// the 8-bit windows that start at the lowest varying bit not yet sorted by.
+constexpr int kClusterCtas = 16;
+constexpr int kClusterThreads = 512;
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kClusterItemsSmall = 4, kClusterItemsLarge = 12;
+constexpr int64_t kClusterSort = (int64_t)kClusterCtas * kClusterThreads * kClusterItemsLarge;   // 98304 rows
+
+template <int ITEMS>
+struct ClusterSmem {
+  static constexpr int kRows = kClusterThreads * ITEMS;
+  uint64_t key[2][kRows];
+  unsigned val[2][kRows];
+  unsigned wcnt[kClusterWarps][kRadix];
+  unsigned count[2][kRadix];         // this CTA's digit counts, by pass parity
+  unsigned base[kRadix];
+  uint64_t bits[2][2];               // OR, AND of this CTA's keys, by key parity
+  unsigned ws[kClusterWarps];
+};
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kClusterThreads) k_sort_cluster(const __grid_constant__ SortKeySet S,
+                                                                  const int64_t* __restrict__ perm_in, int n,
+                                                                  int64_t* __restrict__ perm_out) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  ClusterSmem<ITEMS>& M = *reinterpret_cast<ClusterSmem<ITEMS>*>(raw);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cta = (int)cluster.block_rank();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const unsigned R = ((unsigned)n + kClusterCtas - 1) / kClusterCtas;        // rows per CTA (<= kRows)
+  const int mine = max(0, min((int)R, n - cta * (int)R));
+  int cur = 0, pass = 0;
+  for (int i = threadIdx.x; i < mine; i += kClusterThreads) M.val[0][i] = (unsigned)(cta * (int)R + i);
+  __syncthreads();
+  for (int key = S.n - 1; key >= 0; --key) {
+    const SortKey K = S.k[key];
+    uint64_t any = 0, all = ~0ull;
+    for (int i = threadIdx.x; i < mine; i += kClusterThreads) {
+      const unsigned v = M.val[cur][i];
+      const uint64_t u = sort_image(K, perm_in ? perm_in[v] : (int64_t)v);
+      M.key[cur][i] = u;
+      any |= u;
+      all &= u;
+    }
+    if (threadIdx.x == 0) {
+      M.bits[key & 1][0] = 0;
+      M.bits[key & 1][1] = ~0ull;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      any |= __shfl_xor_sync(0xffffffffu, any, o);
+      all &= __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    if (lane == 0) {
+      atomicOr(reinterpret_cast<unsigned long long*>(&M.bits[key & 1][0]), (unsigned long long)any);
+      atomicAnd(reinterpret_cast<unsigned long long*>(&M.bits[key & 1][1]), (unsigned long long)all);
+    }
+    cluster.sync();
+    any = 0;
+    all = ~0ull;
+    if (lane < kClusterCtas) {
+      const uint64_t* b = cluster.map_shared_rank(&M.bits[key & 1][0], lane);
+      any = b[0];
+      all = b[1];
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      any |= __shfl_xor_sync(0xffffffffu, any, o);
+      all &= __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    uint64_t vary = any & ~all;      // the same in every CTA, so all run the same passes
+    while (vary) {
+      const int shift = __ffsll((long long)vary) - 1;
+      vary = shift + 8 < 64 ? vary & (~0ull << (shift + 8)) : 0;
+      for (int i = threadIdx.x; i < kClusterWarps * kRadix; i += kClusterThreads) (&M.wcnt[0][0])[i] = 0;
+      __syncthreads();
+      uint64_t k[ITEMS];
+      unsigned v[ITEMS], rank[ITEMS];
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) {
+        const int i = warp * (32 * ITEMS) + j * 32 + lane;
+        const bool ok = i < mine;
+        k[j] = ok ? M.key[cur][i] : 0;
+        v[j] = ok ? M.val[cur][i] : 0;
+        const unsigned d = (unsigned)(k[j] >> shift) & 255u;
+        unsigned peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          const bool set = (d >> b) & 1u;
+          const unsigned m = __ballot_sync(0xffffffffu, set);
+          peers &= set ? m : ~m;
+        }
+        const int leader = ok ? 31 - __clz(peers) : lane;
+        unsigned old = 0;
+        if (ok && lane == leader) old = atomicAdd(&M.wcnt[warp][d], (unsigned)__popc(peers));
+        rank[j] = __shfl_sync(0xffffffffu, old, leader) + __popc(peers & lt);
+        __syncwarp();
+      }
+      __syncthreads();
+      if (threadIdx.x < kRadix) {
+        unsigned run = 0;
+#pragma unroll
+        for (int w = 0; w < kClusterWarps; ++w) {
+          const unsigned c = M.wcnt[w][threadIdx.x];
+          M.wcnt[w][threadIdx.x] = run;
+          run += c;
+        }
+        M.count[pass & 1][threadIdx.x] = run;
+      }
+      cluster.sync();
+      unsigned total = 0, before = 0, inc = 0;
+      if (threadIdx.x < kRadix) {
+#pragma unroll
+        for (int c = 0; c < kClusterCtas; ++c) {
+          const unsigned x = cluster.map_shared_rank(&M.count[pass & 1][0], c)[threadIdx.x];
+          before += c < cta ? x : 0;
+          total += x;
+        }
+        inc = warp_incl_scan(total);
+        if (lane == 31) M.ws[warp] = inc;
+      }
+      __syncthreads();
+      if (threadIdx.x < kRadix) {
+        unsigned below = 0;
+#pragma unroll
+        for (int w = 0; w < kRadix / 32; ++w) below += w < warp ? M.ws[w] : 0;
+        M.base[threadIdx.x] = below + inc - total + before;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) {
+        if (warp * (32 * ITEMS) + j * 32 + lane < mine) {
+          const unsigned d = (unsigned)(k[j] >> shift) & 255u;
+          const unsigned pos = M.base[d] + M.wcnt[warp][d] + rank[j];
+          const unsigned owner = pos / R, at = pos - owner * R;
+          cluster.map_shared_rank(&M.key[cur ^ 1][0], owner)[at] = k[j];
+          cluster.map_shared_rank(&M.val[cur ^ 1][0], owner)[at] = v[j];
+        }
+      }
+      cluster.sync();
+      cur ^= 1;
+      ++pass;
+    }
+  }
+  for (int i = threadIdx.x; i < mine; i += kClusterThreads) {
+    const unsigned v = M.val[cur][i];
+    perm_out[cta * (int64_t)R + i] = perm_in ? perm_in[v] : (int64_t)v;
+  }
+  cluster.sync();                    // no CTA leaves while another may still read its counts
+}
+
+// One cluster, where the device can hold one (launched is set), else nothing.
+template <int ITEMS>
+static int run_cluster(const SortKeySet& S, const int64_t* perm_in, int n, int64_t* perm_out, bool& launched,
+                       cudaStream_t s) {
+  constexpr size_t smem = sizeof(ClusterSmem<ITEMS>);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kClusterCtas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(kClusterCtas);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  static int fits = -1;
+  if (fits < 0) {
+    int clusters = 0;
+    if (cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, k_sort_cluster<ITEMS>, &cfg) != cudaSuccess)
+      clusters = 0;
+    (void)cudaGetLastError();
+    fits = clusters > 0;
+  }
+  launched = fits > 0;
+  if (!launched) return TQPK_OK;
+  TQPK_CUDA(cudaLaunchKernelEx(&cfg, k_sort_cluster<ITEMS>, S, perm_in, n, perm_out));
+  ++g_launches;
+  return TQPK_OK;
+}
+
+// Rows per thread of a pass.  All tiles of a sort of up to 1.2 M rows are resident at once at eight
+// (two CTAs of 4096 rows per SM); larger sorts take twelve, whose longer runs and fewer look-backs
+// cost less per row.
+constexpr int kItemsSmall = 8, kItemsLarge = 12;
+constexpr int64_t kLargeSort = int64_t(1200) << 10;
 
 static int64_t sort_tiles(int64_t n) {
-  const int64_t t = (n >= kBigSort ? 512 : 256) * kSortItems;
+  const int64_t t = (n > kLargeSort ? kItemsLarge : kItemsSmall) * kSortBlock;
   return n > 0 ? (n + t - 1) / t : 1;
 }
 
@@ -471,24 +805,31 @@ size_t sort_ws_bytes(int64_t n, int nk) {
   return b + 1024;
 }
 
-template <int BLOCK, class V>
-static int run_passes(const SortKeySet& S, PassArgs<V> A, int max_passes, cudaStream_t s) {
-  constexpr size_t smem = pass_smem<BLOCK, V>();
+// The passes of one key.
+template <int ITEMS, class V, class K>
+static int run_key(PassArgs<V> A, cudaStream_t s) {
+  constexpr size_t smem = pass_smem<ITEMS, V, K>();
   static int per_sm = 0;
   if (!per_sm) {
-    TQPK_CUDA(cudaFuncSetAttribute(k_sort_pass<BLOCK, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TQPK_CUDA(cudaFuncSetAttribute(k_sort_pass<ITEMS, V, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int o = 0;
-    TQPK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sort_pass<BLOCK, V>, BLOCK, smem));
+    TQPK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sort_pass<ITEMS, V, K>, kSortBlock, smem));
     per_sm = std::max(o, 1);
   }
-  const int64_t tiles = (A.n + BLOCK * kSortItems - 1) / (BLOCK * kSortItems);
-  const int grid = (int)std::min<int64_t>(tiles, (int64_t)per_sm * num_sms());
-  for (A.p = 0; A.p < max_passes; ++A.p) {
+  const int grid = (int)std::min<int64_t>(sort_tiles(A.n), (int64_t)per_sm * num_sms());
+  const int nd = sort_key_digits(A.key);
+  const int passes = sizeof(K) == 8 ? nd : std::min(nd, kKeyPasses);
+  for (A.q = 0; A.q < passes; ++A.q) {
     timing_before(KID_SORT_PASS, s);
-    k_sort_pass<BLOCK, V><<<grid, BLOCK, smem, s>>>(S, A);
+    k_sort_pass<ITEMS, V, K><<<grid, kSortBlock, smem, s>>>(A);
     timing_after(KID_SORT_PASS, s);
     TQPK_CHECK_LAUNCH();
   }
+  if (passes == nd) return TQPK_OK;
+  k_sort_check<V><<<grid_for(A.n, 8), kBlock, 0, s>>>(A);
+  TQPK_CHECK_LAUNCH();
+  k_sort_fix<V><<<num_sms(), kBlock, 0, s>>>(A);
+  TQPK_CHECK_LAUNCH();
   return TQPK_OK;
 }
 
@@ -508,29 +849,46 @@ static int sort_large(const SortKeySet& S, const int64_t* perm_in, int64_t n, in
   A.vbuf[0] = cur.take<V>(n);
   A.vbuf[1] = cur.take<V>(n);
   if (!ctl || !hist || !status || !offsets || !A.kbuf[0] || !A.kbuf[1] || !A.vbuf[0] || !A.vbuf[1]) return TQPK_ENOMEM;
-  TQPK_CUDA(cudaMemsetAsync(ws, 0, zeroed, s));
-  const int gx = (int)std::max<int64_t>(1, std::min<int64_t>((n + kHistThreads * 16 - 1) / (kHistThreads * 16),
-                                                             (int64_t)num_sms() * 2));
-  k_sort_hist<<<dim3(gx, S.n), kHistThreads, 0, s>>>(S, perm_in, n, hist, offsets, ctl);
-  TQPK_CHECK_LAUNCH();
   A.perm_in = perm_in;
   A.n = n;
   A.perm_out = perm_out;
-  A.offsets = offsets;
   A.status = status;
   A.ctl = ctl;
-  int max_passes = 0;
-  for (int k = 0; k < S.n; ++k) max_passes += sort_key_digits(S.k[k]);
-  const int rc = n >= kBigSort ? run_passes<512, V>(S, A, max_passes, s) : run_passes<256, V>(S, A, max_passes, s);
-  if (rc) return rc;
-  int err = 0;
-  TQPK_CUDA(cudaMemcpyAsync(&err, &ctl->err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  TQPK_CUDA(cudaStreamSynchronize(s));
-  return err;
+  A.nk = S.n;
+  const int gx = (int)std::max<int64_t>(1, std::min<int64_t>((n + kHistThreads * 16 - 1) / (kHistThreads * 16),
+                                                             (int64_t)num_sms() * 2));
+  // eight letters of text rarely differ in the first four only: text is sorted by every digit
+  for (int k = 0; k < S.n; ++k) A.every |= S.k[k].width ? 1u << k : 0u;
+  for (int round = 0; round < 2; ++round) {
+    if (round == 0) {
+      TQPK_CUDA(cudaMemsetAsync(ws, 0, zeroed, s));
+      k_sort_hist<<<dim3(gx, S.n), kHistThreads, 0, s>>>(S, perm_in, n, hist, offsets, ctl);
+      TQPK_CHECK_LAUNCH();
+    } else {                         // the masks and offsets stay
+      A.every = ~0u;
+      TQPK_CUDA(cudaMemsetAsync(ctl, 0, offsetof(SortCtl, mask), s));
+      TQPK_CUDA(cudaMemsetAsync(status, 0, (size_t)sort_tiles(n) * kRadix * sizeof(uint64_t), s));
+    }
+    for (int k = S.n - 1; k >= 0; --k) {
+      A.key = S.k[k];
+      A.k = k;
+      A.offsets = offsets + (size_t)k * kDigits * kRadix;
+      const bool large = n > kLargeSort;
+      const int rc = (A.every >> k) & 1u ? (large ? run_key<kItemsLarge, V, uint64_t>(A, s) : run_key<kItemsSmall, V, uint64_t>(A, s))
+                                         : (large ? run_key<kItemsLarge, V, uint32_t>(A, s) : run_key<kItemsSmall, V, uint32_t>(A, s));
+      if (rc) return rc;
+    }
+    int h[2] = {0, 0};               // [0] error, [1] a key needs every digit
+    TQPK_CUDA(cudaMemcpyAsync(h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s));
+    TQPK_CUDA(cudaStreamSynchronize(s));
+    if (h[0]) return h[0];
+    if (!h[1]) return TQPK_OK;
+  }
+  return TQPK_ETIMEOUT;              // not reached: the second round sorts by every digit
 }
 
 // The stable order of elements perm_in[0..n) (null: 0..n-1) by keys[0], then keys[1], ...  perm_out must
-// not overlap perm_in.  n > kSmallSort synchronises once (the look-back's error word).
+// not overlap perm_in.  n > kClusterSort synchronises once (the look-back's error word).
 int sort_keys(const SortKey* keys, int nk, const int64_t* perm_in, int64_t n, int64_t* perm_out, void* ws,
               size_t ws_bytes, cudaStream_t s) {
   if (nk < 1 || nk > kMaxSortKeys) return TQPK_EUNSUPPORTED;
@@ -545,6 +903,13 @@ int sort_keys(const SortKey* keys, int nk, const int64_t* perm_in, int64_t n, in
   }
   if (!ws) return TQPK_EINVAL;
   if (ws_bytes < sort_ws_bytes(n, nk)) return TQPK_ENOMEM;
+  if (n <= kClusterSort) {
+    bool launched = false;
+    const int rc = n <= kClusterCtas * kClusterThreads * kClusterItemsSmall
+                       ? run_cluster<kClusterItemsSmall>(S, perm_in, (int)n, perm_out, launched, s)
+                       : run_cluster<kClusterItemsLarge>(S, perm_in, (int)n, perm_out, launched, s);
+    if (rc || launched) return rc;
+  }
   if (sort_tiles(n) > INT32_MAX) return TQPK_EUNSUPPORTED;
   if (n < (int64_t(1) << 32)) return sort_large<uint32_t>(S, perm_in, n, perm_out, ws, ws_bytes, s);
   return sort_large<uint64_t>(S, perm_in, n, perm_out, ws, ws_bytes, s);
