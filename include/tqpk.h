@@ -310,11 +310,13 @@ int tqpk_topk_stable(const void* d_keys, int32_t key_dtype, int32_t descending,
 
 /* ---- (c) join ---------------------------------------------------------- */
 enum { TQPK_JOIN_DIRECT = 1, TQPK_JOIN_SORTED = 2 };
+enum { TQPK_JOIN_UNKNOWN = 2 };
 enum { TQPK_JT_INNER = 0, TQPK_JT_SEMI = 1, TQPK_JT_ANTI = 2, TQPK_JT_OUTER = 3 };
 
 typedef struct {
   int32_t mode;        /* TQPK_JOIN_DIRECT (dense key range) or TQPK_JOIN_SORTED */
-  int32_t unique;      /* build keys are unique (set by tqpk_join_build) */
+  int32_t unique;      /* 1: build keys are unique, 0: they repeat, TQPK_JOIN_UNKNOWN: not known yet
+                          (set by the build; + 256: 64-bit directory entries, 2^32 - 1 build rows or more) */
   int64_t nb_rows;     /* build rows passing the build filter */
   int64_t key_min, key_max;
   int64_t slots;       /* DIRECT: key_max - key_min + 1 */
@@ -333,6 +335,17 @@ int tqpk_join_plan_build(const void* d_build_keys, int32_t key_dtype, const uint
 int tqpk_join_build(tqpk_join_plan* h_plan, const void* d_build_keys, int32_t key_dtype,
                     const uint8_t* d_build_mask, int64_t nb, void* d_ws, size_t ws_bytes,
                     tqpk_stream stream);
+/* tqpk_join_build in its two stages.  tqpk_join_directory builds what a unique
+ * build side, or a semi or anti join of any, needs, and does not synchronise
+ * (DIRECT; unique becomes TQPK_JOIN_UNKNOWN).  tqpk_join_rows adds the sorted
+ * build rows that an inner or outer join of repeated keys reads.  Same
+ * arguments and workspace in both.                                          */
+int tqpk_join_directory(tqpk_join_plan* h_plan, const void* d_build_keys, int32_t key_dtype,
+                        const uint8_t* d_build_mask, int64_t nb, void* d_ws, size_t ws_bytes,
+                        tqpk_stream stream);
+int tqpk_join_rows(tqpk_join_plan* h_plan, const void* d_build_keys, int32_t key_dtype,
+                   const uint8_t* d_build_mask, int64_t nb, void* d_ws, size_t ws_bytes,
+                   tqpk_stream stream);
 /* Probes every probe row passing its mask against the directory that
  * tqpk_join_build left in d_build_ws and writes the matches in the
  * reference's order (ascending probe row; inside one build-key bucket,
@@ -341,12 +354,28 @@ int tqpk_join_build(tqpk_join_plan* h_plan, const void* d_build_keys, int32_t ke
  * unused, may be NULL); OUTER writes the pairs, then the unmatched probe rows
  * with build id TQPK_NULL_INDEX.  *h_count is the number of outputs; when it
  * exceeds capacity only the first `capacity` are written and TQPK_ECAPACITY
- * is returned (call again with a larger buffer).  Synchronises.             */
+ * is returned (call again with a larger buffer).  An inner or outer probe of a
+ * directory whose unique is TQPK_JOIN_UNKNOWN writes nothing when a key turns
+ * out to repeat: TQPK_ECAPACITY with *h_count = -1 (call tqpk_join_rows, then
+ * probe again).  Synchronises.                                              */
 size_t tqpk_join_probe_workspace_bytes(int64_t np);
 int tqpk_join_probe(const tqpk_join_plan* h_plan, const void* d_build_ws, const void* d_probe_keys,
                     int32_t probe_dtype, const uint8_t* d_probe_mask, int64_t np, int32_t join_type,
                     int64_t* d_out_build, int64_t* d_out_probe, int64_t capacity, int64_t* h_count,
                     void* d_probe_ws, size_t probe_ws_bytes, tqpk_stream stream);
+
+/* An inner probe in two calls, for exactly sized outputs: tqpk_join_count leaves
+ * the pair offsets of every tile of probe rows in d_probe_ws and their number in
+ * *h_count (synchronises); tqpk_join_write with the same arguments and
+ * d_probe_ws writes the first `capacity` pairs (no synchronisation).  unique
+ * must be known.                                                            */
+int tqpk_join_count(const tqpk_join_plan* h_plan, const void* d_build_ws, const void* d_probe_keys,
+                    int32_t probe_dtype, const uint8_t* d_probe_mask, int64_t np, int64_t* h_count,
+                    void* d_probe_ws, size_t probe_ws_bytes, tqpk_stream stream);
+int tqpk_join_write(const tqpk_join_plan* h_plan, const void* d_build_ws, const void* d_probe_keys,
+                    int32_t probe_dtype, const uint8_t* d_probe_mask, int64_t np, int64_t* d_out_build,
+                    int64_t* d_out_probe, int64_t capacity, void* d_probe_ws, size_t probe_ws_bytes,
+                    tqpk_stream stream);
 
 /* ---- fused pipelines ------------------------------------------------------
  * Filter -> inner join on a unique build key -> sum(expr) group by build key

@@ -7,21 +7,31 @@
 // re-checks key equality and gathers the output columns.
 //
 // Here the build side is turned into a directory once:
-//   DIRECT  dense key range (<= max(4*rows, 2^24) slots): slot = key - min.
-//           Unique keys: dir[slot] = build row.  Duplicate keys: the passing
-//           build rows are radix-sorted stably by key (CSR, ascending row
-//           inside a key) and dir[slot] = start of the key's run.
+//   DIRECT  dense key range (<= max(4*rows, 2^24) slots): dir[slot = key - min]
+//           = a build row of that key.  That answers a unique build side, and a
+//           semi or anti join of any.  Only a join that needs every build row of
+//           a repeated key also gets the rows radix-sorted stably by key (csr,
+//           ascending row inside a key) and run[slot] = the key's csr range.
 //   SORTED  sparse keys: the same stable sort, plus the distinct keys and run
 //           starts; the probe binary-searches the distinct keys (the
 //           reference's searchsorted, on a deduplicated array).
-// The probe is one single-pass kernel per join type: each thread looks up 16
-// probe rows, the per-row match counts are scanned in the block and across
-// tiles with the decoupled look-back, and the pairs are written by ascending
-// probe row, as the reference's are, then ascending build row (the reference
-// sorts build keys with an unstable torch.sort, hashjoin.py:43, so its order
-// of one key's duplicate build rows is not fixed; this is the stable one).  Rows
-// failing either side's filter mask are skipped in place: the inputs are
+// Probes with at most one output per probe row (unique build keys; semi, anti)
+// are one single-pass kernel: warps read 128 consecutive rows at a time, the
+// hits are placed in shared memory by block scan and written contiguously at the
+// tile's decoupled look-back offset.  Repeated build keys take two kernels: the
+// pairs of every tile are counted, then written at the scanned offsets, each
+// thread finding its pair's probe row by a search in the tile's scan, so that
+// consecutive threads write consecutive pairs.  Either way pairs come by
+// ascending probe row, as the reference's do, then ascending build row (the
+// reference sorts build keys with an unstable torch.sort, hashjoin.py:43, so its
+// order of one key's duplicate build rows is not fixed; this is the stable one).
+// Rows failing either side's filter mask are skipped in place: the inputs are
 // never compacted, and the emitted ids index the original columns.
+//
+// Measured on the operators' plans (1.5 M orders, 6 M lines): a semi-join whose
+// build side repeats its keys took 1003 us with the csr it never read; pairs of
+// a key repeated four times (24 M) were written by one thread per probe row,
+// 534 us of the probe.
 #include <algorithm>
 
 #include "common.cuh"
@@ -29,11 +39,11 @@
 namespace tqpk {
 
 struct JoinDir {
-  int mode, unique;
-  int64_t key_min, slots, n_unique, nb_rows;
-  const int64_t* dir;       // DIRECT: row (unique) or run start (dups), -1 = empty
-  const int* cnt;           // DIRECT: rows per slot
-  const int64_t* csr;       // build rows sorted by (key, row)
+  int mode, wide;           // wide: 64-bit entries (2^32 - 1 build rows or more)
+  int64_t key_min, slots, n_unique;
+  const void* dir;          // DIRECT: a build row per slot, all ones = empty
+  const void* run;          // DIRECT, repeated keys: (start, end) in csr per slot
+  const int64_t* csr;       // build rows sorted by (key, row); null: dir holds the one row
   const int64_t* ukeys;     // SORTED: distinct keys
   const int64_t* ustart;    // SORTED: run starts (n_unique + 1 entries)
 };
@@ -43,15 +53,10 @@ __global__ void k_count_status(const int64_t* count, int* err) {
   if (*count < 0) set_error(err, (int)*count);
 }
 
-__global__ void k_join_init_dir(int64_t* dir, int* cnt, int64_t slots) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < slots; i += (int64_t)gridDim.x * blockDim.x) {
-    dir[i] = -1;
-    cnt[i] = 0;
-  }
-}
-
+// dir[slot] = a build row of the key; *dup set when a key has two.  Four exchanges are in flight per thread.
+template <class R>
 __global__ void __launch_bounds__(kBlock) k_join_build_direct(const void* keys, int dt, RowFilter F, int64_t nb,
-                                                              int64_t kmin, int64_t* dir, int* cnt, int* dup) {
+                                                              int64_t kmin, int kvec, R* __restrict__ dir, int* dup) {
   const int64_t groups = (nb + 3) >> 2;
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < groups;
        g += (int64_t)gridDim.x * blockDim.x) {
@@ -65,26 +70,34 @@ __global__ void __launch_bounds__(kBlock) k_join_build_direct(const void* keys, 
     }
     if (!b) continue;
     int64_t x[4];
-    ld4_int(keys, dt, r0, nb, false, x);
+    ld4_int(keys, dt, r0, nb, kvec != 0, x);
+    R old[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      if (!((b >> j) & 1u)) continue;
-      const int64_t slot = x[j] - kmin;
-      const int old = atomicAdd(&cnt[slot], 1);
-      if (old) *dup = 1;
-      dir[slot] = r0 + j;
+      old[j] = R(~R(0));
+      if ((b >> j) & 1u) {
+        if (sizeof(R) == 4) old[j] = (R)atomicExch(reinterpret_cast<unsigned*>(&dir[x[j] - kmin]), (unsigned)(r0 + j));
+        else old[j] = (R)atomicExch(reinterpret_cast<unsigned long long*>(&dir[x[j] - kmin]), (unsigned long long)(r0 + j));
+      }
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (old[j] != R(~R(0))) *dup = 1;
   }
 }
 
-// After the stable sort: csr[i] = i-th build row in (key, row) order.
+// After the stable sort (csr[i] = i-th build row in (key, row) order): each run's range by slot (DIRECT,
+// run zeroed before), or the head flags (SORTED).
+template <class R>
 __global__ void k_join_runs(const void* keys, int dt, const int64_t* csr, int64_t m, int64_t kmin, int direct,
-                            int64_t* dir, int64_t* head_flag_rows) {
+                            R* run, int64_t* head_flag_rows) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t k = ld_int(keys, dt, csr[i]);
     const bool head = (i == 0) || ld_int(keys, dt, csr[i - 1]) != k;
     if (direct) {
-      if (head) dir[k - kmin] = i;
+      const bool tail = i + 1 == m || ld_int(keys, dt, csr[i + 1]) != k;
+      if (head) run[2 * (k - kmin)] = (R)i;
+      if (tail) run[2 * (k - kmin) + 1] = (R)(i + 1);
     } else {
       head_flag_rows[i] = head ? 1 : 0;
     }
@@ -127,115 +140,244 @@ __global__ void __launch_bounds__(kBlock) k_join_unique(const void* keys, int dt
   }
 }
 
-// Looks up one probe key: returns the match count and the first match's
-// position (a build row when unique, else an index into csr).
-__device__ __forceinline__ int64_t join_lookup(const JoinDir& D, int64_t key, int64_t& first) {
-  if (D.mode == TQPK_JOIN_DIRECT) {
-    const int64_t slot = key - D.key_min;
-    if (slot < 0 || slot >= D.slots) return 0;
-    if (D.unique) {
-      first = D.dir[slot];
-      return first >= 0 ? 1 : 0;
-    }
-    const int c = D.cnt[slot];
-    if (c) first = D.dir[slot];
-    return c;
-  }
+// The distinct key at or after `key` in a sorted directory: its index when equal, else -1.
+__device__ __forceinline__ int64_t join_find(const JoinDir& D, int64_t key) {
   int64_t lo = 0, hi = D.n_unique;
   while (lo < hi) {
     const int64_t mid = (lo + hi) >> 1;
     if (D.ukeys[mid] < key) lo = mid + 1; else hi = mid;
   }
-  if (lo >= D.n_unique || D.ukeys[lo] != key) return 0;
-  first = D.ustart[lo];
-  return D.ustart[lo + 1] - D.ustart[lo];
+  return lo < D.n_unique && D.ukeys[lo] == key ? lo : -1;
 }
 
-template <int JT>
+// The csr range [first, first + count) of a probe key's build rows (a unique directory: first is the row).
+__device__ __forceinline__ int64_t join_range(const JoinDir& D, int64_t key, int64_t& first) {
+  if (D.mode != TQPK_JOIN_DIRECT) {
+    const int64_t u = join_find(D, key);
+    if (u < 0) return 0;
+    first = D.ustart[u];
+    return D.ustart[u + 1] - first;
+  }
+  const int64_t slot = key - D.key_min;
+  if (slot < 0 || slot >= D.slots) return 0;
+  if (!D.csr) {
+    if (D.wide) {
+      const uint64_t r = static_cast<const uint64_t*>(D.dir)[slot];
+      first = (int64_t)r;
+      return r != ~0ull;
+    }
+    const unsigned r = static_cast<const unsigned*>(D.dir)[slot];
+    first = r;
+    return r != ~0u;
+  }
+  if (D.wide) {
+    const longlong2 q = static_cast<const longlong2*>(D.run)[slot];
+    first = q.x;
+    return q.y - q.x;
+  }
+  const uint2 q = static_cast<const uint2*>(D.run)[slot];
+  first = q.x;
+  return (int64_t)(q.y - q.x);
+}
+
+constexpr unsigned kNoRow = ~0u;
+
+// Probes with at most one output per row.  dup (inner join of a build side not known to be unique):
+// nothing is done when it is set.
+template <int JT, bool DIRECT, class R>
 __global__ void __launch_bounds__(kBlock) k_join_probe(JoinDir D, const void* pkeys, int pdt, RowFilter F, int64_t np,
                                                        int64_t* __restrict__ out_b, int64_t* __restrict__ out_p,
                                                        int64_t capacity, const int64_t* base_ptr, int64_t* total_out,
-                                                       uint64_t* status, int* tile_ctr, int* err) {
+                                                       uint64_t* status, int* tile_ctr, const int* dup, int* err) {
   __shared__ int s_tile;
   __shared__ uint64_t s_excl;
-  __shared__ int64_t sw[kBlock / 32 + 1];
+  __shared__ int s_warp[kBlock / 32 + 1];
+  __shared__ uint16_t s_p[kTile];                      // row of the tile, by output place
+  __shared__ R s_b[JT == TQPK_JT_INNER ? kTile : 1];   // its build row
+  if (dup && *dup) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1);
   __syncthreads();
   const int64_t tile = s_tile;
-  const int64_t r0 = tile * kTile + threadIdx.x * kItems;
-  int64_t cnt[kItems], first[kItems];
-  int64_t mine = 0;
+  // warp w reads rows [512 w, 512 w + 512) of the tile, 128 consecutive rows a load
+  const int64_t w0 = tile * kTile + warp * (32 * kItems);
   const bool kvec = ((reinterpret_cast<uintptr_t>(pkeys) & 15u) == 0);
+  uint32_t hits = 0;
+  R row[kItems];
+  uint32_t live[kItems / 4];
+  int64_t key[kItems];
 #pragma unroll
   for (int q = 0; q < kItems / 4; ++q) {
-    const int64_t g0 = r0 + 4 * q;
-    int64_t valid = np - g0;
+    const int64_t g0 = w0 + 128 * q + 4 * lane;
+    const int64_t valid = np - g0;
     uint32_t b = valid >= 4 ? 0xfu : (valid <= 0 ? 0u : ((1u << valid) - 1));
     if (F.mask && b) {
       int64_t m[4];
       ld4_int(F.mask, TQPK_U8, g0, np, F.mask_vec, m);
       b &= (m[0] != 0) | ((m[1] != 0) << 1) | ((m[2] != 0) << 2) | ((m[3] != 0) << 3);
     }
-    int64_t x[4] = {0, 0, 0, 0};
-    if (b) ld4_int(pkeys, pdt, g0, np, kvec, x);
+    live[q] = b;
+  }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int64_t c = 0, f = 0;
-      if ((b >> j) & 1u) {
-        c = join_lookup(D, x[j], f);
-        if (JT == TQPK_JT_SEMI) c = c ? 1 : 0;
-        if (JT == TQPK_JT_ANTI) c = c ? 0 : 1;
-      }
-      cnt[4 * q + j] = c;
-      first[4 * q + j] = f;
-      mine += c;
+  for (int q = 0; q < kItems / 4; ++q) {
+    int64_t x[4] = {0, 0, 0, 0};
+    if (live[q]) ld4_int(pkeys, pdt, w0 + 128 * q + 4 * lane, np, kvec, x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) key[4 * q + j] = x[j];
+  }
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const bool on = (live[i / 4] >> (i & 3)) & 1u;
+    row[i] = R(~R(0));
+    if (DIRECT) {
+      const int64_t slot = key[i] - D.key_min;
+      if (on && slot >= 0 && slot < D.slots) row[i] = static_cast<const R*>(D.dir)[slot];
+    } else if (on && join_find(D, key[i]) >= 0) {
+      row[i] = 0;
     }
   }
-  int64_t total;
-  const int64_t excl = block_excl_scan<kBlock, int64_t>(mine, total, sw);
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const bool on = (live[i / 4] >> (i & 3)) & 1u;
+    const bool hit = row[i] != R(~R(0));
+    if (JT == TQPK_JT_ANTI ? on && !hit : hit) hits |= 1u << i;
+  }
+  // output places: the four 128-row steps' counts (at most 128 each) share one warp scan
+  unsigned c = 0;
+#pragma unroll
+  for (int q = 0; q < kItems / 4; ++q) c |= __popc((hits >> (4 * q)) & 15u) << (8 * q);
+  unsigned even = c & 0x00ff00ffu, odd = (c >> 8) & 0x00ff00ffu;
+  const unsigned ie = warp_incl_scan(even), io = warp_incl_scan(odd);
+  const unsigned te = __shfl_sync(0xffffffffu, ie, 31), to = __shfl_sync(0xffffffffu, io, 31);
+  const unsigned step_total[4] = {te & 0xffffu, to & 0xffffu, te >> 16, to >> 16};
+  const unsigned xe = ie - even, xo = io - odd;
+  const unsigned before[4] = {xe & 0xffffu, xo & 0xffffu, xe >> 16, xo >> 16};
+  const int wtotal = (int)(step_total[0] + step_total[1] + step_total[2] + step_total[3]);
+  if (lane == 0) s_warp[warp] = wtotal;
+  __syncthreads();
+  int total = 0, wbase = 0;
+#pragma unroll
+  for (int w = 0; w < kBlock / 32; ++w) {
+    if (w == warp) wbase = total;
+    total += s_warp[w];
+  }
+  unsigned at0 = wbase;
+#pragma unroll
+  for (int q = 0; q < kItems / 4; ++q) {
+    unsigned at = at0 + before[q];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if ((hits >> (4 * q + j)) & 1u) {
+        s_p[at] = (uint16_t)(warp * (32 * kItems) + 128 * q + 4 * lane + j);
+        if (JT == TQPK_JT_INNER) s_b[at] = row[4 * q + j];
+        ++at;
+      }
+    }
+    at0 += step_total[q];
+  }
   if (threadIdx.x < 32) {
     uint64_t e = lookback_warp(status, tile, (uint64_t)total, err);
     if (threadIdx.x == 0) s_excl = e;
   }
   __syncthreads();
-  const int64_t base = (base_ptr ? *base_ptr : 0);
-  const bool one_per_row = JT != TQPK_JT_INNER || (D.mode == TQPK_JOIN_DIRECT && D.unique);   // block-uniform
-  if (one_per_row) {
-    // at most one output per row, so the tile's outputs fit kTile slots: each thread places its
-    // outputs at its block offset in shared memory, then the block writes them contiguously
-    // (coalesced) instead of every lane storing its own run
-    __shared__ int64_t s_out[kTile];
-    const int64_t gbase = base + (int64_t)s_excl;
-    int64_t lp = excl;
-#pragma unroll
-    for (int j = 0; j < kItems; ++j)
-      if (cnt[j]) s_out[lp++] = r0 + j;
-    __syncthreads();
-    for (int64_t i = threadIdx.x; i < total; i += kBlock)
-      if (gbase + i < capacity) out_p[gbase + i] = s_out[i];
-    if (JT == TQPK_JT_INNER || (JT == TQPK_JT_ANTI && out_b)) {
-      __syncthreads();
-      lp = excl;
-#pragma unroll
-      for (int j = 0; j < kItems; ++j)
-        if (cnt[j]) s_out[lp++] = (JT == TQPK_JT_INNER) ? first[j] : (int64_t)TQPK_NULL_INDEX;
-      __syncthreads();
-      for (int64_t i = threadIdx.x; i < total; i += kBlock)
-        if (gbase + i < capacity) out_b[gbase + i] = s_out[i];
-    }
-  } else {
-    int64_t pos = base + (int64_t)s_excl + excl;
-#pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-      const int64_t c = cnt[j];
-      for (int64_t t = 0; t < c; ++t, ++pos) {
-        if (pos >= capacity) continue;
-        out_p[pos] = r0 + j;
-        if (JT == TQPK_JT_INNER) out_b[pos] = D.csr[first[j] + t];
-      }
-    }
+  const int64_t gbase = (base_ptr ? *base_ptr : 0) + (int64_t)s_excl;
+  for (int i = threadIdx.x; i < total; i += kBlock) {
+    if (gbase + i >= capacity) break;
+    out_p[gbase + i] = tile * kTile + s_p[i];
+    if (JT == TQPK_JT_INNER) out_b[gbase + i] = (int64_t)s_b[i];
+    else if (JT == TQPK_JT_ANTI && out_b) out_b[gbase + i] = (int64_t)TQPK_NULL_INDEX;
   }
-  if (tile == (int64_t)gridDim.x - 1 && threadIdx.x == 0) *total_out = base + (int64_t)(s_excl + total);
+  if (tile == (int64_t)gridDim.x - 1 && threadIdx.x == 0) *total_out = gbase + total;
+}
+
+// ---- joins whose build key repeats: count the pairs of every tile, scan, write -------------------
+constexpr int kPairRows = 4 * kBlock;        // probe rows per tile
+
+struct PairCtl {
+  unsigned done;          // counting CTAs finished
+  int pad;
+  int64_t total;          // pairs in all
+};
+
+// Pass COUNT leaves each tile's pair count in tile_base; its last CTA scans them into offsets.
+template <bool COUNT>
+__global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pkeys, int pdt, RowFilter F, int64_t np,
+                                                       int kvec, int64_t* __restrict__ out_b,
+                                                       int64_t* __restrict__ out_p, int64_t capacity,
+                                                       int64_t* __restrict__ tile_base, PairCtl* ctl) {
+  __shared__ int64_t sw[kBlock / 32 + 1];
+  __shared__ int64_t s_pre[COUNT ? 1 : kPairRows];     // pairs before each row of the tile
+  __shared__ int64_t s_first[COUNT ? 1 : kPairRows];   // where its build rows start
+  __shared__ int s_last;
+  const int64_t tile = blockIdx.x;
+  const int64_t g0 = tile * kPairRows + 4 * threadIdx.x;
+  const int64_t valid = np - g0;
+  uint32_t b = valid >= 4 ? 0xfu : (valid <= 0 ? 0u : ((1u << valid) - 1));
+  if (F.mask && b) {
+    int64_t m[4];
+    ld4_int(F.mask, TQPK_U8, g0, np, F.mask_vec, m);
+    b &= (m[0] != 0) | ((m[1] != 0) << 1) | ((m[2] != 0) << 2) | ((m[3] != 0) << 3);
+  }
+  int64_t x[4] = {0, 0, 0, 0}, first[4] = {0, 0, 0, 0}, cnt[4];
+  if (b) ld4_int(pkeys, pdt, g0, np, kvec != 0, x);
+  int64_t mine = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    cnt[j] = (b >> j) & 1u ? join_range(D, x[j], first[j]) : 0;
+    mine += cnt[j];
+  }
+  int64_t total;
+  int64_t excl = block_excl_scan<kBlock, int64_t>(mine, total, sw);
+  if (COUNT) {
+    if (threadIdx.x == 0) {
+      tile_base[tile] = total;
+      __threadfence();
+      s_last = atomicAdd(&ctl->done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    int64_t run = 0;
+    for (int64_t t0 = 0; t0 < (int64_t)gridDim.x; t0 += 4 * kBlock) {
+      int64_t c[4], sum = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int64_t t = t0 + 4 * threadIdx.x + q;
+        c[q] = t < (int64_t)gridDim.x ? __ldcg(reinterpret_cast<const long long*>(&tile_base[t])) : 0;
+        sum += c[q];
+      }
+      int64_t all;
+      int64_t at = run + block_excl_scan<kBlock, int64_t>(sum, all, sw);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int64_t t = t0 + 4 * threadIdx.x + q;
+        if (t < (int64_t)gridDim.x) tile_base[t] = at;
+        at += c[q];
+      }
+      run += all;
+    }
+    if (threadIdx.x == 0) ctl->total = run;
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    s_pre[4 * threadIdx.x + j] = excl;
+    s_first[4 * threadIdx.x + j] = first[j];
+    excl += cnt[j];
+  }
+  __syncthreads();
+  const int64_t base = tile_base[tile];
+  for (int64_t o = threadIdx.x; o < total; o += kBlock) {
+    if (base + o >= capacity) break;
+    int lo = 0, hi = kPairRows;                // the last row with s_pre <= o
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (s_pre[mid] <= o) lo = mid; else hi = mid;
+    }
+    const int64_t f = s_first[lo] + (o - s_pre[lo]);
+    out_p[base + o] = tile * kPairRows + lo;
+    out_b[base + o] = D.csr ? D.csr[f] : f;
+  }
 }
 
 __global__ void k_gather(int ncols, const __grid_constant__ ColSet C, const int64_t* __restrict__ idx, int64_t n,
@@ -258,8 +400,8 @@ __global__ void k_gather(int ncols, const __grid_constant__ ColSet C, const int6
 struct BuildLayout {
   int* hdr;            // [0] dup flag, [1] error, [2] tile counter
   int64_t* nu;         // distinct keys (SORTED)
-  int64_t* dir;
-  int* cnt;
+  void* dir;           // one entry per slot (4 bytes, or 8 when wide)
+  void* run;           // two entries per slot
   int64_t* csr;
   int64_t* rows;       // the passing build rows in row order (a masked build side)
   int64_t* ukeys;
@@ -270,18 +412,25 @@ struct BuildLayout {
   uint64_t* status;
 };
 
+// Entries are 4 bytes unless a plan says otherwise; wide plans have unique's bit 8 set.
+constexpr int kWide = 256;
+static bool is_wide(const tqpk_join_plan& p) { return (p.unique & kWide) != 0; }
+static int uniqueness(const tqpk_join_plan& p) { return p.unique & ~kWide; }
+
 static bool layout(const tqpk_join_plan& p, void* ws, size_t bytes, BuildLayout& L) {
   WsCursor c(ws, bytes);
   const int64_t m = p.nb_rows > 0 ? p.nb_rows : 1;
+  const size_t e = is_wide(p) ? 8 : 4;
+  const bool direct = p.mode == TQPK_JOIN_DIRECT;
   L.hdr = c.take<int>(64);
   L.nu = c.take<int64_t>(4);
-  L.dir = c.take<int64_t>(p.mode == TQPK_JOIN_DIRECT ? p.slots : 1);
-  L.cnt = c.take<int>(p.mode == TQPK_JOIN_DIRECT ? p.slots : 1);
+  L.dir = c.take<char>(direct ? p.slots * e : 1);
+  L.run = c.take<char>(direct ? 2 * p.slots * e : 1);
   L.csr = c.take<int64_t>(m);
   L.rows = c.take<int64_t>(m);
-  L.ukeys = c.take<int64_t>(p.mode == TQPK_JOIN_SORTED ? m : 1);
-  L.ustart = c.take<int64_t>(p.mode == TQPK_JOIN_SORTED ? m + 1 : 1);
-  L.head = c.take<int64_t>(p.mode == TQPK_JOIN_SORTED ? m : 1);
+  L.ukeys = c.take<int64_t>(direct ? 1 : m);
+  L.ustart = c.take<int64_t>(direct ? 1 : m + 1);
+  L.head = c.take<int64_t>(direct ? 1 : m);
   L.status = c.take<uint64_t>((m + kTile - 1) / kTile + 1);
   L.sort_bytes = sort_ws_bytes(m);
   L.sort_ws = c.take<char>(L.sort_bytes);
@@ -290,31 +439,99 @@ static bool layout(const tqpk_join_plan& p, void* ws, size_t bytes, BuildLayout&
 
 static size_t layout_bytes(const tqpk_join_plan& p) {
   const int64_t m = p.nb_rows > 0 ? p.nb_rows : 1;
+  const size_t e = is_wide(p) ? 8 : 4;
+  const bool direct = p.mode == TQPK_JOIN_DIRECT;
   size_t b = 256 + 256;
-  if (p.mode == TQPK_JOIN_DIRECT) b += align_up(p.slots * 8, 256) + align_up(p.slots * 4, 256);
-  else b += 512;
+  b += direct ? align_up(p.slots * e, 256) + align_up(2 * p.slots * e, 256) : 512;
   b += 2 * align_up(m * 8, 256);
-  if (p.mode == TQPK_JOIN_SORTED) b += align_up(m * 8, 256) + align_up((m + 1) * 8, 256) + align_up(m * 8, 256);
-  else b += 768;
+  b += direct ? 768 : align_up(m * 8, 256) + align_up((m + 1) * 8, 256) + align_up(m * 8, 256);
   b += align_up(((m + kTile - 1) / kTile + 1) * 8, 256);
   b += align_up(sort_ws_bytes(m), 256);
   return b + 2048;
 }
 
-static JoinDir make_dir(const tqpk_join_plan& p, const BuildLayout& L) {
-  JoinDir D;
+// The directory a probe reads; pairs: of every build row of a key (the csr), when keys repeat.
+static JoinDir make_dir(const tqpk_join_plan& p, const BuildLayout& L, bool pairs) {
+  JoinDir D{};
   D.mode = p.mode;
-  D.unique = p.unique;
+  D.wide = is_wide(p) ? 1 : 0;
   D.key_min = p.key_min;
-  D.slots = p.slots;
+  D.slots = p.nb_rows > 0 ? p.slots : 0;
   D.n_unique = p.n_unique;
-  D.nb_rows = p.nb_rows;
   D.dir = L.dir;
-  D.cnt = L.cnt;
-  D.csr = L.csr;
+  D.run = L.run;
+  D.csr = pairs && uniqueness(p) == 0 ? L.csr : nullptr;
   D.ukeys = L.ukeys;
   D.ustart = L.ustart;
+  if (p.nb_rows == 0) D.mode = TQPK_JOIN_DIRECT;       // no slot at all
   return D;
+}
+
+template <int JT>
+static int launch_probe(const JoinDir& D, const void* pkeys, int pdt, const RowFilter& F, int64_t np, int64_t* out_b,
+                        int64_t* out_p, int64_t capacity, const int64_t* base, int64_t* total, uint64_t* status,
+                        int* tile_ctr, const int* dup, int* err, cudaStream_t s) {
+  const int64_t tiles = (np + kTile - 1) / kTile;
+  timing_before(KID_JOIN_PROBE, s);
+  if (D.mode != TQPK_JOIN_DIRECT) {
+    if constexpr (JT != TQPK_JT_INNER)
+      k_join_probe<JT, false, unsigned><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, out_b, out_p, capacity, base,
+                                                                      total, status, tile_ctr, dup, err);
+  } else if (D.wide) {
+    k_join_probe<JT, true, uint64_t><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, out_b, out_p, capacity, base,
+                                                                   total, status, tile_ctr, dup, err);
+  } else {
+    k_join_probe<JT, true, unsigned><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, out_b, out_p, capacity, base,
+                                                                   total, status, tile_ctr, dup, err);
+  }
+  timing_after(KID_JOIN_PROBE, s);
+  TQPK_CHECK_LAUNCH();
+  return TQPK_OK;
+}
+
+struct ProbeLayout {
+  int* ctl;              // [0] tile counter A, [1] error, [2] tile counter B, [3] a repeated build key
+  int64_t* totals;
+  PairCtl* pair;
+  uint64_t* status_a;
+  uint64_t* status_b;
+  size_t zeroed;
+  int64_t* tile_base;
+};
+
+static bool probe_layout(int64_t np, void* pws, size_t bytes, ProbeLayout& W) {
+  const int64_t tiles = (np + kTile - 1) / kTile;
+  WsCursor cur(pws, bytes);
+  W.ctl = cur.take<int>(64);
+  W.totals = cur.take<int64_t>(8);
+  W.pair = cur.take<PairCtl>(1);
+  W.status_a = cur.take<uint64_t>(tiles + 1);
+  W.status_b = cur.take<uint64_t>(tiles + 1);
+  W.zeroed = cur.off;
+  W.tile_base = cur.take<int64_t>((np + kPairRows - 1) / kPairRows + 1);
+  return W.tile_base != nullptr;
+}
+
+// Pair counts of every tile of probe rows and their sum (W.pair->total), on the device.
+static int count_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFilter& F, int64_t np,
+                       const ProbeLayout& W, cudaStream_t s) {
+  const int64_t tiles = (np + kPairRows - 1) / kPairRows;
+  if (tiles > INT32_MAX) return TQPK_EUNSUPPORTED;
+  k_join_pairs<true><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, nullptr, nullptr, 0,
+                                                   W.tile_base, W.pair);
+  TQPK_CHECK_LAUNCH();
+  return TQPK_OK;
+}
+
+static int write_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFilter& F, int64_t np,
+                       const ProbeLayout& W, int64_t* out_b, int64_t* out_p, int64_t capacity, cudaStream_t s) {
+  const int64_t tiles = (np + kPairRows - 1) / kPairRows;
+  timing_before(KID_JOIN_PROBE, s);
+  k_join_pairs<false><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, out_b, out_p,
+                                                    capacity, W.tile_base, W.pair);
+  timing_after(KID_JOIN_PROBE, s);
+  TQPK_CHECK_LAUNCH();
+  return TQPK_OK;
 }
 
 }  // namespace tqpk
@@ -335,20 +552,74 @@ extern "C" int tqpk_join_plan_build(const void* keys, int32_t dt, const uint8_t*
   plan->key_min = rows ? mn : 0;
   plan->key_max = rows ? mx : -1;
   const int64_t range = rows ? (mx - mn + 1) : 1;
-  // direct addressing costs 12 B per slot of the key range; up to 2^24 slots (~200 MB) that is
-  // cheaper than a binary search per probe row even for a sparse build side (a filtered
+  // direct addressing costs 4 B per slot of the key range (12 B when keys repeat); up to 2^24 slots
+  // that is cheaper than a binary search per probe row even for a sparse build side (a filtered
   // dimension of 2 M keys joined by a 60 M-row fact table: 7.6 ms sorted, ~0.1 ms direct)
   const bool dense = rows == 0 || (range > 0 && range <= std::max<int64_t>(4 * rows, int64_t(1) << 24) &&
                                    range < (int64_t(1) << 31));
   plan->mode = dense ? TQPK_JOIN_DIRECT : TQPK_JOIN_SORTED;
   plan->slots = dense ? range : 0;
-  plan->unique = 1;
+  plan->unique = 1 | (nb >= (int64_t)0xffffffffu ? kWide : 0);
   plan->ws_bytes = layout_bytes(*plan);
   return TQPK_OK;
 }
 
-extern "C" int tqpk_join_build(tqpk_join_plan* plan, const void* keys, int32_t dt, const uint8_t* mask, int64_t nb,
-                               void* ws, size_t ws_bytes, tqpk_stream stream) {
+extern "C" int tqpk_join_rows(tqpk_join_plan* plan, const void* keys, int32_t dt, const uint8_t* mask, int64_t nb,
+                              void* ws, size_t ws_bytes, tqpk_stream stream) {
+  if (!plan || nb < 0 || (nb > 0 && !keys)) return TQPK_EINVAL;
+  if (!is_int_dtype(dt)) return TQPK_EDTYPE;
+  if (!ws || ws_bytes < plan->ws_bytes) return TQPK_ENOMEM;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  BuildLayout L;
+  if (!layout(*plan, ws, ws_bytes, L)) return TQPK_ENOMEM;
+  plan->unique = is_wide(*plan) ? kWide : 0;
+  if (plan->nb_rows == 0) return TQPK_OK;
+  // Passing build rows in row order (all of them without a mask), then a stable sort by key -> CSR.
+  if (mask) {
+    ColSet C;
+    C.n = 1;
+    C.in[0] = nullptr;
+    C.out[0] = L.rows;
+    C.size[0] = 0;  // row ids
+    int64_t* d_m = L.nu + 1;
+    TQPK_CUDA(cudaMemsetAsync(L.rows, 0, plan->nb_rows * 8, s));   // row ids even if the compaction fails
+    int rc = compact_launch(nullptr, mask, nb, C, d_m, L.sort_ws, L.sort_bytes, s);
+    if (rc) return rc;
+    k_count_status<<<1, 1, 0, s>>>(d_m, L.hdr + 1);   // a failed compaction's status joins the error word
+    TQPK_CHECK_LAUNCH();
+  }
+  const SortKey by_key{keys, nullptr, dt, 0, 0, 0};
+  int rc = sort_keys(&by_key, 1, mask ? L.rows : nullptr, plan->nb_rows, L.csr, L.sort_ws, L.sort_bytes, s);
+  if (rc) return rc;
+  const int direct = plan->mode == TQPK_JOIN_DIRECT;
+  if (direct) TQPK_CUDA(cudaMemsetAsync(L.run, 0, 2 * plan->slots * (is_wide(*plan) ? 8 : 4), s));
+  if (is_wide(*plan))
+    k_join_runs<uint64_t><<<grid_for(plan->nb_rows, 8), kBlock, 0, s>>>(keys, dt, L.csr, plan->nb_rows, plan->key_min,
+                                                                        direct, static_cast<uint64_t*>(L.run), L.head);
+  else
+    k_join_runs<unsigned><<<grid_for(plan->nb_rows, 8), kBlock, 0, s>>>(keys, dt, L.csr, plan->nb_rows, plan->key_min,
+                                                                        direct, static_cast<unsigned*>(L.run), L.head);
+  TQPK_CHECK_LAUNCH();
+  if (!direct) {
+    const int64_t tiles = (plan->nb_rows + kTile - 1) / kTile;
+    TQPK_CUDA(cudaMemsetAsync(L.status, 0, (tiles + 1) * 8, s));
+    TQPK_CUDA(cudaMemsetAsync(L.hdr + 2, 0, sizeof(int), s));
+    k_join_unique<<<(int)tiles, kBlock, 0, s>>>(keys, dt, L.csr, L.head, plan->nb_rows, L.ukeys, L.ustart, L.nu,
+                                                L.status, L.hdr + 2, L.hdr + 1);
+    TQPK_CHECK_LAUNCH();
+    int64_t nu = 0;
+    TQPK_CUDA(cudaMemcpyAsync(&nu, L.nu, 8, cudaMemcpyDeviceToHost, s));
+    TQPK_CUDA(cudaStreamSynchronize(s));
+    plan->n_unique = nu;
+  }
+  int err = 0;
+  TQPK_CUDA(cudaMemcpyAsync(&err, L.hdr + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+  TQPK_CUDA(cudaStreamSynchronize(s));
+  return err;
+}
+
+extern "C" int tqpk_join_directory(tqpk_join_plan* plan, const void* keys, int32_t dt, const uint8_t* mask, int64_t nb,
+                                   void* ws, size_t ws_bytes, tqpk_stream stream) {
   if (!plan || nb < 0 || (nb > 0 && !keys)) return TQPK_EINVAL;
   if (!is_int_dtype(dt)) return TQPK_EDTYPE;
   if (!ws || ws_bytes < plan->ws_bytes) return TQPK_ENOMEM;
@@ -356,69 +627,38 @@ extern "C" int tqpk_join_build(tqpk_join_plan* plan, const void* keys, int32_t d
   BuildLayout L;
   if (!layout(*plan, ws, ws_bytes, L)) return TQPK_ENOMEM;
   TQPK_CUDA(cudaMemsetAsync(L.hdr, 0, 64 * sizeof(int), s));
-  RowFilter F = make_filter(nullptr, mask);
-  bool need_sort = plan->mode == TQPK_JOIN_SORTED;
-  if (plan->mode == TQPK_JOIN_DIRECT) {
-    k_join_init_dir<<<grid_for(plan->slots, 4), kBlock, 0, s>>>(L.dir, L.cnt, plan->slots);
-    TQPK_CHECK_LAUNCH();
-    if (plan->nb_rows > 0) {
-      k_join_build_direct<<<grid_for((nb + 3) / 4, 8), kBlock, 0, s>>>(keys, dt, F, nb, plan->key_min, L.dir, L.cnt,
-                                                                      L.hdr);
-      TQPK_CHECK_LAUNCH();
-    }
-    int h[2] = {0, 0};   // [0] a repeated key, [1] error word: one read
-    TQPK_CUDA(cudaMemcpyAsync(h, L.hdr, sizeof(h), cudaMemcpyDeviceToHost, s));
-    TQPK_CUDA(cudaStreamSynchronize(s));
-    if (h[1]) return h[1];
-    plan->unique = h[0] ? 0 : 1;
-    need_sort = h[0] != 0;
-    if (!need_sort) return TQPK_OK;
-  }
-  if (need_sort && plan->nb_rows > 0) {
-    plan->unique = 0;
-    // Passing build rows in row order (all of them without a mask), then a stable sort by key -> CSR.
-    if (mask) {
-      ColSet C;
-      C.n = 1;
-      C.in[0] = nullptr;
-      C.out[0] = L.rows;
-      C.size[0] = 0;  // row ids
-      int64_t* d_m = L.nu + 1;
-      TQPK_CUDA(cudaMemsetAsync(L.rows, 0, plan->nb_rows * 8, s));   // row ids even if the compaction fails
-      int rc = compact_launch(nullptr, mask, nb, C, d_m, L.sort_ws, L.sort_bytes, s);
-      if (rc) return rc;
-      k_count_status<<<1, 1, 0, s>>>(d_m, L.hdr + 1);   // a failed compaction's status joins the error word
-      TQPK_CHECK_LAUNCH();
-    }
-    const SortKey by_key{keys, nullptr, dt, 0, 0, 0};
-    int rc = sort_keys(&by_key, 1, mask ? L.rows : nullptr, plan->nb_rows, L.csr, L.sort_ws, L.sort_bytes, s);
-    if (rc) return rc;
-    const int direct = plan->mode == TQPK_JOIN_DIRECT;
-    k_join_runs<<<grid_for(plan->nb_rows, 4), kBlock, 0, s>>>(keys, dt, L.csr, plan->nb_rows, plan->key_min, direct,
-                                                             L.dir, L.head);
-    TQPK_CHECK_LAUNCH();
-    if (!direct) {
-      const int64_t tiles = (plan->nb_rows + kTile - 1) / kTile;
-      TQPK_CUDA(cudaMemsetAsync(L.status, 0, (tiles + 1) * 8, s));
-      TQPK_CUDA(cudaMemsetAsync(L.hdr + 2, 0, sizeof(int), s));
-      k_join_unique<<<(int)tiles, kBlock, 0, s>>>(keys, dt, L.csr, L.head, plan->nb_rows, L.ukeys, L.ustart, L.nu,
-                                                  L.status, L.hdr + 2, L.hdr + 1);
-      TQPK_CHECK_LAUNCH();
-      int64_t nu = 0;
-      TQPK_CUDA(cudaMemcpyAsync(&nu, L.nu, 8, cudaMemcpyDeviceToHost, s));
-      TQPK_CUDA(cudaStreamSynchronize(s));
-      plan->n_unique = nu;
-    }
-  }
-  int err = 0;
-  TQPK_CUDA(cudaMemcpyAsync(&err, L.hdr + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-  TQPK_CUDA(cudaStreamSynchronize(s));
-  return err ? err : TQPK_OK;
+  const int wide = plan->unique & kWide;
+  if (plan->mode == TQPK_JOIN_SORTED) return tqpk_join_rows(plan, keys, dt, mask, nb, ws, ws_bytes, stream);
+  plan->unique = (plan->nb_rows > 0 ? TQPK_JOIN_UNKNOWN : 1) | wide;
+  TQPK_CUDA(cudaMemsetAsync(L.dir, 0xff, plan->slots * (wide ? 8 : 4), s));
+  if (plan->nb_rows == 0) return TQPK_OK;
+  const RowFilter F = make_filter(nullptr, mask);
+  const int kvec = aligned16(keys) ? 1 : 0;
+  if (wide)
+    k_join_build_direct<uint64_t><<<grid_for((nb + 3) / 4, 8), kBlock, 0, s>>>(keys, dt, F, nb, plan->key_min, kvec,
+                                                                              static_cast<uint64_t*>(L.dir), L.hdr);
+  else
+    k_join_build_direct<unsigned><<<grid_for((nb + 3) / 4, 8), kBlock, 0, s>>>(keys, dt, F, nb, plan->key_min, kvec,
+                                                                              static_cast<unsigned*>(L.dir), L.hdr);
+  TQPK_CHECK_LAUNCH();
+  return TQPK_OK;
+}
+
+extern "C" int tqpk_join_build(tqpk_join_plan* plan, const void* keys, int32_t dt, const uint8_t* mask, int64_t nb,
+                               void* ws, size_t ws_bytes, tqpk_stream stream) {
+  int rc = tqpk_join_directory(plan, keys, dt, mask, nb, ws, ws_bytes, stream);
+  if (rc || uniqueness(*plan) != TQPK_JOIN_UNKNOWN) return rc;
+  int dup = 0;
+  TQPK_CUDA(cudaMemcpyAsync(&dup, ws, sizeof(dup), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
+  TQPK_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+  if (dup) return tqpk_join_rows(plan, keys, dt, mask, nb, ws, ws_bytes, stream);
+  plan->unique = (plan->unique & kWide) | 1;
+  return TQPK_OK;
 }
 
 extern "C" size_t tqpk_join_probe_workspace_bytes(int64_t np) {
   const int64_t tiles = (np + kTile - 1) / kTile;
-  return 1024 + 2 * align_up((size_t)(tiles + 1) * 8, 256);
+  return 2048 + 2 * align_up((size_t)(tiles + 1) * 8, 256) + align_up(((size_t)np / kPairRows + 2) * 8, 256);
 }
 
 extern "C" int tqpk_join_probe(const tqpk_join_plan* plan, const void* build_ws, const void* pkeys, int32_t pdt,
@@ -433,55 +673,97 @@ extern "C" int tqpk_join_probe(const tqpk_join_plan* plan, const void* build_ws,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BuildLayout L;
   if (!layout(*plan, const_cast<void*>(build_ws), plan->ws_bytes, L)) return TQPK_ENOMEM;
-  const JoinDir D = make_dir(*plan, L);
-  const int64_t tiles = (np + kTile - 1) / kTile;
-  WsCursor cur(pws, pws_bytes);
-  int* ctl = cur.take<int>(64);        // [0] tile counter A, [1] error, [2] tile counter B
-  int64_t* totals = cur.take<int64_t>(8);
-  uint64_t* status_a = cur.take<uint64_t>(tiles + 1);
-  uint64_t* status_b = cur.take<uint64_t>(tiles + 1);
-  if (!status_b) return TQPK_ENOMEM;
-  TQPK_CUDA(cudaMemsetAsync(pws, 0, cur.off, s));
+  const JoinDir D = make_dir(*plan, L, jt == TQPK_JT_INNER || jt == TQPK_JT_OUTER);
+  ProbeLayout W;
+  if (!probe_layout(np, pws, pws_bytes, W)) return TQPK_ENOMEM;
   *h_count = 0;
   if (np == 0) return TQPK_OK;
+  TQPK_CUDA(cudaMemsetAsync(pws, 0, W.zeroed, s));
   const RowFilter F = make_filter(nullptr, pmask);
-  const bool empty_build = plan->nb_rows == 0;
+  int* dup = nullptr;
+  int64_t* pair_total = W.totals;
+  int rc;
   if (jt == TQPK_JT_INNER || jt == TQPK_JT_OUTER) {
-    if (!empty_build) {
-      timing_before(KID_JOIN_PROBE, s);
-      k_join_probe<TQPK_JT_INNER><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, out_b, out_p, capacity, nullptr,
-                                                               totals, status_a, ctl, ctl + 1);
-      timing_after(KID_JOIN_PROBE, s);
-      TQPK_CHECK_LAUNCH();
+    const bool one = D.mode == TQPK_JOIN_DIRECT && !D.csr;       // at most one build row per key
+    if (uniqueness(*plan) == TQPK_JOIN_UNKNOWN) dup = L.hdr;
+    if (plan->nb_rows > 0) {
+      if (one) {
+        rc = launch_probe<TQPK_JT_INNER>(D, pkeys, pdt, F, np, out_b, out_p, capacity, nullptr, W.totals, W.status_a,
+                                         W.ctl, dup, W.ctl + 1, s);
+      } else {
+        pair_total = &W.pair->total;
+        rc = count_pairs(D, pkeys, pdt, F, np, W, s);
+        if (!rc && capacity > 0) rc = write_pairs(D, pkeys, pdt, F, np, W, out_b, out_p, capacity, s);
+      }
+      if (rc) return rc;
     }
     if (jt == TQPK_JT_OUTER) {
-      JoinDir E = D;
-      if (empty_build) { E.mode = TQPK_JOIN_DIRECT; E.unique = 1; E.slots = 0; }
-      k_join_probe<TQPK_JT_ANTI><<<(int)tiles, kBlock, 0, s>>>(E, pkeys, pdt, F, np, out_b, out_p, capacity, totals,
-                                                              totals + 1, status_b, ctl + 2, ctl + 1);
-      TQPK_CHECK_LAUNCH();
+      rc = launch_probe<TQPK_JT_ANTI>(D, pkeys, pdt, F, np, out_b, out_p, capacity, pair_total, W.totals + 1,
+                                      W.status_b, W.ctl + 2, dup, W.ctl + 1, s);
+      if (rc) return rc;
     }
   } else if (jt == TQPK_JT_SEMI) {
-    if (!empty_build) {
-      k_join_probe<TQPK_JT_SEMI><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, nullptr, out_p, capacity, nullptr,
-                                                              totals, status_a, ctl, ctl + 1);
-      TQPK_CHECK_LAUNCH();
+    if (plan->nb_rows > 0) {
+      rc = launch_probe<TQPK_JT_SEMI>(D, pkeys, pdt, F, np, nullptr, out_p, capacity, nullptr, W.totals, W.status_a,
+                                      W.ctl, nullptr, W.ctl + 1, s);
+      if (rc) return rc;
     }
   } else {
-    JoinDir E = D;
-    if (empty_build) { E.mode = TQPK_JOIN_DIRECT; E.unique = 1; E.slots = 0; }
-    k_join_probe<TQPK_JT_ANTI><<<(int)tiles, kBlock, 0, s>>>(E, pkeys, pdt, F, np, nullptr, out_p, capacity, nullptr,
-                                                            totals, status_a, ctl, ctl + 1);
-    TQPK_CHECK_LAUNCH();
+    rc = launch_probe<TQPK_JT_ANTI>(D, pkeys, pdt, F, np, nullptr, out_p, capacity, nullptr, W.totals, W.status_a,
+                                    W.ctl, nullptr, W.ctl + 1, s);
+    if (rc) return rc;
   }
-  int64_t h[2] = {0, 0};
-  int err = 0;
-  TQPK_CUDA(cudaMemcpyAsync(h, totals, sizeof(h), cudaMemcpyDeviceToHost, s));
-  TQPK_CUDA(cudaMemcpyAsync(&err, ctl + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+  // one read: control words, totals and the pair total lie beside each other
+  struct { int ctl[64]; int64_t totals[32]; PairCtl pair; } h;
+  if (dup) TQPK_CUDA(cudaMemcpyAsync(W.ctl + 3, dup, sizeof(int), cudaMemcpyDeviceToDevice, s));
+  TQPK_CUDA(cudaMemcpyAsync(&h, W.ctl, sizeof(h), cudaMemcpyDeviceToHost, s));
   TQPK_CUDA(cudaStreamSynchronize(s));
-  if (err) return err;
-  *h_count = (jt == TQPK_JT_OUTER) ? h[1] : h[0];
+  if (h.ctl[1]) return h.ctl[1];
+  if (dup && h.ctl[3]) {
+    *h_count = -1;               // the build keys repeat: tqpk_join_rows first
+    return TQPK_ECAPACITY;
+  }
+  *h_count = jt == TQPK_JT_OUTER ? h.totals[1] : pair_total == W.totals ? h.totals[0] : h.pair.total;
   return *h_count > capacity ? TQPK_ECAPACITY : TQPK_OK;
+}
+
+extern "C" int tqpk_join_count(const tqpk_join_plan* plan, const void* build_ws, const void* pkeys, int32_t pdt,
+                               const uint8_t* pmask, int64_t np, int64_t* h_count, void* pws, size_t pws_bytes,
+                               tqpk_stream stream) {
+  if (!plan || !build_ws || np < 0 || (np > 0 && !pkeys) || !h_count) return TQPK_EINVAL;
+  if (uniqueness(*plan) == TQPK_JOIN_UNKNOWN) return TQPK_EINVAL;
+  if (!is_int_dtype(pdt)) return TQPK_EDTYPE;
+  if (!pws || pws_bytes < tqpk_join_probe_workspace_bytes(np)) return TQPK_ENOMEM;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  BuildLayout L;
+  ProbeLayout W;
+  if (!layout(*plan, const_cast<void*>(build_ws), plan->ws_bytes, L)) return TQPK_ENOMEM;
+  if (!probe_layout(np, pws, pws_bytes, W)) return TQPK_ENOMEM;
+  *h_count = 0;
+  if (np == 0) return TQPK_OK;
+  TQPK_CUDA(cudaMemsetAsync(pws, 0, W.zeroed, s));
+  const int rc = count_pairs(make_dir(*plan, L, true), pkeys, pdt, make_filter(nullptr, pmask), np, W, s);
+  if (rc) return rc;
+  TQPK_CUDA(cudaMemcpyAsync(h_count, &W.pair->total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  TQPK_CUDA(cudaStreamSynchronize(s));
+  return TQPK_OK;
+}
+
+extern "C" int tqpk_join_write(const tqpk_join_plan* plan, const void* build_ws, const void* pkeys, int32_t pdt,
+                               const uint8_t* pmask, int64_t np, int64_t* out_b, int64_t* out_p, int64_t capacity,
+                               void* pws, size_t pws_bytes, tqpk_stream stream) {
+  if (!plan || !build_ws || np < 0 || (np > 0 && !pkeys) || capacity < 0) return TQPK_EINVAL;
+  if (capacity > 0 && (!out_b || !out_p)) return TQPK_EINVAL;
+  if (uniqueness(*plan) == TQPK_JOIN_UNKNOWN) return TQPK_EINVAL;
+  if (!is_int_dtype(pdt)) return TQPK_EDTYPE;
+  if (!pws || pws_bytes < tqpk_join_probe_workspace_bytes(np)) return TQPK_ENOMEM;
+  if (np == 0 || capacity == 0) return TQPK_OK;
+  BuildLayout L;
+  ProbeLayout W;
+  if (!layout(*plan, const_cast<void*>(build_ws), plan->ws_bytes, L)) return TQPK_ENOMEM;
+  if (!probe_layout(np, pws, pws_bytes, W)) return TQPK_ENOMEM;
+  return write_pairs(make_dir(*plan, L, true), pkeys, pdt, make_filter(nullptr, pmask), np, W, out_b, out_p, capacity,
+                     static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tqpk_gather(int32_t ncols, const void* const* cols_in, const int32_t* dts, const int64_t* idx,

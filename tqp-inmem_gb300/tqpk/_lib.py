@@ -31,6 +31,7 @@ ACC_SUM, ACC_COUNT_NOTNULL, ACC_COUNT_ROWS, ACC_MIN, ACC_MAX = 1, 2, 3, 4, 5
 GB_GLOBAL_ONE, GB_DENSE_PRIVATE, GB_DENSE_SHARED, GB_DENSE_GLOBAL, GB_HASH = 0, 1, 2, 3, 4
 OUT_ACC, OUT_AVG = 0, 1
 JOIN_DIRECT, JOIN_SORTED = 1, 2
+JOIN_UNKNOWN, JOIN_WIDE = 2, 256         # values of JoinPlan.unique
 JT_INNER, JT_SEMI, JT_ANTI, JT_OUTER = 0, 1, 2, 3
 
 
@@ -100,6 +101,10 @@ SIGNATURES = {
     "tqpk_topk_stable": (C.c_int, [_VP, _I32, _I32, _VP, _I64, _I64, _VP, _VP, _SZ, _VP]),
     "tqpk_join_plan_build": (C.c_int, [_VP, _I32, _VP, _I64, _P(JoinPlan), _VP, _VP]),
     "tqpk_join_build": (C.c_int, [_P(JoinPlan), _VP, _I32, _VP, _I64, _VP, _SZ, _VP]),
+    "tqpk_join_directory": (C.c_int, [_P(JoinPlan), _VP, _I32, _VP, _I64, _VP, _SZ, _VP]),
+    "tqpk_join_rows": (C.c_int, [_P(JoinPlan), _VP, _I32, _VP, _I64, _VP, _SZ, _VP]),
+    "tqpk_join_count": (C.c_int, [_P(JoinPlan), _VP, _VP, _I32, _VP, _I64, _P(_I64), _VP, _SZ, _VP]),
+    "tqpk_join_write": (C.c_int, [_P(JoinPlan), _VP, _VP, _I32, _VP, _I64, _VP, _VP, _I64, _VP, _SZ, _VP]),
     "tqpk_join_probe_workspace_bytes": (_SZ, [_I64]),
     "tqpk_join_probe": (C.c_int, [_P(JoinPlan), _VP, _VP, _I32, _VP, _I64, _I32, _VP, _VP, _I64, _P(_I64), _VP,
                                   _SZ, _VP]),

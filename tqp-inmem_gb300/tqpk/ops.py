@@ -374,26 +374,38 @@ class JoinBuild:
     ws: torch.Tensor
     keys: torch.Tensor
     device: torch.device
+    mask: Optional[torch.Tensor] = None
+
+    def _call(self, fn, what: str) -> None:
+        n = int(self.keys.numel())
+        L.check(fn(C.byref(self.plan), self.keys.data_ptr() if n else None, code_of(self.keys.dtype),
+                   self.mask.data_ptr() if self.mask is not None else None, n, self.ws.data_ptr(), self.ws.numel(),
+                   _stream(self.device)), what)
+
+    @property
+    def unique(self) -> int:
+        """1: the build keys are unique, 0: they repeat, L.JOIN_UNKNOWN: not known yet."""
+        return self.plan.unique & ~L.JOIN_WIDE
 
 
 def join_build(keys: torch.Tensor, mask: Optional[torch.Tensor] = None) -> JoinBuild:
+    """The build side's directory (one host read, of the key range).  Whether a key repeats, and the
+    sorted rows of repeated keys, are left to the first probe that needs them."""
     lib = L.load()
     keys = _col1d(keys)
     _check_cuda(keys, mask)
     if keys.dtype == torch.float64:
         raise NotImplementedError("join on a float64 key is not on the kernel path")
     dev = keys.device
-    s = _stream(dev)
     plan = L.JoinPlan()
     scratch = _ws(256, dev)
-    mp = mask.data_ptr() if mask is not None else None
     n = int(keys.numel())
-    L.check(lib.tqpk_join_plan_build(keys.data_ptr() if n else None, code_of(keys.dtype), mp, n, C.byref(plan),
-                                     scratch.data_ptr(), s), "tqpk_join_plan_build")
-    ws = _ws(plan.ws_bytes, dev)
-    L.check(lib.tqpk_join_build(C.byref(plan), keys.data_ptr() if n else None, code_of(keys.dtype), mp, n,
-                                ws.data_ptr(), ws.numel(), s), "tqpk_join_build")
-    return JoinBuild(plan, ws, keys, dev)
+    L.check(lib.tqpk_join_plan_build(keys.data_ptr() if n else None, code_of(keys.dtype),
+                                     mask.data_ptr() if mask is not None else None, n, C.byref(plan),
+                                     scratch.data_ptr(), _stream(dev)), "tqpk_join_plan_build")
+    build = JoinBuild(plan, _ws(plan.ws_bytes, dev), keys, dev, mask)
+    build._call(lib.tqpk_join_directory, "tqpk_join_directory")
+    return build
 
 
 def join_probe(build: JoinBuild, probe_keys: torch.Tensor, probe_mask: Optional[torch.Tensor] = None,
@@ -409,22 +421,42 @@ def join_probe(build: JoinBuild, probe_keys: torch.Tensor, probe_mask: Optional[
     s = _stream(dev)
     n = int(pk.numel())
     pws = _ws(lib.tqpk_join_probe_workspace_bytes(n), dev)
-    mp = probe_mask.data_ptr() if probe_mask is not None else None
-    # Unique build keys (and semi/anti joins) give at most one output per probe row.
-    cap = n if (build.plan.unique or jt in (L.JT_SEMI, L.JT_ANTI)) else 0
+    head = (build.ws.data_ptr(), pk.data_ptr() if n else None, code_of(pk.dtype),
+            probe_mask.data_ptr() if probe_mask is not None else None, n)
+    cnt = C.c_int64(0)
+
+    def outputs(cap):
+        return torch.empty(cap, dtype=torch.int64, device=dev), torch.empty(cap, dtype=torch.int64, device=dev)
+
+    if build.unique != 0 or jt in (L.JT_SEMI, L.JT_ANTI):
+        # at most one output per probe row, unless a key of the build side turns out to repeat
+        ob, op = outputs(n)
+        st = lib.tqpk_join_probe(C.byref(build.plan), *head, jt, ob.data_ptr() if n else None,
+                                 op.data_ptr() if n else None, n, C.byref(cnt), pws.data_ptr(), pws.numel(), s)
+        if not (st == L.ECAPACITY and cnt.value < 0):
+            L.check(st, "tqpk_join_probe")
+            if jt in (L.JT_INNER, L.JT_OUTER) and n:
+                build.plan.unique = 1 | (build.plan.unique & L.JOIN_WIDE)
+            return ob[:cnt.value], op[:cnt.value]
+        build._call(lib.tqpk_join_rows, "tqpk_join_rows")
+    if jt == L.JT_INNER:
+        L.check(lib.tqpk_join_count(C.byref(build.plan), *head, C.byref(cnt), pws.data_ptr(), pws.numel(), s),
+                "tqpk_join_count")
+        ob, op = outputs(cnt.value)
+        L.check(lib.tqpk_join_write(C.byref(build.plan), *head, ob.data_ptr() if cnt.value else None,
+                                    op.data_ptr() if cnt.value else None, cnt.value, pws.data_ptr(), pws.numel(), s),
+                "tqpk_join_write")
+        return ob, op
+    cap = 0
     for _ in range(2):
-        ob = torch.empty(cap, dtype=torch.int64, device=dev)
-        op = torch.empty(cap, dtype=torch.int64, device=dev)
-        cnt = C.c_int64(0)
-        st = lib.tqpk_join_probe(C.byref(build.plan), build.ws.data_ptr(), pk.data_ptr() if n else None,
-                                 code_of(pk.dtype), mp, n, jt, ob.data_ptr() if cap else None,
+        ob, op = outputs(cap)
+        st = lib.tqpk_join_probe(C.byref(build.plan), *head, jt, ob.data_ptr() if cap else None,
                                  op.data_ptr() if cap else None, cap, C.byref(cnt), pws.data_ptr(), pws.numel(), s)
         if st == L.ECAPACITY:
             cap = cnt.value
             continue
         L.check(st, "tqpk_join_probe")
-        m = cnt.value
-        return ob[:m], op[:m]
+        return ob[:cnt.value], op[:cnt.value]
     raise RuntimeError("tqpk_join_probe: output size changed between calls")
 
 
