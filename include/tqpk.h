@@ -364,17 +364,21 @@ int tqpk_join_probe(const tqpk_join_plan* h_plan, const void* d_build_ws, const 
                     int64_t* d_out_build, int64_t* d_out_probe, int64_t capacity, int64_t* h_count,
                     void* d_probe_ws, size_t probe_ws_bytes, tqpk_stream stream);
 
-/* An inner probe in two calls, for exactly sized outputs: tqpk_join_count leaves
- * the pair offsets of every tile of probe rows in d_probe_ws and their number in
- * *h_count (synchronises); tqpk_join_write with the same arguments and
- * d_probe_ws writes the first `capacity` pairs (no synchronisation).  unique
- * must be known.                                                            */
+/* An inner probe in two calls, for exactly sized outputs and for joins with extra
+ * conditions (hashjoin.py:100-108): tqpk_join_count leaves the pair offsets of
+ * every tile of probe rows in d_probe_ws and their number in *h_count
+ * (synchronises); tqpk_join_write with the same arguments and d_probe_ws writes
+ * the first `capacity` pairs (no synchronisation).  h_cond (may be NULL) is a
+ * numeric predicate program over the two sides' columns, evaluated for every
+ * key-equal pair; bit c of probe_cols: its column c is the probe side's.  A
+ * string instruction is TQPK_EUNSUPPORTED.  A directory whose unique is
+ * TQPK_JOIN_UNKNOWN gives TQPK_ECAPACITY and *h_count = -1 when a key repeats. */
 int tqpk_join_count(const tqpk_join_plan* h_plan, const void* d_build_ws, const void* d_probe_keys,
-                    int32_t probe_dtype, const uint8_t* d_probe_mask, int64_t np, int64_t* h_count,
-                    void* d_probe_ws, size_t probe_ws_bytes, tqpk_stream stream);
+                    int32_t probe_dtype, const uint8_t* d_probe_mask, int64_t np, const tqpk_predicate* h_cond,
+                    uint32_t probe_cols, int64_t* h_count, void* d_probe_ws, size_t probe_ws_bytes, tqpk_stream stream);
 int tqpk_join_write(const tqpk_join_plan* h_plan, const void* d_build_ws, const void* d_probe_keys,
-                    int32_t probe_dtype, const uint8_t* d_probe_mask, int64_t np, int64_t* d_out_build,
-                    int64_t* d_out_probe, int64_t capacity, void* d_probe_ws, size_t probe_ws_bytes,
+                    int32_t probe_dtype, const uint8_t* d_probe_mask, int64_t np, const tqpk_predicate* h_cond,
+                    uint32_t probe_cols, int64_t* d_out_build, int64_t* d_out_probe, int64_t capacity, void* d_probe_ws, size_t probe_ws_bytes,
                     tqpk_stream stream);
 
 /* ---- fused pipelines ------------------------------------------------------

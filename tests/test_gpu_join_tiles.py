@@ -61,6 +61,36 @@ def test_pairs(kind, nb, npr):
                 np.testing.assert_array_equal(bi.cpu().numpy(), ebi, err_msg=jtype)
 
 
+CONDS = [[["#12", "=", "#22"]], [["#12", "<", "#22"], ["f#13", ">=", "100.25"]], [["NOT", [["#12", "=", "#22"]]]],
+         [["f#13", "=", "500.5"]], [[["f#23", ">", "f#13"], "OR", ["#22", "IN", ["1", "3"]]]], [["#12", "<=", "1.5"]],
+         [["#12", ">", "99"]]]
+
+
+@pytest.mark.parametrize("conds", CONDS)
+@pytest.mark.parametrize("kind,nb,npr", [("unique", 700, 1025), ("repeated", 5000, 4097), ("one key", 300, 90),
+                                         ("sparse", 900, 20_001)])
+def test_conditions_of_a_join(kind, nb, npr, conds):
+    """Conditions evaluated by the probe against the oracle's filter over the key-equal pairs."""
+    from oracle import tqp_oracle as O
+    from tqpk.operators import join_vortex
+    from tqpk.variable import Variable
+    rng = np.random.default_rng(nb + npr)
+    bk = _keys(kind, rng, nb)
+    pk = bk[rng.integers(0, nb, npr)]
+    cols = {11: bk, 12: rng.integers(0, 5, nb).astype(np.int32), 13: rng.integers(0, 2001, nb) * 0.5,
+            21: pk, 22: rng.integers(0, 5, npr).astype(np.int64), 23: rng.integers(0, 2001, npr) * 0.5}
+    bi, pi = _expected(bk, np.ones(nb, bool), pk, np.ones(npr, bool), "inner")
+    pairs = {c: cols[c][bi] if c < 20 else cols[c][pi] for c in cols}
+    keep = np.ones(bi.size, bool)
+    for c in conds:
+        keep &= O.eval_filter(c, pairs)
+    tg = {c: Variable(torch.from_numpy(a).cuda(), "int") for c, a in cols.items()}
+    args = {"left group": [11, 12, 13], "right group": [21, 22, 23], "materialized in": [11, 12, 13, 21, 22, 23]}
+    assert join_vortex(True, tg, args, 11, 21, conds, "inner", None, None, "j") == int(keep.sum())
+    for c in cols:
+        np.testing.assert_array_equal(tg[c].tensor.cpu().numpy(), pairs[c][keep], err_msg=str(c))
+
+
 def test_staged_build_equals_the_whole_build():
     import ctypes as C
     from tqpk import _lib as L

@@ -299,15 +299,65 @@ struct PairCtl {
   int64_t total;          // pairs in all
 };
 
-// Pass COUNT leaves each tile's pair count in tile_base; its last CTA scans them into offsets.
-template <bool COUNT>
+// The join's extra conditions: a numeric predicate program over columns of both sides (bit c of
+// probe_cols: column c is the probe side's).
+struct PairCond {
+  tqpk_predicate P;
+  unsigned probe_cols;
+};
+
+__device__ __forceinline__ bool pair_cmp(const PairCond& C, const tqpk_pred_insn& I, int64_t b, int64_t p) {
+  const int64_t r = (C.probe_cols >> I.col) & 1u ? p : b;
+  const void* col = C.P.cols[I.col];
+  const int dt = C.P.dtypes[I.col];
+  if (I.op == TQPK_P_MASK) return ld_int(col, TQPK_U8, r) != 0;
+  if (I.op == TQPK_P_CMPCOL) {
+    const int c2 = (int)I.lit_i;
+    const int64_t r2 = (C.probe_cols >> c2) & 1u ? p : b;
+    if (I.domain == TQPK_DOM_F64) return cmp_op<double>(I.cmp, ld_f64(col, dt, r), ld_f64(C.P.cols[c2], C.P.dtypes[c2], r2));
+    return cmp_op<int64_t>(I.cmp, ld_int(col, dt, r), ld_int(C.P.cols[c2], C.P.dtypes[c2], r2));
+  }
+  if (I.domain == TQPK_DOM_F64) {
+    const double x = ld_f64(col, dt, r);
+    if (I.cmp != TQPK_ISCLOSE) return cmp_op<double>(I.cmp, x, I.lit_f);
+    const double err = fabs(__dsub_rn(x, I.lit_f));
+    return (x == I.lit_f) || (isfinite(err) && err <= I.lit_aux);
+  }
+  const int64_t x = ld_int(col, dt, r);
+  if (I.domain == TQPK_DOM_F32) return cmp_op<float>(I.cmp, static_cast<float>(x), static_cast<float>(I.lit_f));
+  return cmp_op<int64_t>(I.cmp, x, I.lit_i);
+}
+
+// The program for build row b and probe row p; the stack is a word of bits (at most 32 deep).
+__device__ __forceinline__ bool pair_holds(const PairCond& C, int64_t b, int64_t p) {
+  unsigned st = 0;
+  for (int k = 0; k < C.P.n_insn; ++k) {
+    const tqpk_pred_insn& I = C.P.insn[k];
+    switch (I.op) {
+      case TQPK_P_AND: st = ((st >> 1) & ~1u) | ((st >> 1) & st & 1u); break;
+      case TQPK_P_OR: st = (st >> 1) | (st & 1u); break;
+      case TQPK_P_NOT: st ^= 1u; break;
+      case TQPK_P_TRUE: st = (st << 1) | 1u; break;
+      case TQPK_P_FALSE: st <<= 1; break;
+      default: st = (st << 1) | (pair_cmp(C, I, b, p) ? 1u : 0u); break;
+    }
+  }
+  return st & 1u;
+}
+
+// Pass COUNT leaves each tile's pair count in tile_base; its last CTA scans them into offsets.  COND: only
+// the pairs that satisfy C count; both passes evaluate it (24 M pairs of a key repeated four times, one in
+// four kept: materialising them, gathering the condition's columns and compacting took ~600 us).
+template <bool COUNT, bool COND>
 __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pkeys, int pdt, RowFilter F, int64_t np,
                                                        int kvec, int64_t* __restrict__ out_b,
                                                        int64_t* __restrict__ out_p, int64_t capacity,
-                                                       int64_t* __restrict__ tile_base, PairCtl* ctl) {
+                                                       int64_t* __restrict__ tile_base, PairCtl* ctl,
+                                                       const __grid_constant__ PairCond C) {
+  constexpr bool kRows = !COUNT || COND;
   __shared__ int64_t sw[kBlock / 32 + 1];
-  __shared__ int64_t s_pre[COUNT ? 1 : kPairRows];     // pairs before each row of the tile
-  __shared__ int64_t s_first[COUNT ? 1 : kPairRows];   // where its build rows start
+  __shared__ int64_t s_pre[kRows ? kPairRows : 1];     // pairs before each row of the tile
+  __shared__ int64_t s_first[kRows ? kPairRows : 1];   // where its build rows start
   __shared__ int s_last;
   const int64_t tile = blockIdx.x;
   const int64_t g0 = tile * kPairRows + 4 * threadIdx.x;
@@ -328,6 +378,36 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
   }
   int64_t total;
   int64_t excl = block_excl_scan<kBlock, int64_t>(mine, total, sw);
+  // pair o of the tile: its probe row (the last one with s_pre <= o) and build row
+  auto pair = [&](int64_t o, int& row, int64_t& build) {
+    int lo = 0, hi = kPairRows;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (s_pre[mid] <= o) lo = mid; else hi = mid;
+    }
+    const int64_t f = s_first[lo] + (o - s_pre[lo]);
+    row = lo;
+    build = D.csr ? D.csr[f] : f;
+  };
+  if (kRows) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s_pre[4 * threadIdx.x + j] = excl;
+      s_first[4 * threadIdx.x + j] = first[j];
+      excl += cnt[j];
+    }
+    __syncthreads();
+  }
+  if (COUNT && COND) {
+    int64_t kept = 0;
+    for (int64_t o = threadIdx.x; o < total; o += kBlock) {
+      int row;
+      int64_t build;
+      pair(o, row, build);
+      kept += pair_holds(C, build, tile * kPairRows + row) ? 1 : 0;
+    }
+    block_excl_scan<kBlock, int64_t>(kept, total, sw);
+  }
   if (COUNT) {
     if (threadIdx.x == 0) {
       tile_base[tile] = total;
@@ -359,24 +439,43 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
     if (threadIdx.x == 0) ctl->total = run;
     return;
   }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    s_pre[4 * threadIdx.x + j] = excl;
-    s_first[4 * threadIdx.x + j] = first[j];
-    excl += cnt[j];
-  }
-  __syncthreads();
-  const int64_t base = tile_base[tile];
-  for (int64_t o = threadIdx.x; o < total; o += kBlock) {
-    if (base + o >= capacity) break;
-    int lo = 0, hi = kPairRows;                // the last row with s_pre <= o
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (s_pre[mid] <= o) lo = mid; else hi = mid;
+  int64_t base = tile_base[tile];
+  if (!COND) {
+    for (int64_t o = threadIdx.x; o < total; o += kBlock) {
+      if (base + o >= capacity) break;
+      int row;
+      int64_t build;
+      pair(o, row, build);
+      out_p[base + o] = tile * kPairRows + row;
+      out_b[base + o] = build;
     }
-    const int64_t f = s_first[lo] + (o - s_pre[lo]);
-    out_p[base + o] = tile * kPairRows + lo;
-    out_b[base + o] = D.csr ? D.csr[f] : f;
+    return;
+  }
+  __shared__ unsigned s_kept[2][kBlock / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int64_t o0 = 0; o0 < total; o0 += kBlock) {
+    const int64_t o = o0 + threadIdx.x;
+    int row = 0;
+    int64_t build = 0;
+    bool keep = false;
+    if (o < total) {
+      pair(o, row, build);
+      keep = pair_holds(C, build, tile * kPairRows + row);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    unsigned* kept = s_kept[(o0 / kBlock) & 1];
+    if (lane == 0) kept[warp] = __popc(m);
+    __syncthreads();                 // two buffers: the next chunk's counts do not overwrite this one's
+    int64_t at = base + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w) {
+      at += w < warp ? kept[w] : 0;
+      base += kept[w];
+    }
+    if (keep && at < capacity) {
+      out_p[at] = tile * kPairRows + row;
+      out_b[at] = build;
+    }
   }
 }
 
@@ -514,21 +613,23 @@ static bool probe_layout(int64_t np, void* pws, size_t bytes, ProbeLayout& W) {
 
 // Pair counts of every tile of probe rows and their sum (W.pair->total), on the device.
 static int count_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFilter& F, int64_t np,
-                       const ProbeLayout& W, cudaStream_t s) {
+                       const PairCond& C, const ProbeLayout& W, cudaStream_t s) {
   const int64_t tiles = (np + kPairRows - 1) / kPairRows;
   if (tiles > INT32_MAX) return TQPK_EUNSUPPORTED;
-  k_join_pairs<true><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, nullptr, nullptr, 0,
-                                                   W.tile_base, W.pair);
+  auto kernel = C.P.n_insn ? k_join_pairs<true, true> : k_join_pairs<true, false>;
+  kernel<<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, nullptr, nullptr, 0, W.tile_base,
+                                       W.pair, C);
   TQPK_CHECK_LAUNCH();
   return TQPK_OK;
 }
 
-static int write_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFilter& F, int64_t np,
+static int write_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFilter& F, int64_t np, const PairCond& C,
                        const ProbeLayout& W, int64_t* out_b, int64_t* out_p, int64_t capacity, cudaStream_t s) {
   const int64_t tiles = (np + kPairRows - 1) / kPairRows;
+  auto kernel = C.P.n_insn ? k_join_pairs<false, true> : k_join_pairs<false, false>;
   timing_before(KID_JOIN_PROBE, s);
-  k_join_pairs<false><<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, out_b, out_p,
-                                                    capacity, W.tile_base, W.pair);
+  kernel<<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, out_b, out_p, capacity,
+                                       W.tile_base, W.pair, C);
   timing_after(KID_JOIN_PROBE, s);
   TQPK_CHECK_LAUNCH();
   return TQPK_OK;
@@ -692,8 +793,9 @@ extern "C" int tqpk_join_probe(const tqpk_join_plan* plan, const void* build_ws,
                                          W.ctl, dup, W.ctl + 1, s);
       } else {
         pair_total = &W.pair->total;
-        rc = count_pairs(D, pkeys, pdt, F, np, W, s);
-        if (!rc && capacity > 0) rc = write_pairs(D, pkeys, pdt, F, np, W, out_b, out_p, capacity, s);
+        const PairCond none{};
+        rc = count_pairs(D, pkeys, pdt, F, np, none, W, s);
+        if (!rc && capacity > 0) rc = write_pairs(D, pkeys, pdt, F, np, none, W, out_b, out_p, capacity, s);
       }
       if (rc) return rc;
     }
@@ -727,12 +829,27 @@ extern "C" int tqpk_join_probe(const tqpk_join_plan* plan, const void* build_ws,
   return *h_count > capacity ? TQPK_ECAPACITY : TQPK_OK;
 }
 
+// The conditions of a call (null: none): numeric instructions only.
+static int pair_cond(const tqpk_predicate* cond, uint32_t probe_cols, PairCond& C) {
+  C = PairCond{};
+  if (!cond) return TQPK_OK;
+  const int rc = check_pred(cond);
+  if (rc) return rc;
+  for (int k = 0; k < cond->n_insn; ++k)
+    if (cond->insn[k].op > TQPK_P_CMPCOL) return TQPK_EUNSUPPORTED;
+  C.P = *cond;
+  C.probe_cols = probe_cols;
+  return TQPK_OK;
+}
+
 extern "C" int tqpk_join_count(const tqpk_join_plan* plan, const void* build_ws, const void* pkeys, int32_t pdt,
-                               const uint8_t* pmask, int64_t np, int64_t* h_count, void* pws, size_t pws_bytes,
-                               tqpk_stream stream) {
+                               const uint8_t* pmask, int64_t np, const tqpk_predicate* cond, uint32_t probe_cols,
+                               int64_t* h_count, void* pws, size_t pws_bytes, tqpk_stream stream) {
   if (!plan || !build_ws || np < 0 || (np > 0 && !pkeys) || !h_count) return TQPK_EINVAL;
-  if (uniqueness(*plan) == TQPK_JOIN_UNKNOWN) return TQPK_EINVAL;
   if (!is_int_dtype(pdt)) return TQPK_EDTYPE;
+  PairCond C;
+  int rc = pair_cond(cond, probe_cols, C);
+  if (rc) return rc;
   if (!pws || pws_bytes < tqpk_join_probe_workspace_bytes(np)) return TQPK_ENOMEM;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BuildLayout L;
@@ -741,8 +858,17 @@ extern "C" int tqpk_join_count(const tqpk_join_plan* plan, const void* build_ws,
   if (!probe_layout(np, pws, pws_bytes, W)) return TQPK_ENOMEM;
   *h_count = 0;
   if (np == 0) return TQPK_OK;
+  if (uniqueness(*plan) == TQPK_JOIN_UNKNOWN) {
+    int dup = 0;
+    TQPK_CUDA(cudaMemcpyAsync(&dup, L.hdr, sizeof(dup), cudaMemcpyDeviceToHost, s));
+    TQPK_CUDA(cudaStreamSynchronize(s));
+    if (dup) {
+      *h_count = -1;             // the build keys repeat: tqpk_join_rows first
+      return TQPK_ECAPACITY;
+    }
+  }
   TQPK_CUDA(cudaMemsetAsync(pws, 0, W.zeroed, s));
-  const int rc = count_pairs(make_dir(*plan, L, true), pkeys, pdt, make_filter(nullptr, pmask), np, W, s);
+  rc = count_pairs(make_dir(*plan, L, true), pkeys, pdt, make_filter(nullptr, pmask), np, C, W, s);
   if (rc) return rc;
   TQPK_CUDA(cudaMemcpyAsync(h_count, &W.pair->total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   TQPK_CUDA(cudaStreamSynchronize(s));
@@ -750,20 +876,23 @@ extern "C" int tqpk_join_count(const tqpk_join_plan* plan, const void* build_ws,
 }
 
 extern "C" int tqpk_join_write(const tqpk_join_plan* plan, const void* build_ws, const void* pkeys, int32_t pdt,
-                               const uint8_t* pmask, int64_t np, int64_t* out_b, int64_t* out_p, int64_t capacity,
-                               void* pws, size_t pws_bytes, tqpk_stream stream) {
+                               const uint8_t* pmask, int64_t np, const tqpk_predicate* cond, uint32_t probe_cols,
+                               int64_t* out_b, int64_t* out_p, int64_t capacity, void* pws, size_t pws_bytes,
+                               tqpk_stream stream) {
   if (!plan || !build_ws || np < 0 || (np > 0 && !pkeys) || capacity < 0) return TQPK_EINVAL;
   if (capacity > 0 && (!out_b || !out_p)) return TQPK_EINVAL;
-  if (uniqueness(*plan) == TQPK_JOIN_UNKNOWN) return TQPK_EINVAL;
   if (!is_int_dtype(pdt)) return TQPK_EDTYPE;
+  PairCond C;
+  const int rc = pair_cond(cond, probe_cols, C);
+  if (rc) return rc;
   if (!pws || pws_bytes < tqpk_join_probe_workspace_bytes(np)) return TQPK_ENOMEM;
   if (np == 0 || capacity == 0) return TQPK_OK;
   BuildLayout L;
   ProbeLayout W;
   if (!layout(*plan, const_cast<void*>(build_ws), plan->ws_bytes, L)) return TQPK_ENOMEM;
   if (!probe_layout(np, pws, pws_bytes, W)) return TQPK_ENOMEM;
-  return write_pairs(make_dir(*plan, L, true), pkeys, pdt, make_filter(nullptr, pmask), np, W, out_b, out_p, capacity,
-                     static_cast<cudaStream_t>(stream));
+  return write_pairs(make_dir(*plan, L, true), pkeys, pdt, make_filter(nullptr, pmask), np, C, W, out_b, out_p,
+                     capacity, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tqpk_gather(int32_t ncols, const void* const* cols_in, const int32_t* dts, const int64_t* idx,

@@ -14,9 +14,11 @@ which changes a result:
   (:153-175, with index_with_null for right-outer, conversion.py:52-57).
 
 Extra join conditions (:100-108, e.g. the second key of a two-key join,
-main.py:208-217) are evaluated on the gathered pair columns with the
-predicate kernel and the pairs compacted; the semi, anti and outer forms are
-then derived from the probe rows that keep a pair (:110-151).
+main.py:208-217) on numeric columns are evaluated by the probe for every
+key-equal pair before it is written; conditions on text run on the gathered
+pair columns with the predicate kernel, and the pairs are compacted.  The semi,
+anti and outer forms are then derived from the probe rows that keep a pair
+(:110-151).
 """
 from __future__ import annotations
 
@@ -25,8 +27,8 @@ from typing import Dict, List
 import torch
 
 from .. import _lib as L
-from ..ops import check_deferred, compact, filter_mask, gather, join_build, join_probe, mark_rows
-from ..predicate import compile_filter
+from ..ops import check_deferred, compact, filter_mask, gather, join_build, join_pairs, join_probe, mark_rows
+from ..predicate import compile_filter, has_strings
 from ..variable import make_like, wait_ready
 from ._materialize import materialize
 from .filter import _require_gpu
@@ -60,8 +62,12 @@ def _pairs(tensors_left, tensors_right, left_key, right_key, condition_list, jty
     b = join_build(lk, left_mask)
     wait_ready(tensors_right[right_key])
     # with extra conditions every form starts from the key-equal pairs (hashjoin.py:100-108)
-    bi, pi = join_probe(b, rk, right_mask, "inner" if condition_list else jtype)
-    for cond in condition_list:                       # hashjoin.py:100-108
+    pred = _pair_predicate(tensors_left, tensors_right, condition_list) if condition_list and rk.is_cuda else None
+    if pred is not None:
+        bi, pi = join_pairs(b, rk, right_mask, *pred)
+    else:
+        bi, pi = join_probe(b, rk, right_mask, "inner" if condition_list else jtype)
+    for cond in condition_list if pred is None else []:
         ids = set()
         _collect_ids(cond, ids)
         cols = {}
@@ -79,6 +85,31 @@ def _pairs(tensors_left, tensors_right, left_key, right_key, condition_list, jty
         bi, pi = _non_inner(bi, pi, rk, right_mask, jtype)
     key_range = (int(b.plan.key_min), int(b.plan.key_max)) if b.plan.key_max >= b.plan.key_min else None
     return bi, pi, b.plan.nb_rows, key_range
+
+
+def _pair_predicate(tensors_left, tensors_right, condition_list):
+    """The conditions as one numeric predicate over the two sides' columns and the mask of its
+    probe-side columns, evaluated by the probe itself; None for conditions on text or beyond one
+    program's limits (they run on the gathered pair columns instead)."""
+    ids = set()
+    for cond in condition_list:
+        _collect_ids(cond, ids)
+    cols, tree = {}, condition_list[0]
+    for cond in condition_list[1:]:
+        tree = [tree, "AND", cond]
+    for cid in ids:
+        v = tensors_left[cid] if cid in tensors_left else tensors_right[cid]
+        if v.tensor.dim() != 1:
+            return None
+        cols[cid] = v.tensor
+    try:
+        pred = compile_filter(tree, cols)
+    except NotImplementedError:
+        return None
+    if has_strings(pred.struct):
+        return None
+    wait_ready(*[tensors_left[c] if c in tensors_left else tensors_right[c] for c in ids])
+    return pred, sum(1 << i for i, c in enumerate(pred.col_ids) if c not in tensors_left)
 
 
 def _non_inner(bi, pi, rk, right_mask, jtype):

@@ -440,13 +440,7 @@ def join_probe(build: JoinBuild, probe_keys: torch.Tensor, probe_mask: Optional[
             return ob[:cnt.value], op[:cnt.value]
         build._call(lib.tqpk_join_rows, "tqpk_join_rows")
     if jt == L.JT_INNER:
-        L.check(lib.tqpk_join_count(C.byref(build.plan), *head, C.byref(cnt), pws.data_ptr(), pws.numel(), s),
-                "tqpk_join_count")
-        ob, op = outputs(cnt.value)
-        L.check(lib.tqpk_join_write(C.byref(build.plan), *head, ob.data_ptr() if cnt.value else None,
-                                    op.data_ptr() if cnt.value else None, cnt.value, pws.data_ptr(), pws.numel(), s),
-                "tqpk_join_write")
-        return ob, op
+        return join_pairs(build, pk, probe_mask)
     cap = 0
     for _ in range(2):
         ob, op = outputs(cap)
@@ -458,6 +452,35 @@ def join_probe(build: JoinBuild, probe_keys: torch.Tensor, probe_mask: Optional[
         L.check(st, "tqpk_join_probe")
         return ob[:cnt.value], op[:cnt.value]
     raise RuntimeError("tqpk_join_probe: output size changed between calls")
+
+
+def join_pairs(build: JoinBuild, probe_keys: torch.Tensor, probe_mask: Optional[torch.Tensor] = None,
+               cond: Optional[CompiledPredicate] = None, probe_cols: int = 0) -> Tuple[torch.Tensor, torch.Tensor]:
+    """(build_idx, probe_idx) of an inner join, counted before they are written.  cond, when given, is a
+    numeric predicate over both sides' columns that every pair must satisfy; bit c of probe_cols says
+    that its column c is the probe side's."""
+    lib = L.load()
+    pk = _col1d(probe_keys)
+    _check_cuda(pk, probe_mask, *(cond.tensors if cond is not None else ()))
+    dev = build.device
+    s = _stream(dev)
+    n = int(pk.numel())
+    pws = _ws(lib.tqpk_join_probe_workspace_bytes(n), dev)
+    args = (build.ws.data_ptr(), pk.data_ptr() if n else None, code_of(pk.dtype),
+            probe_mask.data_ptr() if probe_mask is not None else None, n,
+            C.byref(cond.struct) if cond is not None else None, probe_cols)
+    cnt = C.c_int64(0)
+    st = lib.tqpk_join_count(C.byref(build.plan), *args, C.byref(cnt), pws.data_ptr(), pws.numel(), s)
+    if st == L.ECAPACITY and cnt.value < 0:
+        build._call(lib.tqpk_join_rows, "tqpk_join_rows")
+        st = lib.tqpk_join_count(C.byref(build.plan), *args, C.byref(cnt), pws.data_ptr(), pws.numel(), s)
+    L.check(st, "tqpk_join_count")
+    m = cnt.value
+    ob, op = torch.empty(m, dtype=torch.int64, device=dev), torch.empty(m, dtype=torch.int64, device=dev)
+    if m:
+        L.check(lib.tqpk_join_write(C.byref(build.plan), *args, ob.data_ptr(), op.data_ptr(), m, pws.data_ptr(),
+                                    pws.numel(), s), "tqpk_join_write")
+    return ob, op
 
 
 def gather_rows(col: torch.Tensor, idx: torch.Tensor) -> torch.Tensor:
