@@ -211,83 +211,100 @@ __global__ void __launch_bounds__(256) k_groupby_dense(const __grid_constant__ t
 // ascending key-tuple order of the dense modes.
 constexpr uint64_t kHashEmpty = ~0ull;
 
-__device__ __forceinline__ int64_t hash_slot(uint64_t packed, int64_t C) {
-  return (int64_t)((packed * 0x9E3779B97F4A7C15ull) >> 20) & (C - 1);
+// The splitmix64 finaliser (S. Vigna).  Packed keys are arithmetic progressions more often than not (a
+// part's suppliers); one multiplication, of whose product the middle bits were taken, sent them into
+// long runs of linear probing.
+__device__ __forceinline__ int64_t hash_slot(uint64_t z, int64_t C) {
+  z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+  z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+  return (int64_t)(z ^ (z >> 31)) & (C - 1);
 }
 
 __global__ void k_fill_u64(uint64_t* p, int64_t n, uint64_t v) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
-__global__ void __launch_bounds__(256) k_groupby_hash(const __grid_constant__ tqpk_groupby_spec S,
-                                                      const __grid_constant__ tqpk_predicate P, RowFilter F, int64_t n,
-                                                      GbDev G, uint64_t* __restrict__ gacc,
-                                                      unsigned long long* __restrict__ hkeys, int keys_vec,
-                                                      int cols_vec, int* err) {
+// What bounds it: per passing row one compare-and-swap and A reductions at scattered L2 lines.  A tile's
+// passing rows are gathered first, so that the program runs with full warps whatever the filter's
+// selectivity (4 rows a thread in place, one in seven passing, executed it almost seven times as often:
+// 576 us for 0.9 M of 6 M rows), and by the plain loop: the unrolled form with operand selects costs
+// ~2500 instructions a row.  A claimed slot goes on the group list at once (pk, cslot; one counter update
+// per 256 rows), which saves the passes over the table that counted and collected the occupied slots.
+__global__ void __launch_bounds__(kBlock) k_groupby_hash(const __grid_constant__ tqpk_groupby_spec S,
+                                                         const __grid_constant__ tqpk_predicate P, RowFilter F,
+                                                         int64_t n, GbDev G, uint64_t* __restrict__ gacc,
+                                                         unsigned long long* __restrict__ hkeys,
+                                                         int64_t* __restrict__ pk, int64_t* __restrict__ cslot,
+                                                         unsigned long long* groups, int64_t cap, int* err) {
+  __shared__ uint16_t s_row[kTile];
+  __shared__ int sw[kBlock / 32 + 1];
+  __shared__ unsigned s_claims[kBlock / 32];
+  __shared__ unsigned long long s_at;
   const int A = S.n_accs;
   const int64_t C = G.slots;
-  const int64_t groups = (n + 3) >> 2;
-  const bool small = S.n_expr <= 16;
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < groups; g += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r0 = g << 2;
-    const uint32_t b = filter4(F, P, r0, n);
-    if (!b) continue;
-    uint64_t packed[4] = {0, 0, 0, 0};
-    for (int k = 0; k < G.nk; ++k) {
-      int64_t x[4];
-      ld4_int(S.keys[k], S.key_dtypes[k], r0, n, keys_vec, x);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int64_t t0 = blockIdx.x * (int64_t)kTile; t0 < n; t0 += (int64_t)gridDim.x * kTile) {
+    uint32_t bits = 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) packed[j] += (uint64_t)(x[j] - G.kmin[k]) * (uint64_t)G.kstride[k];
+    for (int q = 0; q < kItems / 4; ++q) {
+      const int64_t r0 = t0 + (q * kBlock + threadIdx.x) * 4;
+      if (r0 < n) bits |= filter4(F, P, r0, n) << (4 * q);
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (!((b >> j) & 1u)) continue;
-      int64_t h = hash_slot(packed[j], C);
-      int64_t probes = 0;
-      while (true) {
-        const unsigned long long cur = __ldcg(&hkeys[h]);
-        if (cur == packed[j]) break;
-        if (cur == kHashEmpty) {
-          const unsigned long long prev = atomicCAS(&hkeys[h], kHashEmpty, (unsigned long long)packed[j]);
-          if (prev == kHashEmpty || prev == packed[j]) break;
+    int total;
+    int at = block_excl_scan<kBlock, int>(__popc(bits), total, sw);
+    for (uint32_t b = bits; b; b &= b - 1) {
+      const int j = __ffs(b) - 1;
+      s_row[at++] = (uint16_t)(((j >> 2) * kBlock + threadIdx.x) * 4 + (j & 3));
+    }
+    __syncthreads();
+    for (int i0 = 0; i0 < total; i0 += kBlock) {
+      const int i = i0 + threadIdx.x;
+      bool claimed = false;
+      uint64_t packed = 0;
+      int64_t h = -1;
+      if (i < total) {
+        const int64_t row = t0 + s_row[i];
+        for (int k = 0; k < G.nk; ++k)
+          packed += (uint64_t)(ld_int(S.keys[k], S.key_dtypes[k], row) - G.kmin[k]) * (uint64_t)G.kstride[k];
+        h = hash_slot(packed, C);
+        for (int64_t probes = 0;; h = (h + 1) & (C - 1)) {
+          const unsigned long long prev = atomicCAS(&hkeys[h], kHashEmpty, (unsigned long long)packed);
+          claimed = prev == kHashEmpty;
+          if (claimed || prev == packed) break;
+          if (++probes > C) {              // table full: cannot happen (C >= 2 rows)
+            set_error(err, TQPK_ECAPACITY);
+            h = -1;
+            break;
+          }
         }
-        h = (h + 1) & (C - 1);
-        if (++probes > C) { set_error(err, TQPK_ECAPACITY); h = -1; break; }   // table full: cannot happen (C >= 2 rows)
+        if (h >= 0) {
+          uint64_t r[TQPK_MAX_EXPR];
+          expr_eval_generic(S.expr, S.n_expr, S.cols, S.col_dtypes, row, r);
+          for (int a = 0; a < A; ++a)
+            acc_merge_global(&gacc[(int64_t)a * C + h], S.accs[a],
+                             acc_value(S.accs[a], S.accs[a].kind == TQPK_ACC_COUNT_ROWS ? 0 : r[S.accs[a].reg]));
+        }
       }
-      if (h < 0) continue;
-      if (small) {
-        uint64_t r[16];
-        expr_eval_small<16>(S.expr, S.n_expr, S.cols, S.col_dtypes, r0 + j, r);
-        for (int a = 0; a < A; ++a)
-          acc_merge_global(&gacc[(int64_t)a * C + h], S.accs[a], acc_value(S.accs[a], reg_pick<16>(r, S.accs[a].reg)));
-      } else {
-        uint64_t r[TQPK_MAX_EXPR];
-        expr_eval_generic(S.expr, S.n_expr, S.cols, S.col_dtypes, r0 + j, r);
-        for (int a = 0; a < A; ++a)
-          acc_merge_global(&gacc[(int64_t)a * C + h], S.accs[a], acc_value(S.accs[a], r[S.accs[a].reg]));
+      const unsigned m = __ballot_sync(0xffffffffu, claimed);
+      if (lane == 0) s_claims[warp] = __popc(m);
+      __syncthreads();
+      unsigned before = 0, all = 0;
+#pragma unroll
+      for (int w = 0; w < kBlock / 32; ++w) {
+        before += w < warp ? s_claims[w] : 0;
+        all += s_claims[w];
+      }
+      if (threadIdx.x == 0) s_at = all ? atomicAdd(groups, (unsigned long long)all) : 0;
+      __syncthreads();
+      if (claimed) {
+        const int64_t o = (int64_t)s_at + before + __popc(m & ((1u << lane) - 1u));
+        if (o < cap) {
+          pk[o] = (int64_t)packed;
+          cslot[o] = h;
+        }
       }
     }
-  }
-}
-
-// Appends (packed key, slot) of every occupied slot (unordered).
-__global__ void k_hash_collect(const uint64_t* __restrict__ count0, const unsigned long long* __restrict__ hkeys,
-                               int64_t C, int64_t* __restrict__ pk, int64_t* __restrict__ cslot,
-                               unsigned long long* counter, int64_t cap) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t base = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); base < C;
-       base += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t s = base + lane;
-    const bool occ = s < C && count0[s] != 0;
-    const unsigned bal = __ballot_sync(0xffffffffu, occ);
-    if (!bal) continue;
-    unsigned long long at = 0;
-    if (lane == 0) at = atomicAdd(counter, (unsigned long long)__popc(bal));
-    at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
-    if (occ && (int64_t)at < cap) {
-      pk[at] = (int64_t)hkeys[s];
-      cslot[at] = s;
-    }
+    __syncthreads();
   }
 }
 
@@ -637,15 +654,11 @@ extern "C" int tqpk_groupby_run(const tqpk_groupby_spec* S, const tqpk_gb_plan* 
     k_fill_u64<<<grid_for(C, 4), kBlock, 0, s>>>(reinterpret_cast<uint64_t*>(H.hkeys), C, kHashEmpty);
     TQPK_CHECK_LAUNCH();
     if (n > 0 && plan->n_rows > 0) {
-      bool kvec = true;
-      for (int k = 0; k < S->n_keys; ++k) kvec = kvec && aligned16(S->keys[k]);
       const GbDev G = to_dev(*plan, S->n_keys);
       timing_before(KID_GROUPBY, s);
-      k_groupby_hash<<<grid_for((n + 3) / 4, 8), 256, 0, s>>>(*S, *pred_or_empty(pred), make_filter(pred, mask), n, G,
-                                                               H.gacc, H.hkeys, kvec, spec_cols_vec(S) ? 1 : 0, err);
+      k_groupby_hash<<<grid_for((n + kItems - 1) / kItems, 8), kBlock, 0, s>>>(
+          *S, *pred_or_empty(pred), make_filter(pred, mask), n, G, H.gacc, H.hkeys, H.pk, H.cslot, d_groups, C / 2, err);
       timing_after(KID_GROUPBY, s);
-      TQPK_CHECK_LAUNCH();
-      k_count_groups<<<grid_for(C, 4), kBlock, 0, s>>>(H.gacc, C, d_groups);
       TQPK_CHECK_LAUNCH();
     }
     unsigned long long h[2] = {0, 0};
@@ -740,12 +753,8 @@ extern "C" int tqpk_groupby_emit(const tqpk_groupby_spec* S, const tqpk_gb_plan*
   const int64_t K = plan->slots, A = S->n_accs;
   char* base = static_cast<char*>(ws);
   if (plan->mode == TQPK_GB_HASH) {
-    // the occupied slots (unordered), sorted by packed key = ascending key tuple
+    // the groups in the order their slots were claimed, sorted by packed key = ascending key tuple
     HashLayout H = hash_layout(ws, K, (int)A);
-    unsigned long long* counter = reinterpret_cast<unsigned long long*>(base + 16);
-    TQPK_CUDA(cudaMemsetAsync(counter, 0, 8, s));
-    k_hash_collect<<<grid_for(K, 4), kBlock, 0, s>>>(H.gacc, H.hkeys, K, H.pk, H.cslot, counter, groups);
-    TQPK_CHECK_LAUNCH();
     if (groups > K / 2) return TQPK_EINVAL;       // the table has two slots per row
     const SortKey by_packed{H.pk, nullptr, TQPK_I64, 0, 0, 0};
     int rc2 = sort_keys(&by_packed, 1, nullptr, groups, H.perm, H.sort_ws, H.sort_bytes, s);
