@@ -14,6 +14,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "tqpk.h"
 
@@ -613,6 +614,222 @@ __device__ __forceinline__ uint32_t eval_pred4(const tqpk_predicate& P, int64_t 
   return (sp > 0 ? st[0] : 0xfu) & vm;
 }
 
+// ---- 4 Q rows at a time: four consecutive rows at each of r0[0..Q-1] (ascending), typed, so that the
+// dtype is decided once and the Q loads are in flight together ----
+template <class T, int Q>
+__device__ __forceinline__ void load_rows(const void* p, const int64_t (&r0)[Q], int64_t n, bool vec, T (&x)[4 * Q]) {
+  const T* c = static_cast<const T*>(p);
+  if (vec && r0[Q - 1] + 4 <= n) {           // every group is whole
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if constexpr (sizeof(T) == 8) {
+        const ulonglong2* v = reinterpret_cast<const ulonglong2*>(c + r0[q]);
+        const ulonglong2 a = v[0], b = v[1];
+        memcpy(&x[4 * q], &a, 16);
+        memcpy(&x[4 * q + 2], &b, 16);
+      } else if constexpr (sizeof(T) == 4) {
+        const uint4 a = *reinterpret_cast<const uint4*>(c + r0[q]);
+        memcpy(&x[4 * q], &a, 16);
+      } else {
+        const uint32_t a = *reinterpret_cast<const uint32_t*>(c + r0[q]);
+        memcpy(&x[4 * q], &a, 4);
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 4 * Q; ++i) {
+    const int64_t r = r0[i >> 2] + (i & 3);
+    x[i] = r < n ? c[r] : T(0);
+  }
+}
+
+// Bit i: f(i).
+template <int N, class F>
+__device__ __forceinline__ uint32_t bits_of(F f) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) m |= (uint32_t)f(i) << i;
+  return m;
+}
+
+// x[i] <op> b, the operator decided once.
+template <class T, int N>
+__device__ __forceinline__ uint32_t cmp_rows(int op, const T (&x)[N], T b) {
+  switch (op) {
+    case TQPK_LT: return bits_of<N>([&](int i) { return x[i] < b; });
+    case TQPK_LE: return bits_of<N>([&](int i) { return x[i] <= b; });
+    case TQPK_GT: return bits_of<N>([&](int i) { return x[i] > b; });
+    case TQPK_GE: return bits_of<N>([&](int i) { return x[i] >= b; });
+    case TQPK_EQ: return bits_of<N>([&](int i) { return x[i] == b; });
+    case TQPK_NE: return bits_of<N>([&](int i) { return x[i] != b; });
+  }
+  return 0;
+}
+
+// Integer column against an int64 literal, compared in the column's own width.
+template <class T, int N>
+__device__ __forceinline__ uint32_t int_leaf(const tqpk_pred_insn& I, const T (&x)[N]) {
+  const T b = (T)I.lit_i;
+  if ((int64_t)b == I.lit_i) return cmp_rows<T, N>(I.cmp, x, b);
+  const bool below = sizeof(T) == 8 || I.lit_i > 0;       // every value of the column is below the literal
+  const bool holds = below ? I.cmp == TQPK_LT || I.cmp == TQPK_LE || I.cmp == TQPK_NE
+                           : I.cmp == TQPK_GT || I.cmp == TQPK_GE || I.cmp == TQPK_NE;
+  return holds ? ~0u : 0u;
+}
+
+template <class T, int Q>
+__device__ __forceinline__ uint32_t num_leaf(const tqpk_predicate& P, const tqpk_pred_insn& I, const int64_t (&r0)[Q],
+                                             int64_t n, bool vec) {
+  T x[4 * Q];
+  load_rows<T, Q>(P.cols[I.col], r0, n, vec, x);
+  if (I.domain == TQPK_DOM_I64) return int_leaf<T, 4 * Q>(I, x);
+  if (I.domain == TQPK_DOM_F32) {
+    float y[4 * Q];
+#pragma unroll
+    for (int i = 0; i < 4 * Q; ++i) y[i] = static_cast<float>(static_cast<int64_t>(x[i]));
+    return cmp_rows<float, 4 * Q>(I.cmp, y, static_cast<float>(I.lit_f));   // exact: the host stores a float32 value
+  }
+  double y[4 * Q];                             // an integer column (isclose takes float columns only)
+#pragma unroll
+  for (int i = 0; i < 4 * Q; ++i) y[i] = static_cast<double>(static_cast<int64_t>(x[i]));
+  return cmp_rows<double, 4 * Q>(I.cmp, y, I.lit_f);
+}
+
+// Float64 column: comparisons on the order-preserving integer image (an FP64 compare costs 64 FP32 ones on
+// this part); NaN compares false except under !=.
+template <int Q>
+__device__ __forceinline__ uint32_t f64_leaf(const tqpk_predicate& P, const tqpk_pred_insn& I, const int64_t (&r0)[Q],
+                                             int64_t n, bool vec) {
+  double x[4 * Q];
+  load_rows<double, Q>(P.cols[I.col], r0, n, vec, x);
+  if (I.cmp == TQPK_ISCLOSE)
+    return bits_of<4 * Q>([&](int i) {
+      const double err = fabs(__dsub_rn(x[i], I.lit_f));
+      return (x[i] == I.lit_f) || (isfinite(err) && err <= I.lit_aux);
+    });
+  constexpr uint64_t kInf = 0x7ff0000000000000ull;
+  const uint64_t lit = d2u(I.lit_f);
+  if ((lit << 1) > (kInf << 1)) return I.cmp == TQPK_NE ? ~0u : 0u;       // a NaN literal
+  int64_t y[4 * Q];
+  uint32_t nan = 0;
+#pragma unroll
+  for (int i = 0; i < 4 * Q; ++i) {
+    const uint64_t u = d2u(x[i]);
+    nan |= (uint32_t)((u << 1) > (kInf << 1)) << i;
+    // sign-magnitude to two's complement; both zeros become 0
+    y[i] = (int64_t)u < 0 ? (int64_t)(0x8000000000000000ull - u) : (int64_t)u;
+  }
+  const int64_t b = (int64_t)lit < 0 ? (int64_t)(0x8000000000000000ull - lit) : (int64_t)lit;
+  const uint32_t m = cmp_rows<int64_t, 4 * Q>(I.cmp, y, b);
+  return I.cmp == TQPK_NE ? m | nan : m & ~nan;
+}
+
+// One comparison leaf (rows >= n: unspecified bits).
+template <int Q>
+__device__ __forceinline__ uint32_t pred_leaf(const tqpk_predicate& P, const tqpk_pred_insn& I, const int64_t (&r0)[Q],
+                                              int64_t n, bool vec) {
+  switch (P.dtypes[I.col]) {
+    case TQPK_F64: return f64_leaf<Q>(P, I, r0, n, vec);
+    case TQPK_I64: return num_leaf<int64_t, Q>(P, I, r0, n, vec);
+    case TQPK_I32: return num_leaf<int32_t, Q>(P, I, r0, n, vec);
+    case TQPK_I8: return num_leaf<int8_t, Q>(P, I, r0, n, vec);
+    default: return num_leaf<uint8_t, Q>(P, I, r0, n, vec);
+  }
+}
+
+template <class T, int Q>
+__device__ __forceinline__ uint32_t cmpcol_rows(const tqpk_predicate& P, const tqpk_pred_insn& I, const int64_t (&r0)[Q],
+                                                int64_t n, bool vec) {
+  T a[4 * Q], b[4 * Q];
+  load_rows<T, Q>(P.cols[I.col], r0, n, vec, a);
+  load_rows<T, Q>(P.cols[(int)I.lit_i], r0, n, vec, b);
+  switch (I.cmp) {
+    case TQPK_LT: return bits_of<4 * Q>([&](int i) { return a[i] < b[i]; });
+    case TQPK_LE: return bits_of<4 * Q>([&](int i) { return a[i] <= b[i]; });
+    case TQPK_GT: return bits_of<4 * Q>([&](int i) { return a[i] > b[i]; });
+    case TQPK_GE: return bits_of<4 * Q>([&](int i) { return a[i] >= b[i]; });
+    case TQPK_EQ: return bits_of<4 * Q>([&](int i) { return a[i] == b[i]; });
+    case TQPK_NE: return bits_of<4 * Q>([&](int i) { return a[i] != b[i]; });
+  }
+  return 0;
+}
+
+// Two columns: in their own type when it is the same, else row by row.
+template <int Q>
+__device__ __forceinline__ uint32_t pred_cmpcol(const tqpk_predicate& P, const tqpk_pred_insn& I, const int64_t (&r0)[Q],
+                                                int64_t n, bool vec) {
+  const int c2 = (int)I.lit_i, dt = P.dtypes[I.col], dt2 = P.dtypes[c2];
+  if (dt == dt2 && I.domain == TQPK_DOM_I64 && dt == TQPK_I64) return cmpcol_rows<int64_t, Q>(P, I, r0, n, vec);
+  if (dt == dt2 && I.domain == TQPK_DOM_I64 && dt == TQPK_I32) return cmpcol_rows<int32_t, Q>(P, I, r0, n, vec);
+  uint32_t m = 0;
+#pragma unroll 1
+  for (int i = 0; i < 4 * Q; ++i) {
+    const int64_t r = r0[i >> 2] + (i & 3);
+    if (r >= n) break;
+    const bool c = I.domain == TQPK_DOM_F64 ? cmp_op<double>(I.cmp, ld_f64(P.cols[I.col], dt, r), ld_f64(P.cols[c2], dt2, r))
+                                            : cmp_op<int64_t>(I.cmp, ld_int(P.cols[I.col], dt, r), ld_int(P.cols[c2], dt2, r));
+    m |= (uint32_t)c << i;
+  }
+  return m;
+}
+
+template <int Q>
+__device__ __forceinline__ uint32_t valid_rows(const int64_t (&r0)[Q], int64_t n) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int64_t v = n - r0[q];
+    m |= (v >= 4 ? 0xfu : (v <= 0 ? 0u : ((1u << v) - 1))) << (4 * q);
+  }
+  return m;
+}
+
+// The predicate for 4 Q rows -> mask (rows >= n are 0).  As eval_pred4, with the program, the types and the
+// operators decided once for them.
+template <int Q>
+__device__ __forceinline__ uint32_t eval_pred_rows(const tqpk_predicate& P, const int64_t (&r0)[Q], int64_t n, bool vec) {
+  const uint32_t valid = valid_rows<Q>(r0, n);
+  if (!valid) return 0;
+  uint32_t st[TQPK_MAX_PRED];
+  uint32_t top = ~0u;                      // the top of the stack; st[0..sp-2] below it
+  int sp = 0;
+  for (int k = 0; k < P.n_insn; ++k) {
+    const tqpk_pred_insn& I = P.insn[k];
+    if (I.op == TQPK_P_AND || I.op == TQPK_P_OR) {
+      --sp;
+      top = I.op == TQPK_P_AND ? top & st[sp - 1] : top | st[sp - 1];
+      continue;
+    }
+    if (I.op == TQPK_P_NOT) {
+      top = ~top;
+      continue;
+    }
+    if (sp > 0) st[sp - 1] = top;
+    ++sp;
+    switch (I.op) {
+      case TQPK_P_CMP: top = pred_leaf<Q>(P, I, r0, n, vec); break;
+      case TQPK_P_TRUE: top = ~0u; break;
+      case TQPK_P_FALSE: top = 0u; break;
+      case TQPK_P_CMPCOL: top = pred_cmpcol<Q>(P, I, r0, n, vec); break;
+      case TQPK_P_MASK: {
+        uint8_t x[4 * Q];
+        load_rows<uint8_t, Q>(P.cols[I.col], r0, n, vec, x);
+        top = bits_of<4 * Q>([&](int i) { return x[i] != 0; });
+        break;
+      }
+      default: {                           // text
+        top = 0;
+#pragma unroll 1
+        for (int q = 0; q < Q; ++q)
+          if (r0[q] < n) top |= str_leaf4(P, I, r0[q], n) << (4 * q);
+        break;
+      }
+    }
+  }
+  return top & valid;
+}
+
 // Row filter: a u8 mask column, a predicate program, or neither (all rows).
 struct RowFilter {
   const uint8_t* mask;
@@ -629,6 +846,18 @@ __device__ __forceinline__ uint32_t filter4(const RowFilter& F, const tqpk_predi
   int64_t x[4];
   ld4_int(F.mask, TQPK_U8, r0, n, F.mask_vec, x);
   return ((x[0] != 0) | ((x[1] != 0) << 1) | ((x[2] != 0) << 2) | ((x[3] != 0) << 3)) & vm;
+}
+
+// filter4 for 4 Q rows; PRED: F may hold a predicate (callers with masks only leave its code out).
+template <int Q, bool PRED>
+__device__ __forceinline__ uint32_t filter_rows(const RowFilter& F, const tqpk_predicate& P, const int64_t (&r0)[Q],
+                                                int64_t n) {
+  if (PRED && F.use_pred) return eval_pred_rows<Q>(P, r0, n, F.pred_vec);
+  const uint32_t valid = valid_rows<Q>(r0, n);
+  if (!F.mask || !valid) return valid;
+  uint8_t x[4 * Q];
+  load_rows<uint8_t, Q>(F.mask, r0, n, F.mask_vec, x);
+  return bits_of<4 * Q>([&](int i) { return x[i] != 0; }) & valid;
 }
 
 // ---- scans --------------------------------------------------------------------

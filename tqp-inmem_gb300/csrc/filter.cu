@@ -10,6 +10,8 @@
 // keeps row order (what tensor[mask] gives).
 #include <stdio.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace tqpk {
@@ -48,21 +50,29 @@ int num_sms() {
   return cached[dev];
 }
 
-__global__ void __launch_bounds__(kBlock) k_filter_mask(const __grid_constant__ tqpk_predicate P, int64_t n,
-                                                        uint8_t* __restrict__ mask, unsigned long long* count,
-                                                        int vec, int mask_vec) {
-  const int64_t groups = (n + 3) >> 2;
+// 4 Q rows per thread, four at a time 1024 rows apart (coalesced): a thread's loads of a column are all in
+// flight, and type, operator and program are decided once for them.
+template <int Q>
+__global__ void __launch_bounds__(kBlock, Q == 1 ? 6 : 3) k_filter_mask(const __grid_constant__ tqpk_predicate P,
+                                                                        int64_t n, uint8_t* __restrict__ mask,
+                                                                        unsigned long long* count, int vec,
+                                                                        int mask_vec) {
   unsigned local = 0;
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < groups;
-       g += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r0 = g << 2;
-    const uint32_t b = eval_pred4(P, r0, n, vec);
-    local += __popc(b);
-    if (mask_vec && r0 + 4 <= n) {
-      const uint32_t w = (b & 1u) | ((b & 2u) << 7) | ((b & 4u) << 14) | ((b & 8u) << 21);
-      *reinterpret_cast<uint32_t*>(mask + r0) = w;
-    } else {
-      for (int j = 0; j < 4 && r0 + j < n; ++j) mask[r0 + j] = (b >> j) & 1u;
+  for (int64_t t0 = blockIdx.x * (int64_t)(4 * Q * kBlock); t0 < n; t0 += (int64_t)gridDim.x * (4 * Q * kBlock)) {
+    int64_t r0[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) r0[q] = t0 + (q * kBlock + threadIdx.x) * 4;
+    const uint32_t bits = eval_pred_rows<Q>(P, r0, n, vec);
+    local += __popc(bits);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const uint32_t b = (bits >> (4 * q)) & 0xfu;
+      if (mask_vec && r0[q] + 4 <= n) {
+        const uint32_t w = (b & 1u) | ((b & 2u) << 7) | ((b & 4u) << 14) | ((b & 8u) << 21);
+        *reinterpret_cast<uint32_t*>(mask + r0[q]) = w;
+      } else {
+        for (int j = 0; j < 4 && r0[q] + j < n; ++j) mask[r0[q] + j] = (b >> j) & 1u;
+      }
     }
   }
   if (count) {
@@ -70,6 +80,10 @@ __global__ void __launch_bounds__(kBlock) k_filter_mask(const __grid_constant__ 
     if ((threadIdx.x & 31) == 0 && local) atomicAdd(count, (unsigned long long)local);
   }
 }
+
+// Sixteen rows a thread from here on (four CTAs of 4096 rows per SM), four below, where more warps matter
+// more than fewer instructions.
+constexpr int64_t kManyRows = int64_t(5) << 19;
 
 // Control block of one compaction (zeroed before the launch).
 struct CompactCtl {
@@ -171,43 +185,88 @@ __global__ void k_init_range(int64_t* out, unsigned long long* count) {
   if (threadIdx.x == 0) *count = 0;
 }
 
+// Min and max of 4 Q rows' keys where their bit is set, in the column's own width.
+template <class T, int Q>
+__device__ __forceinline__ void range_rows(const void* col, const int64_t (&r0)[Q], int64_t n, bool vec, uint32_t bits,
+                                           int64_t& mn, int64_t& mx) {
+  T x[4 * Q];
+  load_rows<T, Q>(col, r0, n, vec, x);
+  using W = std::conditional_t<sizeof(T) == 8, int64_t, int>;
+  constexpr W kMost = sizeof(T) == 8 ? (W)INT64_MAX : (W)INT32_MAX, kLeast = -kMost - 1;
+  W lo = kMost, hi = kLeast;
+#pragma unroll
+  for (int i = 0; i < 4 * Q; ++i) {
+    lo = min(lo, (bits >> i) & 1u ? (W)x[i] : kMost);
+    hi = max(hi, (bits >> i) & 1u ? (W)x[i] : kLeast);
+  }
+  mn = min(mn, (int64_t)lo);
+  mx = max(mx, (int64_t)hi);
+}
+
+// 4 Q rows per thread and step, each column's type decided once for them, and one update per CTA: four rows
+// at a time spent ~260 instructions on two one-byte keys, and an update per warp (9.7 K on the same words)
+// queued.
+template <int Q, bool PRED>
 __global__ void __launch_bounds__(kBlock) k_key_range(const __grid_constant__ tqpk_predicate P, RowFilter F, int64_t n,
                                                       KeySet K, int64_t* out, unsigned long long* count, int vec) {
+  __shared__ int64_t s_mn[TQPK_MAX_KEYS][kBlock / 32], s_mx[TQPK_MAX_KEYS][kBlock / 32];
+  __shared__ unsigned s_cnt[kBlock / 32];
   int64_t mn[TQPK_MAX_KEYS], mx[TQPK_MAX_KEYS];
 #pragma unroll
   for (int k = 0; k < TQPK_MAX_KEYS; ++k) { mn[k] = INT64_MAX; mx[k] = INT64_MIN; }
   unsigned cnt = 0;
-  const int64_t groups = (n + 3) >> 2;
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < groups;
-       g += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r0 = g << 2;
-    const uint32_t b = filter4(F, P, r0, n);
-    if (!b) continue;
-    cnt += __popc(b);
+  for (int64_t t0 = blockIdx.x * (int64_t)(4 * Q * kBlock); t0 < n; t0 += (int64_t)gridDim.x * (4 * Q * kBlock)) {
+    int64_t r0[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) r0[q] = t0 + (q * kBlock + threadIdx.x) * 4;
+    const uint32_t bits = filter_rows<Q, PRED>(F, P, r0, n);
+    if (!bits) continue;
+    cnt += __popc(bits);
 #pragma unroll
     for (int k = 0; k < TQPK_MAX_KEYS; ++k) {
       if (k >= K.n) break;
-      int64_t x[4];
-      ld4_int(K.col[k], K.dt[k], r0, n, vec, x);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if ((b >> j) & 1u) { mn[k] = min(mn[k], x[j]); mx[k] = max(mx[k], x[j]); }
+      switch (K.dt[k]) {
+        case TQPK_I64: range_rows<int64_t, Q>(K.col[k], r0, n, vec, bits, mn[k], mx[k]); break;
+        case TQPK_I32: range_rows<int32_t, Q>(K.col[k], r0, n, vec, bits, mn[k], mx[k]); break;
+        case TQPK_I8: range_rows<int8_t, Q>(K.col[k], r0, n, vec, bits, mn[k], mx[k]); break;
+        default: range_rows<uint8_t, Q>(K.col[k], r0, n, vec, bits, mn[k], mx[k]); break;
+      }
     }
   }
-  for (int k = 0; k < K.n; ++k) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < TQPK_MAX_KEYS; ++k) {
+    if (k >= K.n) break;
     int64_t a = mn[k], z = mx[k];
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
       a = min(a, (int64_t)__shfl_xor_sync(0xffffffffu, (long long)a, o));
       z = max(z, (int64_t)__shfl_xor_sync(0xffffffffu, (long long)z, o));
     }
-    if ((threadIdx.x & 31) == 0 && a <= z) {
+    if (lane == 0) {
+      s_mn[k][warp] = a;
+      s_mx[k][warp] = z;
+    }
+  }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane == 0) s_cnt[warp] = cnt;
+  __syncthreads();
+  if (warp) return;
+  for (int k = 0; k < K.n; ++k) {
+    int64_t a = lane < kBlock / 32 ? s_mn[k][lane] : INT64_MAX, z = lane < kBlock / 32 ? s_mx[k][lane] : INT64_MIN;
+#pragma unroll
+    for (int o = 4; o; o >>= 1) {
+      a = min(a, (int64_t)__shfl_xor_sync(0xffffffffu, (long long)a, o));
+      z = max(z, (int64_t)__shfl_xor_sync(0xffffffffu, (long long)z, o));
+    }
+    if (lane == 0 && a <= z) {
       atomicMin(reinterpret_cast<long long*>(&out[k]), (long long)a);
       atomicMax(reinterpret_cast<long long*>(&out[TQPK_MAX_KEYS + k]), (long long)z);
     }
   }
-  cnt = __reduce_add_sync(0xffffffffu, cnt);
-  if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(count, (unsigned long long)cnt);
+  unsigned c = lane < kBlock / 32 ? s_cnt[lane] : 0;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if (lane == 0 && c) atomicAdd(count, (unsigned long long)c);
 }
 
 // ---------------------------------------------------------------- host side
@@ -337,7 +396,11 @@ int key_ranges(const tqpk_predicate* pred, const uint8_t* mask, int64_t n, int n
   TQPK_CHECK_LAUNCH();
   if (n > 0) {
     RowFilter F = make_filter(pred, mask);
-    k_key_range<<<grid_for((n + 3) / 4, 4), kBlock, 0, s>>>(*pred_or_empty(pred), F, n, K, out, cnt, vec ? 1 : 0);
+    const bool many = n >= kManyRows;
+    auto kernel = F.use_pred ? (many ? k_key_range<4, true> : k_key_range<1, true>)
+                             : (many ? k_key_range<4, false> : k_key_range<1, false>);
+    kernel<<<grid_for((n + 3) / 4 / (many ? 4 : 1), 8), kBlock, 0, s>>>(*pred_or_empty(pred), F, n, K, out, cnt,
+                                                                        vec ? 1 : 0);
     TQPK_CHECK_LAUNCH();
   }
   int64_t host[2 * TQPK_MAX_KEYS + 1];
@@ -441,8 +504,13 @@ extern "C" int tqpk_filter_mask(const tqpk_predicate* h_pred, int64_t n, uint8_t
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int mask_vec = (reinterpret_cast<uintptr_t>(d_mask) & 3u) == 0;
   timing_before(KID_FILTER_MASK, s);
-  k_filter_mask<<<grid_for((n + 3) / 4, 8), kBlock, 0, s>>>(*h_pred, n, d_mask, d_count, pred_vec_ok(h_pred) ? 1 : 0,
-                                                          mask_vec);
+  // text programs keep every warp busy with their bytes: four rows a thread spread them over more warps
+  bool text = false;
+  for (int k = 0; k < h_pred->n_insn; ++k) text = text || h_pred->insn[k].op >= TQPK_P_STRCMP;
+  const bool many = n >= kManyRows && !text;
+  auto kernel = many ? k_filter_mask<4> : k_filter_mask<1>;
+  kernel<<<grid_for((n + 3) / 4 / (many ? 4 : 1), 8), kBlock, 0, s>>>(*h_pred, n, d_mask, d_count,
+                                                                      pred_vec_ok(h_pred) ? 1 : 0, mask_vec);
   timing_after(KID_FILTER_MASK, s);
   TQPK_CHECK_LAUNCH();
   return TQPK_OK;

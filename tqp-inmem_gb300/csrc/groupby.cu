@@ -230,6 +230,7 @@ __global__ void k_fill_u64(uint64_t* p, int64_t n, uint64_t v) {
 // 576 us for 0.9 M of 6 M rows), and by the plain loop: the unrolled form with operand selects costs
 // ~2500 instructions a row.  A claimed slot goes on the group list at once (pk, cslot; one counter update
 // per 256 rows), which saves the passes over the table that counted and collected the occupied slots.
+template <bool PRED>
 __global__ void __launch_bounds__(kBlock) k_groupby_hash(const __grid_constant__ tqpk_groupby_spec S,
                                                          const __grid_constant__ tqpk_predicate P, RowFilter F,
                                                          int64_t n, GbDev G, uint64_t* __restrict__ gacc,
@@ -244,12 +245,10 @@ __global__ void __launch_bounds__(kBlock) k_groupby_hash(const __grid_constant__
   const int64_t C = G.slots;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int64_t t0 = blockIdx.x * (int64_t)kTile; t0 < n; t0 += (int64_t)gridDim.x * kTile) {
-    uint32_t bits = 0;
+    int64_t r0[4];
 #pragma unroll
-    for (int q = 0; q < kItems / 4; ++q) {
-      const int64_t r0 = t0 + (q * kBlock + threadIdx.x) * 4;
-      if (r0 < n) bits |= filter4(F, P, r0, n) << (4 * q);
-    }
+    for (int q = 0; q < 4; ++q) r0[q] = t0 + (q * kBlock + threadIdx.x) * 4;
+    const uint32_t bits = filter_rows<4, PRED>(F, P, r0, n);
     int total;
     int at = block_excl_scan<kBlock, int>(__popc(bits), total, sw);
     for (uint32_t b = bits; b; b &= b - 1) {
@@ -656,8 +655,10 @@ extern "C" int tqpk_groupby_run(const tqpk_groupby_spec* S, const tqpk_gb_plan* 
     if (n > 0 && plan->n_rows > 0) {
       const GbDev G = to_dev(*plan, S->n_keys);
       timing_before(KID_GROUPBY, s);
-      k_groupby_hash<<<grid_for((n + kItems - 1) / kItems, 8), kBlock, 0, s>>>(
-          *S, *pred_or_empty(pred), make_filter(pred, mask), n, G, H.gacc, H.hkeys, H.pk, H.cslot, d_groups, C / 2, err);
+      const RowFilter F = make_filter(pred, mask);
+      auto kernel = F.use_pred ? k_groupby_hash<true> : k_groupby_hash<false>;
+      kernel<<<grid_for((n + kItems - 1) / kItems, 8), kBlock, 0, s>>>(
+          *S, *pred_or_empty(pred), F, n, G, H.gacc, H.hkeys, H.pk, H.cslot, d_groups, C / 2, err);
       timing_after(KID_GROUPBY, s);
       TQPK_CHECK_LAUNCH();
     }
