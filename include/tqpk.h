@@ -308,6 +308,20 @@ int tqpk_topk_stable(const void* d_keys, int32_t key_dtype, int32_t descending,
                      const int64_t* d_perm_in, int64_t n, int64_t k, int64_t* d_perm_out,
                      void* d_ws, size_t ws_bytes, tqpk_stream stream);
 
+/* The elements (d_cand[i], or i when d_cand is NULL) of n whose key equals that of
+ * d_top[m - 1], the last of the m (<= 256) entries tqpk_topk_stable gave for the
+ * same keys and elements: *h_ties counts them and *h_less the entries strictly
+ * before it (synchronises); tqpk_topk_ties_write, after it and with its workspace,
+ * lists them in input order.  With these a sort by several keys with a limit
+ * (sort.py:26-42) looks at the later keys of the tied rows only.             */
+size_t tqpk_topk_ties_workspace_bytes(int64_t n);
+int tqpk_topk_ties(const void* d_keys, int32_t key_dtype, int32_t descending, const int64_t* d_cand, int64_t n,
+                   const int64_t* d_top, int64_t m, int64_t* h_less, int64_t* h_ties, void* d_ws,
+                   size_t ws_bytes, tqpk_stream stream);
+int tqpk_topk_ties_write(const void* d_keys, int32_t key_dtype, int32_t descending, const int64_t* d_cand,
+                         int64_t n, const int64_t* d_top, int64_t m, int64_t* d_out, void* d_ws,
+                         size_t ws_bytes, tqpk_stream stream);
+
 /* ---- (c) join ---------------------------------------------------------- */
 enum { TQPK_JOIN_DIRECT = 1, TQPK_JOIN_SORTED = 2 };
 enum { TQPK_JOIN_UNKNOWN = 2 };

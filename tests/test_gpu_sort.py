@@ -97,3 +97,24 @@ def test_too_many_words_raise():
     wide = torch.zeros((3000, 8 * 33), dtype=torch.int8, device="cuda")
     with pytest.raises(NotImplementedError):
         argsort_keys([wide], [False])
+
+
+@pytest.mark.parametrize("n", [1, 300, 4096, 4097, 98_305, 300_001])
+@pytest.mark.parametrize("limit", [1, 10, 255, 256])
+def test_topk_by_several_keys(n, limit):
+    """Few ties, ties at the cut, a first key that ties everywhere, text keys, NaN and both zeros."""
+    from tqpk.ops import topk_keys
+    rng = np.random.default_rng(n + limit)
+    price = rng.integers(90000, 10495001, n) / 100.0
+    coarse = rng.integers(0, 4, n) * 0.5
+    coarse[: min(n, 3)] = [-0.0, np.nan, 0.0][: min(n, 3)]
+    text = np.zeros((n, 11), np.int8)
+    text[:, 4] = rng.integers(0, 3, n)
+    text[:, 10] = rng.integers(-2, 2, n)
+    ids = rng.permutation(n).astype(np.int64)
+    same = np.full(n, 3, np.int32)
+    for keys, descs in (([price, ids], [True, False]), ([coarse, same, price], [False, True, True]),
+                        ([same, coarse, text], [True, True, False]), ([text, coarse], [True, False]),
+                        ([same, coarse], [False, False])):
+        got = topk_keys([torch.from_numpy(k).cuda() for k in keys], descs, limit)
+        np.testing.assert_array_equal(got.cpu().numpy(), _expected(keys, descs)[:limit])

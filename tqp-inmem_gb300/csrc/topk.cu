@@ -82,9 +82,140 @@ __global__ void k_topk_positions_to_perm(const int64_t* idx, const int64_t* coun
   }
 }
 
+// Elements (cand[i], or i) whose key ties with the m-th of a top-k's entries, counted per 4096-element tile
+// and then (WRITE) listed in input order; also how many of the entries come strictly before it.  A row of
+// several keys is in the first k only if it is in the first k by the first key or ties with the k-th, so a
+// sort with a limit looks at the later keys of these rows only.  Bound: one read of the key column.
+struct TieCtl {
+  unsigned done;
+  int pad;
+  int64_t less, ties;
+};
+
+template <bool WRITE>
+__global__ void __launch_bounds__(kBlock) k_topk_ties(const void* __restrict__ keys, int dt, int desc,
+                                                      const int64_t* __restrict__ cand, int64_t n,
+                                                      const int64_t* __restrict__ top, int m, TieCtl* ctl,
+                                                      int64_t* __restrict__ tile_base, int64_t* __restrict__ out) {
+  __shared__ int64_t sw[kBlock / 32 + 1];
+  __shared__ int s_cnt[kItems * (kBlock / 32)];      // ties of (step, warp), then their exclusive scan
+  __shared__ uint64_t s_cut;
+  __shared__ int s_last;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_cut = sort_key(keys, dt, top[m - 1], desc);
+  __syncthreads();
+  const uint64_t cut = s_cut;
+  const int64_t t0 = blockIdx.x * (int64_t)kTile;
+  uint64_t k[kItems];
+#pragma unroll
+  for (int j = 0; j < kItems; ++j) {
+    const int64_t i = t0 + j * kBlock + threadIdx.x;
+    k[j] = i < n ? sort_key(keys, dt, cand ? cand[i] : i, desc) : 0;
+  }
+  uint32_t hits = 0;
+#pragma unroll
+  for (int j = 0; j < kItems; ++j)
+    hits |= (uint32_t)(t0 + j * kBlock + threadIdx.x < n && k[j] == cut) << j;
+  if (!WRITE) {
+    int64_t total;
+    block_excl_scan<kBlock, int64_t>(__popc(hits), total, sw);
+    if (threadIdx.x == 0) {
+      tile_base[blockIdx.x] = total;
+      __threadfence();
+      s_last = atomicAdd(&ctl->done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    int64_t run = 0;
+    for (int64_t b = 0; b < (int64_t)gridDim.x; b += kBlock) {
+      const int64_t t = b + threadIdx.x;
+      const int64_t c = t < (int64_t)gridDim.x ? __ldcg(reinterpret_cast<const long long*>(&tile_base[t])) : 0;
+      int64_t all;
+      const int64_t at = block_excl_scan<kBlock, int64_t>(c, all, sw);
+      if (t < (int64_t)gridDim.x) tile_base[t] = run + at;
+      run += all;
+    }
+    int64_t before = 0, all;
+    for (int e = threadIdx.x; e < m; e += kBlock) before += sort_key(keys, dt, top[e], desc) < cut;
+    block_excl_scan<kBlock, int64_t>(before, all, sw);
+    if (threadIdx.x == 0) {
+      ctl->ties = run;
+      ctl->less = all;
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < kItems; ++j) {
+    const unsigned b = __ballot_sync(0xffffffffu, (hits >> j) & 1u);
+    if (lane == 0) s_cnt[j * (kBlock / 32) + warp] = __popc(b);
+  }
+  __syncthreads();
+  int mine = threadIdx.x < kItems * (kBlock / 32) ? s_cnt[threadIdx.x] : 0, total;
+  __shared__ int si[kBlock / 32 + 1];
+  mine = block_excl_scan<kBlock, int>(mine, total, si);
+  if (threadIdx.x < kItems * (kBlock / 32)) s_cnt[threadIdx.x] = mine;
+  __syncthreads();
+  const int64_t base = tile_base[blockIdx.x];
+#pragma unroll
+  for (int j = 0; j < kItems; ++j) {
+    const unsigned b = __ballot_sync(0xffffffffu, (hits >> j) & 1u);
+    if ((hits >> j) & 1u) {
+      const int64_t i = t0 + j * kBlock + threadIdx.x;
+      out[base + s_cnt[j * (kBlock / 32) + warp] + __popc(b & ((1u << lane) - 1u))] = cand ? cand[i] : i;
+    }
+  }
+}
+
 }  // namespace tqpk
 
 using namespace tqpk;
+
+static int topk_ties(bool write, const void* keys, int32_t dt, int32_t desc, const int64_t* cand, int64_t n,
+                     const int64_t* top, int64_t m, int64_t* out, int64_t* h_less, int64_t* h_ties, void* ws,
+                     size_t ws_bytes, tqpk_stream stream) {
+  if (n < 1 || m < 1 || m > 256 || m > n || !keys || !top || !ws) return TQPK_EINVAL;
+  if (!dtype_size(dt)) return TQPK_EDTYPE;
+  const int64_t tiles = (n + kTile - 1) / kTile;
+  if (tiles > INT32_MAX) return TQPK_EUNSUPPORTED;
+  WsCursor cur(ws, ws_bytes);
+  TieCtl* ctl = cur.take<TieCtl>(1);
+  int64_t* base = cur.take<int64_t>(tiles);
+  if (!ctl || !base) return TQPK_ENOMEM;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (write) {
+    k_topk_ties<true><<<(int)tiles, kBlock, 0, s>>>(keys, dt, desc ? 1 : 0, cand, n, top, (int)m, ctl, base, out);
+    TQPK_CHECK_LAUNCH();
+    return TQPK_OK;
+  }
+  TQPK_CUDA(cudaMemsetAsync(ctl, 0, sizeof(TieCtl), s));
+  k_topk_ties<false><<<(int)tiles, kBlock, 0, s>>>(keys, dt, desc ? 1 : 0, cand, n, top, (int)m, ctl, base, nullptr);
+  TQPK_CHECK_LAUNCH();
+  TieCtl h;
+  TQPK_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s));
+  TQPK_CUDA(cudaStreamSynchronize(s));
+  *h_less = h.less;
+  *h_ties = h.ties;
+  return TQPK_OK;
+}
+
+extern "C" size_t tqpk_topk_ties_workspace_bytes(int64_t n) {
+  return 512 + align_up((size_t)((std::max<int64_t>(n, 0) + kTile - 1) / kTile) * 8, 256);
+}
+
+extern "C" int tqpk_topk_ties(const void* d_keys, int32_t dt, int32_t desc, const int64_t* d_cand, int64_t n,
+                              const int64_t* d_top, int64_t m, int64_t* h_less, int64_t* h_ties, void* ws,
+                              size_t ws_bytes, tqpk_stream stream) {
+  if (!h_less || !h_ties) return TQPK_EINVAL;
+  return topk_ties(false, d_keys, dt, desc, d_cand, n, d_top, m, nullptr, h_less, h_ties, ws, ws_bytes, stream);
+}
+
+extern "C" int tqpk_topk_ties_write(const void* d_keys, int32_t dt, int32_t desc, const int64_t* d_cand, int64_t n,
+                                    const int64_t* d_top, int64_t m, int64_t* d_out, void* ws, size_t ws_bytes,
+                                    tqpk_stream stream) {
+  if (!d_out) return TQPK_EINVAL;
+  return topk_ties(true, d_keys, dt, desc, d_cand, n, d_top, m, d_out, nullptr, nullptr, ws, ws_bytes, stream);
+}
 
 // Test hook: the poll limit of the single-launch top-k's grid barrier, and arrivals it also waits
 // for that never come (its bounded wait then runs out: TQPK_ETIMEOUT in the caller's error word).

@@ -18,6 +18,8 @@ OK, EINVAL, ENOMEM, ETIMEOUT, EDTYPE, ECUDA, ECAPACITY, EUNSUPPORTED = 0, -1, -2
 ROWID, I8, U8, I32, I64, F64, BOOL = 0, 1, 2, 3, 4, 5, 6
 MAX_COLS, MAX_PRED, MAX_KEYS, MAX_EXPR, MAX_ACCS = 16, 32, 4, 32, 16
 MAX_SORT_WORDS = 32
+CLUSTER_SORT_ROWS = 98304                # rows one cluster sorts in a single launch
+TOPK_MAX = 256                           # limits the threshold top-k takes
 NULL_INDEX = -64
 
 P_CMP, P_AND, P_OR, P_NOT, P_TRUE, P_FALSE, P_MASK, P_CMPCOL = 1, 2, 3, 4, 5, 6, 7, 8
@@ -99,6 +101,9 @@ SIGNATURES = {
     "tqpk_argsort_keys": (C.c_int, [_I32, _P(_VP), _P(_I32), _P(_I32), _P(_I32), _VP, _I64, _VP, _VP, _SZ, _VP]),
     "tqpk_topk_workspace_bytes": (_SZ, [_I64, _I64]),
     "tqpk_topk_stable": (C.c_int, [_VP, _I32, _I32, _VP, _I64, _I64, _VP, _VP, _SZ, _VP]),
+    "tqpk_topk_ties_workspace_bytes": (_SZ, [_I64]),
+    "tqpk_topk_ties": (C.c_int, [_VP, _I32, _I32, _VP, _I64, _VP, _I64, _P(_I64), _P(_I64), _VP, _SZ, _VP]),
+    "tqpk_topk_ties_write": (C.c_int, [_VP, _I32, _I32, _VP, _I64, _VP, _I64, _VP, _VP, _SZ, _VP]),
     "tqpk_join_plan_build": (C.c_int, [_VP, _I32, _VP, _I64, _P(JoinPlan), _VP, _VP]),
     "tqpk_join_build": (C.c_int, [_P(JoinPlan), _VP, _I32, _VP, _I64, _VP, _SZ, _VP]),
     "tqpk_join_directory": (C.c_int, [_P(JoinPlan), _VP, _I32, _VP, _I64, _VP, _SZ, _VP]),

@@ -3,8 +3,9 @@
 The reference runs one stable torch.sort per key, last key first, each time
 gathering the key through ``perm`` (:26-35), then slices ``perm[:limit]``
 (:41-42) and gathers every input column (:44-54).  Here that loop is one
-tqpk_argsort_keys call; with a limit the first key uses the stable top-k, which
-returns the same rows as the full sort followed by the slice.  A [N, w] key (the
+tqpk_argsort_keys call; with a limit the stable top-k of the first key, and of
+the rows tied at its end by the next keys, returns the same rows as the full sort
+followed by the slice.  A [N, w] key (the
 reference ranks its rows with unique(dim=0)) is sorted by its 8-byte words,
 which gives the same lexicographic order and ties; keys of more words than one
 call takes are sorted key by key (tqpk_argsort_stable), last word of the last
@@ -17,8 +18,9 @@ from __future__ import annotations
 
 import torch
 
-from .._lib import MAX_SORT_WORDS
-from ..ops import argsort_keys, argsort_stable, check_deferred, gather, gather_rows, sort_words, string_words, topk_stable
+from .._lib import CLUSTER_SORT_ROWS, MAX_SORT_WORDS, TOPK_MAX
+from ..ops import (argsort_keys, argsort_stable, check_deferred, gather, gather_rows, sort_words, string_words, topk_keys,
+                   topk_stable)
 from ..variable import make_like, wait_ready
 from .filter import _require_gpu
 
@@ -56,9 +58,17 @@ def tqp_sort(gpu_enable, tensor_group, args, with_limit, name="sort"):
     if len(cols) == len(key_descs) and all(
             c.is_cuda and (c.dim() == 1 or c.shape[1] == 1 or
                            (c.shape[1] > 1 and c.dtype in (torch.int8, torch.uint8))) for c in cols):
-        # one call for every key, or for all but the first when a limit ends the sort in a top-k
-        many = list(zip(cols, key_descs))[1 if limit is not None else 0:]
-        if many and sort_words([c for c, _ in many]) <= MAX_SORT_WORDS and (limit is None or not _is_text(cols[0])):
+        many = list(zip(cols, key_descs))
+        few = sort_words(cols) <= MAX_SORT_WORDS
+        if (limit is not None and 0 < limit <= TOPK_MAX and few and sort_words(cols) > 1
+                and cols[0].shape[0] > CLUSTER_SORT_ROWS):
+            # the top-k key by key: 6 M rows by a price and a tie-breaking id took 560 us of sorting the
+            # ids first.  A table that one cluster sorts in a launch (~30-60 us) is sorted.
+            perm = topk_keys(cols, key_descs, limit)
+            many, key_ids = [], []
+        elif limit is not None:              # all keys but the first, which ends the sort in a top-k
+            many = many[1:] if not _is_text(cols[0]) else []
+        if many and few:
             perm = argsort_keys([c for c, _ in many], [d for _, d in many])
             key_ids, key_descs = key_ids[:len(key_ids) - len(many)], key_descs[:len(key_descs) - len(many)]
     for key_id, desc in zip(reversed(key_ids), reversed(key_descs)):

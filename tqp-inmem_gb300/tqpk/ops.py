@@ -364,6 +364,46 @@ def topk_stable(keys: torch.Tensor, k: int, descending: bool = False,
     return out
 
 
+def topk_keys(cols: Sequence[torch.Tensor], descs: Sequence[bool], k: int) -> torch.Tensor:
+    """The first k (<= L.TOPK_MAX) rows of the stable order by cols[0], then cols[1], ...: the top-k by
+    the first key, and only where more rows tie with its k-th than it took, the top-k of the tied rows
+    by the next key."""
+    lib = L.load()
+    n = int(cols[0].shape[0])
+    device = cols[0].device
+    need = min(int(k), n)
+    if need <= 0:
+        return torch.empty(0, dtype=torch.int64, device=device)
+    levels = [(c, w, d) for c, d in zip(cols, descs)
+              for w in range((c.shape[1] + 7) // 8 if c.dim() == 2 and c.shape[1] > 1 else 1)]
+    picked, cand = [], None
+    for i, (col, word, desc) in enumerate(levels):
+        key = string_words(col, word) if col.dim() == 2 and col.shape[1] > 1 else _col1d(col)
+        top = topk_stable(key, need, desc, cand)
+        if i + 1 == len(levels):
+            picked.append(top)
+            break
+        m = n if cand is None else int(cand.numel())
+        ws = _ws(lib.tqpk_topk_ties_workspace_bytes(m), device)
+        args = (key.data_ptr(), code_of(key.dtype), int(bool(desc)), cand.data_ptr() if cand is not None else None, m,
+                top.data_ptr(), need)
+        less, ties = C.c_int64(0), C.c_int64(0)
+        L.check(lib.tqpk_topk_ties(*args, C.byref(less), C.byref(ties), ws.data_ptr(), ws.numel(), _stream(device)),
+                "tqpk_topk_ties")
+        if ties.value == need - less.value:          # every row tied with the last one is in
+            picked.append(top)
+            break
+        if less.value:
+            picked.append(top[:less.value])
+        rows = torch.empty(ties.value, dtype=torch.int64, device=device)
+        L.check(lib.tqpk_topk_ties_write(*args, rows.data_ptr(), ws.data_ptr(), ws.numel(), _stream(device)),
+                "tqpk_topk_ties_write")
+        need -= less.value
+        cand = rows
+    # rows equal in every key were picked together, in row order
+    return argsort_keys(cols, descs, picked[0] if len(picked) == 1 else torch.cat(picked))
+
+
 # ---------------------------------------------------------------- (c) join
 JOIN_TYPES = {"inner": L.JT_INNER, "right-semi": L.JT_SEMI, "right-anti": L.JT_ANTI, "right-outer": L.JT_OUTER}
 
