@@ -87,24 +87,18 @@ __global__ void k_topk_positions_to_perm(const int64_t* idx, const int64_t* coun
 // several keys is in the first k only if it is in the first k by the first key or ties with the k-th, so a
 // sort with a limit looks at the later keys of these rows only.  Bound: one read of the key column.
 struct TieCtl {
-  unsigned done;
-  int pad;
-  int64_t less, ties;
+  unsigned long long less, ties;
 };
 
 template <bool WRITE>
 __global__ void __launch_bounds__(kBlock) k_topk_ties(const void* __restrict__ keys, int dt, int desc,
                                                       const int64_t* __restrict__ cand, int64_t n,
                                                       const int64_t* __restrict__ top, int m, TieCtl* ctl,
-                                                      int64_t* __restrict__ tile_base, int64_t* __restrict__ out) {
-  __shared__ int64_t sw[kBlock / 32 + 1];
+                                                      int* __restrict__ tile_ties, int64_t* __restrict__ out) {
   __shared__ int s_cnt[kItems * (kBlock / 32)];      // ties of (step, warp), then their exclusive scan
-  __shared__ uint64_t s_cut;
-  __shared__ int s_last;
+  __shared__ int si[kBlock / 32 + 1];
+  __shared__ int64_t sw[kBlock / 32 + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) s_cut = sort_key(keys, dt, top[m - 1], desc);
-  __syncthreads();
-  const uint64_t cut = s_cut;
   const int64_t t0 = blockIdx.x * (int64_t)kTile;
   uint64_t k[kItems];
 #pragma unroll
@@ -112,51 +106,36 @@ __global__ void __launch_bounds__(kBlock) k_topk_ties(const void* __restrict__ k
     const int64_t i = t0 + j * kBlock + threadIdx.x;
     k[j] = i < n ? sort_key(keys, dt, cand ? cand[i] : i, desc) : 0;
   }
+  const uint64_t cut = sort_key(keys, dt, top[m - 1], desc);
   uint32_t hits = 0;
 #pragma unroll
   for (int j = 0; j < kItems; ++j)
     hits |= (uint32_t)(t0 + j * kBlock + threadIdx.x < n && k[j] == cut) << j;
   if (!WRITE) {
-    int64_t total;
-    block_excl_scan<kBlock, int64_t>(__popc(hits), total, sw);
+    int total;
+    block_excl_scan<kBlock, int>(__popc(hits), total, si);
     if (threadIdx.x == 0) {
-      tile_base[blockIdx.x] = total;
-      __threadfence();
-      s_last = atomicAdd(&ctl->done, 1u) == gridDim.x - 1;
+      tile_ties[blockIdx.x] = total;
+      if (total) atomicAdd(&ctl->ties, (unsigned long long)total);
     }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    int64_t run = 0;
-    for (int64_t b = 0; b < (int64_t)gridDim.x; b += kBlock) {
-      const int64_t t = b + threadIdx.x;
-      const int64_t c = t < (int64_t)gridDim.x ? __ldcg(reinterpret_cast<const long long*>(&tile_base[t])) : 0;
-      int64_t all;
-      const int64_t at = block_excl_scan<kBlock, int64_t>(c, all, sw);
-      if (t < (int64_t)gridDim.x) tile_base[t] = run + at;
-      run += all;
-    }
-    int64_t before = 0, all;
-    for (int e = threadIdx.x; e < m; e += kBlock) before += sort_key(keys, dt, top[e], desc) < cut;
-    block_excl_scan<kBlock, int64_t>(before, all, sw);
-    if (threadIdx.x == 0) {
-      ctl->ties = run;
-      ctl->less = all;
-    }
+    if (blockIdx.x == 0)
+      for (int e = threadIdx.x; e < m; e += kBlock)
+        if (sort_key(keys, dt, top[e], desc) < cut) atomicAdd(&ctl->less, 1ull);
     return;
   }
+  int64_t before = 0, base;                          // the ties of the tiles before this one
+  for (int t = threadIdx.x; t < (int)blockIdx.x; t += kBlock) before += tile_ties[t];
+  block_excl_scan<kBlock, int64_t>(before, base, sw);
 #pragma unroll
   for (int j = 0; j < kItems; ++j) {
     const unsigned b = __ballot_sync(0xffffffffu, (hits >> j) & 1u);
     if (lane == 0) s_cnt[j * (kBlock / 32) + warp] = __popc(b);
   }
   __syncthreads();
-  int mine = threadIdx.x < kItems * (kBlock / 32) ? s_cnt[threadIdx.x] : 0, total;
-  __shared__ int si[kBlock / 32 + 1];
+  int total, mine = threadIdx.x < kItems * (kBlock / 32) ? s_cnt[threadIdx.x] : 0;
   mine = block_excl_scan<kBlock, int>(mine, total, si);
   if (threadIdx.x < kItems * (kBlock / 32)) s_cnt[threadIdx.x] = mine;
   __syncthreads();
-  const int64_t base = tile_base[blockIdx.x];
 #pragma unroll
   for (int j = 0; j < kItems; ++j) {
     const unsigned b = __ballot_sync(0xffffffffu, (hits >> j) & 1u);
@@ -180,7 +159,7 @@ static int topk_ties(bool write, const void* keys, int32_t dt, int32_t desc, con
   if (tiles > INT32_MAX) return TQPK_EUNSUPPORTED;
   WsCursor cur(ws, ws_bytes);
   TieCtl* ctl = cur.take<TieCtl>(1);
-  int64_t* base = cur.take<int64_t>(tiles);
+  int* base = cur.take<int>(tiles);
   if (!ctl || !base) return TQPK_ENOMEM;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (write) {
@@ -194,13 +173,13 @@ static int topk_ties(bool write, const void* keys, int32_t dt, int32_t desc, con
   TieCtl h;
   TQPK_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s));
   TQPK_CUDA(cudaStreamSynchronize(s));
-  *h_less = h.less;
-  *h_ties = h.ties;
+  *h_less = (int64_t)h.less;
+  *h_ties = (int64_t)h.ties;
   return TQPK_OK;
 }
 
 extern "C" size_t tqpk_topk_ties_workspace_bytes(int64_t n) {
-  return 512 + align_up((size_t)((std::max<int64_t>(n, 0) + kTile - 1) / kTile) * 8, 256);
+  return 512 + align_up((size_t)((std::max<int64_t>(n, 0) + kTile - 1) / kTile) * 4, 256);
 }
 
 extern "C" int tqpk_topk_ties(const void* d_keys, int32_t dt, int32_t desc, const int64_t* d_cand, int64_t n,

@@ -175,7 +175,29 @@ struct ArraySource {
   int desc;
   __device__ __forceinline__ bool get(int64_t i, uint64_t& k) const;
   __device__ __forceinline__ unsigned bits4(int64_t) const { return 0xfu; }
+  // Four items: of an 8- or 4-byte column in its own order as 16-byte loads (one item at a time, each
+  // behind the type's switch, a pass over 6 M float64 took 35 us, 5x its bytes' time).
   __device__ __forceinline__ unsigned get4(int64_t i0, uint64_t* k) const {
+    if (!perm && i0 + 4 <= n && (reinterpret_cast<uintptr_t>(keys) & 15u) == 0) {
+      if (dt == TQPK_F64 || dt == TQPK_I64) {
+        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(static_cast<const uint64_t*>(keys) + i0);
+        const ulonglong2 a = p[0], b = p[1];
+        const int f = dt == TQPK_F64;
+        k[0] = sort_key_bits(a.x, f, desc);
+        k[1] = sort_key_bits(a.y, f, desc);
+        k[2] = sort_key_bits(b.x, f, desc);
+        k[3] = sort_key_bits(b.y, f, desc);
+        return 0xfu;
+      }
+      if (dt == TQPK_I32) {
+        const int4 a = *reinterpret_cast<const int4*>(static_cast<const int32_t*>(keys) + i0);
+        k[0] = sort_key_bits((uint64_t)(int64_t)a.x, 0, desc);
+        k[1] = sort_key_bits((uint64_t)(int64_t)a.y, 0, desc);
+        k[2] = sort_key_bits((uint64_t)(int64_t)a.z, 0, desc);
+        k[3] = sort_key_bits((uint64_t)(int64_t)a.w, 0, desc);
+        return 0xfu;
+      }
+    }
     unsigned ok = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) ok |= (get(i0 + q, k[q]) ? 1u : 0u) << q;
