@@ -322,12 +322,6 @@ __global__ void k_count_groups(const uint64_t* cnt, int64_t K, unsigned long lon
   if ((threadIdx.x & 31) == 0 && local) atomicAdd(groups, (unsigned long long)local);
 }
 
-__global__ void k_count_one(unsigned long long* groups) { *groups = 1; }
-
-__global__ void k_groups_or_error(const int* err, const unsigned long long* groups, int64_t* out) {
-  *out = *err ? (int64_t)*err : (int64_t)*groups;
-}
-
 struct EmitOut {
   int n;
   int op[TQPK_MAX_ACCS];
@@ -349,74 +343,148 @@ __device__ __forceinline__ void store_as(void* col, int dt, int64_t i, uint64_t 
   }
 }
 
-// Ordered emission of the occupied slots (ascending slot = ascending key tuple).
+// Control words of one emission (zeroed before the launch).
+struct EmitCtl {
+  int tile_ctr;          // next tile to take
+  int err;               // first error status of any CTA
+  int finished;          // CTAs done
+  int pad;
+  int64_t groups;        // written by the CTA of the last tile
+};
+
+// Output column c of the group in slot s.
+__device__ __forceinline__ void emit_value(const tqpk_groupby_spec& S, const GbDev& G, const EmitOut& E,
+                                           const uint64_t* __restrict__ gacc, int64_t s, int64_t pos, int c) {
+  const int64_t K = G.slots;
+  if (c < G.nk) {
+    const int64_t q = K < (int64_t(1) << 31)         // slot indices fit 32 bits: 32-bit key decoding
+                          ? (int64_t)(((uint32_t)s / (uint32_t)G.kstride[c]) % (uint32_t)G.krange[c])
+                          : (s / G.kstride[c]) % G.krange[c];
+    store_as(E.key[c], E.key_dt[c], pos, (uint64_t)(G.kmin[c] + q), false);
+    return;
+  }
+  const int o = c - G.nk;
+  const tqpk_acc& a = S.accs[E.a[o]];
+  uint64_t v = gacc[(int64_t)E.a[o] * K + s];
+  bool f = a.type == TQPK_F64 && a.kind != TQPK_ACC_COUNT_ROWS && a.kind != TQPK_ACC_COUNT_NOTNULL;
+  if (f && (a.kind == TQPK_ACC_MIN || a.kind == TQPK_ACC_MAX)) v = d2u(f64_from_ordered(v));
+  if (E.op[o] == TQPK_OUT_AVG) {
+    const double num = f ? u2d(v) : (double)(int64_t)v;
+    const double den = (double)(int64_t)gacc[(int64_t)E.b[o] * K + s];
+    v = d2u(__ddiv_rn(num, den));
+    f = true;
+  } else if (a.kind == TQPK_ACC_COUNT_ROWS || a.kind == TQPK_ACC_COUNT_NOTNULL) {
+    f = false;
+  }
+  store_as(E.col[o], E.dt[o], pos, v, f);
+}
+
+// Ordered emission of the occupied slots (ascending slot = ascending key tuple), ITEMS slots per thread.
+// A warp reads 32 consecutive slots at a time and ranks them by ballots; the tile's groups are then written
+// column by column, consecutive threads to consecutive rows.  Tiles with fewer groups than that fills give
+// every (group, column) pair its own thread instead: a group's outputs (an average is an FP64 division, a
+// key a division of the slot index) are independent, and one thread per group made a few groups a serial
+// chain.  The last tile's prefix is the group count, so no pass over the table counts it.
+// 6 M slots, 1.5 M groups, three columns: 56 us (70, and 14 for the count, with 16 consecutive slots per
+// thread).
+template <int ITEMS>
 __global__ void __launch_bounds__(kBlock) k_emit_dense(const __grid_constant__ tqpk_groupby_spec S, GbDev G,
                                                        const uint64_t* __restrict__ gacc, int force_one,
                                                        const __grid_constant__ EmitOut E, uint64_t* status,
-                                                       int* tile_ctr, int* err) {
+                                                       EmitCtl* ctl, int64_t* groups_out) {
+  constexpr int kSlots = kBlock * ITEMS;
+  constexpr int kWarpSlots = 32 * ITEMS;
   __shared__ int s_tile;
   __shared__ uint64_t s_excl;
-  __shared__ int sw[kBlock / 32 + 1];
-  if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1);
+  __shared__ int s_warp[kBlock / 32];
+  __shared__ uint16_t e_off[kSlots];                 // slot offset in the tile of its r-th group
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_tile = atomicAdd(&ctl->tile_ctr, 1);
   __syncthreads();
   const int64_t tile = s_tile;
   const int64_t K = G.slots;
-  const int64_t s0 = tile * kTile + threadIdx.x * kItems;
-  uint32_t bits = 0;
-  for (int j = 0; j < kItems; ++j) {
-    const int64_t s = s0 + j;
-    if (s < K && (gacc[s] != 0 || force_one)) bits |= 1u << j;
+  const int64_t w0 = tile * kSlots + warp * kWarpSlots;
+  uint32_t occ[ITEMS];
+  {
+    uint64_t c[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const int64_t s = w0 + j * 32 + lane;
+      c[j] = s < K ? (force_one ? 1 : gacc[s]) : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) occ[j] = __ballot_sync(0xffffffffu, c[j] != 0);
   }
-  int total;
-  const int excl = block_excl_scan<kBlock, int>(__popc(bits), total, sw);
+  int mine = 0;
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) mine += __popc(occ[j]);
+  if (lane == 0) s_warp[warp] = mine;
+  __syncthreads();
+  int total = 0, r = 0;
+#pragma unroll
+  for (int w = 0; w < kBlock / 32; ++w) {
+    if (w == warp) r = total;
+    total += s_warp[w];
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    if ((occ[j] >> lane) & 1u)
+      e_off[r + __popc(occ[j] & ((1u << lane) - 1u))] = (uint16_t)(warp * kWarpSlots + j * 32 + lane);
+    r += __popc(occ[j]);
+  }
   if (threadIdx.x < 32) {
-    uint64_t e = lookback_warp(status, tile, (uint64_t)total, err);
+    uint64_t e = lookback_warp(status, tile, (uint64_t)total, &ctl->err);
     if (threadIdx.x == 0) s_excl = e;
   }
-  // The tile's groups in output order (entry r: the slot offset in the tile; its output row is
-  // s_excl + r), then every (group, column) pair on its own thread.  A group's outputs (an average is an FP64
-  // division, a key a division of the slot index) are independent, and on this part FP64 runs at
-  // 1/64 rate: one thread per group made a few groups a long serial chain (6 groups, 8 outputs:
-  // 25 us for one CTA).
-  __shared__ uint16_t e_off[kTile];
-  {
-    int r = excl;
-    uint32_t b = bits;
-    while (b) {
-      const int j = __ffs(b) - 1;
-      b &= b - 1;
-      e_off[r++] = (uint16_t)(threadIdx.x * kItems + j);
-    }
-  }
   __syncthreads();
-  const int per = G.nk + E.n;                       // columns written per group
-  const bool small = K < (int64_t(1) << 31);       // slot indices fit 32 bits: 32-bit key decoding
-  for (int w = threadIdx.x; w < total * per; w += kBlock) {
-    const int r = w / per, c = w - r * per;
-    const int64_t s = tile * kTile + e_off[r];
-    const int64_t pos = (int64_t)s_excl + r;
-    if (c < G.nk) {
-      const int k = c;
-      const int64_t q = small ? (int64_t)(((uint32_t)s / (uint32_t)G.kstride[k]) % (uint32_t)G.krange[k])
-                              : (s / G.kstride[k]) % G.krange[k];
-      store_as(E.key[k], E.key_dt[k], pos, (uint64_t)(G.kmin[k] + q), false);
-      continue;
+  const int per = G.nk + E.n;                        // columns written per group
+  const int64_t first = (int64_t)s_excl;
+  if (total >= kBlock / 2) {
+    for (int c = 0; c < per; ++c)
+      for (int g = threadIdx.x; g < total; g += kBlock)
+        emit_value(S, G, E, gacc, tile * kSlots + e_off[g], first + g, c);
+  } else {
+    for (int w = threadIdx.x; w < total * per; w += kBlock) {
+      const int g = w / per;
+      emit_value(S, G, E, gacc, tile * kSlots + e_off[g], first + g, w - g * per);
     }
-    const int o = c - G.nk;
-    const tqpk_acc& a = S.accs[E.a[o]];
-    uint64_t v = gacc[(int64_t)E.a[o] * K + s];
-    bool f = a.type == TQPK_F64 && a.kind != TQPK_ACC_COUNT_ROWS && a.kind != TQPK_ACC_COUNT_NOTNULL;
-    if (f && (a.kind == TQPK_ACC_MIN || a.kind == TQPK_ACC_MAX)) v = d2u(f64_from_ordered(v));
-    if (E.op[o] == TQPK_OUT_AVG) {
-      const double num = f ? u2d(v) : (double)(int64_t)v;
-      const double den = (double)(int64_t)gacc[(int64_t)E.b[o] * K + s];
-      v = d2u(__ddiv_rn(num, den));
-      f = true;
-    } else if (a.kind == TQPK_ACC_COUNT_ROWS || a.kind == TQPK_ACC_COUNT_NOTNULL) {
-      f = false;
-    }
-    store_as(E.col[o], E.dt[o], pos, v, f);
   }
+  if (tile == (int64_t)gridDim.x - 1 && threadIdx.x == 0) ctl->groups = first + total;
+  // the last CTA to finish writes the group count, or the error of a look-back that gave up
+  if (!groups_out) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&ctl->finished, 1) == (int)gridDim.x - 1) {
+      __threadfence();
+      const int e = *reinterpret_cast<volatile int*>(&ctl->err);
+      *groups_out = e ? (int64_t)e : *reinterpret_cast<volatile int64_t*>(&ctl->groups);
+    }
+  }
+}
+
+// Look-back tiles: 4096 slots for tables that fill the GPU with them, 512 for smaller ones (27 K slots were
+// seven CTAs, 51 us).  A tile's life is ~12 us of counter, loads and look-back plus ~1 us per slot a thread
+// holds: 6 M slots take 57 us in tiles of 4096, 75 in 2048, 115 in 1024.
+constexpr int64_t kBigTable = int64_t(1) << 21;
+constexpr int kEmitItems = 16;
+static int64_t emit_tiles(int64_t K) {
+  const int64_t t = (K >= kBigTable ? kEmitItems : 2) * kBlock;
+  return (K + t - 1) / t;
+}
+static size_t emit_ws_bytes(int64_t K) { return 256 + align_up((size_t)emit_tiles(K) * 8, 256); }
+
+static int launch_emit(const tqpk_groupby_spec& S, const GbDev& G, const uint64_t* gacc, const EmitOut& E, void* ws,
+                       int64_t* groups_out, EmitCtl** ctl_out, cudaStream_t s) {
+  EmitCtl* ctl = static_cast<EmitCtl*>(ws);
+  uint64_t* status = reinterpret_cast<uint64_t*>(static_cast<char*>(ws) + 256);
+  const int64_t tiles = emit_tiles(G.slots);
+  TQPK_CUDA(cudaMemsetAsync(ws, 0, 256 + tiles * 8, s));
+  auto kernel = G.slots >= kBigTable ? k_emit_dense<kEmitItems> : k_emit_dense<2>;
+  kernel<<<(int)tiles, kBlock, 0, s>>>(S, G, gacc, S.n_keys == 0 ? 1 : 0, E, status, ctl, groups_out);
+  TQPK_CHECK_LAUNCH();
+  *ctl_out = ctl;
+  return TQPK_OK;
 }
 
 // Groups of a hash table in key order: position j holds slot cslot[perm[j]].
@@ -595,7 +663,7 @@ static int plan_from_ranges(const tqpk_groupby_spec* S, const int64_t* mn, const
     plan->ws_bytes = hash_ws_bytes(C, (int)A);
     return TQPK_OK;
   }
-  plan->ws_bytes = 512 + align_up((size_t)(K * A * 8), 256) + compact_status_bytes(K);
+  plan->ws_bytes = 512 + align_up((size_t)(K * A * 8), 256) + emit_ws_bytes(K);
   return TQPK_OK;
 }
 
@@ -768,23 +836,17 @@ extern "C" int tqpk_groupby_emit(const tqpk_groupby_spec* S, const tqpk_gb_plan*
   }
   uint64_t* gacc = reinterpret_cast<uint64_t*>(base + 512);
   void* cws = base + 512 + align_up((size_t)(K * A * 8), 256);
-  const int64_t tiles = (K + kTile - 1) / kTile;
-  WsCursor cur(cws, compact_status_bytes(K));
-  int* ctl = cur.take<int>(64);
-  uint64_t* status = cur.take<uint64_t>(tiles);
-  if (!ctl || !status) return TQPK_ENOMEM;
-  TQPK_CUDA(cudaMemsetAsync(cws, 0, cur.off, s));
-  const GbDev G = to_dev(*plan, S->n_keys);
-  k_emit_dense<<<(int)tiles, kBlock, 0, s>>>(*S, G, gacc, S->n_keys == 0 ? 1 : 0, E, status, ctl, ctl + 1);
-  TQPK_CHECK_LAUNCH();
+  EmitCtl* ctl = nullptr;
+  rc = launch_emit(*S, to_dev(*plan, S->n_keys), gacc, E, cws, nullptr, &ctl, s);
+  if (rc) return rc;
   int err = 0;
-  TQPK_CUDA(cudaMemcpyAsync(&err, ctl + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+  TQPK_CUDA(cudaMemcpyAsync(&err, &ctl->err, sizeof(int), cudaMemcpyDeviceToHost, s));
   TQPK_CUDA(cudaStreamSynchronize(s));
   return err ? err : TQPK_OK;
 }
 
 // tqpk_groupby_emit without a host synchronisation: the group count is
-// counted on the device and written to *d_groups_out (a negative status
+// found on the device and written to *d_groups_out (a negative status
 // there if the emit's look-back failed).  The output columns must hold
 // plan->slots rows (the largest possible group count).
 extern "C" int tqpk_groupby_emit_async(const tqpk_groupby_spec* S, const tqpk_gb_plan* plan, void* ws,
@@ -813,28 +875,10 @@ extern "C" int tqpk_groupby_emit_async(const tqpk_groupby_spec* S, const tqpk_gb
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int64_t K = plan->slots, A = S->n_accs;
   char* base = static_cast<char*>(ws);
-  unsigned long long* d_groups = reinterpret_cast<unsigned long long*>(base);
   uint64_t* gacc = reinterpret_cast<uint64_t*>(base + 512);
   void* cws = base + 512 + align_up((size_t)(K * A * 8), 256);
-  const int64_t tiles = (K + kTile - 1) / kTile;
-  WsCursor cur(cws, compact_status_bytes(K));
-  int* ctl = cur.take<int>(64);
-  uint64_t* status = cur.take<uint64_t>(tiles);
-  if (!ctl || !status) return TQPK_ENOMEM;
-  TQPK_CUDA(cudaMemsetAsync(cws, 0, cur.off, s));
-  TQPK_CUDA(cudaMemsetAsync(d_groups, 0, 8, s));
-  if (S->n_keys == 0) {
-    k_count_one<<<1, 1, 0, s>>>(d_groups);
-  } else {
-    k_count_groups<<<grid_for(K, 4), kBlock, 0, s>>>(gacc, K, d_groups);
-  }
-  TQPK_CHECK_LAUNCH();
-  const GbDev G = to_dev(*plan, S->n_keys);
-  k_emit_dense<<<(int)tiles, kBlock, 0, s>>>(*S, G, gacc, S->n_keys == 0 ? 1 : 0, E, status, ctl, ctl + 1);
-  TQPK_CHECK_LAUNCH();
-  k_groups_or_error<<<1, 1, 0, s>>>(ctl + 1, d_groups, d_groups_out);
-  TQPK_CHECK_LAUNCH();
-  return TQPK_OK;
+  EmitCtl* ctl = nullptr;
+  return launch_emit(*S, to_dev(*plan, S->n_keys), gacc, E, cws, d_groups_out, &ctl, s);
 }
 
 // Stages of tqpk_groupby_run for callers that launch their own accumulation
