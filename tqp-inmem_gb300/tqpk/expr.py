@@ -41,8 +41,9 @@ expression language compiles too:
 """
 from __future__ import annotations
 
+import itertools
 from dataclasses import dataclass, field
-from typing import Any, Dict, List, Tuple
+from typing import Any, Dict, List, Optional, Tuple
 
 import torch
 
@@ -118,6 +119,9 @@ class AggregateProgram:
     # reference's 2-step path, which stays float64 there: aggregate.py:170)
     casts: Dict[int, Tuple[torch.dtype, bool]] = field(default_factory=dict)
     encoded: bool = False     # the kernel groups by one int32 code column standing for the key tuple
+    # number of the program among the memoised ones (None: not memoised): two programs of one number
+    # differ in their column pointers only
+    sig: Optional[int] = None
 
 
 def needs_key_codes(args: dict, columns: Dict[int, torch.Tensor]) -> bool:
@@ -444,6 +448,7 @@ def _add_output(b: _Builder, prog: AggregateProgram, oid: int, fn: str, arg):
 # parsing its trees again (tens of microseconds of host time per call).
 _AGG_MEMO: Dict[tuple, Tuple[AggregateProgram, List[int]]] = {}
 _AGG_MEMO_MAX = 256
+_numbers = itertools.count(1)
 
 
 def _as_1d(t: torch.Tensor) -> torch.Tensor:
@@ -466,6 +471,7 @@ def compile_aggregate(args: dict, columns: Dict[int, torch.Tensor], derived: boo
     if sig is not None and not prog.masks and all(c < _HIDDEN_ID for c in col_ids):   # no derived columns
         if len(_AGG_MEMO) >= _AGG_MEMO_MAX:
             _AGG_MEMO.clear()
+        prog.sig = next(_numbers)
         _AGG_MEMO[sig] = (prog, col_ids)
     return prog
 
@@ -484,7 +490,7 @@ def _rebind(proto: AggregateProgram, col_ids: List[int], columns: Dict[int, torc
         s.cols[i] = t.data_ptr()
     return AggregateProgram(spec=s, tensors=tensors, key_ids=list(proto.key_ids),
                             key_outputs=list(proto.key_outputs), outputs=list(proto.outputs), masks=[],
-                            post=list(proto.post), encoded=False, casts=dict(proto.casts))
+                            post=list(proto.post), encoded=False, casts=dict(proto.casts), sig=proto.sig)
 
 
 def _compile_aggregate(args: dict, columns: Dict[int, torch.Tensor], derived: bool,

@@ -210,19 +210,47 @@ def _shape_key(*structs) -> bytes:
     return b"|".join(out)
 
 
-def run_groupby(spec, pred, plan, ws, n: int, stream: int, pred_tensors=(), key_tensors=(), col_tensors=(),
-                err_ptr=None):
-    """Accumulation pass of ops.groupby as a query-specialised kernel (table in ws).  The
-    generated kernel is looked up by the shape of the spec, predicate and plan, so a
-    repeated query shape skips the source generation."""
-    lib = L.load()
-    key = _shape_key(spec, pred.struct if pred is not None else None, plan)
-    hit = _gb_memo.get(key)
+_made: Dict[tuple, tuple] = {}
+_MADE_MAX = 1024
+
+
+def made(key: Optional[tuple], make):
+    """make()'s result (a compiled kernel and what goes with it), kept under key: numbers of memoised
+    programs (their `sig`) and the plan's numbers.  A key holding None is not kept."""
+    if key is None or None in key:
+        return make()
+    hit = _made.get(key)
     if hit is None:
-        src, name, T, smem = groupby_source(spec, pred.struct if pred is not None else None, plan)
-        hit = (compile_kernel(src, name), T, smem)
-        _gb_memo[key] = hit
-    h, T, smem = hit
+        hit = make()
+        if len(_made) >= _MADE_MAX:
+            _made.clear()
+        _made[key] = hit
+    return hit
+
+
+def pred_sig(pred) -> Optional[int]:
+    """The number of a memoised predicate, 0 for none, None for one that is not memoised."""
+    return 0 if pred is None else pred.sig
+
+
+def run_groupby(spec, pred, plan, ws, n: int, stream: int, pred_tensors=(), key_tensors=(), col_tensors=(),
+                err_ptr=None, sig: Optional[int] = None):
+    """Accumulation pass of ops.groupby as a query-specialised kernel (table in ws).  The
+    generated kernel is looked up by the numbers of the program (sig) and predicate and the
+    plan's, else by the shape of the spec, predicate and plan, so a repeated query shape skips
+    the source generation."""
+    lib = L.load()
+
+    def make():
+        key = _shape_key(spec, pred.struct if pred is not None else None, plan)
+        hit = _gb_memo.get(key)
+        if hit is None:
+            src, name, T, smem = groupby_source(spec, pred.struct if pred is not None else None, plan)
+            hit = _gb_memo[key] = (compile_kernel(src, name), T, smem)
+        return hit
+    nk = spec.n_keys
+    h, T, smem = made(("groupby", sig, pred_sig(pred), plan.mode, plan.threads, plan.slots, *plan.key_min[:nk],
+                       *plan.key_range[:nk], *plan.key_stride[:nk]), make)
     a = _Args()
     if pred is not None:
         for c in range(pred.struct.n_cols):
@@ -306,10 +334,7 @@ class _Args:
         self.vals.append(C.c_int32(int(v)))
 
     def array(self):
-        arr = (C.c_void_p * len(self.vals))()
-        for i, v in enumerate(self.vals):
-            arr[i] = C.cast(C.pointer(v), C.c_void_p)
-        return arr
+        return (C.c_void_p * len(self.vals))(*[C.addressof(v) for v in self.vals])
 
 
 def launch(handle: int, grid: int, block: int, smem: int, args: _Args, stream: int, timing_kid: int = 0):

@@ -198,7 +198,8 @@ def groupby(prog: AggregateProgram, n: int, device, mask: Optional[torch.Tensor]
         L.check(lib.tqpk_groupby_prepare(C.byref(prog.spec), C.byref(plan), ws.data_ptr(), ws.numel(), s),
                 "tqpk_groupby_prepare")
         jit.run_groupby(prog.spec, pred, plan, ws, n, s, pred.tensors if pred is not None else (),
-                        [t for t in prog.tensors[:prog.spec.n_keys]], prog.tensors[prog.spec.n_keys:])
+                        [t for t in prog.tensors[:prog.spec.n_keys]], prog.tensors[prog.spec.n_keys:],
+                        sig=prog.sig)
     ops = []
     for (_, op, a, b, dt) in prog.outputs:
         ops += [op, a, b, code_of(dt)]
@@ -220,8 +221,9 @@ def groupby(prog: AggregateProgram, n: int, device, mask: Optional[torch.Tensor]
             G = int(gdev.item())
         if G < 0:
             L.check(G, "tqpk_groupby_emit_async")
-        keys = [k[:G] for k in keys]
-        outs = [o[:G] for o in outs]
+        if G != K:
+            keys = [k[:G] for k in keys]
+            outs = [o[:G] for o in outs]
     else:
         L.check(lib.tqpk_groupby_run(C.byref(prog.spec), C.byref(plan), pp, mp, n, ws.data_ptr(), ws.numel(),
                                      C.byref(groups), s), "tqpk_groupby_run")
@@ -297,7 +299,7 @@ def _mask_predicate(mask: torch.Tensor) -> CompiledPredicate:
     p.cols[0] = m.data_ptr()
     p.dtypes[0] = L.BOOL
     p.insn[0] = L.PredInsn(L.P_MASK, 0, 0, 0, 0, 0.0, 0.0)
-    return CompiledPredicate(p, [m], [-1])
+    return CompiledPredicate(p, [m], [-1], -1)
 
 
 # ---------------------------------------------------------------- (b) sort / (e) top-k

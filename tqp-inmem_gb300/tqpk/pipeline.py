@@ -58,10 +58,11 @@ class JoinAggTopK:
         self.k, self.desc = int(k), bool(descending)
         nbytes = self.lib.tqpk_pipeline_join_agg_topk_workspace_bytes(self.key_min, self.key_max)
         self.ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=self.dev)
-        self.out_keys = torch.empty(self.k, dtype=torch.int64, device=self.dev)
-        self.out_vals = torch.empty(self.k, dtype=torch.float64, device=self.dev)
-        self.out_count = torch.zeros(1, dtype=torch.int64, device=self.dev)
-        self.groups = torch.zeros(1, dtype=torch.int64, device=self.dev)
+        # one block, so that the result comes back in one copy: row count, group count, keys, sums
+        self._out = torch.zeros(2 + 2 * self.k, dtype=torch.int64, device=self.dev)
+        self.out_count, self.groups = self._out[:1], self._out[1:2]
+        self.out_keys = self._out[2:2 + self.k]
+        self.out_vals = self._out[2 + self.k:].view(torch.float64)
 
     @property
     def workspace_bytes(self) -> int:
@@ -103,13 +104,17 @@ class JoinAggTopK:
                 src, name, self._probe_smem = jit.join_probe_tma_source(
                     self.prog.spec, self.value_reg, pp, None, code_of(self.pk.dtype),
                     ST=int(os.environ.get("TQPK_TMA_STAGES", "2")))
+                self._probe_handle = jit.compile_kernel(src, name)
             else:
                 # evict-first probe columns; with the row directory, value columns staged by cp.async
                 # (42.3-42.7 -> 41.4 us on the 6,001,215-row probe, this pipeline's timing)
-                src, name = jit.join_probe_source(self.prog.spec, self.value_reg, pp, stream_cs=True,
-                                                  stage_vals=not self._bits, occ_sentinel=True,
-                                                  dir_bits=self._bits)
-            self._probe_handle = jit.compile_kernel(src, name)
+                def make():
+                    src, name = jit.join_probe_source(self.prog.spec, self.value_reg, pp, stream_cs=True,
+                                                      stage_vals=not self._bits, occ_sentinel=True,
+                                                      dir_bits=self._bits)
+                    return (jit.compile_kernel(src, name),)
+                self._probe_handle, = jit.made(("join probe", self.prog.sig, jit.pred_sig(self.ppred), self._bits,
+                                                code_of(self.pk.dtype)), make)
             if self._bits and JOIN_SHARED_PERCENT is not None:
                 L.check(self.lib.tqpk_jit_prefer_shared(self._probe_handle, JOIN_SHARED_PERCENT),
                         "tqpk_jit_prefer_shared")
@@ -138,8 +143,11 @@ class JoinAggTopK:
         from . import jit
         if not hasattr(self, "_build_handle"):
             bp = self.bpred.struct if self.bpred else None
-            src, name = jit.join_build_bits_source(bp)
-            self._build_handle = jit.compile_kernel(src, name)
+
+            def make():
+                src, name = jit.join_build_bits_source(bp)
+                return (jit.compile_kernel(src, name),)
+            self._build_handle, = jit.made(("join build", jit.pred_sig(self.bpred)), make)
             d, su, oc = C.c_void_p(), C.c_void_p(), C.c_void_p()
             L.check(self.lib.tqpk_pipeline_join_tables(self.ws.data_ptr(), self.ws.numel(), self.key_min,
                                                        self.key_max, C.byref(d), C.byref(su), C.byref(oc)),
@@ -191,23 +199,20 @@ class JoinAggTopK:
         key raises NotImplementedError (TQPK_EUNSUPPORTED), an out-of-domain one ValueError."""
         if getattr(self, "_probe_smem", 0):
             self.check_error()                      # the TMA-staged probe keeps its own error word
-        keys = self.out_keys if key_dtype in (None, torch.int64) else self.out_keys.to(key_dtype)
-        if not hasattr(self, "_hdr_host"):
-            self._hdr_host = torch.empty(16, dtype=torch.int32, pin_memory=True)
-            self._vals_host = torch.empty(self.k, dtype=torch.float64, pin_memory=True)
-        if getattr(self, "_keys_host", None) is None or self._keys_host.dtype != keys.dtype:
-            self._keys_host = torch.empty(self.k, dtype=keys.dtype, pin_memory=True)
-        hdr = self._hdr_host
+        if not hasattr(self, "_host"):
+            self._host = torch.empty(2 + self._out.numel(), dtype=torch.int64, pin_memory=True)
         cur = torch.cuda.current_stream(self.dev)
-        hdr[:4].copy_(self.ws[:16].view(torch.int32), non_blocking=True)       # hdr[2] = error word
-        hdr[4:6].copy_(self.out_count.view(torch.int32), non_blocking=True)
-        self._keys_host.copy_(keys, non_blocking=True)
-        self._vals_host.copy_(self.out_vals, non_blocking=True)
+        self._host[:2].copy_(self.ws[:16].view(torch.int64), non_blocking=True)       # int 2 = error word
+        self._host[2:].copy_(self._out, non_blocking=True)
+        keys = self.out_keys if key_dtype in (None, torch.int64) else self.out_keys.to(key_dtype)
         cur.synchronize()
-        err, m = int(hdr[2]), int(hdr[4:6].view(torch.int64)[0])
+        h = self._host.numpy()
+        err, m = int(h[1:2].view(np.int32)[0]), int(h[2])
         if err:
             L.check(err, "fused join pipeline (repeated or out-of-domain build key)")
-        self.result_host = (self._keys_host[:m].numpy().copy(), self._vals_host[:m].numpy().copy())
+        hk = h[4:4 + m]
+        self.result_host = (hk.copy() if keys.dtype == torch.int64 else hk.astype(str(keys.dtype).split(".")[-1]),
+                            h[4 + self.k:4 + self.k + m].view(np.float64).copy())
         return keys[:m], self.out_vals[:m], m
 
 
@@ -288,11 +293,13 @@ class StarAggTopK:
         (amn, amx), (bmn, bmx), (cmn, cmx) = self.doms
         nbytes = self.lib.tqpk_pipeline_star_workspace_bytes(amx - amn + 1, bmx - bmn + 1, cmx - cmn + 1)
         self.ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=self.dev)
-        self.out_keys = torch.empty(self.k, dtype=torch.int64, device=self.dev)
-        self.out_vals = torch.empty(self.k, dtype=torch.float64, device=self.dev)
-        self.out_cnts = torch.empty(self.k, dtype=torch.int64, device=self.dev)
-        self.out_count = torch.zeros(1, dtype=torch.int64, device=self.dev)
-        self.groups = torch.zeros(1, dtype=torch.int64, device=self.dev)
+        # one block, so that the result comes back in one copy: the directories' error words (int32),
+        # row count, group count, keys, sums, counts
+        self._out = torch.zeros(4 + 3 * self.k, dtype=torch.int64, device=self.dev)
+        self.out_count, self.groups = self._out[2:3], self._out[3:4]
+        self.out_keys = self._out[4:4 + self.k]
+        self.out_vals = self._out[4 + self.k:4 + 2 * self.k].view(torch.float64)
+        self.out_cnts = self._out[4 + 2 * self.k:]
 
     @property
     def workspace_bytes(self) -> int:
@@ -332,13 +339,16 @@ class StarAggTopK:
         self.dir_c = torch.empty(cmx - cmn + 1, dtype=torch.int32, device=dev)
         self.sum = torch.empty(cmx - cmn + 1, dtype=torch.float64, device=dev)
         self.cnt = torch.empty(cmx - cmn + 1, dtype=torch.int32, device=dev)
-        self.err = torch.zeros(3, dtype=torch.int32, device=dev)
+        self.err = self._out[:2].view(torch.int32)[:3]
         self.tws = torch.empty(self.lib.tqpk_dense_topk_workspace_bytes(self.k), dtype=torch.uint8, device=dev)
         # fkB loaded with fkA and evict-first column loads: 529 -> 507 us on the 59,986,052-row star join
         # + B's directory composed with C's (no C lookup in the probe)
-        src, name = jit.star_probe_source(self.prog.spec, self.value_reg, self.fpred.struct if self.fpred else None,
-                                          None, early_fb=True, stream_cs=True, composed=True, a_bits=self._a_bits)
-        self._probe = jit.compile_kernel(src, name)
+        def make():
+            src, name = jit.star_probe_source(self.prog.spec, self.value_reg,
+                                              self.fpred.struct if self.fpred else None, None, early_fb=True,
+                                              stream_cs=True, composed=True, a_bits=self._a_bits)
+            return (jit.compile_kernel(src, name),)
+        self._probe, = jit.made(("star probe", self.prog.sig, jit.pred_sig(self.fpred), self._a_bits), make)
         if self._a_bits:      # the CTAs' 5 KB of queues per CTA; the rest of the SM's storage as L1
             L.check(self.lib.tqpk_jit_prefer_shared(self._probe, STAR_SHARED_PERCENT), "tqpk_jit_prefer_shared")
         fa, fb = self.t[0], self.t[1]
@@ -439,25 +449,21 @@ class StarAggTopK:
         (`result_host` then holds the rows as numpy arrays).  A repeated dimension key raises
         NotImplementedError, an out-of-domain one ValueError."""
         cur = torch.cuda.current_stream(self.dev)
-        if not hasattr(self, "_hdr_host"):
-            self._hdr_host = torch.empty(8, dtype=torch.int64, pin_memory=True)
-            self._rows_host = [torch.empty(self.k, dtype=t.dtype, pin_memory=True)
-                               for t in (self.out_keys, self.out_vals, self.out_cnts)]
-        hdr = self._hdr_host
-        if getattr(self, "_jit_path", False):        # the three directory builds' error words
-            hdr[:3].copy_(self.err.to(torch.int64), non_blocking=True)
-        else:                                         # the library pipeline's error word (header int 2)
-            hdr[1:3] = 0
-            hdr[:1].copy_(self.ws[8:12].view(torch.int32).to(torch.int64), non_blocking=True)
-        hdr[3:4].copy_(self.out_count, non_blocking=True)
-        for h, t in zip(self._rows_host, (self.out_keys, self.out_vals, self.out_cnts)):
-            h.copy_(t, non_blocking=True)
+        if not hasattr(self, "_host"):
+            self._host = torch.empty(2 + self._out.numel(), dtype=torch.int64, pin_memory=True)
+        jitted = getattr(self, "_jit_path", False)
+        if not jitted:                                # the library pipeline's error word (header int 2)
+            self._host[:2].copy_(self.ws[:16].view(torch.int64), non_blocking=True)
+        self._host[2:].copy_(self._out, non_blocking=True)
         cur.synchronize()
-        errs = [int(x) for x in hdr[:3].tolist() if x]
+        h = self._host.numpy()
+        # the three directory builds' error words
+        errs = [int(x) for x in (h[2:4].view(np.int32)[:3] if jitted else h[1:2].view(np.int32)[:1]) if x]
         if errs:
             L.check(errs[0], "star pipeline (repeated or out-of-domain dimension key)")
-        m = int(hdr[3])
-        self.result_host = tuple(h[:m].numpy().copy() for h in self._rows_host)
+        m, k = int(h[4]), self.k
+        rows = h[6:]
+        self.result_host = (rows[:m].copy(), rows[k:k + m].view(np.float64).copy(), rows[2 * k:2 * k + m].copy())
         return self.out_keys[:m], self.out_vals[:m], self.out_cnts[:m], m
 
     def group_table(self):

@@ -28,8 +28,9 @@ its own width, the column's row stride), usable wherever a string column is.
 from __future__ import annotations
 
 import datetime as _dt
+import itertools
 from dataclasses import dataclass, field
-from typing import Any, Dict, List
+from typing import Any, Dict, List, Optional
 
 import numpy as np
 
@@ -81,9 +82,30 @@ class CompiledPredicate:
     struct: Any
     tensors: List[Any] = field(default_factory=list)
     col_ids: List[int] = field(default_factory=list)
+    # number of the program among the memoised ones (None: not memoised): two predicates of one
+    # number differ in their column pointers only
+    sig: Optional[int] = None
 
     def bind(self):
         return self.struct
+
+
+# Compiled filter programs by tree, literals, and the columns' dtypes and widths: a repeated filter
+# re-binds the column pointers of the cached program (a plan's filters cost ~30 us each to parse).
+_FILTER_MEMO: Dict[tuple, tuple] = {}
+_FILTER_MEMO_MAX = 256
+_numbers = itertools.count(1)
+
+
+def _filter_key(tree, columns, subquery, agg):
+    """The memo's key, or None for operands it cannot hold by value."""
+    if subquery is not None and not isinstance(subquery, (int, float, str)):
+        return None
+    try:
+        return (repr(tree), agg, type(subquery), subquery,
+                tuple((c, t.dtype, t.dim(), t.shape[1] if t.dim() == 2 else 0) for c, t in columns.items()))
+    except (AttributeError, TypeError):
+        return None
 
 
 class _Compiler:
@@ -382,6 +404,18 @@ def compile_filter(tree, columns: Dict[int, Any], subquery=None, agg: bool = Fal
     aggregate.py:203-233 does: torch.le/ge/eq/ne without the filter's eps and isclose,
     `<>` allowed, a multi-character string literal tested for equality whatever the
     operator (:229-231), IN/LIKE and functions other than NOT/StartsWith rejected."""
+    key = _filter_key(tree, columns, subquery, agg)
+    hit = _FILTER_MEMO.get(key) if key is not None else None
+    if hit is not None:
+        proto, slots, number = hit
+        p = L.Predicate.from_buffer_copy(proto)
+        tensors = []
+        for s, (cid, start, text) in enumerate(slots):
+            t = columns[cid]
+            t = (t if text or t.dim() == 1 else t.reshape(-1)).contiguous()
+            tensors.append(t)
+            p.cols[s] = t.data_ptr() + start
+        return CompiledPredicate(p, tensors, [cid for cid, _, _ in slots], number)
     c = _Compiler(columns, subquery, agg)
     c.emit(tree)
     if len(c.insn) > L.MAX_PRED:
@@ -391,11 +425,13 @@ def compile_filter(tree, columns: Dict[int, Any], subquery=None, agg: bool = Fal
     p.n_cols = len(c.slots)
     tensors = []
     ids = [None] * len(c.slots)
-    for cid, s in c.slots.items():
+    slots = []                                         # (column, byte offset, text) by slot
+    for cid, s in c.slots.items():                     # in slot order
         if isinstance(cid, tuple):                     # substring view: offset pointer, own width, row stride
             _, base_id, start, width = cid
             t = c.str_tensor(base_id).contiguous()
             tensors.append(t)
+            slots.append((base_id, start, True))
             ids[s] = base_id
             p.cols[s] = t.data_ptr() + start
             p.widths[s] = width
@@ -408,6 +444,7 @@ def compile_filter(tree, columns: Dict[int, Any], subquery=None, agg: bool = Fal
         else:
             t = c.col_tensor(cid).contiguous()
         tensors.append(t)
+        slots.append((cid, 0, cid in c.str_cols))
         ids[s] = cid
         p.cols[s] = t.data_ptr()
         p.dtypes[s] = code_of(t.dtype)
@@ -415,7 +452,13 @@ def compile_filter(tree, columns: Dict[int, Any], subquery=None, agg: bool = Fal
         p.insn[i] = L.PredInsn(op, col, cmp, dom, li, lf, la)
     for i, b in enumerate(c.pool):
         p.strpool[i] = b
-    return CompiledPredicate(p, tensors, ids)
+    number = None
+    if key is not None:
+        number = next(_numbers)
+        if len(_FILTER_MEMO) >= _FILTER_MEMO_MAX:
+            _FILTER_MEMO.clear()
+        _FILTER_MEMO[key] = (p, slots, number)
+    return CompiledPredicate(p, tensors, ids, number)
 
 
 def has_strings(P) -> bool:
