@@ -386,7 +386,9 @@ int tqpk_join_probe(const tqpk_join_plan* h_plan, const void* d_build_ws, const 
  * numeric predicate program over the two sides' columns, evaluated for every
  * key-equal pair; bit c of probe_cols: its column c is the probe side's.  A
  * string instruction is TQPK_EUNSUPPORTED.  A directory whose unique is
- * TQPK_JOIN_UNKNOWN gives TQPK_ECAPACITY and *h_count = -1 when a key repeats. */
+ * TQPK_JOIN_UNKNOWN gives TQPK_ECAPACITY and *h_count = -1 when a key repeats.
+ * d_probe_ws holds tqpk_join_pairs_workspace_bytes(plan, np, h_cond != NULL).  */
+size_t tqpk_join_pairs_workspace_bytes(const tqpk_join_plan* h_plan, int64_t np, int32_t with_cond);
 int tqpk_join_count(const tqpk_join_plan* h_plan, const void* d_build_ws, const void* d_probe_keys,
                     int32_t probe_dtype, const uint8_t* d_probe_mask, int64_t np, const tqpk_predicate* h_cond,
                     uint32_t probe_cols, int64_t* h_count, void* d_probe_ws, size_t probe_ws_bytes, tqpk_stream stream);

@@ -304,7 +304,27 @@ struct PairCtl {
 struct PairCond {
   tqpk_predicate P;
   unsigned probe_cols;
+  // The usual condition, one comparison of an integer column of each side (a second key): build <cmp> probe.
+  int two_sided, cmp, build_dt, probe_dt;
+  const void* build_col;
+  const void* probe_col;
+  const int64_t* vals;      // the build column's values in csr order (null: read by build row)
 };
+
+// What the counting pass of a join with conditions leaves for the writing one: per tile whether its threads
+// took their own rows' pairs, then which of them hold (bit 16 j + t: pair t of a thread's row j) and where
+// each row's build rows start (4-byte entries only).
+struct PairKept {
+  uint8_t* by_row;
+  uint64_t* held;
+  unsigned* first;
+};
+
+__global__ void k_pair_vals(const void* __restrict__ col, int dt, const int64_t* __restrict__ csr, int64_t m,
+                            int64_t* __restrict__ vals) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
+    vals[i] = ld_int(col, dt, csr[i]);
+}
 
 __device__ __forceinline__ bool pair_cmp(const PairCond& C, const tqpk_pred_insn& I, int64_t b, int64_t p) {
   const int64_t r = (C.probe_cols >> I.col) & 1u ? p : b;
@@ -346,13 +366,20 @@ __device__ __forceinline__ bool pair_holds(const PairCond& C, int64_t b, int64_t
 }
 
 // Pass COUNT leaves each tile's pair count in tile_base; its last CTA scans them into offsets.  COND: only
-// the pairs that satisfy C count; both passes evaluate it (24 M pairs of a key repeated four times, one in
-// four kept: materialising them, gathering the condition's columns and compacting took ~600 us).
+// the pairs that satisfy C count (24 M pairs of a key repeated four times, one in four kept: materialising
+// them, gathering the condition's columns and compacting took ~600 us).  What bounds it is the L1's handling
+// of scattered lanes, about one a clock: the csr entry and the build column's value of every pair, in both
+// passes, took 248 + 300 us.  So the usual condition's build column is laid out in csr order first, a row's
+// values then come two to a load, and a tile whose rows have at most kRowPairs candidates each gives every
+// thread its own four rows and keeps its verdicts for the writing pass.  Longer runs are spread over the
+// block pair by pair, by a search in the tile's scan, in both passes.
+constexpr int kRowPairs = 16;
+
 template <bool COUNT, bool COND>
 __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pkeys, int pdt, RowFilter F, int64_t np,
                                                        int kvec, int64_t* __restrict__ out_b,
                                                        int64_t* __restrict__ out_p, int64_t capacity,
-                                                       int64_t* __restrict__ tile_base, PairCtl* ctl,
+                                                       int64_t* __restrict__ tile_base, PairCtl* ctl, PairKept W,
                                                        const __grid_constant__ PairCond C) {
   constexpr bool kRows = !COUNT || COND;
   __shared__ int64_t sw[kBlock / 32 + 1];
@@ -361,6 +388,20 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
   __shared__ int s_last;
   const int64_t tile = blockIdx.x;
   const int64_t g0 = tile * kPairRows + 4 * threadIdx.x;
+  if (!COUNT && COND && W.by_row[tile]) {
+    uint64_t held = W.held[tile * kBlock + threadIdx.x];
+    const uint4 f4 = *reinterpret_cast<const uint4*>(&W.first[4 * (tile * kBlock + threadIdx.x)]);
+    int64_t kept;
+    int64_t at = tile_base[tile] + block_excl_scan<kBlock, int64_t>(__popcll(held), kept, sw);
+    for (; held; held &= held - 1, ++at) {
+      const int q = __ffsll((long long)held) - 1, j = q >> 4;
+      const int64_t f = (int64_t)(j == 0 ? f4.x : j == 1 ? f4.y : j == 2 ? f4.z : f4.w) + (q & 15);
+      if (at >= capacity) break;
+      out_p[at] = g0 + j;
+      out_b[at] = D.csr ? D.csr[f] : f;
+    }
+    return;
+  }
   const int64_t valid = np - g0;
   uint32_t b = valid >= 4 ? 0xfu : (valid <= 0 ? 0u : ((1u << valid) - 1));
   if (F.mask && b) {
@@ -389,7 +430,65 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
     row = lo;
     build = D.csr ? D.csr[f] : f;
   };
-  if (kRows) {
+  __shared__ unsigned s_kept[2][kBlock / 32];
+  const bool by_row = COUNT && COND && !__syncthreads_or(D.wide || cnt[0] > kRowPairs || cnt[1] > kRowPairs ||
+                                                         cnt[2] > kRowPairs || cnt[3] > kRowPairs);
+  if (COUNT && COND && threadIdx.x == 0) W.by_row[tile] = by_row;
+  if (by_row) {
+    uint64_t held = 0;
+    int64_t pv[4] = {0, 0, 0, 0};
+    if (b && C.two_sided) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (cnt[j]) pv[j] = ld_int(C.probe_col, C.probe_dt, g0 + j);
+    }
+    const int most = (int)max(max(cnt[0], cnt[1]), max(cnt[2], cnt[3]));
+    for (int t = 0; C.vals && t < most; t += 2) {
+      int64_t v[4][2];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t* p = C.vals + first[j] + t;
+        const int left = (int)cnt[j] - t;
+        if (left >= 2 && (first[j] & 1) == 0) {
+          const longlong2 a = *reinterpret_cast<const longlong2*>(p);
+          v[j][0] = a.x;
+          v[j][1] = a.y;
+        } else {
+          v[j][0] = left >= 1 ? p[0] : 0;
+          v[j][1] = left >= 2 ? p[1] : 0;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int left = (int)cnt[j] - t;
+        const uint64_t two = (left >= 1 && cmp_op<int64_t>(C.cmp, v[j][0], pv[j]) ? 1u : 0u) |
+                             (left >= 2 && cmp_op<int64_t>(C.cmp, v[j][1], pv[j]) ? 2u : 0u);
+        held |= two << (16 * j + t);
+      }
+    }
+    for (int t = 0; !C.vals && t < most; ++t) {
+      int64_t build[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) build[j] = t < cnt[j] ? (D.csr ? D.csr[first[j] + t] : first[j] + t) : -1;
+      if (C.two_sided) {
+        int64_t bv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bv[j] = build[j] >= 0 ? ld_int(C.build_col, C.build_dt, build[j]) : 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          held |= (uint64_t)(build[j] >= 0 && cmp_op<int64_t>(C.cmp, bv[j], pv[j])) << (16 * j + t);
+      } else {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j)
+          if (build[j] >= 0) held |= (uint64_t)pair_holds(C, build[j], g0 + j) << (16 * j + t);
+      }
+    }
+    W.held[tile * kBlock + threadIdx.x] = held;
+    *reinterpret_cast<uint4*>(&W.first[4 * (tile * kBlock + threadIdx.x)]) =
+        make_uint4((unsigned)first[0], (unsigned)first[1], (unsigned)first[2], (unsigned)first[3]);
+    block_excl_scan<kBlock, int64_t>(__popcll(held), total, sw);
+  }
+  if (kRows && !by_row) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       s_pre[4 * threadIdx.x + j] = excl;
@@ -398,7 +497,7 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
     }
     __syncthreads();
   }
-  if (COUNT && COND) {
+  if (COUNT && COND && !by_row) {
     int64_t kept = 0;
     for (int64_t o = threadIdx.x; o < total; o += kBlock) {
       int row;
@@ -451,7 +550,6 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
     }
     return;
   }
-  __shared__ unsigned s_kept[2][kBlock / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int64_t o0 = 0; o0 < total; o0 += kBlock) {
     const int64_t o = o0 + threadIdx.x;
@@ -596,9 +694,11 @@ struct ProbeLayout {
   uint64_t* status_b;
   size_t zeroed;
   int64_t* tile_base;
+  PairKept kept;         // joins with conditions
+  int64_t* vals;
 };
 
-static bool probe_layout(int64_t np, void* pws, size_t bytes, ProbeLayout& W) {
+static bool probe_layout(int64_t np, void* pws, size_t bytes, ProbeLayout& W, int64_t cond_build_rows = -1) {
   const int64_t tiles = (np + kTile - 1) / kTile;
   WsCursor cur(pws, bytes);
   W.ctl = cur.take<int>(64);
@@ -607,8 +707,14 @@ static bool probe_layout(int64_t np, void* pws, size_t bytes, ProbeLayout& W) {
   W.status_a = cur.take<uint64_t>(tiles + 1);
   W.status_b = cur.take<uint64_t>(tiles + 1);
   W.zeroed = cur.off;
-  W.tile_base = cur.take<int64_t>((np + kPairRows - 1) / kPairRows + 1);
-  return W.tile_base != nullptr;
+  const int64_t ptiles = (np + kPairRows - 1) / kPairRows;
+  W.tile_base = cur.take<int64_t>(ptiles + 1);
+  if (cond_build_rows < 0) return W.tile_base != nullptr;
+  W.kept.by_row = cur.take<uint8_t>(ptiles + 1);
+  W.kept.held = cur.take<uint64_t>(ptiles * kBlock + 1);
+  W.kept.first = cur.take<unsigned>(ptiles * kPairRows + 4);
+  W.vals = cur.take<int64_t>(cond_build_rows + 2);
+  return W.vals != nullptr;
 }
 
 // Pair counts of every tile of probe rows and their sum (W.pair->total), on the device.
@@ -618,7 +724,7 @@ static int count_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFi
   if (tiles > INT32_MAX) return TQPK_EUNSUPPORTED;
   auto kernel = C.P.n_insn ? k_join_pairs<true, true> : k_join_pairs<true, false>;
   kernel<<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, nullptr, nullptr, 0, W.tile_base,
-                                       W.pair, C);
+                                       W.pair, W.kept, C);
   TQPK_CHECK_LAUNCH();
   return TQPK_OK;
 }
@@ -629,7 +735,7 @@ static int write_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFi
   auto kernel = C.P.n_insn ? k_join_pairs<false, true> : k_join_pairs<false, false>;
   timing_before(KID_JOIN_PROBE, s);
   kernel<<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, out_b, out_p, capacity,
-                                       W.tile_base, W.pair, C);
+                                       W.tile_base, W.pair, W.kept, C);
   timing_after(KID_JOIN_PROBE, s);
   TQPK_CHECK_LAUNCH();
   return TQPK_OK;
@@ -762,6 +868,14 @@ extern "C" size_t tqpk_join_probe_workspace_bytes(int64_t np) {
   return 2048 + 2 * align_up((size_t)(tiles + 1) * 8, 256) + align_up(((size_t)np / kPairRows + 2) * 8, 256);
 }
 
+extern "C" size_t tqpk_join_pairs_workspace_bytes(const tqpk_join_plan* plan, int64_t np, int32_t with_cond) {
+  if (!plan || np < 0) return 0;
+  const size_t base = tqpk_join_probe_workspace_bytes(np), t = (size_t)np / kPairRows + 2;
+  if (!with_cond) return base;
+  return base + align_up(t, 256) + align_up(t * kBlock * 8, 256) + align_up(t * kPairRows * 4, 256) +
+         align_up(((size_t)plan->nb_rows + 2) * 8, 256);
+}
+
 extern "C" int tqpk_join_probe(const tqpk_join_plan* plan, const void* build_ws, const void* pkeys, int32_t pdt,
                                const uint8_t* pmask, int64_t np, int32_t jt, int64_t* out_b, int64_t* out_p,
                                int64_t capacity, int64_t* h_count, void* pws, size_t pws_bytes, tqpk_stream stream) {
@@ -839,6 +953,21 @@ static int pair_cond(const tqpk_predicate* cond, uint32_t probe_cols, PairCond& 
     if (cond->insn[k].op > TQPK_P_CMPCOL) return TQPK_EUNSUPPORTED;
   C.P = *cond;
   C.probe_cols = probe_cols;
+  const tqpk_pred_insn& I = cond->insn[0];
+  if (cond->n_insn == 1 && I.op == TQPK_P_CMPCOL && I.domain == TQPK_DOM_I64) {
+    const int c1 = I.col, c2 = (int)I.lit_i;
+    const bool p1 = (probe_cols >> c1) & 1u, p2 = (probe_cols >> c2) & 1u;
+    if (p1 != p2 && is_int_dtype(cond->dtypes[c1]) && is_int_dtype(cond->dtypes[c2])) {
+      const int bc = p1 ? c2 : c1, pc = p1 ? c1 : c2;
+      static const int flipped[] = {TQPK_GT, TQPK_GE, TQPK_LT, TQPK_LE, TQPK_EQ, TQPK_NE};   // of LT, LE, GT, ...
+      C.two_sided = 1;
+      C.cmp = p1 ? flipped[I.cmp - TQPK_LT] : I.cmp;
+      C.build_col = cond->cols[bc];
+      C.build_dt = cond->dtypes[bc];
+      C.probe_col = cond->cols[pc];
+      C.probe_dt = cond->dtypes[pc];
+    }
+  }
   return TQPK_OK;
 }
 
@@ -850,12 +979,12 @@ extern "C" int tqpk_join_count(const tqpk_join_plan* plan, const void* build_ws,
   PairCond C;
   int rc = pair_cond(cond, probe_cols, C);
   if (rc) return rc;
-  if (!pws || pws_bytes < tqpk_join_probe_workspace_bytes(np)) return TQPK_ENOMEM;
+  if (!pws || pws_bytes < tqpk_join_pairs_workspace_bytes(plan, np, cond != nullptr)) return TQPK_ENOMEM;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BuildLayout L;
   ProbeLayout W;
   if (!layout(*plan, const_cast<void*>(build_ws), plan->ws_bytes, L)) return TQPK_ENOMEM;
-  if (!probe_layout(np, pws, pws_bytes, W)) return TQPK_ENOMEM;
+  if (!probe_layout(np, pws, pws_bytes, W, cond ? plan->nb_rows : -1)) return TQPK_ENOMEM;
   *h_count = 0;
   if (np == 0) return TQPK_OK;
   if (uniqueness(*plan) == TQPK_JOIN_UNKNOWN) {
@@ -868,7 +997,13 @@ extern "C" int tqpk_join_count(const tqpk_join_plan* plan, const void* build_ws,
     }
   }
   TQPK_CUDA(cudaMemsetAsync(pws, 0, W.zeroed, s));
-  rc = count_pairs(make_dir(*plan, L, true), pkeys, pdt, make_filter(nullptr, pmask), np, C, W, s);
+  const JoinDir D = make_dir(*plan, L, true);
+  if (C.two_sided && D.csr && !D.wide && plan->nb_rows > 0) {
+    k_pair_vals<<<grid_for(plan->nb_rows, 8), kBlock, 0, s>>>(C.build_col, C.build_dt, D.csr, plan->nb_rows, W.vals);
+    TQPK_CHECK_LAUNCH();
+    C.vals = W.vals;
+  }
+  rc = count_pairs(D, pkeys, pdt, make_filter(nullptr, pmask), np, C, W, s);
   if (rc) return rc;
   TQPK_CUDA(cudaMemcpyAsync(h_count, &W.pair->total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   TQPK_CUDA(cudaStreamSynchronize(s));
@@ -885,12 +1020,12 @@ extern "C" int tqpk_join_write(const tqpk_join_plan* plan, const void* build_ws,
   PairCond C;
   const int rc = pair_cond(cond, probe_cols, C);
   if (rc) return rc;
-  if (!pws || pws_bytes < tqpk_join_probe_workspace_bytes(np)) return TQPK_ENOMEM;
+  if (!pws || pws_bytes < tqpk_join_pairs_workspace_bytes(plan, np, cond != nullptr)) return TQPK_ENOMEM;
   if (np == 0 || capacity == 0) return TQPK_OK;
   BuildLayout L;
   ProbeLayout W;
   if (!layout(*plan, const_cast<void*>(build_ws), plan->ws_bytes, L)) return TQPK_ENOMEM;
-  if (!probe_layout(np, pws, pws_bytes, W)) return TQPK_ENOMEM;
+  if (!probe_layout(np, pws, pws_bytes, W, cond ? plan->nb_rows : -1)) return TQPK_ENOMEM;
   return write_pairs(make_dir(*plan, L, true), pkeys, pdt, make_filter(nullptr, pmask), np, C, W, out_b, out_p,
                      capacity, static_cast<cudaStream_t>(stream));
 }

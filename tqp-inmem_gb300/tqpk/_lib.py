@@ -108,6 +108,7 @@ SIGNATURES = {
     "tqpk_join_build": (C.c_int, [_P(JoinPlan), _VP, _I32, _VP, _I64, _VP, _SZ, _VP]),
     "tqpk_join_directory": (C.c_int, [_P(JoinPlan), _VP, _I32, _VP, _I64, _VP, _SZ, _VP]),
     "tqpk_join_rows": (C.c_int, [_P(JoinPlan), _VP, _I32, _VP, _I64, _VP, _SZ, _VP]),
+    "tqpk_join_pairs_workspace_bytes": (_SZ, [_P(JoinPlan), _I64, _I32]),
     "tqpk_join_count": (C.c_int, [_P(JoinPlan), _VP, _VP, _I32, _VP, _I64, _P(Predicate), C.c_uint32, _P(_I64), _VP,
                                   _SZ, _VP]),
     "tqpk_join_write": (C.c_int, [_P(JoinPlan), _VP, _VP, _I32, _VP, _I64, _P(Predicate), C.c_uint32, _VP, _VP, _I64,

@@ -507,7 +507,7 @@ def join_pairs(build: JoinBuild, probe_keys: torch.Tensor, probe_mask: Optional[
     dev = build.device
     s = _stream(dev)
     n = int(pk.numel())
-    pws = _ws(lib.tqpk_join_probe_workspace_bytes(n), dev)
+    pws = _ws(lib.tqpk_join_pairs_workspace_bytes(C.byref(build.plan), n, int(cond is not None)), dev)
     args = (build.ws.data_ptr(), pk.data_ptr() if n else None, code_of(pk.dtype),
             probe_mask.data_ptr() if probe_mask is not None else None, n,
             C.byref(cond.struct) if cond is not None else None, probe_cols)
