@@ -92,6 +92,21 @@ def test_keys_of_more_digits_than_are_sorted_by(make, n):
     _check([rng.integers(0, 3, n).astype(np.int32), f], [False, False], rng.permutation(n))
 
 
+@pytest.mark.parametrize("n", [3000, 40_000, 150_001])
+@pytest.mark.parametrize("dtype", [np.int8, np.uint8])
+def test_text_widths(n, dtype):
+    """Words cut short by the row's end, rows at every alignment, every byte value, both orders."""
+    rng = np.random.default_rng(n)
+    for w in (2, 3, 7, 8, 9, 10, 11, 16, 19, 25):
+        t = rng.integers(0, 256, (n, w)).astype(np.uint8).view(dtype)
+        t[:, : w // 2] = t[: 3, : w // 2][rng.integers(0, 3, n)]           # few values in front: ties decided behind
+        for desc in (False, True):
+            _check([t], [desc])
+    t = np.zeros((n, 9), dtype)
+    t[:, 8] = rng.integers(60, 70, n)
+    _check([t], [True])
+
+
 def test_too_many_words_raise():
     from tqpk.ops import argsort_keys
     wide = torch.zeros((3000, 8 * 33), dtype=torch.int8, device="cuda")
