@@ -88,3 +88,44 @@ def test_key_ranges_under_a_mask(n):
             s = c if m is None else c[m]
             assert plan.nb_rows == s.size
             assert (plan.key_min, plan.key_max) == ((int(s.min()), int(s.max())) if s.size else (0, -1))
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 1023, 1025, 5000])
+@pytest.mark.parametrize("width", [6, 25, 188, 189])
+def test_text_programs(n, width):
+    """Text staged in shared memory (rows of up to 188 bytes) and in place, beside numeric comparisons."""
+    from oracle import tqp_oracle as O
+    from tqpk.ops import filter_mask
+    from tqpk.predicate import compile_filter
+    rng = np.random.default_rng(n + width)
+    words = [b"ECONOMY", b"TIN", b"MED", b"AB", b"CANADA", b""]
+    t = np.zeros((n, width), np.int8)
+    for i in range(n):
+        s = b" ".join(words[j] for j in rng.integers(0, 6, 1 + width // 8))[:width]
+        t[i, :len(s)] = np.frombuffer(s, np.int8)
+    cols = {1: t, 2: rng.integers(0, 9, n), 3: np.ascontiguousarray(t[:, : min(width, 9)])}
+    dev = {c: torch.from_numpy(a).cuda() for c, a in cols.items()}
+    trees = [["StartsWith", ["t#1", "AB"]], ["t#1", "LIKE", "%MED%TIN%"], ["Contains", ["t#1", "NOM"]],
+             [["NOT", [["StartsWith", ["t#1", "MED"]]]], "AND", [["k#2", "<", "5"], "OR", ["Contains", ["s#3", "IN"]]]],
+             [["substring", ["t#1", "2", "3"]], "IN", ["CON", "ANA", "IN "]], ["s#3", "=", "CANADA"],
+             [["substring", ["t#1", str(width - 1), "2"]], "=", "ED"]]
+    for tree in trees:
+        if "CANADA" in repr(tree) and min(width, 9) < 6:
+            continue
+        pred = compile_filter(tree, dev)
+        mask, count = filter_mask(pred, n, dev[1].device, with_count=True)
+        exp = np.asarray(O.eval_filter(tree, cols), bool).reshape(-1)
+        np.testing.assert_array_equal(mask.cpu().numpy(), exp, err_msg=repr(tree))
+        assert int(count.item()) == int(exp.sum())
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 5000])
+@pytest.mark.parametrize("width", [2, 15, 16, 25, 160, 161])
+def test_gather_of_text_rows(n, width):
+    from tqpk.ops import gather_rows
+    rng = np.random.default_rng(n + width)
+    t = rng.integers(-128, 128, (700, width)).astype(np.int8)
+    idx = rng.integers(0, 700, n)
+    idx[0] = 699
+    got = gather_rows(torch.from_numpy(t).cuda(), torch.from_numpy(idx).cuda())
+    np.testing.assert_array_equal(got.cpu().numpy(), t[idx])

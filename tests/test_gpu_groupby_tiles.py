@@ -75,3 +75,27 @@ def test_dense_keys(n, slots_a, slots_b):
     v, w = rng.integers(-5000, 5000, n) * 0.25, rng.integers(0, 50, n).astype(np.int32)
     for mask in _masks(rng, n):
         _check([a, b], v, w, mask)
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 60_000])
+@pytest.mark.parametrize("width", [1, 3, 8, 10, 25])
+def test_key_codes_of_text(n, width):
+    """Codes in key-tuple order of a text key (rows at every alignment) beside a float key, under masks."""
+    from tqpk.ops import encode_keys
+    rng = np.random.default_rng(n + width)
+    words = rng.integers(-128, 128, (40, width)).astype(np.int8)
+    words[20:, : width // 2] = words[:20, : width // 2]
+    t = words[rng.integers(0, 40, n)]
+    f = rng.integers(-2, 3, n) * 0.5
+    f[f == 0] = np.where(rng.integers(0, 2, (f == 0).sum()) > 0, 0.0, -0.0)
+    dev = [torch.from_numpy(t).cuda().reshape(n, width), torch.from_numpy(f).cuda()]
+    for mask in _masks(rng, n):
+        m = np.ones(n, bool) if mask is None else mask
+        codes, reps, g = encode_keys(dev, torch.from_numpy(mask).cuda() if mask is not None else None)
+        rows = np.concatenate([t.astype(np.float64), (f + 0.0)[:, None]], 1)[m]
+        u, inv = np.unique(rows, axis=0, return_inverse=True)
+        assert g == len(u)
+        np.testing.assert_array_equal(codes.cpu().numpy()[m], inv.reshape(-1))
+        r = reps.cpu().numpy()
+        assert m[r].all()
+        np.testing.assert_array_equal(np.concatenate([t.astype(np.float64), (f + 0.0)[:, None]], 1)[r], u)

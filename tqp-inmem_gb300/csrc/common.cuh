@@ -205,6 +205,31 @@ __device__ __forceinline__ uint64_t sort_key(const void* keys, int dt, int64_t i
   return sort_key_bits(raw, dt == TQPK_F64, desc);
 }
 
+// Eight bytes at s as a little-endian word, zero past `left` bytes (the bytes from s to the end of its
+// row); inner: the up to three bytes before s belong to the column too.  Two or three aligned words where
+// those lie in the row (or before it), the bytes past the second word one by one where the third would
+// leave it.
+__device__ __forceinline__ uint64_t load_bytes8(const uint8_t* s, int left, bool inner) {
+  const unsigned off = (unsigned)(reinterpret_cast<uintptr_t>(s) & 3u);
+  if (left >= 8 && (off == 0 || inner)) {
+    const unsigned* a = reinterpret_cast<const unsigned*>(s - off);
+    const unsigned w0 = a[0], w1 = a[1];
+    unsigned w2 = 0;
+    if (off && left >= 11) {
+      w2 = a[2];
+    } else {
+#pragma unroll 1
+      for (unsigned i = 0; i < off; ++i) w2 |= (unsigned)s[8 - off + i] << (8 * i);
+    }
+    return ((uint64_t)__funnelshift_r(w1, w2, 8 * off) << 32) | __funnelshift_r(w0, w1, 8 * off);
+  }
+  const int m = left < 8 ? left : 8;
+  uint64_t w = 0;
+#pragma unroll 1
+  for (int i = 0; i < m; ++i) w |= static_cast<uint64_t>(s[i]) << (8 * i);
+  return w;
+}
+
 // Loads four consecutive rows r0..r0+3 (r0 % 4 == 0); rows >= n read as 0.
 // `vec` means the base pointer is 16-byte aligned, so a full group can use
 // 128-bit loads.
@@ -536,25 +561,28 @@ __device__ __forceinline__ bool str_like2(const int8_t* row, int w, const uint8_
   }
   return false;
 }
-static __device__ uint32_t str_leaf4(const tqpk_predicate& P, const tqpk_pred_insn& I, int64_t r0, int64_t n) {
+// One text instruction on one row.
+__device__ __forceinline__ bool str_leaf(const tqpk_predicate& P, const tqpk_pred_insn& I, const int8_t* row) {
   const int w = P.widths[I.col];
-  const int64_t stride = P.strides[I.col] > 0 ? P.strides[I.col] : w;
-  const int8_t* base = static_cast<const int8_t*>(P.cols[I.col]);
   const uint64_t L = (uint64_t)I.lit_i;
+  switch (I.op) {
+    case TQPK_P_STRCMP: return str_all_cmp(row, w, P.strpool + (L & 0xffffffffu), I.cmp);
+    case TQPK_P_PREFIX: return str_at(row, P.strpool + (L & 0xffffffffu), (int)(L >> 32));
+    case TQPK_P_CONTAINS: return str_contains(row, w, P.strpool + (L & 0xffffffffu), (int)(L >> 32));
+  }
+  return str_like2(row, w, P.strpool + (L & 0xffff), (int)((L >> 16) & 0xffff), P.strpool + ((L >> 32) & 0xffff),
+                   (int)(L >> 48));
+}
+__host__ __device__ __forceinline__ int64_t str_stride(const tqpk_predicate& P, int col) {
+  return P.strides[col] > 0 ? P.strides[col] : P.widths[col];
+}
+static __device__ uint32_t str_leaf4(const tqpk_predicate& P, const tqpk_pred_insn& I, int64_t r0, int64_t n) {
+  const int64_t stride = str_stride(P, I.col);
+  const int8_t* base = static_cast<const int8_t*>(P.cols[I.col]);
   uint32_t m = 0;
   for (int j = 0; j < 4; ++j) {
     if (r0 + j >= n) break;
-    const int8_t* row = base + (r0 + j) * stride;
-    bool ok;
-    switch (I.op) {
-      case TQPK_P_STRCMP: ok = str_all_cmp(row, w, P.strpool + (L & 0xffffffffu), I.cmp); break;
-      case TQPK_P_PREFIX: ok = str_at(row, P.strpool + (L & 0xffffffffu), (int)(L >> 32)); break;
-      case TQPK_P_CONTAINS: ok = str_contains(row, w, P.strpool + (L & 0xffffffffu), (int)(L >> 32)); break;
-      default:
-        ok = str_like2(row, w, P.strpool + (L & 0xffff), (int)((L >> 16) & 0xffff), P.strpool + ((L >> 32) & 0xffff),
-                       (int)(L >> 48));
-    }
-    m |= (uint32_t)ok << j;
+    m |= (uint32_t)str_leaf(P, I, base + (r0 + j) * stride) << j;
   }
   return m;
 }
@@ -786,11 +814,10 @@ __device__ __forceinline__ uint32_t valid_rows(const int64_t (&r0)[Q], int64_t n
 }
 
 // The predicate for 4 Q rows -> mask (rows >= n are 0).  As eval_pred4, with the program, the types and the
-// operators decided once for them.
-template <int Q>
-__device__ __forceinline__ uint32_t eval_pred_rows(const tqpk_predicate& P, const int64_t (&r0)[Q], int64_t n, bool vec) {
-  const uint32_t valid = valid_rows<Q>(r0, n);
-  if (!valid) return 0;
+// operators decided once for them; text(I) evaluates a text instruction.
+template <int Q, class Text>
+__device__ __forceinline__ uint32_t eval_pred_with(const tqpk_predicate& P, const int64_t (&r0)[Q], int64_t n, bool vec,
+                                                   Text text) {
   uint32_t st[TQPK_MAX_PRED];
   uint32_t top = ~0u;                      // the top of the stack; st[0..sp-2] below it
   int sp = 0;
@@ -818,16 +845,22 @@ __device__ __forceinline__ uint32_t eval_pred_rows(const tqpk_predicate& P, cons
         top = bits_of<4 * Q>([&](int i) { return x[i] != 0; });
         break;
       }
-      default: {                           // text
-        top = 0;
-#pragma unroll 1
-        for (int q = 0; q < Q; ++q)
-          if (r0[q] < n) top |= str_leaf4(P, I, r0[q], n) << (4 * q);
-        break;
-      }
+      default: top = text(I); break;
     }
   }
-  return top & valid;
+  return top & valid_rows<Q>(r0, n);
+}
+
+template <int Q>
+__device__ __forceinline__ uint32_t eval_pred_rows(const tqpk_predicate& P, const int64_t (&r0)[Q], int64_t n, bool vec) {
+  if (r0[0] >= n) return 0;
+  return eval_pred_with<Q>(P, r0, n, vec, [&](const tqpk_pred_insn& I) {
+    uint32_t m = 0;
+#pragma unroll 1
+    for (int q = 0; q < Q; ++q)
+      if (r0[q] < n) m |= str_leaf4(P, I, r0[q], n) << (4 * q);
+    return m;
+  });
 }
 
 // Row filter: a u8 mask column, a predicate program, or neither (all rows).

@@ -10,6 +10,8 @@
 // keeps row order (what tensor[mask] gives).
 #include <stdio.h>
 
+#include <algorithm>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -73,6 +75,55 @@ __global__ void __launch_bounds__(kBlock, Q == 1 ? 6 : 3) k_filter_mask(const __
       } else {
         for (int j = 0; j < 4 && r0[q] + j < n; ++j) mask[r0[q] + j] = (b >> j) & 1u;
       }
+    }
+  }
+  if (count) {
+    local = __reduce_add_sync(0xffffffffu, local);
+    if ((threadIdx.x & 31) == 0 && local) atomicAdd(count, (unsigned long long)local);
+  }
+}
+
+// Programs with text: the block takes 1024 rows through the program together, and a text instruction stages
+// their bytes 256 rows at a time in shared memory (coalesced), where each thread searches one row; the
+// verdicts go back to the rows' owners as bits.  Searched in place, every byte of a warp's rows was a scattered
+// load (54 us for a prefix and a two-part pattern on 800 K rows of 25 bytes).
+__global__ void __launch_bounds__(kBlock) k_filter_text(const __grid_constant__ tqpk_predicate P, int64_t n,
+                                                        uint8_t* __restrict__ mask, unsigned long long* count, int vec,
+                                                        int mask_vec) {
+  extern __shared__ __align__(16) int8_t stage[];
+  __shared__ unsigned s_bits[4 * kBlock / 32];
+  unsigned local = 0;
+  for (int64_t t0 = blockIdx.x * (int64_t)(4 * kBlock); t0 < n; t0 += (int64_t)gridDim.x * (4 * kBlock)) {
+    const int64_t r0[1] = {t0 + 4 * threadIdx.x};
+    const uint32_t b = eval_pred_with<1>(P, r0, n, vec, [&](const tqpk_pred_insn& I) {
+      const int64_t stride = str_stride(P, I.col);
+      const int8_t* base = static_cast<const int8_t*>(P.cols[I.col]);
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        const int64_t q0 = t0 + j * kBlock;
+        const int rows = (int)(n - q0 < kBlock ? (n - q0 < 0 ? 0 : n - q0) : kBlock);
+        __syncthreads();
+        if (rows > 0) {                      // a substring's last row ends before its stride does
+          const int bytes = (int)((rows - 1) * stride) + P.widths[I.col];
+          const int8_t* s = base + q0 * stride;
+          const int whole = (reinterpret_cast<uintptr_t>(s) & 15u) == 0 ? bytes / 16 : 0;
+          for (int i = threadIdx.x; i < whole; i += kBlock)
+            reinterpret_cast<uint4*>(stage)[i] = reinterpret_cast<const uint4*>(s)[i];
+          for (int i = whole * 16 + threadIdx.x; i < bytes; i += kBlock) stage[i] = s[i];
+        }
+        __syncthreads();
+        const bool ok = (int)threadIdx.x < rows && str_leaf(P, I, stage + (int)threadIdx.x * (int)stride);
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        if ((threadIdx.x & 31) == 0) s_bits[(j * kBlock + threadIdx.x) >> 5] = m;
+      }
+      __syncthreads();
+      return (s_bits[threadIdx.x >> 3] >> (4 * (threadIdx.x & 7))) & 0xfu;
+    });
+    local += __popc(b);
+    if (mask_vec && r0[0] + 4 <= n) {
+      *reinterpret_cast<uint32_t*>(mask + r0[0]) = (b & 1u) | ((b & 2u) << 7) | ((b & 4u) << 14) | ((b & 8u) << 21);
+    } else {
+      for (int j = 0; j < 4 && r0[0] + j < n; ++j) mask[r0[0] + j] = (b >> j) & 1u;
     }
   }
   if (count) {
@@ -504,9 +555,17 @@ extern "C" int tqpk_filter_mask(const tqpk_predicate* h_pred, int64_t n, uint8_t
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int mask_vec = (reinterpret_cast<uintptr_t>(d_mask) & 3u) == 0;
   timing_before(KID_FILTER_MASK, s);
-  // text programs keep every warp busy with their bytes: four rows a thread spread them over more warps
-  bool text = false;
-  for (int k = 0; k < h_pred->n_insn; ++k) text = text || h_pred->insn[k].op >= TQPK_P_STRCMP;
+  int64_t text = 0;              // the widest text row read
+  for (int k = 0; k < h_pred->n_insn; ++k)
+    if (h_pred->insn[k].op >= TQPK_P_STRCMP) text = std::max(text, str_stride(*h_pred, h_pred->insn[k].col));
+  if (text > 0 && text * kBlock <= 47 * 1024) {       // beside the verdicts in 48 KB
+    k_filter_text<<<grid_for((n + 3) / 4, 8), kBlock, (size_t)text * kBlock, s>>>(
+        *h_pred, n, d_mask, d_count, pred_vec_ok(h_pred) ? 1 : 0, mask_vec);
+    timing_after(KID_FILTER_MASK, s);
+    TQPK_CHECK_LAUNCH();
+    return TQPK_OK;
+  }
+  // wider text stays four rows a thread: its bytes keep every warp busy
   const bool many = n >= kManyRows && !text;
   auto kernel = many ? k_filter_mask<4> : k_filter_mask<1>;
   kernel<<<grid_for((n + 3) / 4 / (many ? 4 : 1), 8), kBlock, 0, s>>>(*h_pred, n, d_mask, d_count,

@@ -81,30 +81,12 @@ __host__ __device__ __forceinline__ int sort_key_digits(const SortKey& K) {
 __device__ __forceinline__ uint64_t sort_image(const SortKey& K, int64_t e) {
   const int64_t r = K.rows ? K.rows[e] : e;
   if (K.width) {                     // bytes word*8 .. word*8+7, big-endian, zero past the width
-    const uint8_t* s = static_cast<const uint8_t*>(K.col) + r * K.width + K.word * 8;
     const int left = K.width - K.word * 8;
-    const unsigned off = (unsigned)(reinterpret_cast<uintptr_t>(s) & 3u);
-    uint64_t w = 0;
-    // Eight bytes as two or three aligned words where those lie in this row or the one before it, the bytes
-    // past the second word one by one where the third would leave the row: byte loads a row, each behind the
-    // last, made a text key's set-up 12 us of 27.6 K rows, now ~4.
-    if (left >= 8 && (off == 0 || K.word > 0 || r > 0)) {
-      const unsigned* a = reinterpret_cast<const unsigned*>(s - off);
-      const unsigned w0 = a[0], w1 = a[1];
-      unsigned w2 = 0;
-      if (off && left >= 11) {
-        w2 = a[2];
-      } else {
-#pragma unroll 1
-        for (unsigned i = 0; i < off; ++i) w2 |= (unsigned)s[8 - off + i] << (8 * i);
-      }
-      const unsigned lo = __funnelshift_r(w0, w1, 8 * off), hi = __funnelshift_r(w1, w2, 8 * off);
-      w = ((uint64_t)__byte_perm(lo, 0, 0x0123) << 32) | __byte_perm(hi, 0, 0x0123);
-    } else {
-      const int m = left < 8 ? left : 8;
-#pragma unroll 1
-      for (int i = 0; i < m; ++i) w |= static_cast<uint64_t>(s[i]) << (56 - 8 * i);
-    }
+    // big-endian; read byte by byte, each load behind the last, it made a text key's set-up 12 us of 27.6 K
+    // rows, as words ~4
+    const uint64_t le = load_bytes8(static_cast<const uint8_t*>(K.col) + r * K.width + K.word * 8, left,
+                                    K.word > 0 || r > 0);
+    uint64_t w = ((uint64_t)__byte_perm((unsigned)le, 0, 0x0123) << 32) | __byte_perm((unsigned)(le >> 32), 0, 0x0123);
     if (K.dt == TQPK_I8)             // int8 bytes order as signed values
       w ^= left >= 8 ? 0x8080808080808080ull : 0x8080808080808080ull & ~(~0ull >> (8 * left));
     return K.desc ? ~w : w;
