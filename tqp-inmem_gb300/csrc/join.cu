@@ -57,6 +57,7 @@ __global__ void k_count_status(const int64_t* count, int* err) {
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_join_build_direct(const void* keys, int dt, RowFilter F, int64_t nb,
                                                               int64_t kmin, int kvec, R* __restrict__ dir, int* dup) {
+  bool repeated = false;
   const int64_t groups = (nb + 3) >> 2;
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < groups;
        g += (int64_t)gridDim.x * blockDim.x) {
@@ -71,19 +72,27 @@ __global__ void __launch_bounds__(kBlock) k_join_build_direct(const void* keys, 
     if (!b) continue;
     int64_t x[4];
     ld4_int(keys, dt, r0, nb, kvec != 0, x);
+    // of neighbouring rows with one key (a table stored by it) only the last is exchanged
+    unsigned last = b;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (((b >> j) & 3u) == 3u && x[j] == x[j + 1]) last &= ~(1u << j);
+    repeated |= last != b;
     R old[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       old[j] = R(~R(0));
-      if ((b >> j) & 1u) {
+      if ((last >> j) & 1u) {
         if (sizeof(R) == 4) old[j] = (R)atomicExch(reinterpret_cast<unsigned*>(&dir[x[j] - kmin]), (unsigned)(r0 + j));
         else old[j] = (R)atomicExch(reinterpret_cast<unsigned long long*>(&dir[x[j] - kmin]), (unsigned long long)(r0 + j));
       }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (old[j] != R(~R(0))) *dup = 1;
+    for (int j = 0; j < 4; ++j) repeated |= old[j] != R(~R(0));
   }
+  // one store per CTA: a store per repeated row queued on the word (6 M rows of a key repeated four times: 50
+  // us, 77 with a row count per key beside the directory)
+  if (__syncthreads_or(repeated) && threadIdx.x == 0) *dup = 1;
 }
 
 // After the stable sort (csr[i] = i-th build row in (key, row) order): each run's range by slot (DIRECT,
@@ -577,17 +586,39 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
   }
 }
 
-__global__ void k_gather(int ncols, const __grid_constant__ ColSet C, const int64_t* __restrict__ idx, int64_t n,
-                         int null_aware) {
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = idx[j];
-    const bool isnull = null_aware && i == TQPK_NULL_INDEX;
+// Column c of the rows idx[j], four rows per thread: their reads are all in flight before the first write
+// (one row at a time, a thread waited for every column of it: 41 us for the six columns of 1.5 M joined rows).
+constexpr int kGatherRows = 4;
+
+template <class T>
+__device__ __forceinline__ void gather_column(const void* in, void* out, const int64_t (&i)[kGatherRows], int64_t j0,
+                                              int64_t n, unsigned null, T null_value) {
+  const T* src = static_cast<const T*>(in);
+  T v[kGatherRows];
+#pragma unroll
+  for (int u = 0; u < kGatherRows; ++u) v[u] = j0 + u * kBlock < n && !((null >> u) & 1u) ? src[i[u]] : null_value;
+#pragma unroll
+  for (int u = 0; u < kGatherRows; ++u)
+    if (j0 + u * kBlock < n) static_cast<T*>(out)[j0 + u * kBlock] = v[u];
+}
+
+__global__ void __launch_bounds__(kBlock) k_gather(int ncols, const __grid_constant__ ColSet C,
+                                                   const int64_t* __restrict__ idx, int64_t n, int null_aware) {
+  for (int64_t t0 = blockIdx.x * (int64_t)(kGatherRows * kBlock); t0 < n;
+       t0 += (int64_t)gridDim.x * (kGatherRows * kBlock)) {
+    const int64_t j0 = t0 + threadIdx.x;
+    int64_t i[kGatherRows];
+    unsigned null = 0;
+#pragma unroll
+    for (int u = 0; u < kGatherRows; ++u) i[u] = j0 + u * kBlock < n ? idx[j0 + u * kBlock] : 0;
+#pragma unroll
+    for (int u = 0; u < kGatherRows; ++u) null |= (unsigned)(null_aware && i[u] == TQPK_NULL_INDEX) << u;
     for (int c = 0; c < ncols; ++c) {
       switch (C.size[c]) {
-        case 1: static_cast<uint8_t*>(C.out[c])[j] = isnull ? (uint8_t)(int8_t)TQPK_NULL_INDEX : static_cast<const uint8_t*>(C.in[c])[i]; break;
-        case 4: static_cast<int32_t*>(C.out[c])[j] = isnull ? TQPK_NULL_INDEX : static_cast<const int32_t*>(C.in[c])[i]; break;
-        case 8: static_cast<int64_t*>(C.out[c])[j] = isnull ? TQPK_NULL_INDEX : static_cast<const int64_t*>(C.in[c])[i]; break;
-        default: static_cast<double*>(C.out[c])[j] = isnull ? (double)TQPK_NULL_INDEX : static_cast<const double*>(C.in[c])[i]; break;
+        case 1: gather_column<uint8_t>(C.in[c], C.out[c], i, j0, n, null, (uint8_t)(int8_t)TQPK_NULL_INDEX); break;
+        case 4: gather_column<int32_t>(C.in[c], C.out[c], i, j0, n, null, TQPK_NULL_INDEX); break;
+        case 8: gather_column<int64_t>(C.in[c], C.out[c], i, j0, n, null, TQPK_NULL_INDEX); break;
+        default: gather_column<double>(C.in[c], C.out[c], i, j0, n, null, (double)TQPK_NULL_INDEX); break;
       }
     }
   }
@@ -1044,7 +1075,7 @@ extern "C" int tqpk_gather(int32_t ncols, const void* const* cols_in, const int3
     C.out[c] = cols_out[c];
     C.size[c] = (dts[c] == TQPK_F64) ? 9 : sz;  // 9: float64 (null fill is -64.0)
   }
-  k_gather<<<grid_for(n_idx, 8), kBlock, 0, static_cast<cudaStream_t>(stream)>>>(ncols, C, idx, n_idx, null_aware);
+  k_gather<<<grid_for((n_idx + kGatherRows - 1) / kGatherRows, 8), kBlock, 0, static_cast<cudaStream_t>(stream)>>>(ncols, C, idx, n_idx, null_aware);
   TQPK_CHECK_LAUNCH();
   return TQPK_OK;
 }

@@ -945,8 +945,9 @@ static int sort_large(const SortKeySet& S, const int64_t* perm_in, int64_t n, in
   A.status = status;
   A.ctl = ctl;
   A.nk = S.n;
-  const int gx = (int)std::max<int64_t>(1, std::min<int64_t>((n + kHistThreads * 16 - 1) / (kHistThreads * 16),
-                                                             (int64_t)num_sms() * 2));
+  // four rows a thread for one key (0.8 M rows: 13 us, 18 with sixteen); several keys fill the SMs together
+  const int64_t per_cta = (int64_t)kHistThreads * (S.n == 1 ? 4 : 16);
+  const int gx = (int)std::max<int64_t>(1, std::min<int64_t>((n + per_cta - 1) / per_cta, (int64_t)num_sms() * 2));
   // eight letters of text rarely differ in the first four only: text is sorted by every digit
   for (int k = 0; k < S.n; ++k) A.every |= S.k[k].width ? 1u << k : 0u;
   for (int round = 0; round < 2; ++round) {
