@@ -622,6 +622,9 @@ def groupby_source(spec, pred, plan) -> Tuple[str, str, int, int]:
         src += ["    " + l for l in _load_lines(pcols, pred.dtypes, "P", "pp", "n", "vp != 0")]
     src += ["    " + l for l in _load_lines(kcols, S.key_dtypes, "Kc", "kp", "n", "vk != 0")]
     src += ["    " + l for l in _load_lines(ecols, S.col_dtypes, "Cv", "cp", "n", "vc != 0")]
+    if not private and not shared:
+        src.append("    i64 held = -1;")
+        src.append("    u64 " + ", ".join(f"h{a} = 0" for a in range(A)) + ";")
     src.append("#pragma unroll")
     src.append("    for (int j = 0; j < 4; ++j) {")
     src.append("      if (r0 + j >= n) break;")
@@ -649,8 +652,24 @@ def groupby_source(spec, pred, plan) -> Tuple[str, str, int, int]:
         elif shared:
             src.append("      " + _merge_atomic(acc, f"&sm[slot * A + {a}]", v))
         else:
-            src.append("      " + _merge_atomic(acc, f"&gacc[{a} * K + slot]", v, glob=True))
+            src.append(f"      const u64 x{a} = {v};")
+    if not private and not shared:
+        # rows of one thread with one slot (a table stored by its key) are combined before the table is
+        # updated: 6 M lines of 1.5 M orders took 18 M scattered reductions
+        src.append("      if (slot == held) {")
+        src += [f"        h{a} = {_combine(S.accs[a], f'h{a}', f'x{a}')};" for a in range(A)]
+        src.append("      } else {")
+        src.append("        if (held >= 0) {")
+        src += ["          " + _merge_atomic(S.accs[a], f"&gacc[{a} * K + held]", f"h{a}", glob=True) for a in range(A)]
+        src.append("        }")
+        src.append("        held = slot;")
+        src += [f"        h{a} = x{a};" for a in range(A)]
+        src.append("      }")
     src.append("    }")
+    if not private and not shared:
+        src.append("    if (held >= 0) {")
+        src += ["      " + _merge_atomic(S.accs[a], f"&gacc[{a} * K + held]", f"h{a}", glob=True) for a in range(A)]
+        src.append("    }")
     src.append("  }")
     if private:
         src.append("  __syncthreads();")
