@@ -237,6 +237,11 @@ int tqpk_compact_noalloc(const tqpk_predicate* h_pred, const uint8_t* d_mask, in
 int tqpk_key_range(const void* d_col, int32_t dtype, int64_t n, void* d_scratch, int64_t* h_min,
                    int64_t* h_max, tqpk_stream stream);
 
+/* The same for several columns, each over its own rows, with one
+ * synchronisation in all.  d_scratch: 128 bytes per column.                */
+int tqpk_key_ranges(int32_t n_cols, const void* const* d_cols, const int32_t* h_dtypes, const int64_t* h_rows,
+                    void* d_scratch, int64_t* h_min, int64_t* h_max, tqpk_stream stream);
+
 /* Test hook, no counterpart in the reference: the poll limit of the
  * compaction's look-back (<= its default) and a tile whose CTA publishes
  * nothing (-1: none).  With a tile stalled, its successors' bounded waits run

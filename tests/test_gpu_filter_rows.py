@@ -129,3 +129,11 @@ def test_gather_of_text_rows(n, width):
     idx[0] = 699
     got = gather_rows(torch.from_numpy(t).cuda(), torch.from_numpy(idx).cuda())
     np.testing.assert_array_equal(got.cpu().numpy(), t[idx])
+
+
+def test_key_ranges_of_several_columns():
+    from tqpk.ops import key_range, key_ranges
+    rng = np.random.default_rng(2)
+    cols = [torch.from_numpy(c).cuda() for n in (1, 5000, MANY + 3) for c in _columns(rng, n)[:4]]
+    cols.append(torch.empty(0, dtype=torch.int32, device="cuda"))
+    assert key_ranges(cols) == [key_range(c) for c in cols]

@@ -228,12 +228,15 @@ __global__ void __launch_bounds__(kBlock) k_compact(const __grid_constant__ tqpk
 
 // Min/max of up to four integer key columns over the rows passing a filter,
 // plus the passing-row count.  out = [min0..min3, max0..max3].
-__global__ void k_init_range(int64_t* out, unsigned long long* count) {
+// Range record blockIdx.x of kRangeWords words.
+constexpr int kRangeWords = 16;
+__global__ void k_init_range(int64_t* out) {
+  out += blockIdx.x * kRangeWords;
   if (threadIdx.x < TQPK_MAX_KEYS) {
     out[threadIdx.x] = INT64_MAX;
     out[TQPK_MAX_KEYS + threadIdx.x] = INT64_MIN;
   }
-  if (threadIdx.x == 0) *count = 0;
+  if (threadIdx.x == 0) out[2 * TQPK_MAX_KEYS] = 0;
 }
 
 // Min and max of 4 Q rows' keys where their bit is set, in the column's own width.
@@ -418,6 +421,19 @@ int grid_for(int64_t work_items, int per_sm) {
   return (int)(g < 1 ? 1 : g);
 }
 
+// The range record of the key columns K over the filtered rows, on the device (record initialised before).
+static int launch_range(const tqpk_predicate* pred, const uint8_t* mask, int64_t n, const KeySet& K, bool vec,
+                        int64_t* out, cudaStream_t s) {
+  const RowFilter F = make_filter(pred, mask);
+  const bool many = n >= kManyRows;
+  auto kernel = F.use_pred ? (many ? k_key_range<4, true> : k_key_range<1, true>)
+                           : (many ? k_key_range<4, false> : k_key_range<1, false>);
+  kernel<<<grid_for((n + 3) / 4 / (many ? 4 : 1), 8), kBlock, 0, s>>>(
+      *pred_or_empty(pred), F, n, K, out, reinterpret_cast<unsigned long long*>(out + 2 * TQPK_MAX_KEYS), vec ? 1 : 0);
+  TQPK_CHECK_LAUNCH();
+  return TQPK_OK;
+}
+
 // Shared by the group-by and join planners: min/max of key columns over the
 // filtered rows.  scratch holds 8 int64 + 1 counter; synchronises.
 int key_ranges(const tqpk_predicate* pred, const uint8_t* mask, int64_t n, int nk, const void* const* cols,
@@ -442,18 +458,10 @@ int key_ranges(const tqpk_predicate* pred, const uint8_t* mask, int64_t n, int n
     vec = vec && aligned16(cols[k]);
   }
   int64_t* out = static_cast<int64_t*>(scratch);
-  unsigned long long* cnt = reinterpret_cast<unsigned long long*>(out + 2 * TQPK_MAX_KEYS);
-  k_init_range<<<1, 32, 0, s>>>(out, cnt);
+  k_init_range<<<1, 32, 0, s>>>(out);
   TQPK_CHECK_LAUNCH();
-  if (n > 0) {
-    RowFilter F = make_filter(pred, mask);
-    const bool many = n >= kManyRows;
-    auto kernel = F.use_pred ? (many ? k_key_range<4, true> : k_key_range<1, true>)
-                             : (many ? k_key_range<4, false> : k_key_range<1, false>);
-    kernel<<<grid_for((n + 3) / 4 / (many ? 4 : 1), 8), kBlock, 0, s>>>(*pred_or_empty(pred), F, n, K, out, cnt,
-                                                                        vec ? 1 : 0);
-    TQPK_CHECK_LAUNCH();
-  }
+  const int rc = launch_range(pred, mask, n, K, vec, out, s);
+  if (rc) return rc;
   int64_t host[2 * TQPK_MAX_KEYS + 1];
   TQPK_CUDA(cudaMemcpyAsync(host, out, sizeof(host), cudaMemcpyDeviceToHost, s));
   TQPK_CUDA(cudaStreamSynchronize(s));
@@ -595,6 +603,40 @@ extern "C" int tqpk_key_range(const void* d_col, int32_t dtype, int64_t n, void*
   const int32_t dts[1] = {dtype};
   return key_ranges(nullptr, nullptr, n, 1, cols, dts, h_min, h_max, &cnt, d_scratch,
                     static_cast<cudaStream_t>(stream));
+}
+
+// tqpk_key_range of several columns, each over its own rows, with one host synchronisation; d_scratch holds
+// 128 bytes per column.
+extern "C" int tqpk_key_ranges(int32_t n_cols, const void* const* d_cols, const int32_t* dtypes, const int64_t* rows,
+                               void* d_scratch, int64_t* h_min, int64_t* h_max, tqpk_stream stream) {
+  if (n_cols < 0 || n_cols > TQPK_MAX_COLS || !d_cols || !dtypes || !rows || !d_scratch || !h_min || !h_max)
+    return TQPK_EINVAL;
+  if (n_cols == 0) return TQPK_OK;
+  for (int c = 0; c < n_cols; ++c) {
+    if (rows[c] < 0 || (rows[c] > 0 && !d_cols[c])) return TQPK_EINVAL;
+    if (!is_int_dtype(dtypes[c])) return TQPK_EDTYPE;
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  int64_t* out = static_cast<int64_t*>(d_scratch);
+  k_init_range<<<n_cols, 32, 0, s>>>(out);
+  TQPK_CHECK_LAUNCH();
+  for (int c = 0; c < n_cols; ++c) {
+    if (rows[c] == 0) continue;
+    KeySet K{};
+    K.n = 1;
+    K.col[0] = d_cols[c];
+    K.dt[0] = dtypes[c];
+    const int rc = launch_range(nullptr, nullptr, rows[c], K, aligned16(d_cols[c]), out + c * kRangeWords, s);
+    if (rc) return rc;
+  }
+  int64_t host[TQPK_MAX_COLS * kRangeWords];
+  TQPK_CUDA(cudaMemcpyAsync(host, out, (size_t)n_cols * kRangeWords * 8, cudaMemcpyDeviceToHost, s));
+  TQPK_CUDA(cudaStreamSynchronize(s));
+  for (int c = 0; c < n_cols; ++c) {
+    h_min[c] = rows[c] ? host[c * kRangeWords] : 0;
+    h_max[c] = rows[c] ? host[c * kRangeWords + TQPK_MAX_KEYS] : -1;
+  }
+  return TQPK_OK;
 }
 
 extern "C" size_t tqpk_compact_workspace_bytes(int64_t n) { return compact_status_bytes(n < 0 ? 0 : n); }

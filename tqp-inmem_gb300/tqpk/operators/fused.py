@@ -324,7 +324,7 @@ def _match_star_agg_topk(tensor_group, ops, args, start) -> Optional[dict]:
 
 
 def _run_star_agg_topk(tensor_group, m) -> bool:
-    from ..ops import key_range
+    from ..ops import key_ranges
     from ..pipeline import StarAggTopK
     ak, fka, bk, fkb, ck, fkc = m["keys"]
     v = {c: tensor_group[c] for c in (ak, fka, bk, fkb, ck, fkc)}
@@ -336,14 +336,11 @@ def _run_star_agg_topk(tensor_group, m) -> bool:
         ([tensor_group[c] for c in ff["materialized in"]] if ff else [])
     wait_ready(*dim_vars)
     col = lambda c: tensor_group[c].tensor.reshape(-1)          # noqa: E731
-    doms = []
-    for c in (ak, bk, ck):                                      # the dimension key domains (host reads)
-        if col(c).numel() == 0:
-            return False
-        lo, hi = key_range(col(c))
-        if hi - lo + 1 > (1 << 31):
-            return False
-        doms.append((lo, hi))
+    if any(col(c).numel() == 0 for c in (ak, bk, ck)):
+        return False
+    doms = key_ranges([col(c) for c in (ak, bk, ck)])           # the dimension key domains (one host read)
+    if any(hi - lo + 1 > (1 << 31) for lo, hi in doms):
+        return False
     fact_cols = {c: col(c) for c in set(m["vcols"]) | (set(ff["materialized in"]) if ff else set())}
     a_cols = {c: col(c) for c in fa["materialized in"]} if fa else {}
     try:

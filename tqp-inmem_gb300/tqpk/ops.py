@@ -129,6 +129,21 @@ def key_range(col: torch.Tensor) -> Tuple[int, int]:
     return int(lo.value), int(hi.value)
 
 
+def key_ranges(cols: Sequence[torch.Tensor]) -> List[Tuple[int, int]]:
+    """key_range of several columns with one host read."""
+    lib = L.load()
+    cols = [_col1d(c) for c in cols]
+    _check_cuda(*cols)
+    m = len(cols)
+    lo, hi = (C.c_int64 * m)(), (C.c_int64 * m)()
+    rows = (C.c_int64 * m)(*[c.numel() for c in cols])
+    scratch = _ws(128 * m, cols[0].device)
+    L.check(lib.tqpk_key_ranges(m, _vp_array([c.data_ptr() if c.numel() else None for c in cols]),
+                                _i32_array([code_of(c.dtype) for c in cols]), rows, scratch.data_ptr(), lo, hi,
+                                _stream(cols[0].device)), "tqpk_key_ranges")
+    return list(zip(lo, hi))
+
+
 # ---------------------------------------------------------------- (d) group-by
 def _count_groups_from_keys(prog: AggregateProgram, plan, pred, n: int, device, s: int) -> int:
     """Occupied slots of the group table, from the key columns (and the mask) alone: a
