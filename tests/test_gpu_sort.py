@@ -133,3 +133,37 @@ def test_topk_by_several_keys(n, limit):
                         ([same, coarse], [False, False])):
         got = topk_keys([torch.from_numpy(k).cuda() for k in keys], descs, limit)
         np.testing.assert_array_equal(got.cpu().numpy(), _expected(keys, descs)[:limit])
+
+
+@pytest.mark.parametrize("n", [2049, 8193, 32_768, 32_769, 98_304])
+@pytest.mark.parametrize("first", ["int", "text"])
+def test_rows_that_come_in_order(n, first):
+    """The cluster leaves out the keys by which the rows already stand in order: all of them, or those
+    behind the first column, here as groups come out of an aggregate.  One pair out of order anywhere
+    (inside a CTA's rows, across two CTAs, at the end) is a full sort again."""
+    rng = np.random.default_rng(n)
+    text = np.zeros((n, 11), np.int8)
+    text[:] = np.frombuffer(b"a-c-e-g-i-k", np.int8)
+    text[:, 9] = rng.integers(97, 110, n)
+    keys = [text, rng.integers(0, 40, n).astype(np.int64), rng.integers(-9, 9, n) * 0.5]
+    descs = [True, False, True]
+    at = _expected(keys, descs)
+    keys = [k[at] for k in keys]
+    _check(keys, descs)                                                   # in order already
+    if first == "int":
+        lead, lead_desc = rng.integers(0, 300, n).astype(np.int64), True
+    else:
+        lead, lead_desc = rng.integers(97, 101, (n, 17)).astype(np.int8), False
+    _check([lead] + keys, [lead_desc] + descs)                            # behind the first column
+    rows = (n + 15) // 16                                                 # of one CTA
+    for p in (0, rows - 1, 5 * rows - 1, min(rows + 600, n - 2), n - 2):
+        other = [k.copy() for k in keys]
+        for k in other:
+            k[[p, p + 1]] = k[[p + 1, p]]
+        _check(other, descs)
+        _check([lead] + other, [lead_desc] + descs)
+    perm = rng.permutation(n)
+    back = [np.empty_like(k) for k in keys]
+    for b, k in zip(back, keys):
+        b[perm] = k
+    _check(back, descs, perm)                                             # in order through the given rows

@@ -1047,7 +1047,7 @@ struct SortKey {
 constexpr int kMaxSortKeys = 32;
 size_t sort_ws_bytes(int64_t n, int nk = 1);
 int sort_keys(const SortKey* keys, int nk, const int64_t* perm_in, int64_t n, int64_t* perm_out, void* ws,
-              size_t ws_bytes, cudaStream_t s);
+              size_t ws_bytes, cudaStream_t s, bool mixed = false);
 
 bool spec_cols_vec(const tqpk_groupby_spec* S);   // all spec columns 16-byte aligned
 

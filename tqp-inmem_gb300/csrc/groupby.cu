@@ -826,7 +826,7 @@ extern "C" int tqpk_groupby_emit(const tqpk_groupby_spec* S, const tqpk_gb_plan*
     HashLayout H = hash_layout(ws, K, (int)A);
     if (groups > K / 2) return TQPK_EINVAL;       // the table has two slots per row
     const SortKey by_packed{H.pk, nullptr, TQPK_I64, 0, 0, 0};
-    int rc2 = sort_keys(&by_packed, 1, nullptr, groups, H.perm, H.sort_ws, H.sort_bytes, s);
+    int rc2 = sort_keys(&by_packed, 1, nullptr, groups, H.perm, H.sort_ws, H.sort_bytes, s, true);
     if (rc2) return rc2;
     const GbDev G = to_dev(*plan, S->n_keys);
     k_emit_hash<<<grid_for(groups, 4), kBlock, 0, s>>>(*S, G, H.gacc, groups, H.pk, H.cslot, H.perm, E);

@@ -324,7 +324,7 @@ extern "C" int tqpk_key_encode(int32_t n_keys, const void* const* h_keys, const 
       run[kMaxSortKeys - 1 - m++] = SortKey{K.col[k], rep_of_gid, K.dt[k], 0, K.width[k], w};
       if (--left == 0 || m == kMaxSortKeys) {
         int64_t* out = (cur == perm_a) ? perm_b : perm_a;
-        const int rc = sort_keys(run + kMaxSortKeys - m, m, cur, G, out, sort_ws, sort_ws_bytes(n, kMaxSortKeys), s);
+        const int rc = sort_keys(run + kMaxSortKeys - m, m, cur, G, out, sort_ws, sort_ws_bytes(n, kMaxSortKeys), s, true);
         if (rc) return rc;
         cur = out;
         m = 0;

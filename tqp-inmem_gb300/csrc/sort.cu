@@ -57,6 +57,7 @@ constexpr int kHistThreads = 512;
 struct SortKeySet {
   SortKey k[kMaxSortKeys];
   int n;
+  int mixed;                         // the caller knows that the rows come in no order
 };
 
 struct SortCtl {
@@ -621,7 +622,42 @@ struct ClusterSmem {
   unsigned values[8][8];             // the same over the cluster
   uint8_t rank[8][256];              // a value's place among them
   int width[8];                      // bits of a position's rank
+  unsigned broken;                   // this CTA's word of cluster_broken
 };
+
+// Whether rows e0, e1 are out of order by keys[from..to).
+__device__ __forceinline__ bool out_of_order(const SortKeySet& S, int from, int to, int64_t e0, int64_t e1) {
+  for (int f = from; f < to; ++f) {
+    const uint64_t a = sort_image(S.k[f], e0), b = sort_image(S.k[f], e1);
+    if (a != b) return a > b;
+  }
+  return false;
+}
+
+// What this CTA's rows (and the row after them) say about the order the rows come in.  Bit 0: not the
+// order of all the keys; bit 1: not the order of the keys behind the first column (from `rest` on).  The
+// groups of an aggregate come in the order of their keys, and most reports sort them by a total and then
+// those keys, or by the keys alone: then the first column's passes are the whole sort, or there are none.
+// Rows in any other order say so within the first 512 of a CTA, and the CTA stops looking.
+// 27.6 K groups by a count and then their three keys, two of them text: 129 us without, 47 with; 27.6 K
+// random integers 25 us without, 27 with, 60 K 39.6 and 39.7.
+template <int ITEMS>
+__device__ __forceinline__ unsigned cluster_broken(const SortKeySet& S, int rest, const int64_t* perm_in, int n,
+                                                   int first, int mine) {
+  unsigned broken = rest < S.n ? 0 : 2;
+  for (int j = 0; j < ITEMS && broken != 3; ++j) {
+    const int i = j * kClusterThreads + threadIdx.x;
+    bool all = false, later = false;
+    if (i < mine && first + i + 1 < n) {
+      const int64_t e0 = perm_in ? perm_in[first + i] : first + i, e1 = perm_in ? perm_in[first + i + 1] : first + i + 1;
+      if (!(broken & 1)) all = out_of_order(S, 0, S.n, e0, e1);
+      if (!(broken & 2)) later = out_of_order(S, rest, S.n, e0, e1);
+    }
+    if (__syncthreads_or(all)) broken |= 1;
+    if (__syncthreads_or(later)) broken |= 2;
+  }
+  return broken;
+}
 
 // Recodes this CTA's rows' words of text (M.key[cur][i]) as the ranks of their bytes; returns the bits used.
 template <int ITEMS>
@@ -695,9 +731,15 @@ __global__ void __launch_bounds__(kClusterThreads) k_sort_cluster(const __grid_c
   const int mine = max(0, min((int)R, n - cta * (int)R));
   int cur = 0, pass = 0;
   for (int i = threadIdx.x; i < mine; i += kClusterThreads) M.val[0][i] = (unsigned)(cta * (int)R + i);
+  int rest = 1;                      // the second column's first key
+  while (rest < S.n && S.k[rest].word > 0) ++rest;
+  const unsigned here = S.mixed ? 3 : cluster_broken<ITEMS>(S, rest, perm_in, n, cta * (int)R, mine);
+  if (threadIdx.x == 0) M.broken = here;
   cluster.sync();                    // every CTA of the cluster runs before any writes to another
+  const unsigned broken = __reduce_or_sync(0xffffffffu, *cluster.map_shared_rank(&M.broken, lane % kClusterCtas));
+  const int sorted_from = !(broken & 1) ? 0 : !(broken & 2) ? rest : S.n;
   bool packed = false;               // where the positions are: in key, or in val
-  for (int key = S.n - 1; key >= 0; --key) {
+  for (int key = sorted_from - 1; key >= 0; --key) {
     SortKey K = S.k[key];
     const bool text = K.width > 0, desc = K.desc != 0;
     if (text) K.desc = 0;            // turned round after the recoding
@@ -950,8 +992,8 @@ static int sort_large(const SortKeySet& S, const int64_t* perm_in, int64_t n, in
   const int gx = (int)std::max<int64_t>(1, std::min<int64_t>((n + per_cta - 1) / per_cta, (int64_t)num_sms() * 2));
   // eight letters of text rarely differ in the first four only: text is sorted by every digit
   for (int k = 0; k < S.n; ++k) A.every |= S.k[k].width ? 1u << k : 0u;
-  for (int round = 0; round < 2; ++round) {
-    if (round == 0) {
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    if (attempt == 0) {
       TQPK_CUDA(cudaMemsetAsync(ws, 0, zeroed, s));
       k_sort_hist<<<dim3(gx, S.n), kHistThreads, 0, s>>>(S, perm_in, n, hist, offsets, ctl);
       TQPK_CHECK_LAUNCH();
@@ -975,17 +1017,19 @@ static int sort_large(const SortKeySet& S, const int64_t* perm_in, int64_t n, in
     if (h[0]) return h[0];
     if (!h[1]) return TQPK_OK;
   }
-  return TQPK_ETIMEOUT;              // not reached: the second round sorts by every digit
+  return TQPK_ETIMEOUT;              // not reached: the second attempt sorts by every digit
 }
 
 // The stable order of elements perm_in[0..n) (null: 0..n-1) by keys[0], then keys[1], ...  perm_out must
-// not overlap perm_in.  n > kClusterSort synchronises once (the look-back's error word).
+// not overlap perm_in.  n > kClusterSort synchronises once (the look-back's error word).  mixed: the rows are
+// known to come in no order (entries of a hash table in the order they were claimed), so nothing looks for one.
 int sort_keys(const SortKey* keys, int nk, const int64_t* perm_in, int64_t n, int64_t* perm_out, void* ws,
-              size_t ws_bytes, cudaStream_t s) {
+              size_t ws_bytes, cudaStream_t s, bool mixed) {
   if (nk < 1 || nk > kMaxSortKeys) return TQPK_EUNSUPPORTED;
   if (n == 0) return TQPK_OK;
   SortKeySet S{};
   S.n = nk;
+  S.mixed = mixed;
   for (int k = 0; k < nk; ++k) S.k[k] = keys[k];
   if (n <= kSmallSort) {   // no workspace needed
     k_sort_small<<<1, 1024, 0, s>>>(S, perm_in, (int)n, perm_out);
