@@ -968,37 +968,6 @@ __device__ __forceinline__ uint64_t lookback_warp(uint64_t* status, int64_t tile
   return excl;
 }
 
-// Per-thread variant (one independent chain per thread, e.g. one radix digit
-// per thread).  status is indexed status[tile * stride + lane_id].
-__device__ __forceinline__ uint64_t lookback_thread(uint64_t* status, int64_t tile, int stride, int id,
-                                                    uint64_t aggregate, int* err) {
-  if (tile == 0) {
-    st_release(&status[id], kFlagInc | aggregate);
-    return 0;
-  }
-  st_release(&status[tile * stride + id], kFlagAgg | aggregate);
-  uint64_t excl = 0;
-  int64_t p = tile - 1;
-  int spins = 0;
-  while (p >= 0) {
-    const uint64_t s = ld_acquire(&status[p * stride + id]);
-    const uint64_t f = s >> 62;
-    if (f == 0) {
-      if (++spins > kSpinLimit) {
-        set_error(err, TQPK_ETIMEOUT);
-        break;
-      }
-      __nanosleep(64);
-      continue;
-    }
-    excl += s & kValMask;
-    if (f == 2) break;
-    --p;
-  }
-  st_release(&status[tile * stride + id], kFlagInc | ((excl + aggregate) & kValMask));
-  return excl;
-}
-
 // ---------------------------------------------------- kernel timing hook
 // tqpk_timing_begin(id) makes every launch of kernel `id` record a pair of
 // CUDA events around itself on its own stream; tqpk_timing_end() sums them.

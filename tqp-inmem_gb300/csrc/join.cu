@@ -189,7 +189,6 @@ __device__ __forceinline__ int64_t join_range(const JoinDir& D, int64_t key, int
   return (int64_t)(q.y - q.x);
 }
 
-constexpr unsigned kNoRow = ~0u;
 
 // Probes with at most one output per row.  dup (inner join of a build side not known to be unique):
 // nothing is done when it is set.
