@@ -40,7 +40,7 @@ def _keys(kind, rng, nb):
 @pytest.mark.parametrize("kind", ["unique", "repeated", "one key", "sparse"])
 @pytest.mark.parametrize("nb,npr", [(1, 1), (300, 127), (300, 1024), (2047, 1025), (40, 4096), (5000, 4097), (900, 70_001)])
 def test_pairs(kind, nb, npr):
-    from tqpk.ops import join_build, join_probe
+    from tqpk.ops import join_build, join_directory, join_probe
     rng = np.random.default_rng(nb * 7 + npr)
     bk = _keys(kind, rng, nb)
     pk = np.where(rng.integers(0, 3, npr) > 0, bk[rng.integers(0, nb, npr)], rng.integers(-10**6, 10**6, npr)).astype(np.int64)
@@ -52,7 +52,16 @@ def test_pairs(kind, nb, npr):
         tb, tp = torch.from_numpy(bk).cuda(), torch.from_numpy(np.concatenate([[0], pk])).cuda()[1:]   # unaligned
         mb = torch.from_numpy(bm).cuda() if masked else None
         mp = torch.from_numpy(np.concatenate([[False], pm])).cuda()[1:] if masked else None
-        build = join_build(tb, mb)
+        build = join_directory(tb, mb)
+        whole = join_build(tb, mb)
+        assert whole.unique in (0, 1)
+        tb.zero_()                                      # a complete build side does not read its keys again
+        for jtype in ("inner", "right-outer"):
+            bi, pi = join_probe(whole, tp, mp, jtype)
+            ebi, epi = _expected(bk, bm, pk, pm, jtype)
+            np.testing.assert_array_equal(pi.cpu().numpy(), epi, err_msg=jtype)
+            np.testing.assert_array_equal(bi.cpu().numpy(), ebi, err_msg=jtype)
+        tb.copy_(torch.from_numpy(bk))
         for jtype in ("right-semi", "inner", "right-anti", "right-outer", "inner"):
             bi, pi = join_probe(build, tp, mp, jtype)
             ebi, epi = _expected(bk, bm, pk, pm, jtype)

@@ -99,14 +99,16 @@ __global__ void __launch_bounds__(kBlock) k_join_build_direct(const void* keys, 
 // run zeroed before), or the head flags (SORTED).
 template <class R>
 __global__ void k_join_runs(const void* keys, int dt, const int64_t* csr, int64_t m, int64_t kmin, int direct,
-                            R* run, int64_t* head_flag_rows) {
+                            int64_t slots, R* run, int64_t* head_flag_rows) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t k = ld_int(keys, dt, csr[i]);
     const bool head = (i == 0) || ld_int(keys, dt, csr[i - 1]) != k;
     if (direct) {
       const bool tail = i + 1 == m || ld_int(keys, dt, csr[i + 1]) != k;
-      if (head) run[2 * (k - kmin)] = (R)i;
-      if (tail) run[2 * (k - kmin) + 1] = (R)(i + 1);
+      const int64_t slot = k - kmin;
+      if (slot < 0 || slot >= slots) continue;          // keys changed since the plan was made: stay in bounds
+      if (head) run[2 * slot] = (R)i;
+      if (tail) run[2 * slot + 1] = (R)(i + 1);
     } else {
       head_flag_rows[i] = head ? 1 : 0;
     }
@@ -832,10 +834,12 @@ extern "C" int tqpk_join_rows(tqpk_join_plan* plan, const void* keys, int32_t dt
   if (direct) TQPK_CUDA(cudaMemsetAsync(L.run, 0, 2 * plan->slots * (is_wide(*plan) ? 8 : 4), s));
   if (is_wide(*plan))
     k_join_runs<uint64_t><<<grid_for(plan->nb_rows, 8), kBlock, 0, s>>>(keys, dt, L.csr, plan->nb_rows, plan->key_min,
-                                                                        direct, static_cast<uint64_t*>(L.run), L.head);
+                                                                        direct, plan->slots, static_cast<uint64_t*>(L.run),
+                                                                        L.head);
   else
     k_join_runs<unsigned><<<grid_for(plan->nb_rows, 8), kBlock, 0, s>>>(keys, dt, L.csr, plan->nb_rows, plan->key_min,
-                                                                        direct, static_cast<unsigned*>(L.run), L.head);
+                                                                        direct, plan->slots, static_cast<unsigned*>(L.run),
+                                                                        L.head);
   TQPK_CHECK_LAUNCH();
   if (!direct) {
     const int64_t tiles = (plan->nb_rows + kTile - 1) / kTile;

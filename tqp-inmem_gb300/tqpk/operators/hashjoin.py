@@ -27,7 +27,7 @@ from typing import Dict, List
 import torch
 
 from .. import _lib as L
-from ..ops import check_deferred, compact, filter_mask, gather, join_build, join_pairs, join_probe, mark_rows
+from ..ops import check_deferred, compact, filter_mask, gather, join_build, join_directory, join_pairs, join_probe, mark_rows
 from ..predicate import compile_filter, has_strings
 from ..variable import make_like, wait_ready
 from ._materialize import materialize
@@ -59,7 +59,7 @@ def _pairs(tensors_left, tensors_right, left_key, right_key, condition_list, jty
     lk = tensors_left[left_key].tensor
     rk = tensors_right[right_key].tensor
     wait_ready(tensors_left[left_key])
-    b = join_build(lk, left_mask)
+    b = join_directory(lk, left_mask) if lk.is_cuda else join_build(lk, left_mask)
     wait_ready(tensors_right[right_key])
     # with extra conditions every form starts from the key-equal pairs (hashjoin.py:100-108)
     pred = _pair_predicate(tensors_left, tensors_right, condition_list) if condition_list and rk.is_cuda else None

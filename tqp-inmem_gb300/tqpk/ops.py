@@ -446,8 +446,19 @@ class JoinBuild:
 
 
 def join_build(keys: torch.Tensor, mask: Optional[torch.Tensor] = None) -> JoinBuild:
-    """The build side's directory (one host read, of the key range).  Whether a key repeats, and the
-    sorted rows of repeated keys, are left to the first probe that needs them."""
+    """The build side, complete when the call returns: it can be probed from any stream or thread, and
+    the keys are not read again."""
+    return _join_build(keys, mask, "tqpk_join_build")
+
+
+def join_directory(keys: torch.Tensor, mask: Optional[torch.Tensor] = None) -> JoinBuild:
+    """The build side's directory only, with one host read (of the key range) instead of two.  Whether a
+    key repeats, and the sorted rows of repeated keys, are left to the first probe that needs them, so
+    keys and mask stay as they are until then, and the probes run on this call's stream."""
+    return _join_build(keys, mask, "tqpk_join_directory")
+
+
+def _join_build(keys: torch.Tensor, mask: Optional[torch.Tensor], stage: str) -> JoinBuild:
     lib = L.load()
     keys = _col1d(keys)
     _check_cuda(keys, mask)
@@ -461,7 +472,7 @@ def join_build(keys: torch.Tensor, mask: Optional[torch.Tensor] = None) -> JoinB
                                      mask.data_ptr() if mask is not None else None, n, C.byref(plan),
                                      scratch.data_ptr(), _stream(dev)), "tqpk_join_plan_build")
     build = JoinBuild(plan, _ws(plan.ws_bytes, dev), keys, dev, mask)
-    build._call(lib.tqpk_join_directory, "tqpk_join_directory")
+    build._call(getattr(lib, stage), stage)
     return build
 
 

@@ -97,9 +97,18 @@ _FILTER_MEMO_MAX = 256
 _numbers = itertools.count(1)
 
 
+def _plain(tree) -> bool:
+    """Whether repr(tree) says all of it: lists of strings and numbers."""
+    if isinstance(tree, (list, tuple)):
+        return all(map(_plain, tree))
+    return tree is None or type(tree) in (str, int, float, bool)
+
+
 def _filter_key(tree, columns, subquery, agg):
     """The memo's key, or None for operands it cannot hold by value."""
     if subquery is not None and not isinstance(subquery, (int, float, str)):
+        return None
+    if not _plain(tree):
         return None
     try:
         return (repr(tree), agg, type(subquery), subquery,
@@ -457,7 +466,7 @@ def compile_filter(tree, columns: Dict[int, Any], subquery=None, agg: bool = Fal
         number = next(_numbers)
         if len(_FILTER_MEMO) >= _FILTER_MEMO_MAX:
             _FILTER_MEMO.clear()
-        _FILTER_MEMO[key] = (p, slots, number)
+        _FILTER_MEMO[key] = (bytes(p), slots, number)
     return CompiledPredicate(p, tensors, ids, number)
 
 
