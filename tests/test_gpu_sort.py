@@ -167,3 +167,19 @@ def test_rows_that_come_in_order(n, first):
     for b, k in zip(back, keys):
         b[perm] = k
     _check(back, descs, perm)                                             # in order through the given rows
+
+
+@pytest.mark.parametrize("n", [2049, 70_003, 2_200_001])
+@pytest.mark.parametrize("make", [lambda r, n: r.integers(0, 2557, n).astype(np.int32), lambda r, n: r.integers(0, 3, n).astype(np.uint8),
+                                  lambda r, n: np.full(n, 2.5), lambda r, n: np.where(r.integers(0, 900, n) == 0, np.nan, 1.0),
+                                  lambda r, n: np.sort(r.integers(0, n // 50 + 1, n)), lambda r, n: -np.arange(n)])
+def test_topk_of_few_values(make, n):
+    """The k first of a column with many ties are the first rows of the stable order."""
+    from tqpk.ops import topk_stable
+    rng = np.random.default_rng(n)
+    a = make(rng, n)
+    d = torch.from_numpy(a).cuda()
+    for desc in (False, True):
+        exp = _expected([a], [desc])
+        for k in (1, 10, 33, 100, 256):
+            np.testing.assert_array_equal(topk_stable(d, k, desc).cpu().numpy(), exp[:k], err_msg=str((k, desc)))

@@ -327,8 +327,9 @@ __device__ __forceinline__ void tk_scan_group(const Src& src, int64_t b0, int64_
   }
 }
 
-// Pass 1: each CTA keeps the best key of its group of G items; the last CTA to finish
-// computes the cut from all groups' bests.
+// Pass 1: each CTA keeps the best key of its group of G items and in how many threads' items it is (at
+// most 256, a lower bound of the items that have it; counting those cost 30 us of 160 for 60 M rows); the
+// last CTA to finish computes the cut from all groups' bests.
 template <class Src>
 __global__ void __launch_bounds__(256) k_tk_group_best(Src src, int64_t G, int k, TopkOut O) {
   __shared__ uint64_t red[8];
@@ -336,11 +337,15 @@ __global__ void __launch_bounds__(256) k_tk_group_best(Src src, int64_t G, int k
   __shared__ unsigned s_valid, s_bits;
   if (threadIdx.x == 0) { s_valid = 0; s_bits = 0; }
   __syncthreads();
+  __shared__ unsigned s_equal;
+  if (threadIdx.x == 0) s_equal = 0;
   uint64_t best = ~0ull;
   unsigned valid = 0, nbits = 0;
   tk_scan_group(src, b0, b1, O.bits_set != nullptr, [&](uint64_t key, int64_t, bool has) {
     if (has && key < best) best = key;          // slots without an item carry no key
   }, valid, nbits);
+  const uint64_t own = best;
+  const bool items = valid != 0;
   // one atomic per CTA for each count: per-warp atomics on one address serialise in the L2
   valid = __reduce_add_sync(0xffffffffu, valid);
   nbits = __reduce_add_sync(0xffffffffu, nbits);
@@ -349,8 +354,12 @@ __global__ void __launch_bounds__(256) k_tk_group_best(Src src, int64_t G, int k
     if (nbits) atomicAdd(&s_bits, nbits);
   }
   block_min_u64(best, red);        // its barriers order the shared counts too
+  const unsigned equal = __popc(__ballot_sync(0xffffffffu, items && own == best));
+  if ((threadIdx.x & 31) == 0 && equal) atomicAdd(&s_equal, equal);
+  __syncthreads();
   if (threadIdx.x == 0) {
     O.cand_key[kTopkCap + blockIdx.x] = best;
+    O.cand_idx[kTopkCap + blockIdx.x] = s_equal;
     if (blockIdx.x == 0) *O.ticket = 0;          // the candidate counter of the next pass
     if (s_valid && O.valid_total) atomicAdd(O.valid_total, (unsigned long long)s_valid);
     if (s_bits && O.bits_set) atomicAdd(O.bits_set, (unsigned long long)s_bits);
@@ -525,17 +534,51 @@ __device__ __forceinline__ void tk_final(const Src& src, int k, TopkOut O) {
 
 // Pass 2: the items at or under the cut are appended to the candidate list; the last CTA
 // to finish sorts them (tk_final).  Same groups of G items as pass 1, 256 threads per CTA
-// (tk_final's 8 warps).
+// (tk_final's 8 warps).  A group whose best lies over the cut is not read again, which for
+// independent keys is all but about k of them.  Of the items that tie with the cut only the first
+// can be among the k: those with k or more at or under the cut before them, by the counts of the
+// groups before and of the warp's own rows, are left out.  Without that a column of few values
+// overflowed the list and went through the warp lists of one CTA: the first 10 of 6 M dates 3489 us, now
+// 39 (20 M: 13952 and 86; float64 of few ties, 6 / 20 / 60 M: 47 / 149 / 320 and 45 / 137 / 287).
 template <int R, class Src>
 __global__ void __launch_bounds__(256) k_tk_filter(Src src, int64_t G, int k, TopkOut O) {
   const int lane = threadIdx.x & 31;
   const uint64_t cut = k <= 32 ? tk_bin_cut((int)gridDim.x, k, O) : __ldcg(O.bound);
   const int64_t b0 = (int64_t)blockIdx.x * G, b1 = b0 + G < src.n ? b0 + G : src.n;
   unsigned valid = 0, nbits = 0;
-  tk_scan_group(src, b0, b1, false, [&](uint64_t key, int64_t idx, bool has) {
-    const bool pass = has && key <= cut;
-    const unsigned bal = __ballot_sync(0xffffffffu, pass);
+  __shared__ unsigned s_before;      // items at or under the cut in the groups before (at least so many)
+  if (threadIdx.x == 0) s_before = 0;
+  __syncthreads();
+  const bool any = __ldcg(&O.cand_key[kTopkCap + blockIdx.x]) <= cut;
+  if (any) {
+    unsigned c = 0;
+    for (int g = threadIdx.x; g < (int)blockIdx.x; g += 256) {
+      const uint64_t v = __ldcg(&O.cand_key[kTopkCap + g]);
+      const unsigned e = (unsigned)__ldcg(reinterpret_cast<const long long*>(&O.cand_idx[kTopkCap + g]));
+      c += v < cut ? 1u : v == cut ? e : 0u;
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0 && c) atomicAdd(&s_before, c);
+  }
+  __syncthreads();
+  const int wanted = k - (int)min(s_before, (unsigned)k);       // items that tie with the cut
+  int ties = 0, ties_now = 0;        // of this warp's rows: in the quads before, and in this one
+  int64_t quad = -1;
+  if (any) tk_scan_group(src, b0, b1, false, [&](uint64_t key, int64_t idx, bool has) {
+    const bool under = has && key <= cut;
+    unsigned bal = __ballot_sync(0xffffffffu, under);
     if (!bal) return;
+    const int64_t here = __shfl_sync(0xffffffffu, idx, 0) >> 2;
+    if (here != quad) {
+      ties += ties_now;
+      ties_now = 0;
+      quad = here;
+    }
+    const unsigned tied = __ballot_sync(0xffffffffu, under && key == cut);
+    if (ties < wanted) ties_now += __popc(tied);
+    else bal &= ~tied;
+    if (!bal) return;
+    const bool pass = (bal >> lane) & 1u;
     unsigned at = 0;
     if (lane == 0) at = atomicAdd(O.ticket, (unsigned)__popc(bal));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
