@@ -461,7 +461,8 @@ __global__ void __launch_bounds__(kBlock) k_sort_check(const __grid_constant__ P
     const int64_t i = i0 + lane;
     const unsigned w = i < n ? word[i] : 0;
     const bool joins = i > 0 && i < n && word[i - 1] == w;
-    const bool next = lane < 31 ? __shfl_down_sync(0xffffffffu, (int)joins, 1) : (__shfl_down_sync(0xffffffffu, (int)joins, 1), false);
+    const int below = __shfl_down_sync(0xffffffffu, (int)joins, 1);     // one shuffle, taken by all lanes
+    const bool next = lane < 31 && below;
     uint64_t u = 0;
     if (joins || next) u = sort_image(A.key, pass_element(A, pos[i]));
     uint64_t prev = __shfl_up_sync(0xffffffffu, u, 1);
