@@ -16,6 +16,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "tqpk.h"
 
 namespace tqpk {
@@ -40,6 +42,23 @@ extern thread_local int64_t g_launches;
       return TQPK_ECUDA;                                      \
     }                                                         \
   } while (0)
+
+// A number that holds for one device: what its occupancy query said, after the launch limits that go with it
+// were asked for there (a function's attributes belong to a device, and a process may use several).  find()
+// returns it, positive, or anything else for an error, which is not kept.
+class PerDevice {
+  std::atomic<int> known_[64] = {};
+
+ public:
+  template <class F>
+  int get(F find) {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return find();
+    int v = known_[dev].load(std::memory_order_acquire);
+    if (v <= 0 && (v = find()) > 0) known_[dev].store(v, std::memory_order_release);
+    return v;
+  }
+};
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -898,18 +898,19 @@ static int run_cluster(const SortKeySet& S, const int64_t* perm_in, int n, int64
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  static int fits = -1;
-  if (fits < 0) {
+  static PerDevice resident;           // clusters the device holds at a time, plus one
+  const int fits = resident.get([&] {
     int clusters = 0;
     if (cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, k_sort_cluster<ITEMS>, &cfg) != cudaSuccess)
-      clusters = 0;
-    (void)cudaGetLastError();
-    fits = clusters > 0;
-  }
-  launched = fits > 0;
+        cudaOccupancyMaxActiveClusters(&clusters, k_sort_cluster<ITEMS>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    return clusters + 1;
+  });
+  launched = fits > 1;
   if (!launched) return TQPK_OK;
   TQPK_CUDA(cudaLaunchKernelEx(&cfg, k_sort_cluster<ITEMS>, S, perm_in, n, perm_out));
   ++g_launches;
@@ -942,13 +943,18 @@ size_t sort_ws_bytes(int64_t n, int nk) {
 template <int ITEMS, class V, class K>
 static int run_key(PassArgs<V> A, cudaStream_t s) {
   constexpr size_t smem = pass_smem<ITEMS, V, K>();
-  static int per_sm = 0;
-  if (!per_sm) {
-    TQPK_CUDA(cudaFuncSetAttribute(k_sort_pass<ITEMS, V, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static PerDevice resident;           // CTAs per SM
+  const int per_sm = resident.get([&] {
     int o = 0;
-    TQPK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sort_pass<ITEMS, V, K>, kSortBlock, smem));
-    per_sm = std::max(o, 1);
-  }
+    if (cudaFuncSetAttribute(k_sort_pass<ITEMS, V, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sort_pass<ITEMS, V, K>, kSortBlock, smem) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    return std::max(o, 1);
+  });
+  if (per_sm <= 0) return TQPK_ECUDA;
   const int grid = (int)std::min<int64_t>(sort_tiles(A.n), (int64_t)per_sm * num_sms());
   const int nd = sort_key_digits(A.key);
   const int passes = sizeof(K) == 8 ? nd : std::min(nd, kKeyPasses);
