@@ -288,7 +288,7 @@ int tqpk_groupby_emit(const tqpk_groupby_spec* h_spec, const tqpk_gb_plan* h_pla
  * n <= 2048 sorts in one CTA without a workspace (d_ws may be NULL) and
  * without a host synchronisation; sorts of more than 98304 rows synchronise
  * once.
- * d_perm_out must not overlap d_perm_in.                                   */
+ * d_perm_out may be d_perm_in (a loop over keys can sort in place).        */
 size_t tqpk_sort_workspace_bytes(int64_t n);
 int tqpk_argsort_stable(const void* d_keys, int32_t key_dtype, int32_t descending,
                         const int64_t* d_perm_in, int64_t n, int64_t* d_perm_out, void* d_ws,

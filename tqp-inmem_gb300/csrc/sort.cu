@@ -590,7 +590,19 @@ __global__ void __launch_bounds__(1024) k_sort_small(const __grid_constant__ Sor
     }
     __syncthreads();
   }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) perm_out[i] = perm_in ? perm_in[order[i]] : order[i];
+  // every read before the first write: perm_out may be perm_in, or a key column
+  int64_t row[kSmallSort / 1024];
+#pragma unroll
+  for (int q = 0; q < kSmallSort / 1024; ++q) {
+    const int i = threadIdx.x + q * 1024;
+    row[q] = i < n ? (perm_in ? perm_in[order[i]] : order[i]) : 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kSmallSort / 1024; ++q) {
+    const int i = threadIdx.x + q * 1024;
+    if (i < n) perm_out[i] = row[q];
+  }
 }
 
 // Mid-size sorts (the groups of an aggregate, small tables): the rows live in the shared memory of one
@@ -720,8 +732,8 @@ __device__ __forceinline__ int cluster_recode(cg::cluster_group& cluster, Cluste
 
 template <int ITEMS>
 __global__ void __launch_bounds__(kClusterThreads) k_sort_cluster(const __grid_constant__ SortKeySet S,
-                                                                  const int64_t* __restrict__ perm_in, int n,
-                                                                  int64_t* __restrict__ perm_out) {
+                                                                  const int64_t* perm_in, int n,
+                                                                  int64_t* perm_out) {
   extern __shared__ __align__(16) unsigned char raw[];
   ClusterSmem<ITEMS>& M = *reinterpret_cast<ClusterSmem<ITEMS>*>(raw);
   cg::cluster_group cluster = cg::this_cluster();
@@ -874,11 +886,24 @@ __global__ void __launch_bounds__(kClusterThreads) k_sort_cluster(const __grid_c
     }
     __syncthreads();
   }
-  for (int i = threadIdx.x; i < mine; i += kClusterThreads) {
-    const unsigned v = packed ? (unsigned)M.key[cur][i] : M.val[cur][i];
-    perm_out[cta * (int64_t)R + i] = perm_in ? perm_in[v] : (int64_t)v;
+  int64_t row[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int i = j * kClusterThreads + threadIdx.x;
+    row[j] = 0;
+    if (i < mine) {
+      const unsigned v = packed ? (unsigned)M.key[cur][i] : M.val[cur][i];
+      row[j] = perm_in ? perm_in[v] : (int64_t)v;
+    }
   }
-  cluster.sync();                    // no CTA leaves while another may still write to it
+  // no CTA leaves while another may still reach into it, and every read of perm_in and the key columns comes
+  // before the first write: perm_out may be one of them
+  cluster.sync();
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int i = j * kClusterThreads + threadIdx.x;
+    if (i < mine) perm_out[cta * (int64_t)R + i] = row[j];
+  }
 }
 
 // One cluster, where the device can hold one (launched is set), else nothing.
@@ -1027,9 +1052,29 @@ static int sort_large(const SortKeySet& S, const int64_t* perm_in, int64_t n, in
   return TQPK_ETIMEOUT;              // not reached: the second attempt sorts by every digit
 }
 
-// The stable order of elements perm_in[0..n) (null: 0..n-1) by keys[0], then keys[1], ...  perm_out must
-// not overlap perm_in.  n > kClusterSort synchronises once (the look-back's error word).  mixed: the rows are
-// known to come in no order (entries of a hash table in the order they were claimed), so nothing looks for one.
+// Whether perm_out shares memory with perm_in or a key column: the passes read both until the last one writes.
+static bool sort_in_place(const SortKey* keys, int nk, const int64_t* perm_in, int64_t n, const int64_t* perm_out) {
+  const uintptr_t o0 = reinterpret_cast<uintptr_t>(perm_out), o1 = o0 + (uintptr_t)n * 8;
+  auto meets = [&](const void* p, uintptr_t bytes) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    return p && a < o1 && o0 < a + bytes;
+  };
+  bool in = meets(perm_in, (uintptr_t)n * 8);
+  for (int k = 0; k < nk && !in; ++k)
+    in = meets(keys[k].col, (uintptr_t)n * (keys[k].width ? keys[k].width : dtype_size(keys[k].dt)));
+  return in;
+}
+
+// Workspace of the exported sorts: sort_ws_bytes, and a permutation for an in-place call.
+static size_t argsort_ws_bytes(int64_t n, int nk) {
+  return sort_ws_bytes(n, nk) + (n > kSmallSort ? align_up((size_t)n * 8, 256) : 0);
+}
+
+// The stable order of elements perm_in[0..n) (null: 0..n-1) by keys[0], then keys[1], ...  perm_out may be
+// perm_in (or a key column) given argsort_ws_bytes: the tiled passes then write to the workspace, and the order
+// is copied out behind them.  n > kClusterSort synchronises once (the look-back's error word).  mixed: the rows
+// are known to come in no order (entries of a hash table in the order they were claimed), so nothing looks for
+// one.
 int sort_keys(const SortKey* keys, int nk, const int64_t* perm_in, int64_t n, int64_t* perm_out, void* ws,
               size_t ws_bytes, cudaStream_t s, bool mixed) {
   if (nk < 1 || nk > kMaxSortKeys) return TQPK_EUNSUPPORTED;
@@ -1053,15 +1098,23 @@ int sort_keys(const SortKey* keys, int nk, const int64_t* perm_in, int64_t n, in
     if (rc || launched) return rc;
   }
   if (sort_tiles(n) > INT32_MAX) return TQPK_EUNSUPPORTED;
-  if (n < (int64_t(1) << 32)) return sort_large<uint32_t>(S, perm_in, n, perm_out, ws, ws_bytes, s);
-  return sort_large<uint64_t>(S, perm_in, n, perm_out, ws, ws_bytes, s);
+  WsCursor cur(ws, ws_bytes);
+  int64_t* order = perm_out;
+  if (sort_in_place(keys, nk, perm_in, n, perm_out)) order = cur.take<int64_t>(n);
+  if (!order) return TQPK_ENOMEM;
+  void* rest = cur.base + cur.off;
+  const int rc = n < (int64_t(1) << 32) ? sort_large<uint32_t>(S, perm_in, n, order, rest, ws_bytes - cur.off, s)
+                                        : sort_large<uint64_t>(S, perm_in, n, order, rest, ws_bytes - cur.off, s);
+  if (rc || order == perm_out) return rc;
+  TQPK_CUDA(cudaMemcpyAsync(perm_out, order, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
+  return TQPK_OK;
 }
 
 }  // namespace tqpk
 
 using namespace tqpk;
 
-extern "C" size_t tqpk_sort_workspace_bytes(int64_t n) { return sort_ws_bytes(n < 0 ? 0 : n); }
+extern "C" size_t tqpk_sort_workspace_bytes(int64_t n) { return argsort_ws_bytes(n < 0 ? 0 : n, 1); }
 
 extern "C" int tqpk_argsort_stable(const void* d_keys, int32_t dt, int32_t desc, const int64_t* d_perm_in, int64_t n,
                                    int64_t* d_perm_out, void* ws, size_t ws_bytes, tqpk_stream stream) {
@@ -1096,7 +1149,7 @@ extern "C" size_t tqpk_argsort_keys_workspace_bytes(int64_t n, int32_t n_keys, c
   SortKey keys[kMaxSortKeys];
   int rc;
   const int m = expand_keys(n_keys, nullptr, dts, widths, nullptr, keys, &rc);
-  return m < 0 ? 0 : sort_ws_bytes(n < 0 ? 0 : n, m);
+  return m < 0 ? 0 : argsort_ws_bytes(n < 0 ? 0 : n, m);
 }
 
 extern "C" int tqpk_argsort_keys(int32_t n_keys, const void* const* d_cols, const int32_t* dts, const int32_t* widths,
