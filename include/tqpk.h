@@ -286,8 +286,8 @@ int tqpk_groupby_emit(const tqpk_groupby_spec* h_spec, const tqpk_gb_plan* h_pla
  * ties in input order (torch.sort(stable=True, descending=True)).
  * Float keys: -0.0 sorts equal to +0.0 and NaN sorts as the largest value.
  * n <= 2048 sorts in one CTA without a workspace (d_ws may be NULL) and
- * without a host synchronisation; sorts of more than 98304 rows synchronise
- * once.
+ * without a host synchronisation; a larger sort is complete, and done with
+ * the keys and the workspace, when the call returns.
  * d_perm_out may be d_perm_in (a loop over keys can sort in place).        */
 size_t tqpk_sort_workspace_bytes(int64_t n);
 int tqpk_argsort_stable(const void* d_keys, int32_t key_dtype, int32_t descending,
@@ -297,7 +297,8 @@ int tqpk_argsort_stable(const void* d_keys, int32_t key_dtype, int32_t descendin
  * then d_cols[1], ... (n_keys columns of dtype h_dtypes[k]; h_widths[k] > 0: an
  * int8/uint8 [n, w] string column, compared byte by byte, one sort word per
  * eight bytes; h_descs[k] != 0: descending).  At most 32 sort words
- * (TQPK_EUNSUPPORTED beyond).  Otherwise as tqpk_argsort_stable.           */
+ * (TQPK_EUNSUPPORTED beyond).  Otherwise as tqpk_argsort_stable, but only
+ * sorts of more than 98304 rows synchronise, once, behind their last kernel. */
 size_t tqpk_argsort_keys_workspace_bytes(int64_t n, int32_t n_keys, const int32_t* h_dtypes, const int32_t* h_widths);
 int tqpk_argsort_keys(int32_t n_keys, const void* const* d_cols, const int32_t* h_dtypes, const int32_t* h_widths,
                       const int32_t* h_descs, const int64_t* d_perm_in, int64_t n, int64_t* d_perm_out,

@@ -1,6 +1,7 @@
-"""A process with several GPUs: limits that a launch needs are asked for on every device.  No GPU is
-used: the sort's object file is linked with a CUDA runtime of this file that keeps a function's
-attributes per device, as the driver does, and refuses a launch that goes beyond them."""
+"""The sort's host side against a CUDA runtime of this file (no GPU is used: its object file is linked
+with it).  A process with several GPUs: limits that a launch needs are asked for on every device, as the
+runtime keeps a function's attributes per device and refuses a launch that goes beyond them.  And which
+calls wait for their work before they return."""
 import ctypes as C
 import shutil
 import subprocess
@@ -18,12 +19,14 @@ RUNTIME = r"""
 static int g_device = 0;
 static std::map<std::pair<int, const void*>, std::pair<int, bool>> g_attr;   // (device, kernel): smem, clusters of 16
 static int g_count[8];
+static bool g_pending = false;          // work enqueued and not waited for
 static cudaError_t g_last = cudaSuccess;
 
 static cudaError_t allowed(const void* f, size_t smem, bool cluster) {
   const auto& a = g_attr[{g_device, f}];
   if ((smem > 48 * 1024 && (size_t)a.first < smem) || (cluster && !a.second)) return g_last = cudaErrorInvalidValue;
   ++g_count[g_device];
+  g_pending = true;
   return cudaSuccess;
 }
 
@@ -38,6 +41,7 @@ void timing_after(int, cudaStream_t) {}
 extern "C" {
 void fake_device(int d) { g_device = d; }
 int fake_launches(int d) { return g_count[d]; }
+int fake_pending() { return g_pending; }
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
@@ -67,10 +71,11 @@ cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunch
 cudaError_t cudaGetDevice(int* d) { *d = g_device; return cudaSuccess; }
 cudaError_t cudaGetLastError() { const cudaError_t e = g_last; g_last = cudaSuccess; return e; }
 cudaError_t cudaPeekAtLastError() { return g_last; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { g_pending = false; return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void*, size_t n, cudaMemcpyKind k, cudaStream_t) {
   if (k == cudaMemcpyDeviceToHost) memset(d, 0, n);
+  g_pending = true;
   return cudaSuccess;
 }
 }
@@ -110,3 +115,18 @@ def test_every_device_sorts(sort_lib, n):
         before = sort_lib.fake_launches(device)
         assert sort_lib.tqpk_argsort_stable(p, L.I64, 0, None, n, p, p, ws, None) == L.OK
         assert sort_lib.fake_launches(device) > before
+
+
+@pytest.mark.parametrize("n", [2048, 2049, 32_769, 98_304, 98_305])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_sorts_beyond_one_cta_are_complete_when_they_return(sort_lib, n, in_place):
+    """More than 2048 rows: the keys are not read again, and the order is written, when the call returns
+    (another stream may use either); up to 2048 nothing waits, so that a capture may hold the call."""
+    from tqpk import _lib as L
+    ws = sort_lib.tqpk_sort_workspace_bytes(n)
+    base = C.create_string_buffer(4096)
+    p = (C.addressof(base) + 255) & ~255
+    perm = p + (1 << 40)                                    # never read or written either
+    sort_lib.fake_device(0)
+    assert sort_lib.tqpk_argsort_stable(p, L.I64, 0, perm if in_place else None, n, perm, p, ws, None) == L.OK
+    assert bool(sort_lib.fake_pending()) == (n <= 2048)

@@ -1121,7 +1121,10 @@ extern "C" int tqpk_argsort_stable(const void* d_keys, int32_t dt, int32_t desc,
   if (n < 0 || (n > 0 && (!d_keys || !d_perm_out))) return TQPK_EINVAL;
   if (!dtype_size(dt)) return TQPK_EDTYPE;
   const SortKey key{d_keys, nullptr, dt, desc ? 1 : 0, 0, 0};
-  return sort_keys(&key, 1, d_perm_in, n, d_perm_out, ws, ws_bytes, static_cast<cudaStream_t>(stream));
+  const int rc = sort_keys(&key, 1, d_perm_in, n, d_perm_out, ws, ws_bytes, static_cast<cudaStream_t>(stream));
+  // one launch or many, a sort beyond one CTA is complete when the call returns
+  if (rc == TQPK_OK && n > kSmallSort) TQPK_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+  return rc;
 }
 
 // Sort words of a key list (a [n, w] column is ceil(w/8) words, most significant first), or -1.
