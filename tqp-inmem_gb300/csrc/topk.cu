@@ -39,19 +39,21 @@ static int launch_r(const Src& src, int k, int grid, TopkOut O, cudaStream_t s) 
   int64_t G = 4;
   while (G * kTopkGroups < src.n) G <<= 1;
   const int ng = (int)std::max<int64_t>(1, (src.n + G - 1) / G);
-  if (R == 1 && G <= kTopkFusedMaxG && O.err && ng <= fused_capacity<Src>()) {
-    // one cooperative launch: all ng CTAs resident together, so the grid barrier inside completes
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.gridDim = dim3(ng);
-    cfg.blockDim = dim3(256);
-    cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    TQPK_CUDA(cudaLaunchKernelEx(&cfg, k_tk_fused<Src>, src, G, k, O, g_tk_spin_limit, g_tk_missing));
-    return TQPK_OK;
+  if constexpr (!Src::kStoredOrder) {
+    if (R == 1 && G <= kTopkFusedMaxG && O.err && ng <= fused_capacity<Src>()) {
+      // one cooperative launch: all ng CTAs resident together, so the grid barrier inside completes
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeCooperative;
+      attr[0].val.cooperative = 1;
+      cfg.gridDim = dim3(ng);
+      cfg.blockDim = dim3(256);
+      cfg.stream = s;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      TQPK_CUDA(cudaLaunchKernelEx(&cfg, k_tk_fused<Src>, src, G, k, O, g_tk_spin_limit, g_tk_missing));
+      return TQPK_OK;
+    }
   }
   k_tk_group_best<Src><<<ng, 256, 0, s>>>(src, G, k, O);
   TQPK_CHECK_LAUNCH();
@@ -62,11 +64,15 @@ static int launch_r(const Src& src, int k, int grid, TopkOut O, cudaStream_t s) 
 
 template <class Src>
 static int launch_src(const Src& src, int k, int grid, TopkOut O, cudaStream_t s) {
-  if (k <= 32) return launch_r<1>(src, k, grid, O, s);
-  if (k <= 64) return launch_r<2>(src, k, grid, O, s);
-  if (k <= 128) return launch_r<4>(src, k, grid, O, s);
-  if (k <= 256) return launch_r<8>(src, k, grid, O, s);
-  return TQPK_EUNSUPPORTED;
+  if (k > 256) return TQPK_EUNSUPPORTED;
+  if constexpr (Src::kStoredOrder) {
+    return launch_r<1>(src, k, grid, O, s);          // stored columns use no warp lists
+  } else {
+    if (k <= 32) return launch_r<1>(src, k, grid, O, s);
+    if (k <= 64) return launch_r<2>(src, k, grid, O, s);
+    if (k <= 128) return launch_r<4>(src, k, grid, O, s);
+    return launch_r<8>(src, k, grid, O, s);
+  }
 }
 
 int topk_warp_launch(int kind, const void* src, int k, int grid, TopkOut O, cudaStream_t s) {
@@ -235,12 +241,13 @@ extern "C" int tqpk_topk_stable(const void* d_keys, int32_t dt, int32_t desc, co
   unsigned* ticket = cur.take<unsigned>(64);
   int64_t* count = cur.take<int64_t>(4);
   int64_t* idx = cur.take<int64_t>(k);
-  uint64_t* ck = cur.take<uint64_t>(topk_cand_entries((int)k));
-  int64_t* ci = cur.take<int64_t>(topk_cand_entries((int)k));
+  uint64_t* ck = cur.take<uint64_t>(topk_list_entries((int)k));
+  int64_t* ci = cur.take<int64_t>(topk_list_entries((int)k));
   if (!ci) return TQPK_ENOMEM;
   TQPK_CUDA(cudaMemsetAsync(ticket, 0, 256, s));
   ArraySource src{d_keys, dt, d_perm_in, n, desc ? 1 : 0};
   TopkOut O{idx, count, ck, ci, ticket, nullptr, reinterpret_cast<unsigned long long*>(ticket + 8), ticket + 16};
+  O.cap = kTopkGroups * topk_list_share((int)k);
   timing_before(KID_PIPE_TOPK, s);
   int rc = topk_warp_launch(1, &src, (int)k, grid, O, s);
   timing_after(KID_PIPE_TOPK, s);

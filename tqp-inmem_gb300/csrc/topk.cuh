@@ -94,6 +94,7 @@ struct DenseSumSource {
                          // occupied exactly when its bits are no longer those of -0.0
   int64_t n;
   int desc;
+  static constexpr bool kStoredOrder = false;   // sums come in no order of their slots
   const unsigned* bits = nullptr;   // when set, only slots whose bit is set can be occupied (the join's
                                     // build writes its passing keys' bits and initialises those sums)
   static constexpr uint64_t kEmptySum = 0x8000000000000000ull;
@@ -173,6 +174,7 @@ struct ArraySource {
   const int64_t* perm;
   int64_t n;
   int desc;
+  static constexpr bool kStoredOrder = true;    // a column may be stored sorted
   __device__ __forceinline__ bool get(int64_t i, uint64_t& k) const;
   __device__ __forceinline__ unsigned bits4(int64_t) const { return 0xfu; }
   // Four items: of an 8- or 4-byte column in its own order as 16-byte loads (one item at a time, each
@@ -212,7 +214,8 @@ struct TopkOut {
   int64_t* cand_idx;
   unsigned* ticket;
   unsigned long long* valid_total;  // number of valid items seen (may be null)
-  unsigned long long* bound;        // the cut (written by the first pass)
+  unsigned long long* bound;        // the first pass's: k <= 32 the complement of the tightest cut a group found
+                                    // on its own (0: none), k > 32 the cut
   unsigned* arrive;                 // [2] CTAs done with the group-best and the filter pass (zeroed before the launch)
   // Optional, for a dense group table: the last CTA also writes (key_min + slot, sum[slot]) of the
   // top rows and their number (emit_keys null: not written) ...
@@ -227,6 +230,9 @@ struct TopkOut {
   unsigned long long* bits_set = nullptr;
   const unsigned long long* bits_expected = nullptr;
   int* err = nullptr;
+  // Entries of the candidate list, behind which the groups' bests lie.  A stored column (kStoredOrder) has
+  // topk_list_share(k) of them for each group.
+  int cap = 4096;
 };
 
 // ---------------------------------------------------------------------------
@@ -235,18 +241,23 @@ struct TopkOut {
 // key; the k-th best of those group bests is a cut T with at least k items
 // at or below it (every one of those k groups holds one), so the top k are
 // all among the items with key <= T.  For independent keys only about k
-// items pass T.  A second pass appends them to a candidate list (at most
-// kTopkCap), and the last CTA of that pass sorts the list bitonically by
-// (key, index) in shared memory.  When ties push more than kTopkSortCap items
-// under the cut, that CTA falls back to the warp lists over all items (same
-// result, slower).  For k > 32 the cut is computed by the last CTA of the
-// first pass and the top-k is two launches; for k <= 32 every CTA of the
-// second pass derives the cut from the group bests (tk_bin_cut), and when
-// each CTA's group fits one sweep of its threads the two passes run as one
-// cooperative launch with a grid barrier between them (k_tk_fused below).
+// items pass T.  A second pass appends them to a candidate list, and the last
+// CTA of that pass sorts the list bitonically by (key, index) in shared memory,
+// or, beyond kTopkSortCap entries, in parts.  A group of a stored column that
+// has more items under the cut than its share of the list appends its own best
+// k instead, so the list holds all that is left; of a group table (at most
+// kTopkCap candidates) the last CTA
+// then walks every item (same result, slower).  For k > 32 the cut is computed
+// by the last CTA of the first pass and the top-k is two launches; for k <= 32
+// every CTA of the second pass derives the cut from the group bests
+// (tk_bin_cut), and when each CTA's group fits one sweep of its threads the two
+// passes run as one cooperative launch with a grid barrier between them
+// (k_tk_fused below).
 constexpr int kTopkCap = 4096;
 constexpr int kTopkGroups = 512;     // >= 2 x the largest k: the cut stays near the k-th item
 constexpr int kTopkCand = kTopkCap + kTopkGroups;   // cand_key entries used: candidates, then group bests
+// A group's share of a stored column's candidate list; at least k.
+__host__ __device__ constexpr int topk_list_share(int k) { return k <= 32 ? 128 : 256; }
 
 __device__ __forceinline__ void block_min_u64(uint64_t& v, uint64_t* red) {
 #pragma unroll
@@ -278,10 +289,11 @@ __device__ __forceinline__ bool tk_last_cta(unsigned* arrive) {
   return last;
 }
 
-// The cut for k > 32: the k-th best of the ng group bests (bitonic sort of the bests in one CTA).
-__device__ __forceinline__ void tk_cut(int ng, int k, TopkOut O) {
+// The cut for k > 32: the k-th best of the ng group bests (bitonic sort of the bests in one CTA), or the
+// tightest cut a group found on its own (stored: a source that looks for one).
+__device__ __forceinline__ void tk_cut(int ng, int k, TopkOut O, bool stored) {
   __shared__ uint64_t v[kTopkGroups];
-  for (int i = threadIdx.x; i < kTopkGroups; i += blockDim.x) v[i] = i < ng ? __ldcg(&O.cand_key[kTopkCap + i]) : ~0ull;
+  for (int i = threadIdx.x; i < kTopkGroups; i += blockDim.x) v[i] = i < ng ? __ldcg(&O.cand_key[O.cap + i]) : ~0ull;
   __syncthreads();
   for (int size = 2; size <= kTopkGroups; size <<= 1)
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -293,7 +305,10 @@ __device__ __forceinline__ void tk_cut(int ng, int k, TopkOut O) {
       }
       __syncthreads();
     }
-  if (threadIdx.x == 0) *O.bound = v[(k <= kTopkGroups ? k : kTopkGroups) - 1];
+  if (threadIdx.x == 0) {
+    const uint64_t cut = v[(k <= kTopkGroups ? k : kTopkGroups) - 1];
+    *O.bound = stored ? min(cut, ~(uint64_t)__ldcg(O.bound)) : cut;
+  }
 }
 
 // One CTA's walk over items [b0, b1) in quads (4 items per thread, 256 threads): kTopkQuads
@@ -327,6 +342,30 @@ __device__ __forceinline__ void tk_scan_group(const Src& src, int64_t b0, int64_
   }
 }
 
+// A cut from one CTA's items alone, from every thread's best key (~0: it has none): the k-th best of a warp's
+// threads, the best warp's of the CTA (k <= 32), or the worst of the warps' ceil(k / 8)-th bests (k <= 256);
+// at least k items lie at or under it.  Neighbouring items belong to neighbouring threads, so of a column that
+// is stored sorted, or in sorted runs, it lets at most ~4 k of one group through; the cut from the groups'
+// bests alone lets k whole groups through.  Called by all 256 threads; red: 8 words.
+__device__ __forceinline__ uint64_t tk_own_cut(uint64_t own, int k, uint64_t* red) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      const uint64_t other = __shfl_xor_sync(0xffffffffu, own, stride);
+      const bool low = ((lane & stride) == 0) == ((lane & size) == 0);      // keeps the smaller of the two
+      own = (other < own) == low ? other : own;
+    }
+  const uint64_t mine = __shfl_sync(0xffffffffu, own, (k <= 32 ? k : (k + 7) / 8) - 1);
+  __syncthreads();
+  if (lane == 0) red[threadIdx.x >> 5] = mine;
+  __syncthreads();
+  uint64_t cut = red[0];
+  for (int w = 1; w < 8; ++w) cut = (red[w] < cut) == (k <= 32) ? red[w] : cut;
+  return cut;
+}
+
 // Pass 1: each CTA keeps the best key of its group of G items and in how many threads' items it is (at
 // most 256, a lower bound of the items that have it; counting those cost 30 us of 160 for 60 M rows); the
 // last CTA to finish computes the cut from all groups' bests.
@@ -358,14 +397,18 @@ __global__ void __launch_bounds__(256) k_tk_group_best(Src src, int64_t G, int k
   if ((threadIdx.x & 31) == 0 && equal) atomicAdd(&s_equal, equal);
   __syncthreads();
   if (threadIdx.x == 0) {
-    O.cand_key[kTopkCap + blockIdx.x] = best;
-    O.cand_idx[kTopkCap + blockIdx.x] = s_equal;
+    O.cand_key[O.cap + blockIdx.x] = best;
+    O.cand_idx[O.cap + blockIdx.x] = s_equal;
     if (blockIdx.x == 0) *O.ticket = 0;          // the candidate counter of the next pass
     if (s_valid && O.valid_total) atomicAdd(O.valid_total, (unsigned long long)s_valid);
     if (s_bits && O.bits_set) atomicAdd(O.bits_set, (unsigned long long)s_bits);
   }
+  if constexpr (Src::kStoredOrder) {
+    const uint64_t cut = tk_own_cut(own, k, red);
+    if (threadIdx.x == 0 && cut != ~0ull) atomicMax(O.bound, ~(unsigned long long)cut);     // bound: 0 before
+  }
   if (k <= 32) return;              // the filter pass derives its cut from the group bests itself
-  if (tk_last_cta(O.arrive)) tk_cut((int)gridDim.x, k, O);
+  if (tk_last_cta(O.arrive)) tk_cut((int)gridDim.x, k, O, Src::kStoredOrder);
 }
 
 // The cut for k <= 32, computed by every CTA of the filter pass from the ng group bests (no
@@ -386,7 +429,7 @@ __device__ __forceinline__ uint64_t tk_bin_cut(int ng, int k, const TopkOut& O) 
   __shared__ int wsum[8];
   for (int base = 0; base < ng; base += 256) {
     const int g = base + threadIdx.x;
-    const uint64_t v = g < ng ? __ldcg(&O.cand_key[kTopkCap + g]) : ~0ull;
+    const uint64_t v = g < ng ? __ldcg(&O.cand_key[O.cap + g]) : ~0ull;
     const bool ne = v != ~0ull;
     const unsigned m = __ballot_sync(0xffffffffu, ne);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -435,12 +478,79 @@ __device__ __forceinline__ void tk_finish_warp(int m, const TopkOut& O, const in
   if ((threadIdx.x & 31) == 0) tk_counts(m, O);
 }
 
-// The final step, in one CTA: sort the candidates under the cut by (key, index), or, when
-// ties put more than kTopkSortCap items under it, warp lists over every item.
+// Sorts cnt (<= kTopkSortCap) entries by (key, index), in one CTA of 256 threads.
+__device__ __forceinline__ void tk_sort(int cnt, uint64_t* sk, int64_t* si) {
+  int P = 2;
+  while (P < cnt) P <<= 1;
+  for (int i = cnt + threadIdx.x; i < P; i += blockDim.x) {
+    sk[i] = ~0ull;
+    si[i] = INT64_MAX;
+  }
+  __syncthreads();
+  for (int size = 2; size <= P; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
+        const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+        const bool up = (i & size) == 0;
+        const uint64_t ka = sk[i], kb = sk[j];
+        const int64_t ia = si[i], ib = si[j];
+        if (tk_better(kb, ib, ka, ia) == up) { sk[i] = kb; sk[j] = ka; si[i] = ib; si[j] = ia; }
+      }
+      __syncthreads();
+    }
+}
+
+// The best k (<= 256) of m items at or under the cut, by one CTA of 256 threads: load(i0, key, at) gives items
+// i0..i0+3 and the mask of those there are.  1024 items a step; those better than the k-th so far join the
+// buffer (sk, si: kTopkSortCap entries), which is sorted and cut back to k when the next step might not fit.
+// Returns their number, to every thread.  Warp lists (WarpList) took 0.4 us an insertion at k = 256.
+template <class Load>
+__device__ __forceinline__ int tk_stream_best(int64_t m, int k, uint64_t cut, uint64_t* sk, int64_t* si, Load load) {
+  __shared__ unsigned s_fill;
+  const int lane = threadIdx.x & 31;
+  uint64_t worst_key = cut;
+  int64_t worst_at = INT64_MAX;
+  if (threadIdx.x == 0) s_fill = 0;
+  __syncthreads();
+  int fill = 0;
+  for (int64_t base = 0; base < m; base += 1024) {
+    uint64_t key[4];
+    int64_t at[4];
+    const unsigned ok = load(base + threadIdx.x * 4, key, at);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const bool pass = ((ok >> q) & 1u) && tk_better(key[q], at[q], worst_key, worst_at);
+      const unsigned bal = __ballot_sync(0xffffffffu, pass);
+      if (!bal) continue;
+      unsigned o = 0;
+      if (lane == 0) o = atomicAdd(&s_fill, (unsigned)__popc(bal));
+      o = __shfl_sync(0xffffffffu, o, 0) + __popc(bal & ((1u << lane) - 1u));
+      if (pass) {
+        sk[o] = key[q];
+        si[o] = at[q];
+      }
+    }
+    __syncthreads();
+    fill = (int)s_fill;
+    __syncthreads();
+    if (fill <= kTopkSortCap - 1024 && base + 1024 < m) continue;
+    tk_sort(fill, sk, si);
+    if (fill >= k) {
+      fill = k;
+      worst_key = sk[k - 1];
+      worst_at = si[k - 1];
+    }
+    if (threadIdx.x == 0) s_fill = fill;
+    __syncthreads();
+  }
+  return fill;
+}
+
+// The final step, in one CTA: sort the candidates under the cut by (key, index).  More than kTopkSortCap of
+// them: a stored column's list is gone through; of a group table every item is, by warp lists.  sk, si:
+// kTopkSortCap entries.
 template <int R, class Src>
-__device__ __forceinline__ void tk_final(const Src& src, int k, TopkOut O) {
-  __shared__ uint64_t sk[kTopkSortCap];
-  __shared__ int64_t si[kTopkSortCap];
+__device__ __forceinline__ void tk_final(const Src& src, int k, TopkOut O, uint64_t* sk, int64_t* si) {
   const unsigned cnt = __ldcg(O.ticket);
   if (cnt <= 256u) {
     // few candidates: each thread ranks one against all of them (one pass over shared memory,
@@ -468,26 +578,28 @@ __device__ __forceinline__ void tk_final(const Src& src, int k, TopkOut O) {
     return;
   }
   if (cnt <= (unsigned)kTopkSortCap) {
-    int P = 2;
-    while (P < (int)cnt) P <<= 1;
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-      const bool in = i < (int)cnt;
-      sk[i] = in ? __ldcg(&O.cand_key[i]) : ~0ull;
-      si[i] = in ? __ldcg(&O.cand_idx[i]) : INT64_MAX;
+    for (int i = threadIdx.x; i < (int)cnt; i += blockDim.x) {
+      sk[i] = __ldcg(&O.cand_key[i]);
+      si[i] = __ldcg(&O.cand_idx[i]);
     }
-    __syncthreads();
-    for (int size = 2; size <= P; size <<= 1)
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
-          const int i = 2 * t - (t & (stride - 1)), j = i + stride;
-          const bool up = (i & size) == 0;
-          const uint64_t ka = sk[i], kb = sk[j];
-          const int64_t ia = si[i], ib = si[j];
-          if (tk_better(kb, ib, ka, ia) == up) { sk[i] = kb; sk[j] = ka; si[i] = ib; si[j] = ia; }
-        }
-        __syncthreads();
-      }
+    tk_sort((int)cnt, sk, si);
     const int m = (int)cnt < k ? (int)cnt : k;
+    for (int j = threadIdx.x; j < m; j += blockDim.x) O.out_idx[j] = si[j];
+    tk_finish(m, O, si);
+    return;
+  }
+  if constexpr (Src::kStoredOrder) {        // the list holds every candidate
+    const int m = tk_stream_best((int64_t)cnt, k, ~0ull, sk, si, [&](int64_t i0, uint64_t(&key)[4], int64_t(&at)[4]) {
+      unsigned ok = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const bool in = i0 + q < (int64_t)cnt;
+        key[q] = in ? __ldcg(&O.cand_key[i0 + q]) : 0;
+        at[q] = in ? __ldcg(&O.cand_idx[i0 + q]) : 0;
+        ok |= (unsigned)in << q;
+      }
+      return ok;
+    });
     for (int j = threadIdx.x; j < m; j += blockDim.x) O.out_idx[j] = si[j];
     tk_finish(m, O, si);
     return;
@@ -537,24 +649,32 @@ __device__ __forceinline__ void tk_final(const Src& src, int k, TopkOut O) {
 // (tk_final's 8 warps).  A group whose best lies over the cut is not read again, which for
 // independent keys is all but about k of them.  Of the items that tie with the cut only the first
 // can be among the k: those with k or more at or under the cut before them, by the counts of the
-// groups before and of the warp's own rows, are left out.  Without that a column of few values
-// overflowed the list and went through the warp lists of one CTA: the first 10 of 6 M dates 3489 us, now
-// 39 (20 M: 13952 and 86; float64 of few ties, 6 / 20 / 60 M: 47 / 149 / 320 and 45 / 137 / 287).
+// groups before and of the warp's own rows, are left out (a column of few values: the first 10 of 6 M
+// dates).  A stored column's group gathers its items in shared memory and appends them together, or its
+// best k when they are more than its share.  While a list of 4096 entries that overflowed sent one CTA over the
+// whole table, two keys with a limit over 6 M rows took 3.7 ms (first key stored ascending, k = 10), 47 ms
+// (descending), 5.6 ms (the least values in 62 places, k = 100) and half a second (descending, k = 256); now
+// 0.12, 0.11, 0.19 and 0.13, and 0.11-0.13 as before when it is stored in no order.
 template <int R, class Src>
 __global__ void __launch_bounds__(256) k_tk_filter(Src src, int64_t G, int k, TopkOut O) {
   const int lane = threadIdx.x & 31;
-  const uint64_t cut = k <= 32 ? tk_bin_cut((int)gridDim.x, k, O) : __ldcg(O.bound);
+  uint64_t cut = k <= 32 ? tk_bin_cut((int)gridDim.x, k, O) : __ldcg(O.bound);
+  if constexpr (Src::kStoredOrder)
+    if (k <= 32) cut = min(cut, ~(uint64_t)__ldcg(O.bound));
   const int64_t b0 = (int64_t)blockIdx.x * G, b1 = b0 + G < src.n ? b0 + G : src.n;
   unsigned valid = 0, nbits = 0;
+  __shared__ uint64_t sk[kTopkSortCap];
+  __shared__ int64_t si[kTopkSortCap];
+  __shared__ unsigned s_n, s_at;     // this group's candidates, and their place in the list
   __shared__ unsigned s_before;      // items at or under the cut in the groups before (at least so many)
-  if (threadIdx.x == 0) s_before = 0;
+  if (threadIdx.x == 0) { s_before = 0; s_n = 0; }
   __syncthreads();
-  const bool any = __ldcg(&O.cand_key[kTopkCap + blockIdx.x]) <= cut;
+  const bool any = __ldcg(&O.cand_key[O.cap + blockIdx.x]) <= cut;
   if (any) {
     unsigned c = 0;
     for (int g = threadIdx.x; g < (int)blockIdx.x; g += 256) {
-      const uint64_t v = __ldcg(&O.cand_key[kTopkCap + g]);
-      const unsigned e = (unsigned)__ldcg(reinterpret_cast<const long long*>(&O.cand_idx[kTopkCap + g]));
+      const uint64_t v = __ldcg(&O.cand_key[O.cap + g]);
+      const unsigned e = (unsigned)__ldcg(reinterpret_cast<const long long*>(&O.cand_idx[O.cap + g]));
       c += v < cut ? 1u : v == cut ? e : 0u;
     }
     c = __reduce_add_sync(0xffffffffu, c);
@@ -580,14 +700,43 @@ __global__ void __launch_bounds__(256) k_tk_filter(Src src, int64_t G, int k, To
     if (!bal) return;
     const bool pass = (bal >> lane) & 1u;
     unsigned at = 0;
-    if (lane == 0) at = atomicAdd(O.ticket, (unsigned)__popc(bal));
+    if (lane == 0) at = atomicAdd(Src::kStoredOrder ? &s_n : O.ticket, (unsigned)__popc(bal));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
-    if (pass && at < (unsigned)kTopkCap) {
+    if constexpr (Src::kStoredOrder) {
+      if (pass && at < (unsigned)kTopkSortCap) {
+        sk[at] = key;
+        si[at] = idx;
+      }
+    } else if (pass && at < (unsigned)O.cap) {
       O.cand_key[at] = key;
       O.cand_idx[at] = idx;
     }
   }, valid, nbits);
-  if (tk_last_cta(O.arrive + 1)) tk_final<R>(src, k, O);
+  if constexpr (Src::kStoredOrder) {
+    __syncthreads();
+    if (any) {
+      int c = (int)s_n;
+      if (c > kTopkSortCap) {
+        c = tk_stream_best(b1 - b0, k, cut, sk, si, [&](int64_t i, uint64_t(&key)[4], int64_t(&at)[4]) {
+          const int64_t left = b1 - b0 - i;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) at[q] = b0 + i + q;
+          return left <= 0 ? 0u : src.get4(b0 + i, key) & (left >= 4 ? 0xfu : (1u << left) - 1u);
+        });
+      } else if (c > topk_list_share(k)) {
+        tk_sort(c, sk, si);
+        c = k;
+      }
+      if (threadIdx.x == 0) s_at = c ? atomicAdd(O.ticket, (unsigned)c) : 0;
+      if (threadIdx.x == 0) s_n = c;
+      __syncthreads();
+      for (int i = threadIdx.x; i < (int)s_n; i += 256) {
+        O.cand_key[s_at + i] = sk[i];
+        O.cand_idx[s_at + i] = si[i];
+      }
+    }
+  }
+  if (tk_last_cta(O.arrive + 1)) tk_final<R>(src, k, O, sk, si);
 }
 
 // Both passes in one cooperative launch, for k <= 32 and groups of at most one tk_scan_group
@@ -605,6 +754,8 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 template <class Src>
 __global__ void __launch_bounds__(256) k_tk_fused(Src src, int64_t G, int k, TopkOut O, int spin_limit,
                                                   int missing) {
+  __shared__ uint64_t sk[kTopkSortCap];
+  __shared__ int64_t si[kTopkSortCap];
   __shared__ uint64_t red[8];
   __shared__ unsigned s_valid, s_bits;
   __shared__ int s_fail;
@@ -642,7 +793,7 @@ __global__ void __launch_bounds__(256) k_tk_fused(Src src, int64_t G, int k, Top
   }
   block_min_u64(best, red);
   if (threadIdx.x == 0) {
-    O.cand_key[kTopkCap + blockIdx.x] = best;
+    O.cand_key[O.cap + blockIdx.x] = best;
     if (blockIdx.x == 0) *O.ticket = 0;
     if (s_valid && O.valid_total) atomicAdd(O.valid_total, (unsigned long long)s_valid);
     if (s_bits && O.bits_set) atomicAdd(O.bits_set, (unsigned long long)s_bits);
@@ -668,12 +819,12 @@ __global__ void __launch_bounds__(256) k_tk_fused(Src src, int64_t G, int k, Top
       unsigned at = 0;
       if (lane == 0) at = atomicAdd(O.ticket, (unsigned)__popc(bal));
       at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
-      if (pass && at < (unsigned)kTopkCap) {
+      if (pass && at < (unsigned)O.cap) {
         O.cand_key[at] = key[u][q];
         O.cand_idx[at] = c0 + u * 1024 + q;
       }
     }
-  if (tk_last_cta(O.arrive + 1)) tk_final<1>(src, k, O);
+  if (tk_last_cta(O.arrive + 1)) tk_final<1>(src, k, O, sk, si);
 }
 
 // Host launcher: k <= 256.  The cand arrays hold topk_cand_entries(k) entries each;
@@ -684,9 +835,11 @@ inline size_t topk_cand_entries(int k) {
   const size_t a = (size_t)topk_grid_size() * k;
   return a > (size_t)kTopkCand ? a : (size_t)kTopkCand;
 }
+// A stored column's list (tqpk_topk_stable): a share for every group, and the groups' bests.
+inline size_t topk_list_entries(int k) { return (size_t)kTopkGroups * (topk_list_share(k) + 1); }
 inline size_t topk_scratch_bytes(int k) {
   // ticket block + count + k indices + two candidate arrays, each 256-byte aligned
-  return 2 * align_up(topk_cand_entries(k) * 8, 256) + align_up((size_t)k * 8, 256) + 1024;
+  return 2 * align_up(topk_list_entries(k) * 8, 256) + align_up((size_t)k * 8, 256) + 1024;
 }
 
 }  // namespace tqpk
