@@ -1,0 +1,69 @@
+"""Text programs whose searches are staged and whose equalities and prefixes are not: both in one
+program, at the widths of the staging rule, at row counts around a tile, against a row-by-row model."""
+import time
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _table(n, w, rng):
+    a = rng.choice(np.frombuffer(b"ab1 ", np.int8), (n, w))
+    a[rng.random(n) < 0.3, w - 1] = 0
+    return a
+
+
+def _mask(tree, col, w):
+    from tqpk.ops import filter_mask
+    from tqpk.predicate import compile_filter
+    dev = torch.from_numpy(col).cuda()
+    m, count = filter_mask(compile_filter(tree, {1: dev}), len(col), dev.device, with_count=True)
+    m = m.cpu().numpy()
+    assert int(count.item()) == m.sum()
+    return m
+
+
+@pytest.mark.parametrize("w", [3, 8, 25, 187, 188, 189])
+@pytest.mark.parametrize("n", [1, 255, 1024, 1025, 5000])
+def test_searches_beside_equalities_and_prefixes(w, n):
+    rng = np.random.default_rng(w * 7919 + n)
+    col = _table(n, w, rng)
+    rows = [bytes(r.view(np.uint8)) for r in col]
+    whole = rows[n // 2].rstrip(b"\0").decode()
+    sub = ["substring", ["t#1", "1", "2"]]
+    contains, prefix = ["Contains", ["t#1", "a1"]], ["StartsWith", ["t#1", "ab"]]
+    two = ["t#1", "LIKE", "%a%b%"]
+    inlist = [sub, "IN", ["ab", "1 ", "bb", "11"]]
+    eq = ["t#1", "=", whole]
+    C = np.array([b"a1" in r for r in rows])
+    S = np.array([r.startswith(b"ab") for r in rows])
+    T = np.array([b"a" in r and b"b" in r[r.index(b"a") + 1:] for r in rows])
+    IN = np.array([r[:2] in (b"ab", b"1 ", b"bb", b"11") for r in rows])
+    E = np.array([r == rows[n // 2] for r in rows])
+    for tree, want in ((inlist, IN), (prefix, S), (eq, E), (contains, C), (two, T), ([inlist, "AND", contains], IN & C),
+                       ([[prefix, "OR", two], "AND", ["NOT", [contains]]], (S | T) & ~C), ([eq, "OR", [contains, "AND", two]], E | C & T)):
+        np.testing.assert_array_equal(_mask(tree, col, w), want)
+
+
+def test_an_in_list_of_substrings_reads_its_bytes_in_place():
+    """Seven two-byte substrings of 180-byte rows: the first bytes of every row, not whole rows seven
+    times (1.5 M rows: 0.13 ms against 0.33)."""
+    from tqpk.ops import filter_mask
+    from tqpk.predicate import compile_filter
+    n = 1_500_000
+    rng = np.random.default_rng(1)
+    dev = torch.from_numpy(rng.choice(np.frombuffer(b"0123456789", np.int8), (5000, 180))).cuda()
+    dev = dev[torch.randint(0, 5000, (n,), device="cuda")]
+    p = compile_filter([["substring", ["t#1", "1", "2"]], "IN", ["13", "31", "23", "29", "30", "18", "17"]], {1: dev})
+    filter_mask(p, n, dev.device)
+    best = 1.0
+    for _ in range(10):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        for _ in range(10):
+            filter_mask(p, n, dev.device)
+        torch.cuda.synchronize()
+        best = min(best, (time.perf_counter() - t) / 10)
+    assert best < 0.22e-3

@@ -83,10 +83,16 @@ __global__ void __launch_bounds__(kBlock, Q == 1 ? 6 : 3) k_filter_mask(const __
   }
 }
 
-// Programs with text: the block takes 1024 rows through the program together, and a text instruction stages
-// their bytes 256 rows at a time in shared memory (coalesced), where each thread searches one row; the
-// verdicts go back to the rows' owners as bits.  Searched in place, every byte of a warp's rows was a scattered
-// load (54 us for a prefix and a two-part pattern on 800 K rows of 25 bytes).
+// Programs that search text (Contains, LIKE): the block takes 1024 rows through the program together, and a
+// search stages their bytes 256 rows at a time in shared memory (coalesced), where each thread searches one row;
+// the verdicts go back to the rows' owners as bits.  Searched in place, every byte of a warp's rows was a
+// scattered load.  Equality and prefixes stop at their first different byte and stay in place.  Rows of up to
+// kStagedRow bytes, which 48 KB hold beside the verdicts.  1.5 M rows, us in place / staged: a search without a
+// hit on 25 bytes 44 / 25, 150 bytes 444 / 111, 188 bytes 473 / 174; one that hits early in every row, 25 bytes
+// 37 / 30, 150 bytes 87 / 89, 188 bytes 83 / 120 (a predicate that keeps everything, so the line is not drawn by
+// it).  Seven substrings in an IN list on 25 bytes 33 / 63, a prefix on 150 bytes 36 / 43.
+constexpr int kStagedRow = 188;
+
 __global__ void __launch_bounds__(kBlock) k_filter_text(const __grid_constant__ tqpk_predicate P, int64_t n,
                                                         uint8_t* __restrict__ mask, unsigned long long* count, int vec,
                                                         int mask_vec) {
@@ -96,6 +102,7 @@ __global__ void __launch_bounds__(kBlock) k_filter_text(const __grid_constant__ 
   for (int64_t t0 = blockIdx.x * (int64_t)(4 * kBlock); t0 < n; t0 += (int64_t)gridDim.x * (4 * kBlock)) {
     const int64_t r0[1] = {t0 + 4 * threadIdx.x};
     const uint32_t b = eval_pred_with<1>(P, r0, n, vec, [&](const tqpk_pred_insn& I) {
+      if (I.op < TQPK_P_CONTAINS) return str_leaf4(P, I, r0[0], n);
       const int64_t stride = str_stride(P, I.col);
       const int8_t* base = static_cast<const int8_t*>(P.cols[I.col]);
 #pragma unroll 1
@@ -563,17 +570,21 @@ extern "C" int tqpk_filter_mask(const tqpk_predicate* h_pred, int64_t n, uint8_t
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int mask_vec = (reinterpret_cast<uintptr_t>(d_mask) & 3u) == 0;
   timing_before(KID_FILTER_MASK, s);
-  int64_t text = 0;              // the widest text row read
-  for (int k = 0; k < h_pred->n_insn; ++k)
-    if (h_pred->insn[k].op >= TQPK_P_STRCMP) text = std::max(text, str_stride(*h_pred, h_pred->insn[k].col));
-  if (text > 0 && text * kBlock <= 47 * 1024) {       // beside the verdicts in 48 KB
-    k_filter_text<<<grid_for((n + 3) / 4, 8), kBlock, (size_t)text * kBlock, s>>>(
+  bool text = false;
+  int64_t searched = 0;          // the widest text row that is searched
+  for (int k = 0; k < h_pred->n_insn; ++k) {
+    const tqpk_pred_insn& I = h_pred->insn[k];
+    text = text || I.op >= TQPK_P_STRCMP;
+    if (I.op >= TQPK_P_CONTAINS) searched = std::max(searched, str_stride(*h_pred, I.col));
+  }
+  if (searched > 0 && searched <= kStagedRow) {
+    k_filter_text<<<grid_for((n + 3) / 4, 8), kBlock, (size_t)searched * kBlock, s>>>(
         *h_pred, n, d_mask, d_count, pred_vec_ok(h_pred) ? 1 : 0, mask_vec);
     timing_after(KID_FILTER_MASK, s);
     TQPK_CHECK_LAUNCH();
     return TQPK_OK;
   }
-  // wider text stays four rows a thread: its bytes keep every warp busy
+  // other programs with text stay four rows a thread: its bytes keep every warp busy
   const bool many = n >= kManyRows && !text;
   auto kernel = many ? k_filter_mask<4> : k_filter_mask<1>;
   kernel<<<grid_for((n + 3) / 4 / (many ? 4 : 1), 8), kBlock, 0, s>>>(*h_pred, n, d_mask, d_count,
