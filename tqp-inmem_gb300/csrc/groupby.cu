@@ -224,7 +224,10 @@ __global__ void k_fill_u64(uint64_t* p, int64_t n, uint64_t v) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
-// What bounds it: per passing row one compare-and-swap and A reductions at scattered L2 lines.  A tile's
+// What bounds it: per passing row a slot read and A reductions at scattered L2 lines, and a compare-and-swap
+// where the slot is empty (one for every row instead queued on the words of few groups: 6 M rows of 50 groups
+// far apart 404 us, 343 with the read; 20 K groups 169 and 146, 800 K 539 and 457, 3 M 705 and 670; rows
+// stored by their key find the line in use either way: 300 K groups 227 and 235, 3 M 461 and 477).  A tile's
 // passing rows are gathered first, so that the program runs with full warps whatever the filter's
 // selectivity (4 rows a thread in place, one in seven passing, executed it almost seven times as often:
 // 576 us for 0.9 M of 6 M rows), and by the plain loop: the unrolled form with operand selects costs
@@ -267,9 +270,13 @@ __global__ void __launch_bounds__(kBlock) k_groupby_hash(const __grid_constant__
           packed += (uint64_t)(ld_int(S.keys[k], S.key_dtypes[k], row) - G.kmin[k]) * (uint64_t)G.kstride[k];
         h = hash_slot(packed, C);
         for (int64_t probes = 0;; h = (h + 1) & (C - 1)) {
-          const unsigned long long prev = atomicCAS(&hkeys[h], kHashEmpty, (unsigned long long)packed);
-          claimed = prev == kHashEmpty;
-          if (claimed || prev == packed) break;
+          unsigned long long prev = __ldcg(&hkeys[h]);
+          if (prev == packed) break;
+          if (prev == kHashEmpty) {
+            prev = atomicCAS(&hkeys[h], kHashEmpty, (unsigned long long)packed);
+            claimed = prev == kHashEmpty;
+            if (claimed || prev == packed) break;
+          }
           if (++probes > C) {              // table full: cannot happen (C >= 2 rows)
             set_error(err, TQPK_ECAPACITY);
             h = -1;
