@@ -785,6 +785,18 @@ __device__ __forceinline__ uint32_t pred_leaf(const tqpk_predicate& P, const tqp
   }
 }
 
+// Four rows of a numeric column as float64.
+__device__ __forceinline__ void ld4_as_f64(const void* col, int dt, int64_t r0, int64_t n, bool vec, double (&x)[4]) {
+  if (dt == TQPK_F64) {
+    ld4_f64(col, r0, n, vec, x);
+    return;
+  }
+  int64_t v[4];
+  ld4_int(col, dt, r0, n, vec, v);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] = static_cast<double>(v[j]);
+}
+
 template <class T, int Q>
 __device__ __forceinline__ uint32_t cmpcol_rows(const tqpk_predicate& P, const tqpk_pred_insn& I, const int64_t (&r0)[Q],
                                                 int64_t n, bool vec) {
@@ -802,21 +814,36 @@ __device__ __forceinline__ uint32_t cmpcol_rows(const tqpk_predicate& P, const t
   return 0;
 }
 
-// Two columns: in their own type when it is the same, else row by row.
+// Two columns: in their own type when it is the same, else four rows at a time in the wider one (16 rows of both
+// as int64 or float64 do not fit the registers).
 template <int Q>
 __device__ __forceinline__ uint32_t pred_cmpcol(const tqpk_predicate& P, const tqpk_pred_insn& I, const int64_t (&r0)[Q],
                                                 int64_t n, bool vec) {
   const int c2 = (int)I.lit_i, dt = P.dtypes[I.col], dt2 = P.dtypes[c2];
-  if (dt == dt2 && I.domain == TQPK_DOM_I64 && dt == TQPK_I64) return cmpcol_rows<int64_t, Q>(P, I, r0, n, vec);
-  if (dt == dt2 && I.domain == TQPK_DOM_I64 && dt == TQPK_I32) return cmpcol_rows<int32_t, Q>(P, I, r0, n, vec);
+  if (dt == dt2 && (dt == TQPK_F64) == (I.domain == TQPK_DOM_F64)) {
+    switch (dt) {
+      case TQPK_F64: return cmpcol_rows<double, Q>(P, I, r0, n, vec);
+      case TQPK_I64: return cmpcol_rows<int64_t, Q>(P, I, r0, n, vec);
+      case TQPK_I32: return cmpcol_rows<int32_t, Q>(P, I, r0, n, vec);
+    }
+  }
   uint32_t m = 0;
 #pragma unroll 1
-  for (int i = 0; i < 4 * Q; ++i) {
-    const int64_t r = r0[i >> 2] + (i & 3);
-    if (r >= n) break;
-    const bool c = I.domain == TQPK_DOM_F64 ? cmp_op<double>(I.cmp, ld_f64(P.cols[I.col], dt, r), ld_f64(P.cols[c2], dt2, r))
-                                            : cmp_op<int64_t>(I.cmp, ld_int(P.cols[I.col], dt, r), ld_int(P.cols[c2], dt2, r));
-    m |= (uint32_t)c << i;
+  for (int q = 0; q < Q; ++q) {
+    if (r0[q] >= n) break;
+    if (I.domain == TQPK_DOM_F64) {
+      double a[4], b[4];
+      ld4_as_f64(P.cols[I.col], dt, r0[q], n, vec, a);
+      ld4_as_f64(P.cols[c2], dt2, r0[q], n, vec, b);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) m |= (uint32_t)cmp_op<double>(I.cmp, a[j], b[j]) << (4 * q + j);
+    } else {
+      int64_t a[4], b[4];
+      ld4_int(P.cols[I.col], dt, r0[q], n, vec, a);
+      ld4_int(P.cols[c2], dt2, r0[q], n, vec, b);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) m |= (uint32_t)cmp_op<int64_t>(I.cmp, a[j], b[j]) << (4 * q + j);
+    }
   }
   return m;
 }

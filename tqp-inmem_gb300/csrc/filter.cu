@@ -143,6 +143,18 @@ __global__ void __launch_bounds__(kBlock) k_filter_text(const __grid_constant__ 
 // more than fewer instructions.
 constexpr int64_t kManyRows = int64_t(5) << 19;
 
+// Comparisons of columns of different types keep four rows a thread: sixteen of each do not fit the registers
+// in the wider type, and a thread that takes them four at a time has too few loads in flight (6 M rows, int32
+// against int64 29 us, uint8 against int64 25; 19 and 18 with four rows).
+static bool many_rows(const tqpk_predicate* pred, int64_t n) {
+  if (n < kManyRows) return false;
+  for (int k = 0; pred && k < pred->n_insn; ++k) {
+    const tqpk_pred_insn& I = pred->insn[k];
+    if (I.op == TQPK_P_CMPCOL && pred->dtypes[I.col] != pred->dtypes[(int)I.lit_i]) return false;
+  }
+  return true;
+}
+
 // Control block of one compaction (zeroed before the launch).
 struct CompactCtl {
   int tile_ctr;      // next tile to take
@@ -432,7 +444,7 @@ int grid_for(int64_t work_items, int per_sm) {
 static int launch_range(const tqpk_predicate* pred, const uint8_t* mask, int64_t n, const KeySet& K, bool vec,
                         int64_t* out, cudaStream_t s) {
   const RowFilter F = make_filter(pred, mask);
-  const bool many = n >= kManyRows;
+  const bool many = many_rows(F.use_pred ? pred : nullptr, n);
   auto kernel = F.use_pred ? (many ? k_key_range<4, true> : k_key_range<1, true>)
                            : (many ? k_key_range<4, false> : k_key_range<1, false>);
   kernel<<<grid_for((n + 3) / 4 / (many ? 4 : 1), 8), kBlock, 0, s>>>(
@@ -585,7 +597,7 @@ extern "C" int tqpk_filter_mask(const tqpk_predicate* h_pred, int64_t n, uint8_t
     return TQPK_OK;
   }
   // other programs with text stay four rows a thread: its bytes keep every warp busy
-  const bool many = n >= kManyRows && !text;
+  const bool many = !text && many_rows(h_pred, n);
   auto kernel = many ? k_filter_mask<4> : k_filter_mask<1>;
   kernel<<<grid_for((n + 3) / 4 / (many ? 4 : 1), 8), kBlock, 0, s>>>(*h_pred, n, d_mask, d_count,
                                                                       pred_vec_ok(h_pred) ? 1 : 0, mask_vec);
