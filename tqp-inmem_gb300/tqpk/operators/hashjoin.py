@@ -102,13 +102,13 @@ def _pair_predicate(tensors_left, tensors_right, condition_list):
         if v.tensor.dim() != 1:
             return None
         cols[cid] = v.tensor
+    wait_ready(*[tensors_left[c] if c in tensors_left else tensors_right[c] for c in ids])   # a strided one is copied
     try:
         pred = compile_filter(tree, cols)
     except NotImplementedError:
         return None
     if has_strings(pred.struct):
         return None
-    wait_ready(*[tensors_left[c] if c in tensors_left else tensors_right[c] for c in ids])
     return pred, sum(1 << i for i, c in enumerate(pred.col_ids) if c not in tensors_left)
 
 
