@@ -958,7 +958,9 @@ size_t sort_ws_bytes(int64_t n, int nk) {
   const size_t vb = n < (int64_t(1) << 32) ? 4 : 8;
   size_t b = align_up(sizeof(SortCtl), 256);
   b += align_up((size_t)nk * kDigits * kRadix * 8, 256);            // histograms
-  b += align_up((size_t)sort_tiles(n) * kRadix * 8, 256);           // look-back words
+  // look-back words; just above kLargeSort the tiles are fewer than at it, and a workspace for n rows serves
+  // any fewer
+  b += align_up((size_t)std::max(sort_tiles(n), sort_tiles(std::min(n, kLargeSort))) * kRadix * 8, 256);
   b += align_up((size_t)nk * kDigits * kRadix * 8, 256);            // offsets
   b += 2 * align_up(m * 8, 256) + 2 * align_up(m * vb, 256);
   return b + 1024;
