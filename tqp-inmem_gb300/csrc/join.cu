@@ -661,12 +661,15 @@ static bool layout(const tqpk_join_plan& p, void* ws, size_t bytes, BuildLayout&
   L.ustart = c.take<int64_t>(direct ? 1 : m + 1);
   L.head = c.take<int64_t>(direct ? 1 : m);
   L.status = c.take<uint64_t>((m + kTile - 1) / kTile + 1);
-  L.sort_bytes = sort_ws_bytes(m);
+  // the rest: the sort's, or the compaction's of a masked build side, which goes by its rows before the mask
+  const size_t used = align_up(c.off, 256);
+  L.sort_bytes = bytes > used ? (bytes - used) / 256 * 256 : 0;
   L.sort_ws = c.take<char>(L.sort_bytes);
-  return L.sort_ws != nullptr;
+  return L.sort_ws != nullptr && L.sort_bytes >= sort_ws_bytes(m);
 }
 
-static size_t layout_bytes(const tqpk_join_plan& p) {
+// nb: the build side's rows, those its mask drops among them (0: it has no mask).
+static size_t layout_bytes(const tqpk_join_plan& p, int64_t nb) {
   const int64_t m = p.nb_rows > 0 ? p.nb_rows : 1;
   const size_t e = is_wide(p) ? 8 : 4;
   const bool direct = p.mode == TQPK_JOIN_DIRECT;
@@ -675,7 +678,7 @@ static size_t layout_bytes(const tqpk_join_plan& p) {
   b += 2 * align_up(m * 8, 256);
   b += direct ? 768 : align_up(m * 8, 256) + align_up((m + 1) * 8, 256) + align_up(m * 8, 256);
   b += align_up(((m + kTile - 1) / kTile + 1) * 8, 256);
-  b += align_up(sort_ws_bytes(m), 256);
+  b += align_up(std::max(sort_ws_bytes(m), nb > 0 ? compact_status_bytes(nb) : 0), 256);
   return b + 2048;
 }
 
@@ -799,7 +802,7 @@ extern "C" int tqpk_join_plan_build(const void* keys, int32_t dt, const uint8_t*
   plan->mode = dense ? TQPK_JOIN_DIRECT : TQPK_JOIN_SORTED;
   plan->slots = dense ? range : 0;
   plan->unique = 1 | (nb >= (int64_t)0xffffffffu ? kWide : 0);
-  plan->ws_bytes = layout_bytes(*plan);
+  plan->ws_bytes = layout_bytes(*plan, mask ? nb : 0);
   return TQPK_OK;
 }
 
