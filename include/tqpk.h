@@ -304,6 +304,13 @@ int tqpk_argsort_keys(int32_t n_keys, const void* const* d_cols, const int32_t* 
                       const int32_t* h_descs, const int64_t* d_perm_in, int64_t n, int64_t* d_perm_out,
                       void* d_ws, size_t ws_bytes, tqpk_stream stream);
 
+/* Test hook, no counterpart in the reference: tqpk_argsort_keys by the form that
+ * sorts of 2^32 rows and more take (8-byte positions), for any n above 98304.  Its
+ * workspace: tqpk_argsort_keys_workspace_bytes and 8 bytes a row.            */
+int tqpk_debug_argsort_wide(int32_t n_keys, const void* const* d_cols, const int32_t* h_dtypes,
+                            const int32_t* h_widths, const int32_t* h_descs, const int64_t* d_perm_in, int64_t n,
+                            int64_t* d_perm_out, void* d_ws, size_t ws_bytes, tqpk_stream stream);
+
 /* ---- (e) top-k ------------------------------------------------------------
  * The first k entries of the stable sort of keys[perm_in[i]]:
  * d_perm_out[0..k) = perm_in of the k smallest (largest if descending) keys,

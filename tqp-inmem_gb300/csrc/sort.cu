@@ -1148,6 +1148,19 @@ static int expand_keys(int32_t nk, const void* const* cols, const int32_t* dts, 
   return m;
 }
 
+// Test hook: the form for 2^32 rows and more (8-byte positions) on any number of rows above the cluster's.
+extern "C" int tqpk_debug_argsort_wide(int32_t n_keys, const void* const* d_cols, const int32_t* dts,
+                                       const int32_t* widths, const int32_t* descs, const int64_t* d_perm_in, int64_t n,
+                                       int64_t* d_perm_out, void* ws, size_t ws_bytes, tqpk_stream stream) {
+  if (n_keys < 1 || n_keys > kMaxSortKeys || !d_cols || !dts || !widths || !descs || n <= kClusterSort || !d_perm_out || !ws)
+    return TQPK_EINVAL;
+  SortKeySet S{};
+  int rc;
+  S.n = expand_keys(n_keys, d_cols, dts, widths, descs, S.k, &rc);
+  if (S.n < 0) return rc;
+  return sort_large<uint64_t>(S, d_perm_in, n, d_perm_out, ws, ws_bytes, static_cast<cudaStream_t>(stream));
+}
+
 extern "C" size_t tqpk_argsort_keys_workspace_bytes(int64_t n, int32_t n_keys, const int32_t* dts,
                                                     const int32_t* widths) {
   if (n_keys < 1 || n_keys > kMaxSortKeys || !dts || !widths) return 0;

@@ -99,6 +99,7 @@ SIGNATURES = {
     "tqpk_argsort_stable": (C.c_int, [_VP, _I32, _I32, _VP, _I64, _VP, _VP, _SZ, _VP]),
     "tqpk_argsort_keys_workspace_bytes": (_SZ, [_I64, _I32, _P(_I32), _P(_I32)]),
     "tqpk_argsort_keys": (C.c_int, [_I32, _P(_VP), _P(_I32), _P(_I32), _P(_I32), _VP, _I64, _VP, _VP, _SZ, _VP]),
+    "tqpk_debug_argsort_wide": (C.c_int, [_I32, _P(_VP), _P(_I32), _P(_I32), _P(_I32), _VP, _I64, _VP, _VP, _SZ, _VP]),
     "tqpk_topk_workspace_bytes": (_SZ, [_I64, _I64]),
     "tqpk_topk_stable": (C.c_int, [_VP, _I32, _I32, _VP, _I64, _I64, _VP, _VP, _SZ, _VP]),
     "tqpk_topk_ties_workspace_bytes": (_SZ, [_I64]),
