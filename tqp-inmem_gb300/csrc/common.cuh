@@ -228,6 +228,9 @@ __device__ __forceinline__ uint64_t sort_key(const void* keys, int dt, int64_t i
 // row); inner: the up to three bytes before s belong to the column too.  Two or three aligned words where
 // those lie in the row (or before it), the bytes past the second word one by one where the third would
 // leave it.
+// The byte loops stay loops: with the eight loads unrolled, each under its condition, nvcc 13.0.88 built sort
+// kernels in which a row's single last byte (widths 1, 9, 17, 25) came out as bits of another register, the row
+// number among them (23 M of 490 M words, not the same ones twice); as loops every width is right.
 __device__ __forceinline__ uint64_t load_bytes8(const uint8_t* s, int left, bool inner) {
   const unsigned off = (unsigned)(reinterpret_cast<uintptr_t>(s) & 3u);
   if (left >= 8 && (off == 0 || inner)) {
