@@ -214,8 +214,7 @@ struct TopkOut {
   int64_t* cand_idx;
   unsigned* ticket;
   unsigned long long* valid_total;  // number of valid items seen (may be null)
-  unsigned long long* bound;        // the first pass's: k <= 32 the complement of the tightest cut a group found
-                                    // on its own (0: none), k > 32 the cut
+  unsigned long long* bound;        // the cut (written by the first pass)
   unsigned* arrive;                 // [2] CTAs done with the group-best and the filter pass (zeroed before the launch)
   // Optional, for a dense group table: the last CTA also writes (key_min + slot, sum[slot]) of the
   // top rows and their number (emit_keys null: not written) ...
@@ -246,8 +245,8 @@ struct TopkOut {
 // or, beyond kTopkSortCap entries, in parts.  A group of a stored column that
 // has more items under the cut than its share of the list appends its own best
 // k instead, so the list holds all that is left; of a group table (at most
-// kTopkCap candidates) the last CTA
-// then walks every item (same result, slower).  For k > 32 the cut is computed
+// kTopkCap candidates) the last CTA then walks every item (same result,
+// slower).  For k > 32 the cut is computed
 // by the last CTA of the first pass and the top-k is two launches; for k <= 32
 // every CTA of the second pass derives the cut from the group bests
 // (tk_bin_cut), and when each CTA's group fits one sweep of its threads the two
@@ -290,8 +289,8 @@ __device__ __forceinline__ bool tk_last_cta(unsigned* arrive) {
 }
 
 // The cut for k > 32: the k-th best of the ng group bests (bitonic sort of the bests in one CTA), or the
-// tightest cut a group found on its own (stored: a source that looks for one).
-__device__ __forceinline__ void tk_cut(int ng, int k, TopkOut O, bool stored) {
+// tightest cut a group found on its own (owns: they looked for one).
+__device__ __forceinline__ void tk_cut(int ng, int k, TopkOut O, bool owns) {
   __shared__ uint64_t v[kTopkGroups];
   for (int i = threadIdx.x; i < kTopkGroups; i += blockDim.x) v[i] = i < ng ? __ldcg(&O.cand_key[O.cap + i]) : ~0ull;
   __syncthreads();
@@ -305,10 +304,13 @@ __device__ __forceinline__ void tk_cut(int ng, int k, TopkOut O, bool stored) {
       }
       __syncthreads();
     }
-  if (threadIdx.x == 0) {
-    const uint64_t cut = v[(k <= kTopkGroups ? k : kTopkGroups) - 1];
-    *O.bound = stored ? min(cut, ~(uint64_t)__ldcg(O.bound)) : cut;
-  }
+  const uint64_t cut = v[(k <= kTopkGroups ? k : kTopkGroups) - 1];
+  if (threadIdx.x == 0) *O.bound = cut;
+  if (!owns) return;
+  __syncthreads();
+  uint64_t own = ~0ull;
+  for (int i = threadIdx.x; i < ng; i += blockDim.x) own = min(own, __ldcg(&O.cand_key[O.cap + kTopkGroups + i]));
+  if (own < cut) atomicMin(O.bound, (unsigned long long)own);
 }
 
 // One CTA's walk over items [b0, b1) in quads (4 items per thread, 256 threads): kTopkQuads
@@ -342,27 +344,38 @@ __device__ __forceinline__ void tk_scan_group(const Src& src, int64_t b0, int64_
   }
 }
 
-// A cut from one CTA's items alone, from every thread's best key (~0: it has none): the k-th best of a warp's
-// threads, the best warp's of the CTA (k <= 32), or the worst of the warps' ceil(k / 8)-th bests (k <= 256);
-// at least k items lie at or under it.  Neighbouring items belong to neighbouring threads, so of a column that
-// is stored sorted, or in sorted runs, it lets at most ~4 k of one group through; the cut from the groups'
-// bests alone lets k whole groups through.  Called by all 256 threads; red: 8 words.
-__device__ __forceinline__ uint64_t tk_own_cut(uint64_t own, int k, uint64_t* red) {
-  const int lane = threadIdx.x & 31;
+// Whether groups look for a cut of their own: groups of up to kTopkSortCap items fit the second pass's buffer
+// whole (the search is ~1 us of 40), and for k = 1 the group's best is that cut.
+__host__ __device__ constexpr bool tk_own_cuts(int64_t G, int k) { return k > 1 && G > 2048; }
+
+// The best of every thread's best key (~0: it has none), and from those a cut of this CTA's own: the k-th best
+// of a warp's threads, the best warp's of the CTA (k <= 32), or the worst of the warps' ceil(k / 8)-th bests
+// (k <= 256); at least k items lie at or under it.  Neighbouring items belong to neighbouring threads, so of a
+// column that is stored sorted, or in sorted runs, it lets at most ~4 k of one group through; the cut from the
+// groups' bests alone lets k whole groups through (6 M rows stored descending, two keys: 0.59 ms at k = 10 and
+// 1.29 at k = 256 with each group's parts streamed, 0.11 and 0.13 with this cut).  The group keeps it behind the
+// bests.  Called by all 256 threads; red: 16 words.
+__device__ __forceinline__ uint64_t tk_own_cut(uint64_t& best, int k, uint64_t* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t v = best;                       // sorted by the warp: its least comes with it
 #pragma unroll
   for (int size = 2; size <= 32; size <<= 1)
 #pragma unroll
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      const uint64_t other = __shfl_xor_sync(0xffffffffu, own, stride);
+      const uint64_t other = __shfl_xor_sync(0xffffffffu, v, stride);
       const bool low = ((lane & stride) == 0) == ((lane & size) == 0);      // keeps the smaller of the two
-      own = (other < own) == low ? other : own;
+      v = (other < v) == low ? other : v;
     }
-  const uint64_t mine = __shfl_sync(0xffffffffu, own, (k <= 32 ? k : (k + 7) / 8) - 1);
+  if (lane == 0) red[warp] = v;
+  if (lane == (k <= 32 ? k : (k + 7) / 8) - 1) red[8 + warp] = v;
   __syncthreads();
-  if (lane == 0) red[threadIdx.x >> 5] = mine;
-  __syncthreads();
-  uint64_t cut = red[0];
-  for (int w = 1; w < 8; ++w) cut = (red[w] < cut) == (k <= 32) ? red[w] : cut;
+  best = red[0];
+  uint64_t cut = red[8];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) {
+    best = min(best, red[w]);
+    cut = k <= 32 ? min(cut, red[8 + w]) : max(cut, red[8 + w]);
+  }
   return cut;
 }
 
@@ -371,7 +384,7 @@ __device__ __forceinline__ uint64_t tk_own_cut(uint64_t own, int k, uint64_t* re
 // last CTA to finish computes the cut from all groups' bests.
 template <class Src>
 __global__ void __launch_bounds__(256) k_tk_group_best(Src src, int64_t G, int k, TopkOut O) {
-  __shared__ uint64_t red[8];
+  __shared__ uint64_t red[16];
   const int64_t b0 = (int64_t)blockIdx.x * G, b1 = b0 + G < src.n ? b0 + G : src.n;
   __shared__ unsigned s_valid, s_bits;
   if (threadIdx.x == 0) { s_valid = 0; s_bits = 0; }
@@ -392,7 +405,13 @@ __global__ void __launch_bounds__(256) k_tk_group_best(Src src, int64_t G, int k
     if (valid) atomicAdd(&s_valid, valid);
     if (nbits) atomicAdd(&s_bits, nbits);
   }
-  block_min_u64(best, red);        // its barriers order the shared counts too
+  // (the barriers of either order the shared counts too)
+  if (Src::kStoredOrder && tk_own_cuts(G, k)) {
+    const uint64_t cut = tk_own_cut(best, k, red);
+    if (threadIdx.x == 0) O.cand_key[O.cap + kTopkGroups + blockIdx.x] = cut;
+  } else {
+    block_min_u64(best, red);
+  }
   const unsigned equal = __popc(__ballot_sync(0xffffffffu, items && own == best));
   if ((threadIdx.x & 31) == 0 && equal) atomicAdd(&s_equal, equal);
   __syncthreads();
@@ -403,12 +422,8 @@ __global__ void __launch_bounds__(256) k_tk_group_best(Src src, int64_t G, int k
     if (s_valid && O.valid_total) atomicAdd(O.valid_total, (unsigned long long)s_valid);
     if (s_bits && O.bits_set) atomicAdd(O.bits_set, (unsigned long long)s_bits);
   }
-  if constexpr (Src::kStoredOrder) {
-    const uint64_t cut = tk_own_cut(own, k, red);
-    if (threadIdx.x == 0 && cut != ~0ull) atomicMax(O.bound, ~(unsigned long long)cut);     // bound: 0 before
-  }
   if (k <= 32) return;              // the filter pass derives its cut from the group bests itself
-  if (tk_last_cta(O.arrive)) tk_cut((int)gridDim.x, k, O, Src::kStoredOrder);
+  if (tk_last_cta(O.arrive)) tk_cut((int)gridDim.x, k, O, Src::kStoredOrder && tk_own_cuts(G, k));
 }
 
 // The cut for k <= 32, computed by every CTA of the filter pass from the ng group bests (no
@@ -417,12 +432,13 @@ __global__ void __launch_bounds__(256) k_tk_group_best(Src src, int64_t G, int k
 // an item of its own group, so at least k items lie at or under the cut, and the top k are among
 // them; for independent keys about k ln k items pass.  Fewer than k non-empty groups: ~0 (every
 // item passes).  Called by all threads.
-__device__ __forceinline__ uint64_t tk_bin_cut(int ng, int k, const TopkOut& O) {
+__device__ __forceinline__ uint64_t tk_bin_cut(int ng, int k, const TopkOut& O, bool owns = false) {
   __shared__ unsigned long long bin[32];
   __shared__ unsigned s_ne;
-  __shared__ unsigned long long s_cut;
+  __shared__ unsigned long long s_cut, s_own;
+  uint64_t own = ~0ull;
   if (threadIdx.x < 32) bin[threadIdx.x] = ~0ull;
-  if (threadIdx.x == 0) { s_ne = 0; s_cut = 0; }
+  if (threadIdx.x == 0) { s_ne = 0; s_cut = 0; s_own = ~0ull; }
   __syncthreads();
   // the rank of a non-empty group among the non-empty ones decides its bin: groups are read in
   // index order in chunks of 256, each chunk's non-empty ones numbered by a block scan
@@ -430,6 +446,7 @@ __device__ __forceinline__ uint64_t tk_bin_cut(int ng, int k, const TopkOut& O) 
   for (int base = 0; base < ng; base += 256) {
     const int g = base + threadIdx.x;
     const uint64_t v = g < ng ? __ldcg(&O.cand_key[O.cap + g]) : ~0ull;
+    if (owns && g < ng) own = min(own, __ldcg(&O.cand_key[O.cap + kTopkGroups + g]));
     const bool ne = v != ~0ull;
     const unsigned m = __ballot_sync(0xffffffffu, ne);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -442,6 +459,11 @@ __device__ __forceinline__ uint64_t tk_bin_cut(int ng, int k, const TopkOut& O) 
     if (threadIdx.x == 0) for (int w = 0; w < 8; ++w) s_ne += wsum[w];
     __syncthreads();
   }
+  if (owns) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) own = min(own, __shfl_xor_sync(0xffffffffu, own, o));
+    if ((threadIdx.x & 31) == 0) atomicMin(&s_own, (unsigned long long)own);
+  }
   if (threadIdx.x < 32) {
     unsigned long long c = threadIdx.x < k ? bin[threadIdx.x] : 0ull;
 #pragma unroll
@@ -449,7 +471,7 @@ __device__ __forceinline__ uint64_t tk_bin_cut(int ng, int k, const TopkOut& O) 
     if (threadIdx.x == 0) s_cut = s_ne >= (unsigned)k ? c : ~0ull;
   }
   __syncthreads();
-  return s_cut;
+  return min(s_cut, s_own);
 }
 
 constexpr int kTopkSortCap = 2048;   // candidates the final CTA sorts in shared memory
@@ -479,7 +501,7 @@ __device__ __forceinline__ void tk_finish_warp(int m, const TopkOut& O, const in
 }
 
 // Sorts cnt (<= kTopkSortCap) entries by (key, index), in one CTA of 256 threads.
-__device__ __forceinline__ void tk_sort(int cnt, uint64_t* sk, int64_t* si) {
+static __device__ __noinline__ void tk_sort(int cnt, uint64_t* sk, int64_t* si) {
   int P = 2;
   while (P < cnt) P <<= 1;
   for (int i = cnt + threadIdx.x; i < P; i += blockDim.x) {
@@ -505,7 +527,7 @@ __device__ __forceinline__ void tk_sort(int cnt, uint64_t* sk, int64_t* si) {
 // buffer (sk, si: kTopkSortCap entries), which is sorted and cut back to k when the next step might not fit.
 // Returns their number, to every thread.  Warp lists (WarpList) took 0.4 us an insertion at k = 256.
 template <class Load>
-__device__ __forceinline__ int tk_stream_best(int64_t m, int k, uint64_t cut, uint64_t* sk, int64_t* si, Load load) {
+__device__ __noinline__ int tk_stream_best(int64_t m, int k, uint64_t cut, uint64_t* sk, int64_t* si, Load load) {
   __shared__ unsigned s_fill;
   const int lane = threadIdx.x & 31;
   uint64_t worst_key = cut;
@@ -658,9 +680,7 @@ __device__ __forceinline__ void tk_final(const Src& src, int k, TopkOut O, uint6
 template <int R, class Src>
 __global__ void __launch_bounds__(256) k_tk_filter(Src src, int64_t G, int k, TopkOut O) {
   const int lane = threadIdx.x & 31;
-  uint64_t cut = k <= 32 ? tk_bin_cut((int)gridDim.x, k, O) : __ldcg(O.bound);
-  if constexpr (Src::kStoredOrder)
-    if (k <= 32) cut = min(cut, ~(uint64_t)__ldcg(O.bound));
+  const uint64_t cut = k <= 32 ? tk_bin_cut((int)gridDim.x, k, O, Src::kStoredOrder && tk_own_cuts(G, k)) : __ldcg(O.bound);
   const int64_t b0 = (int64_t)blockIdx.x * G, b1 = b0 + G < src.n ? b0 + G : src.n;
   unsigned valid = 0, nbits = 0;
   __shared__ uint64_t sk[kTopkSortCap];
@@ -835,8 +855,8 @@ inline size_t topk_cand_entries(int k) {
   const size_t a = (size_t)topk_grid_size() * k;
   return a > (size_t)kTopkCand ? a : (size_t)kTopkCand;
 }
-// A stored column's list (tqpk_topk_stable): a share for every group, and the groups' bests.
-inline size_t topk_list_entries(int k) { return (size_t)kTopkGroups * (topk_list_share(k) + 1); }
+// A stored column's list (tqpk_topk_stable): a share for every group, the groups' bests, and their own cuts.
+inline size_t topk_list_entries(int k) { return (size_t)kTopkGroups * (topk_list_share(k) + 2); }
 inline size_t topk_scratch_bytes(int k) {
   // ticket block + count + k indices + two candidate arrays, each 256-byte aligned
   return 2 * align_up(topk_list_entries(k) * 8, 256) + align_up((size_t)k * 8, 256) + 1024;
