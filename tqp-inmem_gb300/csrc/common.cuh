@@ -753,13 +753,20 @@ __device__ __forceinline__ uint32_t f64_leaf(const tqpk_predicate& P, const tqpk
                                              int64_t n, bool vec) {
   double x[4 * Q];
   load_rows<double, Q>(P.cols[I.col], r0, n, vec, x);
-  if (I.cmp == TQPK_ISCLOSE)
-    return bits_of<4 * Q>([&](int i) {
-      const double err = fabs(__dsub_rn(x[i], I.lit_f));
-      return (x[i] == I.lit_f) || (isfinite(err) && err <= I.lit_aux);
-    });
   constexpr uint64_t kInf = 0x7ff0000000000000ull;
   const uint64_t lit = d2u(I.lit_f);
+  if (I.cmp == TQPK_ISCLOSE) {
+    // x == literal, or a finite |x - literal| within the allowed error: the difference is the one FP64
+    // instruction a row (6 M rows 23 us; with the three comparisons 55), the tests are on its bits
+    const int64_t allowed = I.lit_aux >= 0.0 ? (int64_t)(d2u(I.lit_aux) & ~(1ull << 63)) : -1;     // NaN: none
+    const bool number = (lit << 1) <= (kInf << 1);
+    return bits_of<4 * Q>([&](int i) {
+      const uint64_t u = d2u(x[i]);
+      const int64_t err = (int64_t)(d2u(__dsub_rn(x[i], I.lit_f)) & ~(1ull << 63));
+      const bool same = u == lit || ((u | lit) << 1) == 0;
+      return (number && same) || (err < (int64_t)kInf && err <= allowed);
+    });
+  }
   if ((lit << 1) > (kInf << 1)) return I.cmp == TQPK_NE ? ~0u : 0u;       // a NaN literal
   int64_t y[4 * Q];
   uint32_t nan = 0;
