@@ -21,3 +21,24 @@ def test_few_repeated_build_keys_out_of_many_rows(spread):
     bi, pi = join_probe(b, probe)
     np.testing.assert_array_equal(pi.cpu().numpy(), [0, 0, 2, 3, 3])
     np.testing.assert_array_equal(bi.cpu().numpy(), [777_776, 777_777, 5, nb - 2, nb - 1])
+
+
+@pytest.mark.parametrize("cmp", [-3, 6, 7, 1 << 20])
+def test_a_condition_with_an_unknown_operator_holds_for_no_pair(cmp):
+    """As in a filter; the operator is an index into the table that turns a comparison round only when it
+    is one of that table's."""
+    from tqpk import _lib as L
+    from tqpk.ops import join_build, join_pairs
+    from tqpk.predicate import compile_filter
+    keys = torch.arange(600, device="cuda") // 3
+    cols = {1: torch.zeros(600, dtype=torch.int64, device="cuda"), 2: torch.zeros(200, dtype=torch.int64, device="cuda")}
+    cond = compile_filter(["b#2", "<", "a#1"], cols)
+    cond.struct.insn[0].cmp = cmp
+    side = sum(1 << i for i, c in enumerate(cond.col_ids) if c == 2)
+    probe = torch.arange(200, device="cuda")
+    if cmp == L.ISCLOSE:                              # refused, as the filter refuses it
+        with pytest.raises(ValueError):
+            join_pairs(join_build(keys), probe, None, cond, side)
+        return
+    bi, pi = join_pairs(join_build(keys), probe, None, cond, side)
+    assert bi.numel() == 0 and pi.numel() == 0

@@ -994,7 +994,8 @@ static int pair_cond(const tqpk_predicate* cond, uint32_t probe_cols, PairCond& 
   if (cond->n_insn == 1 && I.op == TQPK_P_CMPCOL && I.domain == TQPK_DOM_I64) {
     const int c1 = I.col, c2 = (int)I.lit_i;
     const bool p1 = (probe_cols >> c1) & 1u, p2 = (probe_cols >> c2) & 1u;
-    if (p1 != p2 && is_int_dtype(cond->dtypes[c1]) && is_int_dtype(cond->dtypes[c2])) {
+    const bool known = I.cmp >= TQPK_LT && I.cmp <= TQPK_NE;       // another operator holds for no pair
+    if (known && p1 != p2 && is_int_dtype(cond->dtypes[c1]) && is_int_dtype(cond->dtypes[c2])) {
       const int bc = p1 ? c2 : c1, pc = p1 ? c1 : c2;
       static const int flipped[] = {TQPK_GT, TQPK_GE, TQPK_LT, TQPK_LE, TQPK_EQ, TQPK_NE};   // of LT, LE, GT, ...
       C.two_sided = 1;
