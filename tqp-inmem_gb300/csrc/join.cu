@@ -794,7 +794,8 @@ extern "C" int tqpk_join_plan_build(const void* keys, int32_t dt, const uint8_t*
   plan->key_min = rows ? mn : 0;
   plan->key_max = rows ? mx : -1;
   const int64_t range = rows ? (mx - mn + 1) : 1;
-  // direct addressing costs 4 B per slot of the key range (12 B when keys repeat); up to 2^24 slots
+  // direct addressing reads 4 B per slot of the key range (12 B when keys repeat; the workspace holds 12, and about
+  // 40 per build row, as repeats show while the directory is filled); up to 2^24 slots
   // that is cheaper than a binary search per probe row even for a sparse build side (a filtered
   // dimension of 2 M keys joined by a 60 M-row fact table: 7.6 ms sorted, ~0.1 ms direct)
   const bool dense = rows == 0 || (range > 0 && range <= std::max<int64_t>(4 * rows, int64_t(1) << 24) &&

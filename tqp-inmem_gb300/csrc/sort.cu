@@ -4,7 +4,7 @@
 // key first), permuting `perm` each time, then slices perm[:limit].
 // sort_keys runs that whole loop: keys[0] is the most significant key, and the
 // keys are sorted last to first, each key's digits least significant first.
-// tqpk_argsort_stable is its one-key form.
+// tqpk_argsort_stable is its one-key form, and waits for it beyond one CTA's rows.
 //
 // Up to 2048 rows are sorted by one CTA, up to 98304 by one cluster; more rows
 // by the tiled passes below.
