@@ -59,7 +59,8 @@ class JoinAggTopK:
         nbytes = self.lib.tqpk_pipeline_join_agg_topk_workspace_bytes(self.key_min, self.key_max)
         self.ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=self.dev)
         # one block, so that the result comes back in one copy: row count, group count, keys, sums
-        self._out = torch.zeros(2 + 2 * self.k, dtype=torch.int64, device=self.dev)
+        self._out = torch.empty(2 + 2 * self.k, dtype=torch.int64, device=self.dev)
+        self._out[:2].zero_()          # the counts only: a run on another stream may already be writing the rows
         self.out_count, self.groups = self._out[:1], self._out[1:2]
         self.out_keys = self._out[2:2 + self.k]
         self.out_vals = self._out[2 + self.k:].view(torch.float64)
@@ -295,7 +296,8 @@ class StarAggTopK:
         self.ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=self.dev)
         # one block, so that the result comes back in one copy: the directories' error words (int32),
         # row count, group count, keys, sums, counts
-        self._out = torch.zeros(4 + 3 * self.k, dtype=torch.int64, device=self.dev)
+        self._out = torch.empty(4 + 3 * self.k, dtype=torch.int64, device=self.dev)
+        self._out[2:4].zero_()         # the counts only: a run on another stream may already be writing the rest
         self.out_count, self.groups = self._out[2:3], self._out[3:4]
         self.out_keys = self._out[4:4 + self.k]
         self.out_vals = self._out[4 + self.k:4 + 2 * self.k].view(torch.float64)
@@ -340,6 +342,7 @@ class StarAggTopK:
         self.sum = torch.empty(cmx - cmn + 1, dtype=torch.float64, device=dev)
         self.cnt = torch.empty(cmx - cmn + 1, dtype=torch.int32, device=dev)
         self.err = self._out[:2].view(torch.int32)[:3]
+        self.err.zero_()               # on the run's stream
         self.tws = torch.empty(self.lib.tqpk_dense_topk_workspace_bytes(self.k), dtype=torch.uint8, device=dev)
         # fkB loaded with fkA and evict-first column loads: 529 -> 507 us on the 59,986,052-row star join
         # + B's directory composed with C's (no C lookup in the probe)
