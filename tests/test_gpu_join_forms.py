@@ -42,3 +42,38 @@ def test_a_condition_with_an_unknown_operator_holds_for_no_pair(cmp):
         return
     bi, pi = join_pairs(join_build(keys), probe, None, cond, side)
     assert bi.numel() == 0 and pi.numel() == 0
+
+
+@pytest.mark.parametrize("nb,np_,keys", [(300, 1, 1), (3000, 700, 1), (17, 3000, 1), (2500, 5000, 3), (40_000, 40, 2), (5000, 9000, 2500),
+                                         (4000, 320_000, 200)])
+@pytest.mark.parametrize("conditions", [0, 1, 2])
+def test_long_runs_are_shared_by_several_ctas(nb, np_, keys, conditions):
+    """Few probe rows, many build rows a key: a tile's pairs are split among CTAs, in the pairs' order."""
+    from tqpk.ops import join_build, join_pairs
+    from tqpk.predicate import compile_filter
+    rng = np.random.default_rng(nb + np_)
+    bk, pk = rng.integers(0, keys, nb), rng.integers(-1, keys + 1, np_)
+    a, c = rng.integers(0, 400, nb), rng.integers(0, 400, np_)
+    e, f = rng.integers(0, 100, nb).astype(np.int32), rng.integers(0, 100, np_).astype(np.int32)
+    mask = rng.random(np_) < 0.8
+    dev = {i: torch.from_numpy(v).cuda() for i, v in ((1, a), (2, c), (3, e), (4, f))}
+    cond, side = None, 0
+    if conditions:
+        tree = ["x#1", "=", "y#2"]
+        if conditions == 2:
+            tree = [tree, "OR", [["x#3", "<", "y#4"], "AND", ["y#2", "<", "9"]]]
+        cond = compile_filter(tree, dev)
+        side = sum(1 << i for i, col in enumerate(cond.col_ids) if col in (2, 4))
+    bi, pi = join_pairs(join_build(torch.from_numpy(bk).cuda()), torch.from_numpy(pk).cuda(), torch.from_numpy(mask).cuda(), cond, side)
+    order = np.argsort(bk, kind="stable")
+    starts = np.searchsorted(bk[order], pk, "left")
+    counts = (np.searchsorted(bk[order], pk, "right") - starts) * mask
+    want_p = np.repeat(np.arange(np_), counts)
+    want_b = order[np.repeat(starts, counts) + np.arange(counts.sum()) - np.repeat(np.cumsum(counts) - counts, counts)]
+    if conditions:
+        keep = a[want_b] == c[want_p]
+        if conditions == 2:
+            keep |= (e[want_b] < f[want_p]) & (c[want_p] < 9)
+        want_b, want_p = want_b[keep], want_p[keep]
+    np.testing.assert_array_equal(pi.cpu().numpy(), want_p)
+    np.testing.assert_array_equal(bi.cpu().numpy(), want_b)

@@ -382,7 +382,10 @@ __device__ __forceinline__ bool pair_holds(const PairCond& C, int64_t b, int64_t
 // passes, took 248 + 300 us.  So the usual condition's build column is laid out in csr order first, a row's
 // values then come two to a load, and a tile whose rows have at most kRowPairs candidates each gives every
 // thread its own four rows and keeps its verdicts for the writing pass.  Longer runs are spread over the
-// block pair by pair, by a search in the tile's scan, in both passes.
+// block pair by pair, by a search in the tile's scan, in both passes; where the probe side has too few tiles
+// for the GPU, gridDim.y CTAs share a tile's pairs, each a consecutive part of them (3000 x 3000 rows of one key
+// with a second key, three tiles: 23.4 ms with one CTA a tile, which had to judge its pairs twice, 15.4 when they
+// were written, gathered, filtered and compacted, now 0.49; 20 K probe rows of ordinary runs as before).
 constexpr int kRowPairs = 16;
 
 template <bool COUNT, bool COND>
@@ -397,12 +400,15 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
   __shared__ int64_t s_first[kRows ? kPairRows : 1];   // where its build rows start
   __shared__ int s_last;
   const int64_t tile = blockIdx.x;
+  const int part = blockIdx.y, parts = gridDim.y;
+  const int64_t slot = tile * parts + part;             // of tile_base
   const int64_t g0 = tile * kPairRows + 4 * threadIdx.x;
   if (!COUNT && COND && W.by_row[tile]) {
+    if (part > 0) return;
     uint64_t held = W.held[tile * kBlock + threadIdx.x];
     const uint4 f4 = *reinterpret_cast<const uint4*>(&W.first[4 * (tile * kBlock + threadIdx.x)]);
     int64_t kept;
-    int64_t at = tile_base[tile] + block_excl_scan<kBlock, int64_t>(__popcll(held), kept, sw);
+    int64_t at = tile_base[slot] + block_excl_scan<kBlock, int64_t>(__popcll(held), kept, sw);
     for (; held; held &= held - 1, ++at) {
       const int q = __ffsll((long long)held) - 1, j = q >> 4;
       const int64_t f = (int64_t)(j == 0 ? f4.x : j == 1 ? f4.y : j == 2 ? f4.z : f4.w) + (q & 15);
@@ -443,8 +449,10 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
   __shared__ unsigned s_kept[2][kBlock / 32];
   const bool by_row = COUNT && COND && !__syncthreads_or(D.wide || cnt[0] > kRowPairs || cnt[1] > kRowPairs ||
                                                          cnt[2] > kRowPairs || cnt[3] > kRowPairs);
-  if (COUNT && COND && threadIdx.x == 0) W.by_row[tile] = by_row;
-  if (by_row) {
+  if (COUNT && COND && threadIdx.x == 0 && part == 0) W.by_row[tile] = by_row;
+  int64_t from = total * part / parts, to = total * (part + 1) / parts;       // this CTA's pairs of the tile
+  if (by_row && part > 0) to = from = total = 0;
+  if (by_row && part == 0) {
     uint64_t held = 0;
     int64_t pv[4] = {0, 0, 0, 0};
     if (b && C.two_sided) {
@@ -497,6 +505,8 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
     *reinterpret_cast<uint4*>(&W.first[4 * (tile * kBlock + threadIdx.x)]) =
         make_uint4((unsigned)first[0], (unsigned)first[1], (unsigned)first[2], (unsigned)first[3]);
     block_excl_scan<kBlock, int64_t>(__popcll(held), total, sw);
+  } else {
+    total = to - from;
   }
   if (kRows && !by_row) {
 #pragma unroll
@@ -509,7 +519,7 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
   }
   if (COUNT && COND && !by_row) {
     int64_t kept = 0;
-    for (int64_t o = threadIdx.x; o < total; o += kBlock) {
+    for (int64_t o = from + threadIdx.x; o < to; o += kBlock) {
       int row;
       int64_t build;
       pair(o, row, build);
@@ -518,21 +528,22 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
     block_excl_scan<kBlock, int64_t>(kept, total, sw);
   }
   if (COUNT) {
+    const int64_t slots = (int64_t)gridDim.x * parts;
     if (threadIdx.x == 0) {
-      tile_base[tile] = total;
+      tile_base[slot] = total;
       __threadfence();
-      s_last = atomicAdd(&ctl->done, 1u) == gridDim.x - 1;
+      s_last = atomicAdd(&ctl->done, 1u) == (unsigned)(slots - 1);
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
     int64_t run = 0;
-    for (int64_t t0 = 0; t0 < (int64_t)gridDim.x; t0 += 4 * kBlock) {
+    for (int64_t t0 = 0; t0 < slots; t0 += 4 * kBlock) {
       int64_t c[4], sum = 0;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int64_t t = t0 + 4 * threadIdx.x + q;
-        c[q] = t < (int64_t)gridDim.x ? __ldcg(reinterpret_cast<const long long*>(&tile_base[t])) : 0;
+        c[q] = t < slots ? __ldcg(reinterpret_cast<const long long*>(&tile_base[t])) : 0;
         sum += c[q];
       }
       int64_t all;
@@ -540,7 +551,7 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int64_t t = t0 + 4 * threadIdx.x + q;
-        if (t < (int64_t)gridDim.x) tile_base[t] = at;
+        if (t < slots) tile_base[t] = at;
         at += c[q];
       }
       run += all;
@@ -548,9 +559,10 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
     if (threadIdx.x == 0) ctl->total = run;
     return;
   }
-  int64_t base = tile_base[tile];
+  int64_t base = tile_base[slot];
   if (!COND) {
-    for (int64_t o = threadIdx.x; o < total; o += kBlock) {
+    base -= from;
+    for (int64_t o = from + threadIdx.x; o < to; o += kBlock) {
       if (base + o >= capacity) break;
       int row;
       int64_t build;
@@ -561,17 +573,17 @@ __global__ void __launch_bounds__(kBlock) k_join_pairs(JoinDir D, const void* pk
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int64_t o0 = 0; o0 < total; o0 += kBlock) {
+  for (int64_t o0 = from; o0 < to; o0 += kBlock) {
     const int64_t o = o0 + threadIdx.x;
     int row = 0;
     int64_t build = 0;
     bool keep = false;
-    if (o < total) {
+    if (o < to) {
       pair(o, row, build);
       keep = pair_holds(C, build, tile * kPairRows + row);
     }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
-    unsigned* kept = s_kept[(o0 / kBlock) & 1];
+    unsigned* kept = s_kept[((o0 - from) / kBlock) & 1];
     if (lane == 0) kept[warp] = __popc(m);
     __syncthreads();                 // two buffers: the next chunk's counts do not overwrite this one's
     int64_t at = base + __popc(m & ((1u << lane) - 1u));
@@ -733,6 +745,14 @@ struct ProbeLayout {
   int64_t* vals;
 };
 
+// CTAs that share a tile's pairs: two per SM in all while the tiles are fewer than that.
+constexpr int64_t kMaxParts = 128, kPartSlots = 1024;       // at most tiles + kPartSlots places in tile_base
+static dim3 pair_grid(int64_t tiles) {
+  const int64_t want = std::min<int64_t>(2 * num_sms(), kPartSlots);
+  const int64_t parts = tiles < want ? std::min(kMaxParts, (want + tiles - 1) / tiles) : 1;
+  return dim3((unsigned)tiles, (unsigned)parts);
+}
+
 static bool probe_layout(int64_t np, void* pws, size_t bytes, ProbeLayout& W, int64_t cond_build_rows = -1) {
   const int64_t tiles = (np + kTile - 1) / kTile;
   WsCursor cur(pws, bytes);
@@ -743,7 +763,7 @@ static bool probe_layout(int64_t np, void* pws, size_t bytes, ProbeLayout& W, in
   W.status_b = cur.take<uint64_t>(tiles + 1);
   W.zeroed = cur.off;
   const int64_t ptiles = (np + kPairRows - 1) / kPairRows;
-  W.tile_base = cur.take<int64_t>(ptiles + 1);
+  W.tile_base = cur.take<int64_t>(ptiles + kPartSlots + 1);
   if (cond_build_rows < 0) return W.tile_base != nullptr;
   W.kept.by_row = cur.take<uint8_t>(ptiles + 1);
   W.kept.held = cur.take<uint64_t>(ptiles * kBlock + 1);
@@ -758,8 +778,8 @@ static int count_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFi
   const int64_t tiles = (np + kPairRows - 1) / kPairRows;
   if (tiles > INT32_MAX) return TQPK_EUNSUPPORTED;
   auto kernel = C.P.n_insn ? k_join_pairs<true, true> : k_join_pairs<true, false>;
-  kernel<<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, nullptr, nullptr, 0, W.tile_base,
-                                       W.pair, W.kept, C);
+  kernel<<<pair_grid(tiles), kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, nullptr, nullptr, 0,
+                                             W.tile_base, W.pair, W.kept, C);
   TQPK_CHECK_LAUNCH();
   return TQPK_OK;
 }
@@ -769,8 +789,8 @@ static int write_pairs(const JoinDir& D, const void* pkeys, int pdt, const RowFi
   const int64_t tiles = (np + kPairRows - 1) / kPairRows;
   auto kernel = C.P.n_insn ? k_join_pairs<false, true> : k_join_pairs<false, false>;
   timing_before(KID_JOIN_PROBE, s);
-  kernel<<<(int)tiles, kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, out_b, out_p, capacity,
-                                       W.tile_base, W.pair, W.kept, C);
+  kernel<<<pair_grid(tiles), kBlock, 0, s>>>(D, pkeys, pdt, F, np, aligned16(pkeys) ? 1 : 0, out_b, out_p, capacity,
+                                             W.tile_base, W.pair, W.kept, C);
   timing_after(KID_JOIN_PROBE, s);
   TQPK_CHECK_LAUNCH();
   return TQPK_OK;
@@ -903,7 +923,7 @@ extern "C" int tqpk_join_build(tqpk_join_plan* plan, const void* keys, int32_t d
 
 extern "C" size_t tqpk_join_probe_workspace_bytes(int64_t np) {
   const int64_t tiles = (np + kTile - 1) / kTile;
-  return 2048 + 2 * align_up((size_t)(tiles + 1) * 8, 256) + align_up(((size_t)np / kPairRows + 2) * 8, 256);
+  return 2048 + 2 * align_up((size_t)(tiles + 1) * 8, 256) + align_up(((size_t)np / kPairRows + kPartSlots + 2) * 8, 256);
 }
 
 extern "C" size_t tqpk_join_pairs_workspace_bytes(const tqpk_join_plan* plan, int64_t np, int32_t with_cond) {
