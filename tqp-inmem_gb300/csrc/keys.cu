@@ -197,11 +197,9 @@ __global__ void k_string_words(const uint8_t* __restrict__ src, int64_t n, int w
   }
 }
 
-// Rows of up to kStageRow bytes: a thread reads its row by words into shared memory, and the block writes its
+// Rows of fewer than 16 bytes: a thread reads its row by words into shared memory, and the block writes its
 // 256 rows, which lie one after another, 16 bytes at a time.  A byte per thread with a 64-bit division each
 // took 57 us for 1.5 M rows of 15 bytes.
-constexpr int kStageRow = 160;
-
 __global__ void __launch_bounds__(kBlock) k_gather_short_rows(const uint8_t* __restrict__ src, int w,
                                                               const int64_t* __restrict__ idx, int64_t n_idx,
                                                               int64_t n_src, uint8_t* __restrict__ dst, int vec) {
@@ -228,6 +226,80 @@ __global__ void __launch_bounds__(kBlock) k_gather_short_rows(const uint8_t* __r
       reinterpret_cast<uint4*>(o)[i] = reinterpret_cast<const uint4*>(stage)[i];
     for (int i = whole * 16 + threadIdx.x; i < bytes; i += kBlock) o[i] = stage[i];
     __syncthreads();
+  }
+}
+
+// Sixteen bytes of a column of `total` bytes from byte `at` on (those past its end: 0), by aligned words that
+// lie in it, byte by byte at its ends.
+__device__ __forceinline__ ulonglong2 load_bytes16(const uint8_t* col, int64_t at, int64_t total) {
+  const uint8_t* s = col + at;
+  const unsigned off = (unsigned)(reinterpret_cast<uintptr_t>(s) & 3u);
+  if ((reinterpret_cast<uintptr_t>(s) & 15u) == 0 && at + 16 <= total) return *reinterpret_cast<const ulonglong2*>(s);
+  if (at >= off && at - off + 20 <= total) {
+    const unsigned* a = reinterpret_cast<const unsigned*>(s - off);
+    const unsigned w0 = a[0], w1 = a[1], w2 = a[2], w3 = a[3], w4 = a[4];
+    return make_ulonglong2(((uint64_t)__funnelshift_r(w1, w2, 8 * off) << 32) | __funnelshift_r(w0, w1, 8 * off),
+                           ((uint64_t)__funnelshift_r(w3, w4, 8 * off) << 32) | __funnelshift_r(w2, w3, 8 * off));
+  }
+  uint64_t v[2] = {0, 0};
+  const int m = total - at < 16 ? (int)(total - at) : 16;
+#pragma unroll 1
+  for (int i = 0; i < m; ++i) v[i >> 3] |= static_cast<uint64_t>(s[i]) << (8 * (i & 7));
+  return make_ulonglong2(v[0], v[1]);
+}
+
+// Rows of 16 bytes and more: a thread makes 16 bytes of the output at a time, out of one row or two, so that
+// consecutive threads read consecutive words of a row, and write them at once.  What bounds it: the rows'
+// sectors.  In place of rows staged in shared memory a row per thread, whose byte stores met in one bank when the
+// width was a multiple of 32 (750 K rows of 128 bytes 425 us, 64 bytes 122), or a byte per thread (247 and 119):
+// 40 and 24.
+constexpr int kChunkRow = 16, kWideRow = 4096;
+
+__global__ void __launch_bounds__(kBlock) k_gather_chunks(const uint8_t* __restrict__ src, unsigned w,
+                                                          const int64_t* __restrict__ idx, int64_t n_idx, int64_t n_src,
+                                                          uint8_t* __restrict__ dst) {
+  constexpr int U = 2;                             // chunks a thread has in flight
+  const int64_t total = n_src * w;
+  for (int64_t j0 = blockIdx.x * (int64_t)kBlock; j0 < n_idx; j0 += (int64_t)gridDim.x * kBlock) {
+    const unsigned bytes = (unsigned)(n_idx - j0 < kBlock ? n_idx - j0 : kBlock) * w, chunks = bytes / 16;
+    uint8_t* o = dst + j0 * w;                     // 256 rows: a multiple of 16 bytes
+    for (unsigned c0 = threadIdx.x; c0 < chunks; c0 += U * kBlock) {
+      unsigned at[U], left[U];                     // byte of the row the chunk starts at, and the row's bytes in it
+      int64_t r0[U], r1[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned p = 16 * min(c0 + u * kBlock, chunks - 1), row = p / w;
+        at[u] = p - row * w;
+        left[u] = min(16u, w - at[u]);
+        r0[u] = idx[j0 + row];
+        r1[u] = left[u] < 16 ? idx[j0 + row + 1] : -1;
+      }
+      ulonglong2 a[U], b[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        a[u] = b[u] = make_ulonglong2(0, 0);
+        if (r0[u] >= 0 && r0[u] < n_src) a[u] = load_bytes16(src, r0[u] * w + at[u], total);
+        if (r1[u] >= 0 && r1[u] < n_src) b[u] = load_bytes16(src, r1[u] * w, total);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (c0 + u * kBlock >= chunks) break;
+        const unsigned m = 8 * left[u];            // bits of the first row
+        ulonglong2 x = a[u];
+        if (m < 64) {
+          x.x = (x.x & ((1ull << m) - 1)) | (b[u].x << m);
+          x.y = (b[u].y << m) | (b[u].x >> (64 - m));
+        } else if (m < 128) {
+          x.y = (m > 64 ? x.y & ((1ull << (m - 64)) - 1) : 0) | (b[u].x << (m - 64));
+        }
+        reinterpret_cast<ulonglong2*>(o)[c0 + u * kBlock] = x;
+      }
+    }
+    for (unsigned i = chunks * 16 + threadIdx.x; i < bytes; i += kBlock) {
+      const unsigned row = i / w;
+      const int64_t r = idx[j0 + row];
+      o[i] = r >= 0 && r < n_src ? src[r * w + (i - row * w)] : 0;
+    }
   }
 }
 
@@ -344,10 +416,16 @@ extern "C" int tqpk_gather_rows(const void* d_src, int64_t n_src, int64_t row_by
   if (n_idx == 0) return TQPK_OK;
   if (!d_src || !d_idx || !d_dst) return TQPK_EINVAL;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (row_bytes <= kStageRow) {
+  if (row_bytes < kChunkRow) {
     k_gather_short_rows<<<grid_for(n_idx, 8), kBlock, (size_t)row_bytes * kBlock, s>>>(
         static_cast<const uint8_t*>(d_src), (int)row_bytes, d_idx, n_idx, n_src, static_cast<uint8_t*>(d_dst),
         aligned16(d_dst) ? 1 : 0);
+    TQPK_CHECK_LAUNCH();
+    return TQPK_OK;
+  }
+  if (row_bytes <= kWideRow && aligned16(d_dst)) {
+    k_gather_chunks<<<grid_for(n_idx, 8), kBlock, 0, s>>>(static_cast<const uint8_t*>(d_src), (unsigned)row_bytes, d_idx,
+                                                          n_idx, n_src, static_cast<uint8_t*>(d_dst));
     TQPK_CHECK_LAUNCH();
     return TQPK_OK;
   }
