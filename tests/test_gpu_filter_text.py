@@ -15,17 +15,19 @@ def _table(n, w, rng):
     return a
 
 
-def _mask(tree, col, w):
+def _mask(tree, col, w, start=0):
     from tqpk.ops import filter_mask
     from tqpk.predicate import compile_filter
-    dev = torch.from_numpy(col).cuda()
+    buf = torch.zeros(col.size + 16, dtype=torch.int8, device="cuda")      # the column at any alignment
+    dev = buf[start:start + col.size].view(col.shape)
+    dev.copy_(torch.from_numpy(col))
     m, count = filter_mask(compile_filter(tree, {1: dev}), len(col), dev.device, with_count=True)
     m = m.cpu().numpy()
     assert int(count.item()) == m.sum()
     return m
 
 
-@pytest.mark.parametrize("w", [3, 8, 25, 187, 188, 189])
+@pytest.mark.parametrize("w", [3, 8, 25, 32, 64, 128, 187, 188, 189])
 @pytest.mark.parametrize("n", [1, 255, 1024, 1025, 5000])
 def test_searches_beside_equalities_and_prefixes(w, n):
     rng = np.random.default_rng(w * 7919 + n)
@@ -44,7 +46,8 @@ def test_searches_beside_equalities_and_prefixes(w, n):
     E = np.array([r == rows[n // 2] for r in rows])
     for tree, want in ((inlist, IN), (prefix, S), (eq, E), (contains, C), (two, T), ([inlist, "AND", contains], IN & C),
                        ([[prefix, "OR", two], "AND", ["NOT", [contains]]], (S | T) & ~C), ([eq, "OR", [contains, "AND", two]], E | C & T)):
-        np.testing.assert_array_equal(_mask(tree, col, w), want)
+        for start in (0, 4, 1):
+            np.testing.assert_array_equal(_mask(tree, col, w, start), want)
 
 
 def test_an_in_list_of_substrings_reads_its_bytes_in_place():

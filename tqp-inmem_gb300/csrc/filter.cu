@@ -91,7 +91,11 @@ __global__ void __launch_bounds__(kBlock, Q == 1 ? 6 : 3) k_filter_mask(const __
 // hit on 25 bytes 44 / 25, 150 bytes 444 / 111, 188 bytes 473 / 174; one that hits early in every row, 25 bytes
 // 37 / 30, 150 bytes 87 / 89, 188 bytes 83 / 120 (a predicate that keeps everything, so the line is not drawn by
 // it).  Seven substrings in an IN list on 25 bytes 33 / 63, a prefix on 150 bytes 36 / 43.
+// Rows of 64 or 128 bytes are staged a word apart, or the threads' bytes would meet in two banks or one (128 bytes,
+// without a hit 784 us and in place 787, a word apart 120; 64 bytes 188, 393 and 65).  Multiples of 32 gain less
+// (160 bytes 240 and 152) and lose as much where a hit comes early (95 and 116): staged by words, not 16 bytes.
 constexpr int kStagedRow = 188;
+__host__ __device__ __forceinline__ int64_t staged_pitch(int64_t stride) { return stride % 64 ? stride : stride + 4; }
 
 __global__ void __launch_bounds__(kBlock) k_filter_text(const __grid_constant__ tqpk_predicate P, int64_t n,
                                                         uint8_t* __restrict__ mask, unsigned long long* count, int vec,
@@ -105,6 +109,8 @@ __global__ void __launch_bounds__(kBlock) k_filter_text(const __grid_constant__ 
       if (I.op < TQPK_P_CONTAINS) return str_leaf4(P, I, r0[0], n);
       const int64_t stride = str_stride(P, I.col);
       const int8_t* base = static_cast<const int8_t*>(P.cols[I.col]);
+      const bool apart = stride % 64 == 0 && P.widths[I.col] == stride && (reinterpret_cast<uintptr_t>(base) & 3u) == 0;
+      const int pitch = (int)(apart ? staged_pitch(stride) : stride);
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
         const int64_t q0 = t0 + j * kBlock;
@@ -113,13 +119,19 @@ __global__ void __launch_bounds__(kBlock) k_filter_text(const __grid_constant__ 
         if (rows > 0) {                      // a substring's last row ends before its stride does
           const int bytes = (int)((rows - 1) * stride) + P.widths[I.col];
           const int8_t* s = base + q0 * stride;
-          const int whole = (reinterpret_cast<uintptr_t>(s) & 15u) == 0 ? bytes / 16 : 0;
-          for (int i = threadIdx.x; i < whole; i += kBlock)
-            reinterpret_cast<uint4*>(stage)[i] = reinterpret_cast<const uint4*>(s)[i];
-          for (int i = whole * 16 + threadIdx.x; i < bytes; i += kBlock) stage[i] = s[i];
+          if (apart) {
+            const unsigned words = (unsigned)stride / 4;           // of a row; one more between two
+            for (unsigned i = threadIdx.x; i < words * rows; i += kBlock)
+              reinterpret_cast<unsigned*>(stage)[i + i / words] = reinterpret_cast<const unsigned*>(s)[i];
+          } else {
+            const int whole = (reinterpret_cast<uintptr_t>(s) & 15u) == 0 ? bytes / 16 : 0;
+            for (int i = threadIdx.x; i < whole; i += kBlock)
+              reinterpret_cast<uint4*>(stage)[i] = reinterpret_cast<const uint4*>(s)[i];
+            for (int i = whole * 16 + threadIdx.x; i < bytes; i += kBlock) stage[i] = s[i];
+          }
         }
         __syncthreads();
-        const bool ok = (int)threadIdx.x < rows && str_leaf(P, I, stage + (int)threadIdx.x * (int)stride);
+        const bool ok = (int)threadIdx.x < rows && str_leaf(P, I, stage + (int)threadIdx.x * pitch);
         const unsigned m = __ballot_sync(0xffffffffu, ok);
         if ((threadIdx.x & 31) == 0) s_bits[(j * kBlock + threadIdx.x) >> 5] = m;
       }
@@ -583,11 +595,11 @@ extern "C" int tqpk_filter_mask(const tqpk_predicate* h_pred, int64_t n, uint8_t
   const int mask_vec = (reinterpret_cast<uintptr_t>(d_mask) & 3u) == 0;
   timing_before(KID_FILTER_MASK, s);
   bool text = false;
-  int64_t searched = 0;          // the widest text row that is searched
+  int64_t searched = 0;          // the widest text row that is searched, as staged
   for (int k = 0; k < h_pred->n_insn; ++k) {
     const tqpk_pred_insn& I = h_pred->insn[k];
     text = text || I.op >= TQPK_P_STRCMP;
-    if (I.op >= TQPK_P_CONTAINS) searched = std::max(searched, str_stride(*h_pred, I.col));
+    if (I.op >= TQPK_P_CONTAINS) searched = std::max(searched, staged_pitch(str_stride(*h_pred, I.col)));
   }
   if (searched > 0 && searched <= kStagedRow) {
     k_filter_text<<<grid_for((n + 3) / 4, 8), kBlock, (size_t)searched * kBlock, s>>>(
