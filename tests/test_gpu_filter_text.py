@@ -51,22 +51,24 @@ def test_searches_beside_equalities_and_prefixes(w, n):
 
 
 def test_an_in_list_of_substrings_reads_its_bytes_in_place():
-    """Seven two-byte substrings of 180-byte rows: the first bytes of every row, not whole rows seven
-    times (1.5 M rows: 0.13 ms against 0.33)."""
+    """Seven two-byte substrings of 180-byte rows read the first bytes of every row, not whole rows seven
+    times: less than a search that reads them once (1.5 M rows: 0.13 ms against 0.17; 0.33 when staged)."""
     from tqpk.ops import filter_mask
     from tqpk.predicate import compile_filter
     n = 1_500_000
     rng = np.random.default_rng(1)
     dev = torch.from_numpy(rng.choice(np.frombuffer(b"0123456789", np.int8), (5000, 180))).cuda()
     dev = dev[torch.randint(0, 5000, (n,), device="cuda")]
-    p = compile_filter([["substring", ["t#1", "1", "2"]], "IN", ["13", "31", "23", "29", "30", "18", "17"]], {1: dev})
-    filter_mask(p, n, dev.device)
-    best = 1.0
-    for _ in range(10):
-        torch.cuda.synchronize()
-        t = time.perf_counter()
+    best = []
+    for tree in ([["substring", ["t#1", "1", "2"]], "IN", ["13", "31", "23", "29", "30", "18", "17"]], ["Contains", ["t#1", "ab"]]):
+        p = compile_filter(tree, {1: dev})
+        filter_mask(p, n, dev.device)
+        best.append(1.0)
         for _ in range(10):
-            filter_mask(p, n, dev.device)
-        torch.cuda.synchronize()
-        best = min(best, (time.perf_counter() - t) / 10)
-    assert best < 0.22e-3
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            for _ in range(10):
+                filter_mask(p, n, dev.device)
+            torch.cuda.synchronize()
+            best[-1] = min(best[-1], time.perf_counter() - t)
+    assert best[0] < 1.3 * best[1]
