@@ -214,7 +214,7 @@ extern "C" int tqpk_debug_topk_barrier(int32_t spin_limit, int32_t missing) {
 
 extern "C" size_t tqpk_topk_workspace_bytes(int64_t n, int64_t k) {
   if (n < 0) n = 0;
-  if (k <= 256) return topk_scratch_bytes((int)std::max<int64_t>(k, 1)) + 1024;
+  if (k <= 256) return topk_scratch_bytes(n, (int)std::max<int64_t>(k, 1)) + 1024;
   return sort_ws_bytes(n) + align_up((size_t)n * sizeof(int64_t), 256);
 }
 
@@ -241,13 +241,13 @@ extern "C" int tqpk_topk_stable(const void* d_keys, int32_t dt, int32_t desc, co
   unsigned* ticket = cur.take<unsigned>(64);
   int64_t* count = cur.take<int64_t>(4);
   int64_t* idx = cur.take<int64_t>(k);
-  uint64_t* ck = cur.take<uint64_t>(topk_list_entries((int)k));
-  int64_t* ci = cur.take<int64_t>(topk_list_entries((int)k));
+  uint64_t* ck = cur.take<uint64_t>(topk_list_entries(n, (int)k));
+  int64_t* ci = cur.take<int64_t>(topk_list_entries(n, (int)k));
   if (!ci) return TQPK_ENOMEM;
   TQPK_CUDA(cudaMemsetAsync(ticket, 0, 256, s));
   ArraySource src{d_keys, dt, d_perm_in, n, desc ? 1 : 0};
   TopkOut O{idx, count, ck, ci, ticket, nullptr, reinterpret_cast<unsigned long long*>(ticket + 8), ticket + 16};
-  O.cap = kTopkGroups * topk_list_share((int)k);
+  O.cap = topk_list_cap(n, (int)k);
   timing_before(KID_PIPE_TOPK, s);
   int rc = topk_warp_launch(1, &src, (int)k, grid, O, s);
   timing_after(KID_PIPE_TOPK, s);

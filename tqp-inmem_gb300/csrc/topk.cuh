@@ -855,11 +855,16 @@ inline size_t topk_cand_entries(int k) {
   const size_t a = (size_t)topk_grid_size() * k;
   return a > (size_t)kTopkCand ? a : (size_t)kTopkCand;
 }
-// A stored column's list (tqpk_topk_stable): a share for every group, the groups' bests, and their own cuts.
-inline size_t topk_list_entries(int k) { return (size_t)kTopkGroups * (topk_list_share(k) + 2); }
-inline size_t topk_scratch_bytes(int k) {
+// A stored column's list (tqpk_topk_stable): a share for every group, but no more than the items, with the
+// groups' bests and their own cuts behind it.
+inline int topk_list_cap(int64_t n, int k) {
+  const int64_t most = (int64_t)kTopkGroups * topk_list_share(k);
+  return (int)(n < most ? n : most);
+}
+inline size_t topk_list_entries(int64_t n, int k) { return (size_t)topk_list_cap(n, k) + 2 * kTopkGroups; }
+inline size_t topk_scratch_bytes(int64_t n, int k) {
   // ticket block + count + k indices + two candidate arrays, each 256-byte aligned
-  return 2 * align_up(topk_list_entries(k) * 8, 256) + align_up((size_t)k * 8, 256) + 1024;
+  return 2 * align_up(topk_list_entries(n, k) * 8, 256) + align_up((size_t)k * 8, 256) + 1024;
 }
 
 }  // namespace tqpk

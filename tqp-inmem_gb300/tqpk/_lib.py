@@ -18,6 +18,7 @@ OK, EINVAL, ENOMEM, ETIMEOUT, EDTYPE, ECUDA, ECAPACITY, EUNSUPPORTED = 0, -1, -2
 ROWID, I8, U8, I32, I64, F64, BOOL = 0, 1, 2, 3, 4, 5, 6
 MAX_COLS, MAX_PRED, MAX_KEYS, MAX_EXPR, MAX_ACCS = 16, 32, 4, 32, 16
 MAX_SORT_WORDS = 32
+ONE_CTA_SORT_ROWS = 2048                 # rows one CTA sorts, without a workspace
 CLUSTER_SORT_ROWS = 98304                # rows one cluster sorts in a single launch
 TOPK_MAX = 256                           # limits the threshold top-k takes
 NULL_INDEX = -64

@@ -18,7 +18,7 @@ from __future__ import annotations
 
 import torch
 
-from .._lib import CLUSTER_SORT_ROWS, MAX_SORT_WORDS, TOPK_MAX
+from .._lib import CLUSTER_SORT_ROWS, MAX_SORT_WORDS, ONE_CTA_SORT_ROWS, TOPK_MAX
 from ..ops import (argsort_keys, argsort_stable, check_deferred, gather, gather_rows, sort_words, string_words, topk_keys,
                    topk_stable)
 from ..variable import make_like, wait_ready
@@ -59,16 +59,17 @@ def tqp_sort(gpu_enable, tensor_group, args, with_limit, name="sort"):
             c.is_cuda and (c.dim() == 1 or c.shape[1] == 1 or
                            (c.shape[1] > 1 and c.dtype in (torch.int8, torch.uint8))) for c in cols):
         many = list(zip(cols, key_descs))
-        few = sort_words(cols) <= MAX_SORT_WORDS
-        if (limit is not None and 0 < limit <= TOPK_MAX and few and sort_words(cols) > 1
-                and cols[0].shape[0] > CLUSTER_SORT_ROWS):
+        words = sort_words(cols)
+        few = words <= MAX_SORT_WORDS
+        if limit is not None and 0 < limit <= TOPK_MAX and few and words > 1 and cols[0].shape[0] > CLUSTER_SORT_ROWS:
             # the top-k key by key: 6 M rows by a price and a tie-breaking id took 560 us of sorting the
             # ids first.  A table that one cluster sorts in a launch (~30-60 us) is sorted.
             perm = topk_keys(cols, key_descs, limit)
             many, key_ids = [], []
         elif limit is not None:              # all keys but the first, which ends the sort in a top-k
             many = many[1:] if not _is_text(cols[0]) else []
-        if many and few:
+        # one numeric key of few rows: the one-key call below has less to set up (~5 us of a small limit's 100)
+        if many and few and (len(many) > 1 or _is_text(many[0][0]) or many[0][0].shape[0] > ONE_CTA_SORT_ROWS):
             perm = argsort_keys([c for c, _ in many], [d for _, d in many])
             key_ids, key_descs = key_ids[:len(key_ids) - len(many)], key_descs[:len(key_descs) - len(many)]
     for key_id, desc in zip(reversed(key_ids), reversed(key_descs)):
