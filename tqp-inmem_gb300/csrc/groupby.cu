@@ -226,8 +226,9 @@ __global__ void k_fill_u64(uint64_t* p, int64_t n, uint64_t v) {
 
 // What bounds it: per passing row a slot read and A reductions at scattered L2 lines, and a compare-and-swap
 // where the slot is empty (one for every row instead queued on the words of few groups: 6 M rows of 50 groups
-// far apart 404 us, 343 with the read; 20 K groups 169 and 146, 800 K 539 and 457, 3 M 705 and 670; rows
-// stored by their key find the line in use either way: 300 K groups 227 and 235, 3 M 461 and 477).  A tile's
+// far apart 405 us, 348 with the read; 20 K groups 168 and 136, 800 K 540 and 447, 3 M 699 and 643).  The read
+// is on its way while the row's program runs; behind one another they cost rows of many groups more than the
+// compare-and-swap (0.9 M rows of as many pairs 93 us by compare-and-swap, 105 read first, 88 read early).  A tile's
 // passing rows are gathered first, so that the program runs with full warps whatever the filter's
 // selectivity (4 rows a thread in place, one in seven passing, executed it almost seven times as often:
 // 576 us for 0.9 M of 6 M rows), and by the plain loop: the unrolled form with operand selects costs
@@ -269,14 +270,17 @@ __global__ void __launch_bounds__(kBlock) k_groupby_hash(const __grid_constant__
         for (int k = 0; k < G.nk; ++k)
           packed += (uint64_t)(ld_int(S.keys[k], S.key_dtypes[k], row) - G.kmin[k]) * (uint64_t)G.kstride[k];
         h = hash_slot(packed, C);
-        for (int64_t probes = 0;; h = (h + 1) & (C - 1)) {
-          unsigned long long prev = __ldcg(&hkeys[h]);
+        unsigned long long prev = __ldcg(&hkeys[h]);       // on its way while the row's program runs
+        uint64_t r[TQPK_MAX_EXPR];
+        expr_eval_generic(S.expr, S.n_expr, S.cols, S.col_dtypes, row, r);
+        for (int64_t probes = 0;; prev = __ldcg(&hkeys[h])) {
           if (prev == packed) break;
           if (prev == kHashEmpty) {
             prev = atomicCAS(&hkeys[h], kHashEmpty, (unsigned long long)packed);
             claimed = prev == kHashEmpty;
             if (claimed || prev == packed) break;
           }
+          h = (h + 1) & (C - 1);
           if (++probes > C) {              // table full: cannot happen (C >= 2 rows)
             set_error(err, TQPK_ECAPACITY);
             h = -1;
@@ -284,8 +288,6 @@ __global__ void __launch_bounds__(kBlock) k_groupby_hash(const __grid_constant__
           }
         }
         if (h >= 0) {
-          uint64_t r[TQPK_MAX_EXPR];
-          expr_eval_generic(S.expr, S.n_expr, S.cols, S.col_dtypes, row, r);
           for (int a = 0; a < A; ++a)
             acc_merge_global(&gacc[(int64_t)a * C + h], S.accs[a],
                              acc_value(S.accs[a], S.accs[a].kind == TQPK_ACC_COUNT_ROWS ? 0 : r[S.accs[a].reg]));
