@@ -297,7 +297,7 @@ class StarAggTopK:
         # one block, so that the result comes back in one copy: the directories' error words (int32),
         # row count, group count, keys, sums, counts
         self._out = torch.empty(4 + 3 * self.k, dtype=torch.int64, device=self.dev)
-        self._out[2:4].zero_()         # the counts only: a run on another stream may already be writing the rest
+        self._cleared = False
         self.out_count, self.groups = self._out[2:3], self._out[3:4]
         self.out_keys = self._out[4:4 + self.k]
         self.out_vals = self._out[4 + self.k:4 + 2 * self.k].view(torch.float64)
@@ -306,6 +306,13 @@ class StarAggTopK:
     @property
     def workspace_bytes(self) -> int:
         return int(self.ws.numel())
+
+    def _clear(self):
+        """Error words and counts zeroed once, on the stream of the first run: a fill queued by the
+        constructor could land, on another stream, on what the run writes."""
+        if not self._cleared:
+            self._out[:4].zero_()
+            self._cleared = True
 
     def _jit_ok(self) -> bool:
         from . import jit
@@ -342,7 +349,6 @@ class StarAggTopK:
         self.sum = torch.empty(cmx - cmn + 1, dtype=torch.float64, device=dev)
         self.cnt = torch.empty(cmx - cmn + 1, dtype=torch.int32, device=dev)
         self.err = self._out[:2].view(torch.int32)[:3]
-        self.err.zero_()               # on the run's stream
         self.tws = torch.empty(self.lib.tqpk_dense_topk_workspace_bytes(self.k), dtype=torch.uint8, device=dev)
         # fkB loaded with fkA and evict-first column loads: 529 -> 507 us on the 59,986,052-row star join
         # + B's directory composed with C's (no C lookup in the probe)
@@ -416,10 +422,11 @@ class StarAggTopK:
         make the stream wait for fact columns still being copied)."""
         s = (stream or torch.cuda.current_stream(self.dev)).cuda_stream
         self._jit_path = self._jit_ok()
-        if self._jit_path:
-            with torch.cuda.stream(stream or torch.cuda.current_stream(self.dev)):
+        with torch.cuda.stream(stream or torch.cuda.current_stream(self.dev)):
+            self._clear()
+            if self._jit_path:
                 self._run_jit(s, before_probe)
-            return
+                return
         if before_probe is not None:
             before_probe()
         fa, fb, ak, bk, bc, ck = self.t
@@ -451,6 +458,7 @@ class StarAggTopK:
         with one host read: the error words, the row count and the k result rows together
         (`result_host` then holds the rows as numpy arrays).  A repeated dimension key raises
         NotImplementedError, an out-of-domain one ValueError."""
+        self._clear()                                 # not run: no rows
         cur = torch.cuda.current_stream(self.dev)
         if not hasattr(self, "_host"):
             self._host = torch.empty(2 + self._out.numel(), dtype=torch.int64, pin_memory=True)
@@ -480,6 +488,7 @@ class StarAggTopK:
         return ((idx + cmn).cpu().numpy(), self.sum[idx].cpu().numpy(), self.cnt[idx].to(torch.int64).cpu().numpy())
 
     def result(self):
+        self._clear()                                 # not run: no rows
         s = torch.cuda.current_stream(self.dev).cuda_stream
         err = C.c_int(0)
         if getattr(self, "_jit_path", False):
